@@ -53,8 +53,8 @@ enum Kind {
   K_SOLVE_THIN_FWD, K_SOLVE_THIN_BWD,  // the thin supernodes' steps of a solve level
   K_PACK_TC,                           // the tcgen05 products' operands packed (K-major hi | lo)
   K_LDLT_PANEL,                        // LDL^T: pivoted panel steps (they write the next GEMM's tasks)
-  K_LDLT_AFTER,                        // LDL^T: W21 = L21 D and D out of the fronts
-  K_LDLT_INVERSE                       // LDL^T: the 64 x 64 inverses of the unit lower diagonal blocks
+  K_LDLT_AFTER,                        // LDL^T: W21 = L21 D
+  K_LDLT_INVERSE                       // LDL^T: D out of the fronts and the 64 x 64 unit lower inverses
 };
 
 struct Launch {
@@ -116,14 +116,11 @@ struct fc_chol {
   bool ldlt = false;
   DeviceBuf d_lscale, d_llocal, d_lorder, d_lpivots, d_lpos, d_ltwos, d_lfailed, d_lscratch, d_ldd, d_lde;
   DeviceBuf d_lpanel, d_lafter, d_linv;
-  // the LDL^T solve's structure: the pivot orders folded in after each factorisation (host/
-  // ldlt_fold.cpp), its rows, relative maps and permutation on the device, the L21 rows' move;
-  // the structure's own rows and maps kept for the next fold; the tree the solve's kernels read
-  bool ldlt_folded = false;
-  std::vector<int32_t> ldlt_rows0, ldlt_rel0;
-  std::vector<int64_t> ldlt_sparent, ldlt_from_off;
-  std::vector<int32_t> ldlt_from;
-  DeviceBuf d_lsrows, d_lsrel, d_lsperm, d_lfrom, d_ltmp, d_lperm_t;
+  // the LDL^T solve's view of the pivots, made on the device at the end of each factorisation
+  // (ldlt::launch_fold): its row lists and permutation, each column's place in its vectors, and
+  // the tree its kernels read; whether there has been a factorisation to solve with
+  bool ldlt_ready = false;
+  DeviceBuf d_lsrows, d_lsperm, d_lown;
   fc::Tree stree{};
   fc::Tree tree{};
   std::vector<Launch> program;
@@ -884,7 +881,10 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
       h->d_ltwos.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(h->ns, 1)) != cudaSuccess ||
       h->d_lfailed.alloc(sizeof(unsigned long long)) != cudaSuccess ||
       h->d_ldd.alloc(sizeof(double) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
-      h->d_lde.alloc(sizeof(double) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess) {
+      h->d_lde.alloc(sizeof(double) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
+      h->d_lown.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
+      h->d_lsperm.alloc(sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
+      h->d_lsrows.alloc(sizeof(int32_t) * std::max<size_t>(h->rows.size(), 1)) != cudaSuccess) {
     set_status(st, FC_OUT_OF_MEMORY, -1, h->entries, 0, "device memory for the LDL^T factor");
     return FC_OUT_OF_MEMORY;
   }
@@ -904,13 +904,6 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
   std::vector<int64_t> pan_slot;  // each panel task's first slot in gemm_t (its pointer set at upload)
   std::vector<L::AfterTask> aft_t;
   std::vector<L::InverseTask> inv_t;
-  // the structure's rows and relative maps (the solve's are folded from them after each
-  // factorisation) and the supernodal tree's parents
-  h->ldlt_rows0 = h->rows;
-  h->ldlt_rel0 = h->rel;
-  h->ldlt_sparent.assign(h->ns, -1);
-  for (int64_t s = 0; s < h->ns; ++s)
-    for (int64_t q = h->kid_ptr[s]; q < h->kid_ptr[s + 1]; ++q) h->ldlt_sparent[h->kids[q]] = s;
   for (size_t l = 0; l < lv.size(); ++l) {
     const auto &S = lv[l];
     int64_t off = (int64_t)asm_t.size();
@@ -945,10 +938,12 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
     }
     for (int p = 0; p < P; ++p) {
       const int64_t po = (int64_t)pan_t.size(), go = (int64_t)gemm_t.size();
+      int tallest = 0;
       for (size_t q = 0; q < S.size(); ++q) {
         const int64_t s = S[q];
         const int m = h->height[s], w = h->width[s];
         if (p * L::PANEL >= w) continue;
+        tallest = std::max(tallest, m);
         const int earliest = (p + 1) * L::PANEL;
         const int64_t slots = earliest < w ? L::update_tiles(m, w, earliest) : 0;
         L::PanelTask t{};
@@ -962,26 +957,30 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
           gemm_t.push_back(fc::GemmTask{});  // empty until the panel step writes it
         }
       }
-      push(h->program, K_LDLT_PANEL, po, (int64_t)pan_t.size() - po, (int)l);
+      push(h->program, K_LDLT_PANEL, po, (int64_t)pan_t.size() - po, (int)l, tallest);
       push(h->program, K_GEMM, go, (int64_t)gemm_t.size() - go, (int)l);
     }
     const int64_t ao = (int64_t)aft_t.size();
     for (size_t q = 0; q < S.size(); ++q) {
-      const int64_t f = h->first[S[q]];
-      aft_t.push_back({fronts[q], w21[q], h->d_ldd.as<double>() + f, h->d_lde.as<double>() + f});
+      const int m = h->height[S[q]], w = h->width[S[q]];
+      for (int r0 = w; r0 < m; r0 += L::W21_ROWS)
+        aft_t.push_back({fronts[q], w21[q], r0, std::min(m, r0 + L::W21_ROWS)});
     }
     push(h->program, K_LDLT_AFTER, ao, (int64_t)aft_t.size() - ao, (int)l);
     // the solve's diagonal-block inverses: 64 x 64 ones of the unit lower own blocks, then the
     // doubling to blocks of up to SB columns (as the Cholesky factor's, from its panels' inverses)
     const int64_t io = (int64_t)inv_t.size();
-    for (int64_t s : S) {
-      const int m = h->height[s], w = h->width[s];
+    for (size_t q = 0; q < S.size(); ++q) {
+      const int64_t s = S[q];
+      const int w = h->width[s];
       for (int c0 = 0; c0 < w; c0 += L::PANEL) {
         int bw;
         const int64_t ib = inv_block(h, s, c0 / fc::SB, bw), in = c0 % fc::SB;
         L::InverseTask t{};
-        t.L = Lp(h->loff[s] + c0 + (int64_t)c0 * m);
-        t.ldl = m;
+        t.front = fronts[q];
+        t.d = h->d_ldd.as<double>() + h->first[s];
+        t.e = h->d_lde.as<double>() + h->first[s];
+        t.c0 = c0;
         t.X = h->d_Dinv.as<double>() + ib + in + in * bw;
         t.ldx = bw;
         t.nb = std::min(L::PANEL, w - c0);
@@ -1039,6 +1038,9 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
   for (cudaEvent_t ev : h->lane_events)
     if (ev) cudaEventDestroy(ev);
   h->lane_events.assign(h->program.size(), nullptr);
+  h->stree = h->tree;
+  h->stree.rows = h->d_lsrows.as<int32_t>();
+  h->stree.own = h->d_lown.as<int32_t>();
   return FC_OK;
 }
 
@@ -1352,7 +1354,7 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
 // Enqueues the factor's program (as a replayed graph when it can). Returns FC_CANCELLED when the
 // flag was set between levels.
 int enqueue_factor(fc_chol *h, const double *d_val, const volatile int32_t *cancel) {
-  h->ldlt_folded = false;
+  h->ldlt_ready = false;
   if (cancel || h->profiling || !h->graphs) return enqueue_factor_direct(h, d_val, cancel);
   if (!h->factor_graph || h->factor_graph_val != d_val || h->factor_graph_stream != h->stream) {
     if (!capture(h, &h->factor_graph, [&] { enqueue_factor_direct(h, d_val, nullptr); })) {
@@ -1364,6 +1366,7 @@ int enqueue_factor(fc_chol *h, const double *d_val, const volatile int32_t *canc
   }
   cudaGraphLaunch(h->factor_graph, h->stream);
   h->last_factor_launches = (int64_t)h->program.size();
+  h->ldlt_ready = h->ldlt;
   return FC_OK;
 }
 
@@ -1439,7 +1442,7 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
         break;
       case K_GEMM_F64: fc::launch_gemm(h->d_gemm.as<fc::GemmTask>() + l.off, l.count, fc::GemmKind::F64, st); break;
       case K_LDLT_PANEL:
-        fc::ldlt::launch_panel(h->d_lpanel.as<fc::ldlt::PanelTask>() + l.off, l.count, h->d_lpos.as<int32_t>(),
+        fc::ldlt::launch_panel(h->d_lpanel.as<fc::ldlt::PanelTask>() + l.off, l.count, l.width, h->d_lpos.as<int32_t>(),
                                h->d_ltwos.as<int32_t>(), h->d_lfailed.as<unsigned long long>(), st);
         break;
       case K_LDLT_AFTER: fc::ldlt::launch_after(h->d_lafter.as<fc::ldlt::AfterTask>() + l.off, l.count, st); break;
@@ -1447,6 +1450,12 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
     }
     if (lanes && l.record) cudaEventRecord(h->lane_events[li], st);
     ++launches;
+  }
+  if (h->ldlt) {
+    fc::ldlt::launch_fold(h->n, h->d_llocal.as<int32_t>(), h->d_lorder.as<int32_t>(), h->d_perm.as<int64_t>(),
+                          h->d_lown.as<int32_t>(), h->d_lsperm.as<int64_t>(), (int64_t)h->rows.size(),
+                          h->d_rows.as<int32_t>(), h->d_lsrows.as<int32_t>(), user);
+    h->ldlt_ready = true;
   }
   join();
   h->last_factor_launches = launches;
@@ -1489,66 +1498,6 @@ bool ldlt_refused(const fc_chol *h, fc_status *st) {
   if (!h->ldlt) return false;
   set_status(st, FC_INVALID_ARGUMENT, -1, 0, 0, "the LDL^T factor has no solve without allocation");
   return true;
-}
-
-// The LDL^T solve's structure, once per factorisation: the pivot orders read back and folded
-// into the structure (host/ldlt_fold.cpp), the solve's rows, relative maps and permutation
-// uploaded, each front's rows below moved to their new order, and the solve's plan dropped (the
-// next solve plans on the folded structure). Its own blocks are unit lower (split_d), so the
-// Cholesky solve then runs on them as it is, with D^-1 between its passes.
-int ldlt_prepare_solve(fc_chol *h, fc_status *st) {
-  if (h->ldlt_folded) return FC_OK;
-  const int64_t n = h->n, ns = h->ns;
-  std::vector<int32_t> order(n);
-  cudaError_t e = cudaStreamSynchronize(h->stream);
-  if (e == cudaSuccess && n > 0)
-    e = cudaMemcpy(order.data(), h->d_lorder.p, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(st, e, "the LDL^T factor's pivot orders");
-  std::vector<int64_t> rptr(h->rows_off.begin(), h->rows_off.end());
-  rptr.push_back((int64_t)h->ldlt_rows0.size());
-  if (ns == 0) rptr.assign(1, 0);
-  fc::LdltFold fold;
-  if (!fc::ldlt_fold(n, ns, h->first.data(), rptr.data(), h->ldlt_rows0.data(), h->perm.data(), h->ldlt_sparent.data(),
-                     order.data(), fold)) {
-    set_status(st, FC_INTERNAL, -1, 0, 0, "the LDL^T factor's pivot orders are not permutations");
-    return FC_INTERNAL;
-  }
-  std::vector<fc::ldlt::PermuteTask> moves;
-  if ((e = upload(h->d_lsrows, fold.rows, h->stream)) != cudaSuccess ||
-      (e = upload(h->d_lsrel, fold.rel, h->stream)) != cudaSuccess ||
-      (e = upload(h->d_lsperm, fold.perm, h->stream)) != cudaSuccess ||
-      (e = upload(h->d_lfrom, fold.from, h->stream)) != cudaSuccess ||
-      (e = h->d_ltmp.alloc(sizeof(double) * (size_t)std::max<int64_t>(fold.from_off[ns], 1))) != cudaSuccess)
-    return cuda_fail(st, e, "the LDL^T solve's structure");
-  for (int64_t s = 0; s < ns; ++s) {
-    const int m = h->height[s], w = h->width[s];
-    if (m == w) continue;
-    fc::ldlt::PermuteTask t{};
-    t.front.F = static_cast<double *>(arena_at(h->d_L, h, h->loff[s]));
-    t.front.m = m;
-    t.front.w = w;
-    t.from = h->d_lfrom.as<int32_t>() + fold.from_off[s];
-    t.tmp = h->d_ltmp.as<double>() + fold.from_off[s];
-    moves.push_back(t);
-  }
-  if ((e = upload(h->d_lperm_t, moves, h->stream)) != cudaSuccess) return cuda_fail(st, e, "the LDL^T solve's structure");
-  fc::ldlt::launch_permute(h->d_lperm_t.as<fc::ldlt::PermuteTask>(), (int)moves.size(), h->stream);
-  if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess)
-    return cuda_fail(st, e, "the LDL^T solve's structure");
-  h->ldlt_from = std::move(fold.from);
-  h->ldlt_from_off = std::move(fold.from_off);
-  h->rows = std::move(fold.rows);  // what the solve's planner reads
-  h->rel = std::move(fold.rel);
-  h->stree = h->tree;
-  h->stree.rows = h->d_lsrows.as<int32_t>();
-  h->stree.rel = h->d_lsrel.as<int32_t>();
-  h->solve_R = 0;
-  if (h->solve_graph) {
-    cudaGraphExecDestroy(h->solve_graph);
-    h->solve_graph = nullptr;
-  }
-  h->ldlt_folded = true;
-  return FC_OK;
 }
 
 // The solve's program for R right-hand sides (built once per R). Forward, level by level: a thin
@@ -2452,9 +2401,9 @@ void enqueue_solve_direct(fc_chol *h, double *d_b, int R, int64_t ld);
 // Solves for the R right-hand sides in device memory at d_b (column-major, leading dimension ld),
 // as a replayed graph when it can.
 int enqueue_solve(fc_chol *h, double *d_b, int R, int64_t ld, fc_status *st) {
-  if (h->ldlt) {
-    const int rc = ldlt_prepare_solve(h, st);
-    if (rc != FC_OK) return rc;
+  if (h->ldlt && !h->ldlt_ready) {
+    set_status(st, FC_INTERNAL, -1, 0, 0, "the LDL^T factor's pivot orders are not there yet");
+    return FC_INTERNAL;
   }
   const int before = h->solve_R;
   int rc = plan_solve(h, R, st);
@@ -3330,17 +3279,12 @@ int fc_chol_values(fc_chol *h, double *dst, fc_status *status) {
     if (e == cudaSuccess) e = cudaMemcpy(sub.data(), h->d_lde.p, sizeof(double) * (size_t)h->n, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(piv.data(), h->d_lpivots.p, (size_t)h->n, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(status, e, "values");
-    // after a solve the rows below are in the solve's order: row w + i holds row w + from[i]
     int64_t at = 0;
     for (int64_t s = 0; s < h->ns; ++s) {
       const int64_t m = h->height[s], w = h->width[s], f = h->first[s];
       const double *F = rect.data() + h->loff[s];
-      std::vector<int64_t> to(m - w);  // the structure's row w + j is at row w + to[j]
-      for (int64_t i = 0; i < m - w; ++i) to[i] = i;
-      if (h->ldlt_folded)
-        for (int64_t i = 0; i < m - w; ++i) to[h->ldlt_from[h->ldlt_from_off[s] + i]] = i;
       for (int64_t c = 0; c < w; ++c) {
-        for (int64_t r = c; r < m; ++r) dst[at + r - c] = F[(r >= w ? w + to[r - w] : r) + c * m];
+        for (int64_t r = c; r < m; ++r) dst[at + r - c] = F[r + c * m];
         dst[at] = d[f + c];
         if (piv[f + c] == fc::ldlt::PIVOT_FIRST && c + 1 < m) dst[at + 1] = sub[f + c];
         at += m - c;

@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(256) solve_assemble_kernel(Tree t, double *__r
     for (int64_t e = tid; e < (int64_t)(hi - lo) * R; e += blockDim.x) {
       const int ic = lo + (int)(e / R), j = (int)(e % R);
       const int64_t I = rel[ic];
-      double *dst = I < w ? x + (f + I) * R + j : vs + (I - w) * R + j;
+      double *dst = I < w ? x + (t.own ? t.own[f + I] : f + I) * R + j : vs + (I - w) * R + j;
       *dst += vc[(int64_t)ic * R + j];
     }
     __syncthreads();
@@ -1109,7 +1109,7 @@ __global__ void __launch_bounds__(THIN_THREADS) thin_fwd_kernel(Tree t, const do
     const double *vc = v + voff[c];
     // at most w rows: a warp each
     for (int ic = warp; ic < g.x; ic += THIN_WARPS) {
-      const int row = rel[ic];
+      const int row = t.own ? (int)(t.own[f + rel[ic]] - f) : rel[ic];
       for (int j = lane; j < nj; j += 32) xs[(row << lg) + j] += vc[(int64_t)ic * R + j0 + j];
     }
     __syncthreads();

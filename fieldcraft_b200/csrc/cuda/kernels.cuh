@@ -80,6 +80,8 @@ struct Tree {
   const int32_t *a_row;     // mixed precision: each input entry's postordered row and column
   const int32_t *a_col;
   const double *scale;      // mixed precision: S = diag(A)^-1/2 (postorder); null in FP64
+  const int32_t *own;       // solve of the LDL^T factor: column j's place in the solve's vectors (its
+                            // supernode's columns in pivot order); null: its own place
   void *L;                  // L panels and update matrices: double, or float in mixed precision
   void *U;
   double *D;

@@ -71,11 +71,10 @@ __global__ void __launch_bounds__(MAX_THREADS) ldlt_panel_kernel(const PanelTask
   if (threadIdx.x == 0) pos[task.s] = end;
 }
 
-__global__ void __launch_bounds__(MAX_THREADS) ldlt_after_kernel(const AfterTask *__restrict__ tasks) {
+__global__ void __launch_bounds__(W21_ROWS) ldlt_after_kernel(const AfterTask *__restrict__ tasks) {
   const AfterTask &task = tasks[blockIdx.x];
   DeviceBlock blk;
-  if (task.front.m > task.front.w) front_w21(blk, task.front, task.w21, task.front.m - task.front.w);
-  split_d(blk, task.front, task.d, task.e);
+  front_w21(blk, task.front, task.w21, task.front.m - task.front.w, task.r0, task.r1);
 }
 
 // y <- D^-1 y between the solve's forward and backward passes: n unknowns in postorder, R
@@ -110,16 +109,42 @@ __global__ void ldlt_reset_kernel(int64_t n, const int32_t *__restrict__ local, 
   }
 }
 
-__global__ void __launch_bounds__(64) ldlt_inverse_kernel(const InverseTask *__restrict__ tasks) {
+// D out of a block of columns, then the inverse of its unit lower diagonal block, both sides in
+// shared memory, a step of the substitution a pass over them (one thread a column of global memory
+// took 43 us a launch, this 28 with the split).
+constexpr int INVERSE_THREADS = 256, INVERSE_LD = PANEL + 1;
+__global__ void __launch_bounds__(INVERSE_THREADS) ldlt_inverse_kernel(const InverseTask *__restrict__ tasks) {
+  extern __shared__ double sm[];
+  double *L = sm, *X = sm + PANEL * INVERSE_LD;
   const InverseTask &t = tasks[blockIdx.x];
+  const Front &f = t.front;
   DeviceBlock blk;
-  unit_lower_inverse(blk, t.L, t.ldl, t.nb, t.X, t.ldx);
+  split_d(blk, f, t.d, t.e, t.c0, t.c0 + t.nb);
+  for (int e = threadIdx.x; e < PANEL * t.nb; e += blockDim.x) {
+    const int i = e % PANEL, j = e / PANEL;
+    if (i < t.nb) L[i + j * INVERSE_LD] = i > j ? at(f, t.c0 + i, t.c0 + j) : 0.0;
+  }
+  __syncthreads();
+  unit_lower_inverse(blk, L, INVERSE_LD, t.nb, X, INVERSE_LD);
+  for (int e = threadIdx.x; e < PANEL * t.nb; e += blockDim.x) {
+    const int i = e % PANEL, j = e / PANEL;
+    if (i >= j && i < t.nb) t.X[i + (int64_t)j * t.ldx] = X[i + j * INVERSE_LD];
+  }
 }
 
-__global__ void __launch_bounds__(MAX_THREADS) ldlt_permute_kernel(const PermuteTask *__restrict__ tasks) {
-  const PermuteTask &t = tasks[blockIdx.x];
-  DeviceBlock blk;
-  permute_rows_below(blk, t.front, t.from, t.tmp);
+__global__ void ldlt_fold_kernel(int64_t n, const int32_t *__restrict__ local, const int32_t *__restrict__ order,
+                                 const int64_t *__restrict__ perm, int32_t *__restrict__ own,
+                                 int64_t *__restrict__ perm_out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = i - local[i] + order[i];  // the column at pivot position i
+    own[j] = (int32_t)i;
+    perm_out[i] = perm[j];
+  }
+}
+__global__ void ldlt_rows_kernel(int64_t count, const int32_t *__restrict__ rows, const int32_t *__restrict__ own,
+                                 int32_t *__restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = own[rows[i]];
 }
 
 namespace {
@@ -130,20 +155,29 @@ int grid_for(int64_t count, int threads) {
 }  // namespace
 
 void launch_inverse(const InverseTask *tasks, int count, cudaStream_t st) {
-  if (count > 0) ldlt_inverse_kernel<<<count, 64, 0, st>>>(tasks);
+  constexpr size_t smem = sizeof(double) * 2 * PANEL * INVERSE_LD;
+  if (count <= 0) return;
+  cudaFuncSetAttribute(ldlt_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  ldlt_inverse_kernel<<<count, INVERSE_THREADS, smem, st>>>(tasks);
 }
 
-void launch_permute(const PermuteTask *tasks, int count, cudaStream_t st) {
-  if (count > 0) ldlt_permute_kernel<<<count, MAX_THREADS, 0, st>>>(tasks);
+void launch_fold(int64_t n, const int32_t *local, const int32_t *order, const int64_t *perm, int32_t *own,
+                 int64_t *perm_out, int64_t rows_len, const int32_t *rows, int32_t *rows_out, cudaStream_t st) {
+  if (n > 0) ldlt_fold_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, local, order, perm, own, perm_out);
+  if (rows_len > 0) ldlt_rows_kernel<<<grid_for(rows_len, 256), 256, 0, st>>>(rows_len, rows, own, rows_out);
 }
 
-void launch_panel(const PanelTask *tasks, int count, int32_t *pos, int32_t *twos, unsigned long long *failed,
-                  cudaStream_t st) {
-  if (count > 0) ldlt_panel_kernel<<<count, MAX_THREADS, 0, st>>>(tasks, pos, twos, failed);
+// A thread a row up to 1024: a column step is a chain of loads and barriers (bound by their latency,
+// about 2.6 us a column). With 256 threads a top front's rows went round the block six times a step
+// and one thread formed L D from global memory: 90 ms of panels for 16 x 14 x 13 elements, now 12.
+void launch_panel(const PanelTask *tasks, int count, int tallest, int32_t *pos, int32_t *twos,
+                  unsigned long long *failed, cudaStream_t st) {
+  const int threads = tallest >= MAX_THREADS ? MAX_THREADS : tallest <= 64 ? 64 : (tallest + 31) / 32 * 32;
+  if (count > 0) ldlt_panel_kernel<<<count, threads, 0, st>>>(tasks, pos, twos, failed);
 }
 
 void launch_after(const AfterTask *tasks, int count, cudaStream_t st) {
-  if (count > 0) ldlt_after_kernel<<<count, MAX_THREADS, 0, st>>>(tasks);
+  if (count > 0) ldlt_after_kernel<<<count, W21_ROWS, 0, st>>>(tasks);
 }
 
 void launch_scale(int64_t nnz, const int64_t *a_src, const int32_t *a_row, const int32_t *a_col, const double *val,

@@ -22,40 +22,40 @@ struct PanelTask {
   int32_t s;
 };
 
-// After a level's panels, per front (one CTA each): W21 = L21 D into w21 (leading dimension
-// m - w, for the update-matrix GEMM), then D out of the front into d / e (split_d), leaving its
-// own block unit lower.
+// After a level's panels: rows [r0, r1) of a front's W21 = L21 D into w21 (leading dimension
+// m - w, for the update-matrix GEMM). A CTA takes W21_ROWS rows.
+constexpr int W21_ROWS = 64;
 struct AfterTask {
   Front front;
   double *w21;
-  double *d, *e;
+  int64_t r0, r1;
 };
 
-// The solve's 64 x 64 inverse of one unit lower diagonal block: L (leading dimension ldl, nb
-// columns) into X (leading dimension ldx) in the inverse arena.
+// After that, for the columns [c0, c0 + nb) of a front (nb <= 64): D out of them into d / e
+// (split_d), which leaves the own block unit lower, and the solve's inverse of the diagonal block
+// into X (leading dimension ldx) in the inverse arena.
 struct InverseTask {
-  const double *L;
-  double *X;
-  int64_t ldl, ldx;
-  int32_t nb, pad;
-};
-
-// A front's rows below its own columns put in the solve's order (row w + i takes old row
-// w + from[i]), through `tmp` (m - w entries).
-struct PermuteTask {
   Front front;
-  const int32_t *from;
-  double *tmp;
+  double *d, *e;
+  double *X;
+  int64_t ldx;
+  int32_t c0, nb;
 };
 
 void launch_inverse(const InverseTask *tasks, int count, cudaStream_t st);
-void launch_permute(const PermuteTask *tasks, int count, cudaStream_t st);
-void launch_panel(const PanelTask *tasks, int count, int32_t *pos, int32_t *twos, unsigned long long *failed,
+// `tallest`: the largest m of the launch's fronts (sizes its CTAs).
+void launch_panel(const PanelTask *tasks, int count, int tallest, int32_t *pos, int32_t *twos, unsigned long long *failed,
                   cudaStream_t st);
 void launch_after(const AfterTask *tasks, int count, cudaStream_t st);
 void launch_scale(int64_t nnz, const int64_t *a_src, const int32_t *a_row, const int32_t *a_col, const double *val,
                   unsigned long long *scale_bits, cudaStream_t st);
 void launch_reset(int64_t n, const int32_t *local, int32_t *order, int8_t *pivots, cudaStream_t st);
+// The solve's view of the pivots (after the last panel): own[j] is the place of column j of the
+// structure's postorder in the solve's vectors (its supernode's columns in pivot order), perm_out
+// the input permutation to that order, rows_out the row lists through `own`. local[j]: column j's
+// place in its supernode.
+void launch_fold(int64_t n, const int32_t *local, const int32_t *order, const int64_t *perm, int32_t *own,
+                 int64_t *perm_out, int64_t rows_len, const int32_t *rows, int32_t *rows_out, cudaStream_t st);
 void launch_d_inverse(int64_t n, int R, const double *d, const double *e, const int8_t *pivots, double *y,
                       cudaStream_t st);
 

@@ -17,10 +17,12 @@
 #if defined(__CUDACC__)
 #define FC_LDLT_FN __device__ __forceinline__
 #define FC_LDLT_HD __host__ __device__ __forceinline__  // arithmetic the host plan shares
+#define FC_LDLT_ONCE __device__ __forceinline__
 #else
 #include <cmath>
 #define FC_LDLT_FN inline
 #define FC_LDLT_HD inline
+#define FC_LDLT_ONCE __attribute__((noinline, noclone))  // its barrier stays one call site
 #endif
 
 namespace fc {
@@ -30,7 +32,7 @@ constexpr double ALPHA = 0.6403882032022076;  // (1 + sqrt 17) / 8, ldlt.rs:77
 constexpr int ROOK_STEPS = 64;                // ldlt.rs:81
 constexpr int PANEL = 64;                     // cholesky.rs:54
 constexpr double PIVOT_TOLERANCE = 1e-10;     // cholesky.rs:48
-constexpr int MAX_THREADS = 256;
+constexpr int MAX_THREADS = 1024;
 constexpr int8_t PIVOT_ONE = 0, PIVOT_FIRST = 1, PIVOT_SECOND = 2;
 
 #if defined(__CUDACC__)
@@ -62,12 +64,22 @@ struct Front {
   int64_t ld_w;         // >= w - c0 - PANEL
 };
 
-// Block-shared scratch.
+// Block-shared scratch. The panel's own D is kept here too: a column's update reads all of it, and
+// one by one from the front every element was a load of its own.
 struct Shared {
-  double row[PANEL + 1];  // a row of L D over the panel's factored columns
+  double row[PANEL + 1];   // a row of L D over the panel's factored columns
+  double d[PANEL + 1];     // D's diagonal at the panel's factored columns
+  double e[PANEL + 1];     // its subdiagonal at the first column of a 2 x 2 pivot
+  int8_t kind[PANEL + 1];  // PIVOT_ONE / PIVOT_FIRST / PIVOT_SECOND
+#if defined(__CUDACC__)
+  double best_v[32];  // a warp each
+  int best_i[32];
+  int nan[32];
+#else
   double best_v[MAX_THREADS];
   int best_i[MAX_THREADS];
   int nan[MAX_THREADS];
+#endif
 };
 
 FC_LDLT_FN double &at(const Front &f, int64_t r, int64_t c) { return f.F[r + c * f.m]; }
@@ -79,75 +91,103 @@ FC_LDLT_FN void exchange(T &x, T &y) {
   y = t;
 }
 
-// row[0..len) <- row D for the columns k0.. (times_d, cholesky.rs:458-481); one thread.
-FC_LDLT_FN void times_d(double *row, int len, const Front &f, int k0) {
-  int k = 0;
-  while (k < len) {
-    if (f.pivots[k0 + k] == PIVOT_FIRST) {
-      const double x = row[k], y = k + 1 < len ? row[k + 1] : 0.0;
-      const double d11 = at(f, k0 + k, k0 + k), d21 = at(f, k0 + k + 1, k0 + k), d22 = at(f, k0 + k + 1, k0 + k + 1);
-      row[k] = add(mul(x, d11), mul(y, d21));
-      if (k + 1 < len) row[k + 1] = add(mul(x, d21), mul(y, d22));
-      k += 2;
-    } else {
-      row[k] = mul(row[k], at(f, k0 + k, k0 + k));
-      k += 1;
-    }
-  }
+// Element q of row c of L D over the panel's factored columns (times_d, cholesky.rs:458-481).
+FC_LDLT_FN double times_d(const Shared &sh, const Front &f, int c0, int c, int q) {
+  const double x = at(f, c, c0 + q);
+  if (sh.kind[q] == PIVOT_FIRST) return add(mul(x, sh.d[q]), mul(at(f, c, c0 + q + 1), sh.e[q]));
+  if (sh.kind[q] == PIVOT_SECOND) return add(mul(at(f, c, c0 + q - 1), sh.e[q - 1]), mul(x, sh.d[q]));
+  return mul(x, sh.d[q]);
 }
 
-// Column c (local, >= k) of the part still to factor, rows [k, m), into out: the front's entries
-// less the products with the panel's factored columns [c0, k) (Block::current, ldlt.rs:173-192).
+// The block's largest value bv and its lowest index bi (lo when every value is zero), from each
+// thread's; false when any thread met a NaN. Every thread gets the same answer; a barrier in it
+// comes after the threads' writes before the call.
 template <class Block>
-FC_LDLT_FN void current(Block &blk, Shared &sh, const Front &f, int c0, int k, int c, double *out) {
-  if (blk.tid() == 0) {
-    for (int q = c0; q < k; ++q) sh.row[q - c0] = at(f, c, q);
-    times_d(sh.row, k - c0, f, c0);
-  }
-  blk.sync();
-  for (int64_t r = k + blk.tid(); r < f.m; r += blk.size()) {
-    double v = r >= c ? at(f, r, c) : at(f, c, r);
-    for (int q = c0; q < k; ++q) v = sub(v, mul(at(f, r, q), sh.row[q - c0]));
-    out[r] = v;
-  }
-  blk.sync();
-}
-
-// The largest magnitude of v over [lo, hi) except `skip`, with the lowest such index (largest,
-// ldlt.rs:145-163). Returns false when an entry is not a number (the reference's NaN, which its
-// callers treat as a singular column). Every thread gets the same answer.
-template <class Block>
-FC_LDLT_FN bool largest(Block &blk, Shared &sh, const double *v, int lo, int hi, int skip, int &index, double &value) {
-  double bv = 0.0;
-  int bi = lo, bn = 0;
-  for (int i = lo + blk.tid(); i < hi; i += blk.size()) {
-    if (i == skip) continue;
-    const double x = magnitude(v[i]);
-    if (not_a_number(x)) {
-      bn = 1;
-    } else if (x > bv) {
-      bv = x;
-      bi = i;
+FC_LDLT_ONCE bool block_best(Block &blk, Shared &sh, double bv, int bi, int bn, int lo, int none, int &index,
+                             double &value) {
+  auto better = [](double x, int i, double y, int j) { return x > y || (x == y && i < j); };
+#if defined(__CUDACC__)
+  const int lane = blk.tid() & 31, warps = (blk.size() + 31) >> 5;
+  auto warp_best = [&]() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double x = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int i = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (better(x, i, bv, bi)) bv = x, bi = i;
     }
+    bn = __any_sync(0xffffffffu, bn);
+  };
+  warp_best();
+  if (lane == 0) {
+    sh.best_v[blk.tid() >> 5] = bv;
+    sh.best_i[blk.tid() >> 5] = bi;
+    sh.nan[blk.tid() >> 5] = bn;
   }
+  blk.sync();
+  bv = lane < warps ? sh.best_v[lane] : 0.0;
+  bi = lane < warps ? sh.best_i[lane] : none;
+  bn = lane < warps ? sh.nan[lane] : 0;
+  warp_best();
+#else
   sh.best_v[blk.tid()] = bv;
   sh.best_i[blk.tid()] = bi;
   sh.nan[blk.tid()] = bn;
   blk.sync();
-  double v0 = 0.0;
-  int i0 = lo, n0 = 0;
   for (int t = 0; t < blk.size(); ++t) {
-    n0 |= sh.nan[t];
-    const double x = sh.best_v[t];
-    if (x > v0 || (x == v0 && x > 0.0 && sh.best_i[t] < i0)) {
-      v0 = x;
-      i0 = sh.best_i[t];
+    bn |= sh.nan[t];
+    if (better(sh.best_v[t], sh.best_i[t], bv, bi)) bv = sh.best_v[t], bi = sh.best_i[t];
+  }
+#endif
+  index = bv > 0.0 ? bi : lo;
+  value = bv;
+  return bn == 0;
+}
+
+// Column c (local, >= k) of the part still to factor, rows [k, m), into out: the front's entries
+// less the products with the panel's factored columns [c0, k) (Block::current, ldlt.rs:173-192),
+// a row a thread, 16 columns' loads in flight; and the largest magnitude of it over [lo, w) except
+// row `skip`, with the lowest such index (largest, ldlt.rs:145-163; lo when all are zero). Returns
+// false when one of those entries is not a number (the reference's NaN, which its callers treat
+// as a singular column). Every thread gets the same answer.
+template <class Block>
+FC_LDLT_FN bool current(Block &blk, Shared &sh, const Front &f, int c0, int k, int c, double *out, int lo, int skip,
+                        int &index, double &value) {
+  const int len = k - c0;
+  for (int q = blk.tid(); q < len; q += blk.size()) sh.row[q] = times_d(sh, f, c0, c, q);
+  blk.sync();
+  double bv = 0.0;
+  int bi = lo, bn = 0;
+  for (int64_t r = k + blk.tid(); r < f.m; r += blk.size()) {
+    double v = r >= c ? at(f, r, c) : at(f, c, r);
+    const double *L = &at(f, r, c0);
+    int q = 0;
+    for (; q + 16 <= len; q += 16) {
+      double l[16];
+#if defined(__CUDACC__)
+#pragma unroll
+#endif
+      for (int t = 0; t < 16; ++t) l[t] = L[(q + t) * f.m];
+#if defined(__CUDACC__)
+#pragma unroll
+#endif
+      for (int t = 0; t < 16; ++t) v = sub(v, mul(l[t], sh.row[q + t]));
+    }
+#if defined(__CUDACC__)
+#pragma unroll 4
+#endif
+    for (; q < len; ++q) v = sub(v, mul(L[q * f.m], sh.row[q]));
+    out[r] = v;
+    if (r >= lo && r < f.w && r != skip) {
+      const double x = magnitude(v);
+      if (not_a_number(x)) {
+        bn = 1;
+      } else if (x > bv) {
+        bv = x;
+        bi = (int)r;
+      }
     }
   }
-  blk.sync();
-  index = i0;
-  value = v0;
-  return n0 == 0;
+  return block_best(blk, sh, bv, bi, bn, lo, f.w, index, value);
 }
 
 // Symmetric interchange of local columns p and q (both at pivot positions >= k) in the front,
@@ -174,12 +214,14 @@ FC_LDLT_FN void interchange(Block &blk, const Front &f, int p, int q, double *a,
 
 // A 1 x 1 pivot at k from the current column (Block::one, ldlt.rs:206-221).
 template <class Block>
-FC_LDLT_FN void one(Block &blk, const Front &f, int k, const double *col) {
+FC_LDLT_FN void one(Block &blk, Shared &sh, const Front &f, int c0, int k, const double *col) {
   const double d = col[k];
   for (int64_t r = k + 1 + blk.tid(); r < f.m; r += blk.size()) at(f, r, k) = col[r] / d;
   if (blk.tid() == 0) {
     at(f, k, k) = d;
     f.pivots[k] = PIVOT_ONE;
+    sh.d[k - c0] = d;
+    sh.kind[k - c0] = PIVOT_ONE;
   }
   blk.sync();
 }
@@ -187,7 +229,7 @@ FC_LDLT_FN void one(Block &blk, const Front &f, int k, const double *col) {
 // A 2 x 2 pivot at k, k + 1 from the current columns a (k) and b (k + 1) (Block::two,
 // ldlt.rs:223-248).
 template <class Block>
-FC_LDLT_FN void two(Block &blk, const Front &f, int k, const double *a, const double *b) {
+FC_LDLT_FN void two(Block &blk, Shared &sh, const Front &f, int c0, int k, const double *a, const double *b) {
   const double d11 = a[k], d21 = a[k + 1], d22 = b[k + 1];
   const double det = sub(mul(d11, d22), mul(d21, d21));
   for (int64_t r = k + 2 + blk.tid(); r < f.m; r += blk.size()) {
@@ -201,6 +243,11 @@ FC_LDLT_FN void two(Block &blk, const Front &f, int k, const double *a, const do
     at(f, k + 1, k + 1) = d22;
     f.pivots[k] = PIVOT_FIRST;
     f.pivots[k + 1] = PIVOT_SECOND;
+    sh.d[k - c0] = d11;
+    sh.e[k - c0] = d21;
+    sh.d[k - c0 + 1] = d22;
+    sh.kind[k - c0] = PIVOT_FIRST;
+    sh.kind[k - c0 + 1] = PIVOT_SECOND;
   }
   blk.sync();
 }
@@ -216,11 +263,10 @@ FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_ou
   int k = c0;
   *twos = 0;
   while (k < end) {
-    current(blk, sh, f, c0, k, k, a);
-    const double akk = magnitude(a[k]);
     int r0;
     double omega_k;
-    const bool numbers = largest(blk, sh, a, k + 1, w, -1, r0, omega_k);
+    const bool numbers = current(blk, sh, f, c0, k, k, a, k + 1, -1, r0, omega_k);
+    const double akk = magnitude(a[k]);
     if (!finite(akk) || !numbers || !finite(omega_k)) return f.order[k];
     bool pair = false;
     int p = k, pi = k, pr = k;
@@ -229,10 +275,9 @@ FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_ou
       int i = k, r = r0, step = 0;
       double omega_i = omega_k;
       for (;;) {
-        current(blk, sh, f, c0, k, r, b);
         int s;
         double omega_r;
-        const bool fine = largest(blk, sh, b, k, w, r, s, omega_r);
+        const bool fine = current(blk, sh, f, c0, k, r, b, k, r, s, omega_r);
         const double arr = magnitude(b[r]);
         if (!finite(arr) || !fine || !finite(omega_r)) return f.order[k];
         step += 1;
@@ -256,7 +301,7 @@ FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_ou
     if (!pair) {
       interchange(blk, f, k, p, a, b);
       if (!(magnitude(a[k]) > PIVOT_TOLERANCE * f.scale[f.order[k]])) return f.order[k];
-      one(blk, f, k, a);
+      one(blk, sh, f, c0, k, a);
       k += 1;
     } else {
       // i to k, then r to k + 1 (r was at k if i took its place)
@@ -266,7 +311,7 @@ FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_ou
       const double s0 = f.scale[f.order[k]], s1 = f.scale[f.order[k + 1]];
       const double size = s0 < s1 ? s1 : s0;
       if (!(offdiagonal > PIVOT_TOLERANCE * size)) return f.order[k];
-      two(blk, f, k, a, b);
+      two(blk, sh, f, c0, k, a, b);
       *twos += 1;
       k += 2;
     }
@@ -300,12 +345,13 @@ FC_LDLT_FN void panel_w(Block &blk, const Front &f, int c0, int c1) {
   blk.sync();
 }
 
-// W21 = L21 D: the rows [w, m) of the front times its block diagonal, ld_out x w, for the update
+// W21 = L21 D: the rows [r0, r1) of the front, of those past its columns, times its block diagonal,
+// row r at out[r - w], leading dimension ld_out, for the update
 // matrix U = -L21 W21^T the parent assembles (products' Y for a descendant, cholesky.rs:531-548,
 // with times_d's operations).
 template <class Block>
-FC_LDLT_FN void front_w21(Block &blk, const Front &f, double *out, int64_t ld_out) {
-  for (int64_t r = f.w + blk.tid(); r < f.m; r += blk.size()) {
+FC_LDLT_FN void front_w21(Block &blk, const Front &f, double *out, int64_t ld_out, int64_t r0, int64_t r1) {
+  for (int64_t r = r0 + blk.tid(); r < r1; r += blk.size()) {
     double *o = out + (r - f.w);
     int k = 0;
     while (k < f.w) {
@@ -324,21 +370,32 @@ FC_LDLT_FN void front_w21(Block &blk, const Front &f, double *out, int64_t ld_ou
   blk.sync();
 }
 
-// D out of a factored front: d[c] receives D's diagonal and e[c] its subdiagonal (the 2 x 2
-// pivots' d21 at their first column, else 0); the front's own block becomes unit lower (ones on
-// the diagonal, zeros where a 2 x 2 pivot's d21 was), the form the triangular solve reads.
+// All of W21.
+template <class Block>
+FC_LDLT_FN void front_w21(Block &blk, const Front &f, double *out, int64_t ld_out) {
+  front_w21(blk, f, out, ld_out, f.w, f.m);
+}
+
+// D out of a factored front's columns [c0, c1): d[c] receives D's diagonal and e[c] its
+// subdiagonal (the 2 x 2 pivots' d21 at their first column, else 0); the front's own block becomes
+// unit lower (ones on the diagonal, zeros where a 2 x 2 pivot's d21 was), the form the triangular
+// solve reads.
+template <class Block>
+FC_LDLT_FN void split_d(Block &blk, const Front &f, double *d, double *e, int c0, int c1) {
+  for (int c = c0 + blk.tid(); c < c1; c += blk.size()) {
+    d[c] = at(f, c, c);
+    e[c] = 0.0;
+    at(f, c, c) = 1.0;
+    if (f.pivots[c] == PIVOT_FIRST) {
+      e[c] = at(f, c + 1, c);
+      at(f, c + 1, c) = 0.0;
+    }
+  }
+  blk.sync();
+}
 template <class Block>
 FC_LDLT_FN void split_d(Block &blk, const Front &f, double *d, double *e) {
-  for (int c = blk.tid(); c < f.w; c += blk.size()) {
-    d[c] = at(f, c, c);
-    e[c] = f.pivots[c] == PIVOT_FIRST ? at(f, c + 1, c) : 0.0;
-  }
-  blk.sync();
-  for (int c = blk.tid(); c < f.w; c += blk.size()) {
-    at(f, c, c) = 1.0;
-    if (f.pivots[c] == PIVOT_FIRST) at(f, c + 1, c) = 0.0;
-  }
-  blk.sync();
+  split_d(blk, f, d, e, 0, f.w);
 }
 
 // y <- D^-1 y for the unknowns [0, n) of R right-hand sides (row-major, y[i * R + j]), D given by
@@ -361,18 +418,28 @@ FC_LDLT_FN void apply_d_inverse(int64_t i, int R, const double *d, const double 
 
 // X = L^-1 for an nb x nb unit lower block of a front (nb <= 64; L's diagonal is not read),
 // column-major with leading dimension ldx: column j by forward substitution, x_i = -sum over
-// k in [j, i) of L(i, k) x_k, summed in k order from zero. One thread per column; the strictly
-// upper part of X is left as it is (zero in the solve's inverse arena).
+// k in [j, i) of L(i, k) x_k, summed in k order from zero. Step k adds its term to every sum
+// still open (rows past k, columns up to k), so a step is parallel over up to 1024 entries and
+// each entry's terms still come in k order; until the end X holds the sums themselves. The
+// strictly upper part of X is left as it is (zero in the solve's inverse arena).
 template <class Block>
 FC_LDLT_FN void unit_lower_inverse(Block &blk, const double *Lb, int64_t ldl, int nb, double *X, int64_t ldx) {
-  for (int j = blk.tid(); j < nb; j += blk.size()) {
-    double *x = X + (int64_t)j * ldx;
-    x[j] = 1.0;
-    for (int i = j + 1; i < nb; ++i) {
-      double s = 0.0;
-      for (int k = j; k < i; ++k) s = add(s, mul(Lb[i + (int64_t)k * ldl], x[k]));
-      x[i] = -s;
+  for (int e = blk.tid(); e < nb * nb; e += blk.size())
+    if (e % nb > e / nb) X[e % nb + (int64_t)(e / nb) * ldx] = 0.0;
+  blk.sync();
+  for (int k = 0; k < nb; ++k) {
+    const int rows = nb - 1 - k;
+    for (int e = blk.tid(); e < rows * (k + 1); e += blk.size()) {
+      const int i = k + 1 + e % rows, j = e / rows;
+      const double x = j == k ? 1.0 : -X[k + (int64_t)j * ldx];
+      X[i + (int64_t)j * ldx] = add(X[i + (int64_t)j * ldx], mul(Lb[i + (int64_t)k * ldl], x));
     }
+    blk.sync();
+  }
+  for (int e = blk.tid(); e < nb * nb; e += blk.size()) {
+    const int i = e % nb, j = e / nb;
+    if (i == j) X[i + (int64_t)j * ldx] = 1.0;
+    if (i > j) X[i + (int64_t)j * ldx] = -X[i + (int64_t)j * ldx];
   }
   blk.sync();
 }

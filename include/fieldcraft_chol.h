@@ -40,8 +40,7 @@ extern "C" {
 /* FP64 symmetric indefinite P A P^T = L D L^T (LdltFactor, crates/solver/src/ldlt.rs): bounded
  * Bunch-Kaufman pivots inside supernodes, on the same analysis; values (fc_chol_values, the
  * reference's Block::values), inertia (fc_chol_inertia) and solves through fc_chol_solve and
- * fc_chol_solve_device (the first solve after a factorisation folds the pivot orders into the
- * solve's structure, which waits for the stream), and fc_chol_refine_solve_device by plain
+ * fc_chol_solve_device, and fc_chol_refine_solve_device by plain
  * refinement (FC_OPTION_REFINEMENT = 1; conjugate gradients needs a definite preconditioner);
  * no-alloc and persistent solves return FC_INVALID_ARGUMENT. A column with no pivot is
  * FC_SINGULAR (FactorError::Singular). */
@@ -256,8 +255,8 @@ int64_t fc_chol_trace_read(fc_chol *h, int64_t *out, int64_t cap);
  * `kinds` entries), then clears them. Kinds: 0 front assembly, 1 panel (factor,
  * invert and solve below a diagonal block), 3 GEMM of the factor, 10 and 11 the two GEMMs of a
  * doubling step of the diagonal-block inverses, 12 the tcgen05 GEMM of the mixed-precision factor
- * and 15 the packing of its operands; 16 the LDL^T factor's pivoted panel steps, 17 its W21 and D
- * split, 18 its unit lower block inverses;
+ * and 15 the packing of its operands; 16 the LDL^T factor's pivoted panel steps, 17 its W21, 18 its
+ * D split and unit lower block inverses;
  * 19 GEMM, 20 front assembly, 22 forward inverse, 23
  * backward inverse of the solve (level by level), 24 forward, 25 backward persistent launch of the
  * solve, 29 forward, 30 backward step of the thin supernodes (32 covers all). */
