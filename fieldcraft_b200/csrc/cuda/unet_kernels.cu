@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "spmv.cuh"
 #include "unet_kernels.cuh"
 
 namespace fc {
@@ -13,11 +14,17 @@ namespace unet {
 namespace {
 
 using bf16 = __nv_bfloat16;
-constexpr int THREADS = 128;
+// Programmatic dependent launch, as in kernels.cuh: a convolution loads its weights, which no
+// kernel of a pass writes, before it waits for the kernel whose output it reads.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 constexpr float SLOPE = 0.05f;  // leaky ReLU: x for x > 0, SLOPE x otherwise
 __device__ __forceinline__ float gate(float mask) { return mask > 0.f ? 1.f : SLOPE; }
-constexpr int TX = 8, TY = 8;         // output tile of a convolution CTA: 8 x 8 voxels of one z plane
-constexpr int HX = TX + 2, HY = TY + 2, HV = HX * HY * 3;  // its input halo
+constexpr int TX = 8, TY = 8;         // output tile of a CTA: 8 x 8 voxels of one or two z planes
+constexpr int HX = TX + 2, HY = TY + 2;  // its input halo, with a plane more on either side in z
+constexpr int TZ = 2;                    // planes of a convolution's tile
+constexpr int HV_CONV = HX * HY * (TZ + 2), HV_DW = HX * HY * 3;
+constexpr int CONV_THREADS = 128 * TZ, DW_THREADS = 9 * 32;
 
 __device__ __forceinline__ void cp16(void *smem, const void *gmem, bool ok) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -49,50 +56,70 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 __host__ __device__ constexpr int cstride(int c) { return c + 8; }  // shared-memory channel stride
 template <int CIN, int COUT>
 __host__ __device__ constexpr size_t conv_smem() {
-  return sizeof(bf16) * ((size_t)27 * COUT * cstride(CIN) + (size_t)HV * cstride(CIN));
+  return sizeof(bf16) * ((size_t)27 * COUT * cstride(CIN) + (size_t)HV_CONV * cstride(CIN));
 }
 
-// One CTA per 8 x 8 tile of a z plane (persistent over tiles); all 27 taps' weights stay in
-// shared memory. Warp w computes voxel rows y = 2w, 2w + 1 (16 voxels) x COUT channels.
+// The halo of a tile (planes [z - 1, z - 1 + PLANES) of one grid of the batch) into shared memory,
+// zero outside the grid.
+template <int CIN, int PLANES, int THREADS>
+__device__ __forceinline__ void load_halo(bf16 *ts, const Grid &g, const bf16 *in, int x0, int y0, int z) {
+  constexpr int CS = cstride(CIN);
+  for (int e = threadIdx.x; e < HX * HY * PLANES * (CIN / 8); e += THREADS) {
+    const int hv = e / (CIN / 8), c8 = e % (CIN / 8);
+    const int hx = hv % HX, hy = (hv / HX) % HY, hz = hv / (HX * HY);
+    const int gx = x0 + hx - 1, gy = y0 + hy - 1, gz = z + hz - 1;
+    const bool ok = gx >= 0 && gx < g.X && gy >= 0 && gy < g.Y && gz >= 0 && gz < g.Z;
+    const int64_t v = ok ? ((int64_t)gz * g.Y + gy) * g.X + gx : 0;
+    cp16(ts + hv * CS + c8 * 8, in + v * CIN + c8 * 8, ok);
+  }
+}
+
+// One CTA per 8 x 8 x 2 tile of one of the batch's grids (persistent over tiles); all 27 taps'
+// weights stay in shared memory. Warp w computes voxel rows y = 2 (w & 3), 2 (w & 3) + 1 of plane
+// w / 4 (16 voxels) x COUT channels. The passes of a batch run side by side: alone, a pass on a
+// plate's grid has about one tile an SM and a launch is mostly the weights' load: 16 passes on a
+// 33 x 33 x 9 grid take 33 us (7.6 us each alone). Bound by the fragments' shared-memory reads.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(THREADS) conv3_kernel(Grid g, const bf16 *__restrict__ in,
-                                                       const bf16 *__restrict__ w, const float *__restrict__ bias,
-                                                       int relu, const bf16 *__restrict__ mask, bf16 *__restrict__ out) {
+__global__ void __launch_bounds__(CONV_THREADS, 2)
+    conv3_kernel(Grid g, int batch, const bf16 *__restrict__ in, const bf16 *__restrict__ w,
+                 const float *__restrict__ bias, int relu, const bf16 *__restrict__ mask, bf16 *__restrict__ out) {
   constexpr int CS = cstride(CIN);
   extern __shared__ __align__(16) unsigned char smem[];
   bf16 *ws = reinterpret_cast<bf16 *>(smem);
   bf16 *ts = ws + 27 * COUT * CS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int gq = lane >> 2, tg = lane & 3;
-  for (int e = tid; e < 27 * COUT * (CIN / 8); e += THREADS) {
-    const int row = e / (CIN / 8), c8 = e % (CIN / 8);
-    cp16(ws + row * CS + c8 * 8, w + row * CIN + c8 * 8, true);
+  const int gq = lane >> 2, tg = lane & 3, plane = warp >> 2, row = 2 * (warp & 3);
+  for (int e = tid; e < 27 * COUT * (CIN / 8); e += CONV_THREADS) {
+    const int r = e / (CIN / 8), c8 = e % (CIN / 8);
+    cp16(ws + r * CS + c8 * 8, w + r * CIN + c8 * 8, true);
   }
   commit();
-  const int ntx = (g.X + TX - 1) / TX, nty = (g.Y + TY - 1) / TY;
-  const int ntiles = ntx * nty * g.Z;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int x0 = (tile % ntx) * TX, y0 = ((tile / ntx) % nty) * TY, z = tile / (ntx * nty);
+  pdl_wait();
+  pdl_trigger();
+  const int ntx = (g.X + TX - 1) / TX, nty = (g.Y + TY - 1) / TY, ntz = (g.Z + TZ - 1) / TZ;
+  const int ntiles = ntx * nty * ntz;
+  const int64_t total = (int64_t)ntiles * batch, voxels = g.voxels();
+  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const int tile = (int)(t % ntiles);
+    const int64_t base = t / ntiles * voxels;
+    const int x0 = (tile % ntx) * TX, y0 = ((tile / ntx) % nty) * TY, z0 = tile / (ntx * nty) * TZ;
     __syncthreads();
-    for (int e = tid; e < HV * (CIN / 8); e += THREADS) {
-      const int hv = e / (CIN / 8), c8 = e % (CIN / 8);
-      const int hx = hv % HX, hy = (hv / HX) % HY, hz = hv / (HX * HY);
-      const int gx = x0 + hx - 1, gy = y0 + hy - 1, gz = z + hz - 1;
-      const bool ok = gx >= 0 && gx < g.X && gy >= 0 && gy < g.Y && gz >= 0 && gz < g.Z;
-      const int64_t v = ok ? ((int64_t)gz * g.Y + gy) * g.X + gx : 0;
-      cp16(ts + hv * CS + c8 * 8, in + v * CIN + c8 * 8, ok);
-    }
+    load_halo<CIN, TZ + 2, CONV_THREADS>(ts, g, in + base * CIN, x0, y0, z0);
     commit();
     wait_all();
     __syncthreads();
+    const int z = z0 + plane;
+    if (z >= g.Z) continue;
     float acc[COUT / 8][4];
 #pragma unroll
     for (int nt = 0; nt < COUT / 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
     const int q = lane >> 3, r = lane & 7;
+#pragma unroll 3
     for (int tap = 0; tap < 27; ++tap) {
       const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-      // A rows: voxel (x = r, y = 2 warp + (q & 1)); B rows: output channel
-      const bf16 *arow = ts + (((1 + dz) * HY + (1 + 2 * warp + (q & 1) + dy)) * HX + (1 + r + dx)) * CS + (q >> 1) * 8;
+      // A rows: voxel (x = r, y = row + (q & 1)); B rows: output channel
+      const bf16 *arow =
+          ts + (((1 + plane + dz) * HY + (1 + row + (q & 1) + dy)) * HX + (1 + r + dx)) * CS + (q >> 1) * 8;
 #pragma unroll
       for (int ks = 0; ks < CIN / 16; ++ks) {
         uint32_t a[4];
@@ -109,9 +136,9 @@ __global__ void __launch_bounds__(THREADS) conv3_kernel(Grid g, const bf16 *__re
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int gx = x0 + gq, gy = y0 + 2 * warp + h;
+      const int gx = x0 + gq, gy = y0 + row + h;
       if (gx >= g.X || gy >= g.Y) continue;
-      const int64_t v = ((int64_t)z * g.Y + gy) * g.X + gx;
+      const int64_t v = base + ((int64_t)z * g.Y + gy) * g.X + gx;
 #pragma unroll
       for (int nt = 0; nt < COUT / 8; ++nt) {
         const int co = nt * 8 + 2 * tg;
@@ -129,138 +156,175 @@ __global__ void __launch_bounds__(THREADS) conv3_kernel(Grid g, const bf16 *__re
   }
 }
 
-// Weight gradient: CTA (chunk, tap group of 4): warp w accumulates tap 4 group + w over the
-// chunk's tiles as the GEMM dW_tap (COUT x CIN) += dY^T (COUT x voxels) X_tap (voxels x CIN), both
-// operands read transposed by ldmatrix.trans from channels-last tiles.
+// Weight gradient: CTA blockIdx.x takes a chunk of one pair's tiles (a pair: `passes` grids of the
+// batch, whose gradients add), warp w the three taps along x at (dy, dz) = (w % 3 - 1, w / 3 - 1),
+// each the GEMM dW_tap (COUT x CIN) += dY^T (COUT x voxels) X_tap (voxels x CIN), both operands
+// read transposed by ldmatrix.trans from channels-last tiles and dY's fragments shared by the
+// three. Warp 4 also multiplies dY^T by ones: the bias gradient. A chunk's partial is 28 blocks of
+// COUT x CIN floats, the taps' and one whose first COUT are the bias's. The next tile's copies are
+// in flight while a tile is multiplied (16 passes on a 33 x 33 x 9 grid: 53 us, with one buffer 56). A
+// warp a tap, seven CTAs a chunk, read every tile seven times; a pass at a time, its 8 us launch was
+// latency, 16 of them 131 us.
 template <int CIN, int COUT>
 __host__ __device__ constexpr size_t dw_smem() {
-  return sizeof(bf16) * ((size_t)HV * cstride(CIN) + (size_t)TX * TY * cstride(COUT));
+  return 2 * sizeof(bf16) * ((size_t)HV_DW * cstride(CIN) + (size_t)TX * TY * cstride(COUT));
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(THREADS) conv3_dw_kernel(Grid g, const bf16 *__restrict__ in,
-                                                          const bf16 *__restrict__ dy, int tiles_per_chunk,
-                                                          float *__restrict__ part) {
+__global__ void __launch_bounds__(DW_THREADS) conv3_dw_kernel(Grid g, int passes, int chunks,
+                                                              const bf16 *__restrict__ in,
+                                                              const bf16 *__restrict__ dy, float *__restrict__ part) {
   constexpr int CS = cstride(CIN), DS = cstride(COUT);
   extern __shared__ __align__(16) unsigned char smem[];
-  bf16 *ts = reinterpret_cast<bf16 *>(smem);
-  bf16 *ds = ts + HV * CS;
+  constexpr int BUFFER = HV_DW * CS + TX * TY * DS;
+  bf16 *buffers = reinterpret_cast<bf16 *>(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tg = lane & 3, q = lane >> 3, r = lane & 7;
-  const int tap = blockIdx.y * 4 + warp;
-  const bool active = tap < 27;
-  const int dx = tap % 3 - 1, dyo = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
+  const int dyo = warp % 3 - 1, dz = warp / 3 - 1;
   const int ntx = (g.X + TX - 1) / TX, nty = (g.Y + TY - 1) / TY;
   const int ntiles = ntx * nty * g.Z;
-  float acc[COUT / 16][CIN / 8][4];
+  const int pair = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
+  const int64_t total = (int64_t)ntiles * passes, per = (total + chunks - 1) / chunks, voxels = g.voxels();
+  float acc[3][COUT / 16][CIN / 8][4];
+  float sum[COUT / 16][4];
 #pragma unroll
-  for (int mt = 0; mt < COUT / 16; ++mt)
+  for (int mt = 0; mt < COUT / 16; ++mt) {
+    sum[mt][0] = sum[mt][1] = sum[mt][2] = sum[mt][3] = 0.f;
 #pragma unroll
-    for (int nt = 0; nt < CIN / 8; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = acc[mt][nt][2] = acc[mt][nt][3] = 0.f;
-  const int t0 = blockIdx.x * tiles_per_chunk, t1 = min(ntiles, t0 + tiles_per_chunk);
-  for (int tile = t0; tile < t1; ++tile) {
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+      for (int nt = 0; nt < CIN / 8; ++nt) acc[t][mt][nt][0] = acc[t][mt][nt][1] = acc[t][mt][nt][2] = acc[t][mt][nt][3] = 0.f;
+  }
+  const int64_t t0 = chunk * per, t1 = min(total, t0 + per);
+  auto load = [&](int64_t t) {
+    bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + HV_DW * CS;
+    const int tile = (int)(t % ntiles);
+    const int64_t base = ((int64_t)pair * passes + t / ntiles) * voxels;
     const int x0 = (tile % ntx) * TX, y0 = ((tile / ntx) % nty) * TY, z = tile / (ntx * nty);
-    __syncthreads();
-    for (int e = tid; e < HV * (CIN / 8); e += THREADS) {
-      const int hv = e / (CIN / 8), c8 = e % (CIN / 8);
-      const int hx = hv % HX, hy = (hv / HX) % HY, hz = hv / (HX * HY);
-      const int gx = x0 + hx - 1, gy = y0 + hy - 1, gz = z + hz - 1;
-      const bool ok = gx >= 0 && gx < g.X && gy >= 0 && gy < g.Y && gz >= 0 && gz < g.Z;
-      const int64_t v = ok ? ((int64_t)gz * g.Y + gy) * g.X + gx : 0;
-      cp16(ts + hv * CS + c8 * 8, in + v * CIN + c8 * 8, ok);
-    }
-    for (int e = tid; e < TX * TY * (COUT / 8); e += THREADS) {
+    load_halo<CIN, 3, DW_THREADS>(ts, g, in + base * CIN, x0, y0, z);
+    for (int e = tid; e < TX * TY * (COUT / 8); e += DW_THREADS) {
       const int m = e / (COUT / 8), c8 = e % (COUT / 8);
       const int gx = x0 + m % TX, gy = y0 + m / TX;
       const bool ok = gx < g.X && gy < g.Y;
-      const int64_t v = ok ? ((int64_t)z * g.Y + gy) * g.X + gx : 0;
+      const int64_t v = base + (ok ? ((int64_t)z * g.Y + gy) * g.X + gx : 0);
       cp16(ds + m * DS + c8 * 8, dy + v * COUT + c8 * 8, ok);
     }
+  };
+  if (t0 < t1) load(t0);
+  commit();
+  for (int64_t t = t0; t < t1; ++t) {
+    if (t + 1 < t1) load(t + 1);  // into the buffer that the barrier below the last tile freed
     commit();
-    wait_all();
+    asm volatile("cp.async.wait_group 1;\n" ::);
     __syncthreads();
-    if (!active) continue;
+    const bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + HV_DW * CS;
 #pragma unroll
     for (int ks = 0; ks < TX * TY / 16; ++ks) {
       uint32_t a[COUT / 16][4];
 #pragma unroll
       for (int mt = 0; mt < COUT / 16; ++mt)  // rows: voxel ks 16 + (q >> 1) 8 + r; columns: channel
         ldsm_x4_t(a[mt], ds + (ks * 16 + (q >> 1) * 8 + r) * DS + mt * 16 + (q & 1) * 8);
+      if (warp == 4) {
+#pragma unroll
+        for (int mt = 0; mt < COUT / 16; ++mt) mma_bf16(sum[mt], a[mt], 0x3f803f80u, 0x3f803f80u);  // ones
+      }
       const int k = ks * 16 + (q & 1) * 8 + r;  // B row: voxel k of the tile, shifted by the tap
-      const bf16 *brow = ts + (((1 + dz) * HY + (1 + k / TX + dyo)) * HX + (1 + k % TX + dx)) * CS;
 #pragma unroll
-      for (int np = 0; np < CIN / 16; ++np) {
-        uint32_t b[4];
-        ldsm_x4_t(b, brow + (2 * np + (q >> 1)) * 8);
+      for (int dx = 0; dx < 3; ++dx) {
+        const bf16 *brow = ts + (((1 + dz) * HY + (1 + k / TX + dyo)) * HX + (k % TX + dx)) * CS;
 #pragma unroll
-        for (int mt = 0; mt < COUT / 16; ++mt) {
-          mma_bf16(acc[mt][2 * np], a[mt], b[0], b[1]);
-          mma_bf16(acc[mt][2 * np + 1], a[mt], b[2], b[3]);
+        for (int np = 0; np < CIN / 16; ++np) {
+          uint32_t b[4];
+          ldsm_x4_t(b, brow + (2 * np + (q >> 1)) * 8);
+#pragma unroll
+          for (int mt = 0; mt < COUT / 16; ++mt) {
+            mma_bf16(acc[dx][mt][2 * np], a[mt], b[0], b[1]);
+            mma_bf16(acc[dx][mt][2 * np + 1], a[mt], b[2], b[3]);
+          }
         }
       }
     }
+    __syncthreads();
   }
-  if (!active) return;
-  float *dst = part + ((int64_t)blockIdx.x * 27 + tap) * COUT * CIN;
+  float *chunk_part = part + (int64_t)blockIdx.x * 28 * COUT * CIN;
 #pragma unroll
-  for (int mt = 0; mt < COUT / 16; ++mt)
+  for (int dx = 0; dx < 3; ++dx) {
+    float *dst = chunk_part + (3 * warp + dx) * COUT * CIN;  // tap dx + 3 (dy + 3 dz)
 #pragma unroll
-    for (int nt = 0; nt < CIN / 8; ++nt) {
-      const int co = mt * 16 + gq, ci = nt * 8 + 2 * tg;
-      dst[co * CIN + ci] = acc[mt][nt][0];
-      dst[co * CIN + ci + 1] = acc[mt][nt][1];
-      dst[(co + 8) * CIN + ci] = acc[mt][nt][2];
-      dst[(co + 8) * CIN + ci + 1] = acc[mt][nt][3];
+    for (int mt = 0; mt < COUT / 16; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < CIN / 8; ++nt) {
+        const int co = mt * 16 + gq, ci = nt * 8 + 2 * tg;
+        *reinterpret_cast<float2 *>(dst + co * CIN + ci) = make_float2(acc[dx][mt][nt][0], acc[dx][mt][nt][1]);
+        *reinterpret_cast<float2 *>(dst + (co + 8) * CIN + ci) = make_float2(acc[dx][mt][nt][2], acc[dx][mt][nt][3]);
+      }
+  }
+  if (warp == 4 && tg == 0)
+#pragma unroll
+    for (int mt = 0; mt < COUT / 16; ++mt) {
+      chunk_part[27 * COUT * CIN + mt * 16 + gq] = sum[mt][0];
+      chunk_part[27 * COUT * CIN + mt * 16 + gq + 8] = sum[mt][2];
     }
 }
 
-__global__ void dw_reduce_kernel(int chunks, int64_t per_chunk, const float *__restrict__ part, float *__restrict__ gw) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < per_chunk; e += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int c = 0; c < chunks; ++c) s += part[(int64_t)c * per_chunk + e];
-    gw[e] = s;
+// The chunks' partials of each pair added in a fixed order (8 threads an element take every eighth
+// chunk, then those 8 sums in order), a pair after the other: gw and gb receive the last pair's
+// gradient; accw and accb (null: not kept) the sum of the pairs' gradients times `scale`, added to
+// what they hold when `more`.
+constexpr int REDUCE_WAYS = 8, REDUCE_ELEMENTS = 32, REDUCE_PAIRS = 8;
+__global__ void __launch_bounds__(REDUCE_WAYS * REDUCE_ELEMENTS)
+    dw_reduce_kernel(int pairs, int chunks, int weights, int cout, int64_t stride, const float *__restrict__ part,
+                     float scale, int more, float *__restrict__ accw, float *__restrict__ accb, float *__restrict__ gw,
+                     float *__restrict__ gb) {
+  __shared__ float s[REDUCE_PAIRS][REDUCE_WAYS][REDUCE_ELEMENTS];
+  const int el = threadIdx.x % REDUCE_ELEMENTS, way = threadIdx.x / REDUCE_ELEMENTS;
+  const int e = blockIdx.x * REDUCE_ELEMENTS + el;
+  const bool on = e < weights + cout;
+  float *acc = accw ? (e < weights ? accw + e : accb + (e - weights)) : nullptr;
+  float *grad = e < weights ? gw + e : gb + (e - weights);
+  float sum = on && way == 0 && acc && more ? *acc : 0.f, last = 0.f;
+  for (int p0 = 0; p0 < pairs; p0 += REDUCE_PAIRS) {
+    const int np = min(REDUCE_PAIRS, pairs - p0);
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < REDUCE_PAIRS; ++p) {  // every pair's loads in flight
+      float v = 0.f;
+      if (on && p < np)
+        for (int c = way; c < chunks; c += REDUCE_WAYS) v += part[((int64_t)(p0 + p) * chunks + c) * stride + e];
+      s[p][way][el] = v;
+    }
+    __syncthreads();
+    if (way == 0)
+      for (int p = 0; p < np; ++p) {
+        last = 0.f;
+#pragma unroll
+        for (int k = 0; k < REDUCE_WAYS; ++k) last += s[p][k][el];
+        sum += last * scale;
+      }
+  }
+  if (on && way == 0) {
+    *grad = last;
+    if (acc) *acc = sum;
   }
 }
 
-// gb[c] = sum over voxels of dy[v][c]: CTA b sums its voxel range (4 lanes per channel, each a
-// stride-4 sequence, combined in order); then one CTA sums the CTAs' partials in order.
-constexpr int BIAS_CTAS = 256;
-__global__ void __launch_bounds__(128) bias_part_kernel(int64_t voxels, int cout, const bf16 *__restrict__ dy,
-                                                        float *__restrict__ part) {
-  __shared__ float s[128];
-  const int c = threadIdx.x % 32, lane4 = threadIdx.x / 32;
-  const int64_t per = (voxels + gridDim.x - 1) / gridDim.x;
-  const int64_t v0 = blockIdx.x * per, v1 = min(voxels, v0 + per);
-  float acc = 0.f;
-  if (c < cout)
-    for (int64_t v = v0 + lane4; v < v1; v += 4) acc += __bfloat162float(dy[v * cout + c]);
-  s[threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.x < 32 && c < cout) part[blockIdx.x * 32 + c] = ((s[c] + s[32 + c]) + s[64 + c]) + s[96 + c];
-}
-__global__ void bias_reduce_kernel(int ctas, int cout, const float *__restrict__ part, float *__restrict__ gb) {
-  const int c = threadIdx.x;
-  if (c >= cout) return;
-  float s = 0.f;
-  for (int b = 0; b < ctas; ++b) s += part[b * 32 + c];
-  gb[c] = s;
-}
-
-__global__ void flip_kernel(int cin, int cout, const bf16 *__restrict__ w, bf16 *__restrict__ wt) {
-  const int total = 27 * cin * cout;
+// Every layer's BF16 weights and their flipped transposes from the FP32 parameters, a layer a
+// blockIdx.y.
+__global__ void refresh_kernel(LayerTable t, const float *__restrict__ p, bf16 *__restrict__ w, bf16 *__restrict__ wt) {
+  const int l = blockIdx.y, cin = t.cin[l], cout = t.cout[l], total = 27 * cin * cout;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
     const int ci = e % cin, co = (e / cin) % cout, tap = e / (cin * cout);
-    wt[((26 - tap) * cin + ci) * cout + co] = w[e];
+    const bf16 v = __float2bfloat16_rn(p[t.param[l] + e]);
+    w[t.weight[l] + e] = v;
+    wt[t.weight[l] + ((26 - tap) * cin + ci) * cout + co] = v;
   }
-}
-
-__global__ void to_bf16_kernel(int64_t n, const float *__restrict__ src, bf16 *__restrict__ dst) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-    dst[e] = __float2bfloat16_rn(src[e]);
 }
 
 constexpr int C32 = 32;
+// The grid transfers: blockIdx.y is the grid of the batch.
 __global__ void pool_kernel(Grid gf, Grid gc, const bf16 *__restrict__ fine, bf16 *__restrict__ coarse) {
+  fine += blockIdx.y * gf.voxels() * C32;
+  coarse += blockIdx.y * gc.voxels() * C32;
   const int64_t total = gc.voxels() * (C32 / 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(e % (C32 / 2)) * 2;
@@ -280,6 +344,9 @@ __global__ void pool_kernel(Grid gf, Grid gc, const bf16 *__restrict__ fine, bf1
 
 __global__ void up_add_kernel(Grid gf, Grid gc, const bf16 *__restrict__ coarse, const bf16 *__restrict__ skip,
                               bf16 *__restrict__ fine) {
+  coarse += blockIdx.y * gc.voxels() * C32;
+  skip += blockIdx.y * gf.voxels() * C32;
+  fine += blockIdx.y * gf.voxels() * C32;
   const int64_t total = gf.voxels() * (C32 / 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(e % (C32 / 2)) * 2;
@@ -295,6 +362,9 @@ __global__ void up_add_kernel(Grid gf, Grid gc, const bf16 *__restrict__ coarse,
 
 __global__ void up_adjoint_kernel(Grid gf, Grid gc, const bf16 *__restrict__ dfine, const bf16 *__restrict__ mask,
                                   bf16 *__restrict__ dcoarse) {
+  dfine += blockIdx.y * gf.voxels() * C32;
+  mask += blockIdx.y * gc.voxels() * C32;
+  dcoarse += blockIdx.y * gc.voxels() * C32;
   const int64_t total = gc.voxels() * (C32 / 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(e % (C32 / 2)) * 2;
@@ -317,6 +387,10 @@ __global__ void up_adjoint_kernel(Grid gf, Grid gc, const bf16 *__restrict__ dfi
 
 __global__ void pool_adjoint_kernel(Grid gf, Grid gc, const bf16 *__restrict__ dcoarse, const bf16 *__restrict__ dskip,
                                     const bf16 *__restrict__ mask, bf16 *__restrict__ dfine) {
+  dcoarse += blockIdx.y * gc.voxels() * C32;
+  dskip += blockIdx.y * gf.voxels() * C32;
+  mask += blockIdx.y * gf.voxels() * C32;
+  dfine += blockIdx.y * gf.voxels() * C32;
   const int64_t total = gf.voxels() * (C32 / 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(e % (C32 / 2)) * 2;
@@ -333,50 +407,67 @@ __global__ void pool_adjoint_kernel(Grid gf, Grid gc, const bf16 *__restrict__ d
 }
 
 constexpr int CIO = 16;  // channels of the network's input and output grids
-__global__ void scatter_input_kernel(Grid g, const int64_t *__restrict__ eq, const double *__restrict__ r,
-                                     const float *__restrict__ feat, const double *__restrict__ scale,
+// Pass p of a batch (blockIdx.y) belongs to pair p / per (per passes a pair: r, or r and -r); its
+// scales are scale[2 p] (input) and scale[2 p + 1] (output).
+__global__ void scatter_input_kernel(Grid g, int per, const int64_t *__restrict__ eq, const double *__restrict__ r,
+                                     int64_t ld, const float *__restrict__ feat, const double *__restrict__ scale,
                                      bf16 *__restrict__ x) {
-  const int64_t total = g.voxels() * CIO;
-  const double s = scale[0];
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(e % CIO);
-    const int64_t v = e / CIO;
-    float val = 0.f;
-    if (c < 3) {
-      const int64_t q = eq[3 * v + c];
-      if (q >= 0) val = (float)(r[q] * s);
-    } else if (c == 3) {
-      val = feat[v];
+  const int64_t total = g.voxels();
+  const double s = scale[2 * blockIdx.y];
+  r += blockIdx.y / per * ld;
+  x += blockIdx.y * total * CIO;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < total; v += (int64_t)gridDim.x * blockDim.x) {
+    float c[4];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int64_t q = eq[3 * v + a];
+      c[a] = q >= 0 ? (float)(r[q] * s) : 0.f;
     }
-    x[e] = __float2bfloat16_rn(val);
+    c[3] = feat[v];
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(c[0], c[1]), hi = __floats2bfloat162_rn(c[2], c[3]);
+    uint4 *dst = reinterpret_cast<uint4 *>(x + v * CIO);
+    dst[0] = make_uint4(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi), 0u, 0u);
+    dst[1] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
-__global__ void gather_output_kernel(Grid g, const int64_t *__restrict__ eq, const bf16 *__restrict__ y,
-                                     const double *__restrict__ scale, double *__restrict__ z) {
-  const int64_t total = g.voxels() * 3;
-  const double s = scale[1];
+// z (+)= the passes' outputs of pair blockIdx.y, added in pass order: add != 0 adds them to z.
+__global__ void gather_output_kernel(Grid g, int per, const int64_t *__restrict__ eq, const bf16 *__restrict__ y,
+                                     const double *__restrict__ scale, double *__restrict__ z, int64_t ld, int add) {
+  const int64_t voxels = g.voxels(), total = voxels * 3;
+  z += blockIdx.y * ld;
+  y += blockIdx.y * per * voxels * CIO;
+  scale += 2 * blockIdx.y * per;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = e / 3;
     const int c = (int)(e % 3);
     const int64_t q = eq[3 * v + c];
-    if (q >= 0) z[q] = (double)__bfloat162float(y[v * CIO + c]) * s;
+    if (q < 0) continue;
+    // products and sums rounded one by one: the odd network's output changes sign with r exactly
+    double sum = 0.0;
+    for (int p = 0; p < per; ++p)
+      sum = __dadd_rn(sum, __dmul_rn((double)__bfloat162float(y[(p * voxels + v) * CIO + c]), scale[2 * p + 1]));
+    z[q] = add ? z[q] + sum : sum;
   }
 }
 
-__global__ void scatter_grad_kernel(Grid g, const int64_t *__restrict__ eq, const double *__restrict__ dz,
-                                    const double *__restrict__ scale, bf16 *__restrict__ dy) {
-  const int64_t total = g.voxels() * CIO;
-  const double s = scale[1];
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(e % CIO);
-    const int64_t v = e / CIO;
-    float val = 0.f;
-    if (c < 3) {
-      const int64_t q = eq[3 * v + c];
-      if (q >= 0) val = (float)(dz[q] * s);
+__global__ void scatter_grad_kernel(Grid g, int per, const int64_t *__restrict__ eq, const double *__restrict__ dz,
+                                    int64_t ld, const double *__restrict__ scale, bf16 *__restrict__ dy) {
+  const int64_t total = g.voxels();
+  const double s = scale[2 * blockIdx.y + 1];
+  dz += blockIdx.y / per * ld;
+  dy += blockIdx.y * total * CIO;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < total; v += (int64_t)gridDim.x * blockDim.x) {
+    float c[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int64_t q = eq[3 * v + a];
+      c[a] = q >= 0 ? (float)(dz[q] * s) : 0.f;
     }
-    dy[e] = __float2bfloat16_rn(val);
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(c[0], c[1]), hi = __floats2bfloat162_rn(c[2], 0.f);
+    uint4 *dst = reinterpret_cast<uint4 *>(dy + v * CIO);
+    dst[0] = make_uint4(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi), 0u, 0u);
+    dst[1] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -396,181 +487,319 @@ constexpr int DOT_CTAS = 296, MAX_PAIRS = 8;
 struct PairPtrs {
   const double *a[MAX_PAIRS], *b[MAX_PAIRS];
 };
-__global__ void __launch_bounds__(256) dot_part_kernel(int64_t n, int pairs, PairPtrs pp, double *__restrict__ part) {
-  __shared__ double s[256];
+struct DirPtrs {
+  const double *p[MAX_KEPT];
+  int slot[MAX_KEPT];  // where each direction's denominator p_j.q_j is kept
+};
+// The sum of a CTA's 256 values, in every thread of the first warp: a fixed tree.
+__device__ __forceinline__ double block_sum(double v) {
+  __shared__ double s[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double sum = 0.0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) sum += s[w];
+  return sum;
+}
+// blockIdx.y is the pair
+__global__ void __launch_bounds__(256) dot_part_kernel(int64_t n, PairPtrs pp, double *__restrict__ part) {
   const int64_t per = (n + gridDim.x - 1) / gridDim.x;
   const int64_t i0 = blockIdx.x * per, i1 = min(n, i0 + per);
-  for (int k = 0; k < pairs; ++k) {
-    double acc = 0.0;
-    for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) acc += pp.a[k][i] * pp.b[k][i];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-      if ((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) part[k * gridDim.x + blockIdx.x] = s[0];
-    __syncthreads();
-  }
+  const double *a = pp.a[blockIdx.y], *b = pp.b[blockIdx.y];
+  double acc = 0.0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) acc += a[i] * b[i];
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = acc;
 }
-__global__ void __launch_bounds__(256) dot_final_kernel(int ctas, int pairs, const double *__restrict__ part,
+__global__ void __launch_bounds__(256) dot_final_kernel(int ctas, const double *__restrict__ part,
                                                         double *__restrict__ out) {
-  __shared__ double s[256];
-  for (int k = 0; k < pairs; ++k) {
-    double acc = 0.0;
-    for (int b = threadIdx.x; b < ctas; b += blockDim.x) acc += part[k * ctas + b];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-      if ((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
-      __syncthreads();
+  double acc = 0.0;
+  for (int b = threadIdx.x; b < ctas; b += blockDim.x) acc += part[blockIdx.x * ctas + b];
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) out[blockIdx.x] = acc;
+}
+
+// ---- an iteration of flexible CG, three launches ------------------------------------------------
+// Each is a programmatic dependent of the one before it (its CTAs are there when that one ends),
+// and the scalars between them are finished by the last CTA of the kernel that sums them. Bound by
+// the latency of three launches and two grid-wide sums: 36 us an iteration on 48 x 48 x 8 elements.
+// As eleven launches, with a second launch for every sum, it took 95 us.
+constexpr int FCG_THREADS = 256, STEP_THREADS = 64;
+
+// out[k] = the sum over the grid of v[k], k < count: per CTA a fixed tree and the CTAs' partials in
+// a fixed order by the last CTA to finish, all of its threads' loads in flight together (part:
+// count x gridDim.x; *ticket starts and ends zero).
+template <int K, int THREADS>
+__device__ __forceinline__ void grid_sums(double (&v)[K], int count, double *part, int *ticket, double *const (&out)[K]) {
+  constexpr int WARPS = THREADS / 32;
+  __shared__ double s[K][WARPS];
+  __shared__ int last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto cta_sums = [&]() {  // the CTA's sum of v[k] to thread k
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+      if (lane == 0) s[k][warp] = v[k];
     }
-    if (threadIdx.x == 0) out[k] = s[0];
     __syncthreads();
+    double sum = 0.0;
+    if ((int)threadIdx.x < count) {
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) sum += s[threadIdx.x][w];
+    }
+    return sum;
+  };
+  const double mine = cta_sums();
+  if ((int)threadIdx.x < count) {
+    part[threadIdx.x * gridDim.x + blockIdx.x] = mine;
+    __threadfence();
   }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double sum = 0.0;
+    if (k < count)
+#pragma unroll 8
+      for (int b = threadIdx.x; b < (int)gridDim.x; b += THREADS) sum += __ldcg(part + k * gridDim.x + b);
+    v[k] = sum;
+  }
+  const double total = cta_sums();
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (k < count && (int)threadIdx.x == k) *out[k] = total;
+  if (threadIdx.x == 0) *ticket = 0;
 }
 
-__global__ void axpy_dev_kernel(int64_t n, const double *__restrict__ alpha, double sign, const double *__restrict__ x,
-                                double *__restrict__ y) {
-  const double a = sign * alpha[0];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] += a * x[i];
+// A thread a node (three equations), 64 a CTA (a plate's 20 000 nodes in CTAs of 256 left half the
+// SMs idle): with `update`, x += alpha p and r -= alpha q, alpha = p.r / p.q;
+// then, with `z`, z = B r (inv: B's 3 x 3 blocks; null: z = r) and its products with the kept
+// directions' q_j; always r.r.
+__global__ void __launch_bounds__(STEP_THREADS) fcg_step_kernel(FcgStep a) {
+  pdl_wait();
+  pdl_trigger();
+  double v[1 + MAX_KEPT];
+#pragma unroll
+  for (int k = 0; k <= MAX_KEPT; ++k) v[k] = 0.0;
+  const double alpha = a.update && a.alpha[1] != 0.0 ? a.alpha[0] / a.alpha[1] : 0.0;
+  const int64_t nodes = (a.n + 2) / 3;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nodes; k += (int64_t)gridDim.x * blockDim.x) {
+    double r[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int64_t i = 3 * k + c;
+      r[c] = i < a.n ? a.r[i] : 0.0;
+      if (a.update && i < a.n) {
+        a.x[i] += alpha * a.p[i];
+        r[c] -= alpha * a.q[i];
+        a.r[i] = r[c];
+      }
+      v[0] += r[c] * r[c];
+    }
+    if (!a.z) continue;
+    double z[3] = {r[0], r[1], r[2]};
+    if (a.inv) {
+      const double *o = a.inv + 9 * k;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) z[c] = o[3 * c] * r[0] + o[3 * c + 1] * r[1] + o[3 * c + 2] * r[2];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int64_t i = 3 * k + c;
+      if (i >= a.n) continue;
+      a.z[i] = z[c];
+#pragma unroll
+      for (int j = 0; j < MAX_KEPT; ++j)
+        if (j < a.kept) v[1 + j] += z[c] * a.qj[j][i];
+    }
+  }
+  double *out[1 + MAX_KEPT];
+  out[0] = a.rr;
+#pragma unroll
+  for (int j = 0; j < MAX_KEPT; ++j) out[1 + j] = a.zq + j;
+  grid_sums<1 + MAX_KEPT, STEP_THREADS>(v, 1 + (a.z ? a.kept : 0), a.part, a.ticket, out);
 }
 
-struct DirPtrs {
-  const double *p[MAX_PAIRS];
-  int slot[MAX_PAIRS];  // where each direction's denominator p_j.q_j is kept
-};
-__global__ void fcg_direction_kernel(int64_t n, int m, const double *__restrict__ z, DirPtrs pj,
-                                     const double *__restrict__ num, const double *__restrict__ den,
-                                     double *__restrict__ p) {
-  double beta[MAX_PAIRS];
-  for (int j = 0; j < m; ++j) {
-    const double d = den[pj.slot[j]];
+// p = z - sum_j beta_j p_j, beta_j = num[j] / den[slot[j]]; p may be one of the p_j (an entry is read
+// before it is written).
+__global__ void __launch_bounds__(FCG_THREADS) fcg_direction_kernel(int64_t n, int m, const double *z, DirPtrs pj,
+                                                                    const double *num, const double *den, double *p) {
+  pdl_wait();
+  pdl_trigger();
+  double beta[MAX_KEPT];
+#pragma unroll
+  for (int j = 0; j < MAX_KEPT; ++j) {
+    const double d = j < m ? den[pj.slot[j]] : 0.0;
     beta[j] = d != 0.0 ? num[j] / d : 0.0;
   }
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double v = z[i];
-    for (int j = 0; j < m; ++j) v -= beta[j] * pj.p[j][i];
+    double old[MAX_KEPT], v = z[i];
+#pragma unroll
+    for (int j = 0; j < MAX_KEPT; ++j) old[j] = j < m ? pj.p[j][i] : 0.0;
+#pragma unroll
+    for (int j = 0; j < MAX_KEPT; ++j)
+      if (j < m) v -= beta[j] * old[j];
     p[i] = v;
   }
 }
 
-__global__ void input_scales_kernel(int64_t n, const double *__restrict__ nrm2, double kref, double *__restrict__ s) {
-  const double nr = sqrt(nrm2[0]);
+// q = A p, and p.r, p.q (also into *den).
+__global__ void __launch_bounds__(FCG_THREADS) fcg_product_kernel(int64_t n, const int64_t *__restrict__ ptr,
+                                                                  const int32_t *__restrict__ idx,
+                                                                  const double *__restrict__ val, const double *p,
+                                                                  const double *r, double *q, double *sums, double *den,
+                                                                  double *part, int *ticket) {
+  pdl_wait();
+  pdl_trigger();
+  double v[3] = {0.0, 0.0, 0.0};
+  constexpr int ROWS = FCG_THREADS / SPMV_LANES;
+  const int lane = threadIdx.x % SPMV_LANES;
+  // every lane of a warp goes round as often as its last row: the sums are taken by shuffles
+  const int64_t step = (int64_t)gridDim.x * ROWS;
+  for (int64_t base = blockIdx.x * (int64_t)ROWS; base < n; base += step) {
+    const int64_t row = base + threadIdx.x / SPMV_LANES;
+    const double sum = spmv_row(row < n, row, ptr, idx, val, p, lane);
+    if (row < n && lane == 0) {
+      q[row] = sum;
+      const double pr = p[row];
+      v[0] += pr * r[row];
+      v[1] += pr * sum;
+    }
+  }
+  v[2] = v[1];
+  double *const out[3] = {sums, sums + 1, den};
+  grid_sums<3, FCG_THREADS>(v, 3, part, ticket, out);
+}
+
+// The passes' scales of pair threadIdx.x from nrm2 = ||r||^2: (sqrt(n) / ||r||, ||r|| / (sqrt(n) kref)),
+// for the two passes of an odd network (s0, s1 / 2) and (-s0, -s1 / 2).
+__global__ void input_scales_kernel(int64_t n, const double *__restrict__ nrm2, double kref, int per,
+                                    double *__restrict__ s) {
+  const double nr = sqrt(nrm2[threadIdx.x]);
   const double sn = sqrt((double)n);
-  s[0] = nr > 0.0 ? sn / nr : 0.0;
-  s[1] = nr / (sn * kref);
+  const double s0 = nr > 0.0 ? sn / nr : 0.0, s1 = nr / (sn * kref);
+  s += 2 * per * threadIdx.x;
+  s[0] = s0;
+  s[1] = per == 2 ? 0.5 * s1 : s1;
+  if (per == 2) s[2] = -s0, s[3] = -0.5 * s1;
 }
 
 int grid_for(int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, 148 * 8)); }
 
 template <int CIN, int COUT>
-void conv3_launch(const Grid &g, const bf16 *in, const bf16 *w, const float *bias, bool relu, const bf16 *mask,
-                  bf16 *out, cudaStream_t st) {
-  static bool configured = false;
+void conv3_launch(const Grid &g, int batch, const bf16 *in, const bf16 *w, const float *bias, bool relu,
+                  const bf16 *mask, bf16 *out, cudaStream_t st) {
   constexpr size_t smem = conv_smem<CIN, COUT>();
-  if (!configured) {
+  static const int resident = [] {
     cudaFuncSetAttribute(conv3_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    configured = true;
-  }
-  static int sms = 0, per = 1;
-  if (sms == 0) {
-    int dev = 0;
+    int dev = 0, sms = 0, per = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, conv3_kernel<CIN, COUT>, THREADS, smem);
-    sms = std::max(sms, 1);
-  }
-  const int ntiles = ((g.X + TX - 1) / TX) * ((g.Y + TY - 1) / TY) * g.Z;
-  const int grid = std::max(1, std::min(ntiles, sms * std::max(per, 1)));
-  conv3_kernel<CIN, COUT><<<grid, THREADS, smem, st>>>(g, in, w, bias, relu ? 1 : 0, mask, out);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, conv3_kernel<CIN, COUT>, CONV_THREADS, smem);
+    return std::max(sms, 1) * std::max(per, 1);
+  }();
+  const int64_t tiles =
+      (int64_t)batch * ((g.X + TX - 1) / TX) * ((g.Y + TY - 1) / TY) * ((g.Z + TZ - 1) / TZ);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(tiles, resident)));
+  cfg.blockDim = dim3(CONV_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, conv3_kernel<CIN, COUT>, g, batch, in, w, bias, relu ? 1 : 0, mask, out);
 }
 
 template <int CIN, int COUT>
-void dw_launch(const Grid &g, const bf16 *in, const bf16 *dy, float *part, float *gw, cudaStream_t st) {
-  static bool configured = false;
+void dw_launch(const Grid &g, int pairs, int passes, const bf16 *in, const bf16 *dy, float *part, float scale,
+               bool more, float *accw, float *accb, float *gw, float *gb, cudaStream_t st) {
   constexpr size_t smem = dw_smem<CIN, COUT>();
-  if (!configured) {
-    cudaFuncSetAttribute(conv3_dw_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    configured = true;
-  }
-  const int ntiles = ((g.X + TX - 1) / TX) * ((g.Y + TY - 1) / TY) * g.Z;
-  const int chunks = dw_chunks(g);
-  const int per = (ntiles + chunks - 1) / chunks;
-  conv3_dw_kernel<CIN, COUT><<<dim3(chunks, 7), THREADS, smem, st>>>(g, in, dy, per, part);
-  const int64_t per_chunk = (int64_t)27 * CIN * COUT;
-  dw_reduce_kernel<<<grid_for(per_chunk), 256, 0, st>>>(chunks, per_chunk, part, gw);
+  static const bool configured =
+      cudaFuncSetAttribute(conv3_dw_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+      cudaSuccess;
+  (void)configured;
+  const int chunks = dw_chunks(g, pairs, passes);
+  conv3_dw_kernel<CIN, COUT><<<pairs * chunks, DW_THREADS, smem, st>>>(g, passes, chunks, in, dy, part);
+  const int elements = 27 * CIN * COUT + COUT;
+  dw_reduce_kernel<<<(elements + REDUCE_ELEMENTS - 1) / REDUCE_ELEMENTS, REDUCE_WAYS * REDUCE_ELEMENTS, 0, st>>>(
+      pairs, chunks, 27 * CIN * COUT, COUT, (int64_t)28 * CIN * COUT, part, scale, more ? 1 : 0, accw, accb, gw, gb);
 }
 
 }  // namespace
 
-void conv3(const Grid &g, int cin, int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
-           bool relu, const __nv_bfloat16 *mask, __nv_bfloat16 *out, cudaStream_t st) {
+void conv3(const Grid &g, int batch, int cin, int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
+           const float *bias, bool relu, const __nv_bfloat16 *mask, __nv_bfloat16 *out, cudaStream_t st) {
   if (cin == 32 && cout == 32)
-    conv3_launch<32, 32>(g, in, w, bias, relu, mask, out, st);
+    conv3_launch<32, 32>(g, batch, in, w, bias, relu, mask, out, st);
   else if (cin == 16 && cout == 32)
-    conv3_launch<16, 32>(g, in, w, bias, relu, mask, out, st);
+    conv3_launch<16, 32>(g, batch, in, w, bias, relu, mask, out, st);
   else if (cin == 32 && cout == 16)
-    conv3_launch<32, 16>(g, in, w, bias, relu, mask, out, st);
+    conv3_launch<32, 16>(g, batch, in, w, bias, relu, mask, out, st);
   else
-    conv3_launch<16, 16>(g, in, w, bias, relu, mask, out, st);
+    conv3_launch<16, 16>(g, batch, in, w, bias, relu, mask, out, st);
 }
 
-int dw_chunks(const Grid &g) {
-  const int ntiles = ((g.X + TX - 1) / TX) * ((g.Y + TY - 1) / TY) * g.Z;
-  return std::max(1, std::min(ntiles, 256));
+// About one chunk an SM over all pairs (9 warps and 100 accumulators a thread: one CTA an SM).
+int dw_chunks(const Grid &g, int pairs, int passes) {
+  const int64_t tiles = (int64_t)passes * ((g.X + TX - 1) / TX) * ((g.Y + TY - 1) / TY) * g.Z;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (DW_PARTIALS + pairs - 1) / pairs));
 }
 
-void conv3_dw(const Grid &g, int cin, int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *dy, float *part,
-              float *gw, float *gb, cudaStream_t st) {
+void conv3_dw(const Grid &g, int cin, int cout, int pairs, int passes, const __nv_bfloat16 *in,
+              const __nv_bfloat16 *dy, float *part, float scale, bool more, float *accw, float *accb, float *gw,
+              float *gb, cudaStream_t st) {
   if (cin == 32 && cout == 32)
-    dw_launch<32, 32>(g, in, dy, part, gw, st);
+    dw_launch<32, 32>(g, pairs, passes, in, dy, part, scale, more, accw, accb, gw, gb, st);
   else if (cin == 16 && cout == 32)
-    dw_launch<16, 32>(g, in, dy, part, gw, st);
+    dw_launch<16, 32>(g, pairs, passes, in, dy, part, scale, more, accw, accb, gw, gb, st);
   else if (cin == 32 && cout == 16)
-    dw_launch<32, 16>(g, in, dy, part, gw, st);
+    dw_launch<32, 16>(g, pairs, passes, in, dy, part, scale, more, accw, accb, gw, gb, st);
   else
-    dw_launch<16, 16>(g, in, dy, part, gw, st);
-  bias_part_kernel<<<BIAS_CTAS, 128, 0, st>>>(g.voxels(), cout, dy, part);
-  bias_reduce_kernel<<<1, 32, 0, st>>>(BIAS_CTAS, cout, part, gb);
+    dw_launch<16, 16>(g, pairs, passes, in, dy, part, scale, more, accw, accb, gw, gb, st);
 }
 
-void flip_weights(int cin, int cout, const __nv_bfloat16 *w, __nv_bfloat16 *wt, cudaStream_t st) {
-  flip_kernel<<<grid_for(27 * cin * cout), 256, 0, st>>>(cin, cout, w, wt);
+void refresh(const LayerTable &t, const float *p, __nv_bfloat16 *w, __nv_bfloat16 *wt, cudaStream_t st) {
+  refresh_kernel<<<dim3(27, t.layers), 256, 0, st>>>(t, p, w, wt);
 }
 
-void to_bf16(int64_t n, const float *src, __nv_bfloat16 *dst, cudaStream_t st) {
-  to_bf16_kernel<<<grid_for(n), 256, 0, st>>>(n, src, dst);
+void pool(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *fine, __nv_bfloat16 *coarse,
+          cudaStream_t st) {
+  pool_kernel<<<dim3(grid_for(gc.voxels() * 16), batch), 256, 0, st>>>(gf, gc, fine, coarse);
 }
-
-void pool(const Grid &gf, const Grid &gc, const __nv_bfloat16 *fine, __nv_bfloat16 *coarse, cudaStream_t st) {
-  pool_kernel<<<grid_for(gc.voxels() * 16), 256, 0, st>>>(gf, gc, fine, coarse);
-}
-void up_add(const Grid &gf, const Grid &gc, const __nv_bfloat16 *coarse, const __nv_bfloat16 *skip,
+void up_add(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *coarse, const __nv_bfloat16 *skip,
             __nv_bfloat16 *fine, cudaStream_t st) {
-  up_add_kernel<<<grid_for(gf.voxels() * 16), 256, 0, st>>>(gf, gc, coarse, skip, fine);
+  up_add_kernel<<<dim3(grid_for(gf.voxels() * 16), batch), 256, 0, st>>>(gf, gc, coarse, skip, fine);
 }
-void up_adjoint(const Grid &gf, const Grid &gc, const __nv_bfloat16 *dfine, const __nv_bfloat16 *mask,
+void up_adjoint(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *dfine, const __nv_bfloat16 *mask,
                 __nv_bfloat16 *dcoarse, cudaStream_t st) {
-  up_adjoint_kernel<<<grid_for(gc.voxels() * 16), 256, 0, st>>>(gf, gc, dfine, mask, dcoarse);
+  up_adjoint_kernel<<<dim3(grid_for(gc.voxels() * 16), batch), 256, 0, st>>>(gf, gc, dfine, mask, dcoarse);
 }
-void pool_adjoint(const Grid &gf, const Grid &gc, const __nv_bfloat16 *dcoarse, const __nv_bfloat16 *dskip,
-                  const __nv_bfloat16 *mask, __nv_bfloat16 *dfine, cudaStream_t st) {
-  pool_adjoint_kernel<<<grid_for(gf.voxels() * 16), 256, 0, st>>>(gf, gc, dcoarse, dskip, mask, dfine);
+void pool_adjoint(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *dcoarse,
+                  const __nv_bfloat16 *dskip, const __nv_bfloat16 *mask, __nv_bfloat16 *dfine, cudaStream_t st) {
+  pool_adjoint_kernel<<<dim3(grid_for(gf.voxels() * 16), batch), 256, 0, st>>>(gf, gc, dcoarse, dskip, mask, dfine);
 }
 
-void scatter_input(const Grid &g, const int64_t *eq, const double *r, const float *feat, const double *scale,
-                   __nv_bfloat16 *x, cudaStream_t st) {
-  scatter_input_kernel<<<grid_for(g.voxels() * CIO), 256, 0, st>>>(g, eq, r, feat, scale, x);
+void scatter_input(const Grid &g, int pairs, int per, const int64_t *eq, const double *r, int64_t ld,
+                   const float *feat, const double *scale, __nv_bfloat16 *x, cudaStream_t st) {
+  scatter_input_kernel<<<dim3(grid_for(g.voxels()), pairs * per), 256, 0, st>>>(g, per, eq, r, ld, feat, scale, x);
 }
-void gather_output(const Grid &g, const int64_t *eq, const __nv_bfloat16 *y, const double *scale, double *z,
-                   cudaStream_t st) {
-  gather_output_kernel<<<grid_for(g.voxels() * 3), 256, 0, st>>>(g, eq, y, scale, z);
+void gather_output(const Grid &g, int pairs, int per, const int64_t *eq, const __nv_bfloat16 *y, const double *scale,
+                   double *z, int64_t ld, bool add, cudaStream_t st) {
+  gather_output_kernel<<<dim3(grid_for(g.voxels() * 3), pairs), 256, 0, st>>>(g, per, eq, y, scale, z, ld,
+                                                                              add ? 1 : 0);
 }
-void scatter_grad(const Grid &g, const int64_t *eq, const double *dz, const double *scale, __nv_bfloat16 *dy,
-                  cudaStream_t st) {
-  scatter_grad_kernel<<<grid_for(g.voxels() * CIO), 256, 0, st>>>(g, eq, dz, scale, dy);
+void scatter_grad(const Grid &g, int pairs, int per, const int64_t *eq, const double *dz, int64_t ld,
+                  const double *scale, __nv_bfloat16 *dy, cudaStream_t st) {
+  scatter_grad_kernel<<<dim3(grid_for(g.voxels()), pairs * per), 256, 0, st>>>(g, per, eq, dz, ld, scale, dy);
 }
 
 void adam(int64_t n, float *p, const float *g, float *m, float *v, float lr, float b1, float b2, float eps, int t,
@@ -583,39 +812,51 @@ void dots(int64_t n, int pairs, const double *const *a, const double *const *b, 
           cudaStream_t st) {
   PairPtrs pp{};
   for (int k = 0; k < pairs && k < MAX_PAIRS; ++k) pp.a[k] = a[k], pp.b[k] = b[k];
-  dot_part_kernel<<<DOT_CTAS, 256, 0, st>>>(n, pairs, pp, partial);
-  dot_final_kernel<<<1, 256, 0, st>>>(DOT_CTAS, pairs, partial, out);
+  if (pairs < 1) return;
+  dot_part_kernel<<<dim3(DOT_CTAS, pairs), 256, 0, st>>>(n, pp, partial);
+  dot_final_kernel<<<pairs, 256, 0, st>>>(DOT_CTAS, partial, out);
 }
 
-void axpy_dev(int64_t n, const double *alpha, double sign, const double *x, double *y, cudaStream_t st) {
-  axpy_dev_kernel<<<grid_for(n), 256, 0, st>>>(n, alpha, sign, x, y);
+// A launch that may start while the stream's previous kernel ends (its kernel waits for it).
+template <class... P, class... A>
+static void launch_dependent(void (*kernel)(P...), int64_t grid, int threads, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::max<int64_t>(grid, 1));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+void fcg_step(const FcgStep &a, cudaStream_t st) {
+  const int64_t nodes = (a.n + 2) / 3;
+  launch_dependent(fcg_step_kernel, std::min<int64_t>((nodes + STEP_THREADS - 1) / STEP_THREADS, FCG_CTAS), STEP_THREADS, st,
+                   a);
 }
 
 void fcg_direction(int64_t n, int m, const double *z, const double *const *pj, const int *slot, const double *num,
                    const double *den, double *p, cudaStream_t st) {
   DirPtrs dp{};
-  for (int j = 0; j < m && j < MAX_PAIRS; ++j) dp.p[j] = pj[j], dp.slot[j] = slot[j];
-  fcg_direction_kernel<<<grid_for(n), 256, 0, st>>>(n, m, z, dp, num, den, p);
+  for (int j = 0; j < m && j < MAX_KEPT; ++j) dp.p[j] = pj[j], dp.slot[j] = slot[j];
+  launch_dependent(fcg_direction_kernel, std::min<int64_t>((n + FCG_THREADS - 1) / FCG_THREADS, FCG_CTAS),
+                   FCG_THREADS, st, n, m, z,
+                   dp, num, den, p);
 }
 
-// alpha = s[0] / s[1] (p.r / p.q; 0 when p.q is 0), kept: *den = s[1]; x += alpha p; r -= alpha q
-__global__ void fcg_update_kernel(int64_t n, const double *__restrict__ s, double *__restrict__ den,
-                                  const double *__restrict__ p, const double *__restrict__ q, double *__restrict__ x,
-                                  double *__restrict__ r) {
-  const double alpha = s[1] != 0.0 ? s[0] / s[1] : 0.0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *den = s[1];
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * p[i];
-    r[i] -= alpha * q[i];
-  }
-}
-void fcg_update(int64_t n, const double *s, double *den, const double *p, const double *q, double *x, double *r,
-                cudaStream_t st) {
-  fcg_update_kernel<<<grid_for(n), 256, 0, st>>>(n, s, den, p, q, x, r);
+void fcg_product(int64_t n, const int64_t *ptr, const int32_t *idx, const double *val, const double *p,
+                 const double *r, double *q, double *sums, double *den, double *part, int *ticket, cudaStream_t st) {
+  constexpr int ROWS = FCG_THREADS / SPMV_LANES;
+  launch_dependent(fcg_product_kernel, std::min<int64_t>((n + ROWS - 1) / ROWS, FCG_CTAS), FCG_THREADS, st, n, ptr, idx,
+                   val, p, r,
+                   q, sums, den, part, ticket);
 }
 
-void input_scales(int64_t n, const double *nrm2, double kref, double *s, cudaStream_t st) {
-  input_scales_kernel<<<1, 1, 0, st>>>(n, nrm2, kref, s);
+void input_scales(int64_t n, int pairs, int per, const double *nrm2, double kref, double *s, cudaStream_t st) {
+  input_scales_kernel<<<1, pairs, 0, st>>>(n, nrm2, kref, per, s);
 }
 
 }  // namespace unet

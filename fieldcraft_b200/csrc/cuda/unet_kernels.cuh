@@ -18,46 +18,64 @@ struct Grid {
   __host__ __device__ int64_t voxels() const { return (int64_t)X * Y * Z; }
 };
 
-// out = act(conv3x3x3(in, w) + bias) on grid g; CIN, COUT in {16, 32}. relu: the leaky ReLU
+// Batches: the passes of a batch lie one after the other, each a whole grid.
+
+// out = act(conv3x3x3(in, w) + bias) on the batch's grids g; CIN, COUT in {16, 32}. relu: the leaky ReLU
 // (x for x > 0, 0.05 x otherwise). mask (optional, COUT channels): out *= (mask > 0 ? 1 : 0.05),
 // the derivative of the leaky ReLU whose output is `mask`, applied to a gradient. bias may be null.
-void conv3(const Grid &g, int cin, int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
-           bool relu, const __nv_bfloat16 *mask, __nv_bfloat16 *out, cudaStream_t st);
-// Weight gradient of conv3: part[chunk][tap][cout][cin] = sum over the chunk's voxels of
-// dy[v][cout] in[v + tap][cin]; then gw[tap][cout][cin] = sum of the chunks in order, and
-// gb[cout] = sum_v dy[v][cout]. part must hold dw_chunks(g) * 27 * cin * cout floats.
-int dw_chunks(const Grid &g);
-void conv3_dw(const Grid &g, int cin, int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *dy, float *part,
-              float *gw, float *gb, cudaStream_t st);
-// Weights for the transposed convolution (the input gradient): wt[26 - tap][cin][cout] = w[tap][cout][cin].
-void flip_weights(int cin, int cout, const __nv_bfloat16 *w, __nv_bfloat16 *wt, cudaStream_t st);
-// FP32 master weights -> BF16 copies (n values).
-void to_bf16(int64_t n, const float *src, __nv_bfloat16 *dst, cudaStream_t st);
+// Launched as a programmatic dependent: the weights are read before the stream's previous kernel is
+// done, so that kernel must not be the one that writes them.
+void conv3(const Grid &g, int batch, int cin, int cout, const __nv_bfloat16 *in, const __nv_bfloat16 *w,
+           const float *bias, bool relu, const __nv_bfloat16 *mask, __nv_bfloat16 *out, cudaStream_t st);
+// Weight gradient of conv3 over `pairs` pairs of `passes` passes each: per pair g_w[tap][cout][cin] =
+// sum over its passes' voxels of dy[v][cout] in[v + tap][cin] and g_b[cout] = sum of dy[v][cout],
+// in chunks of tiles whose partials are added in order. gw and gb receive the last pair's; accw and
+// accb (or null) the sum over the pairs of scale g, on top of what they hold when `more`. part must
+// hold pairs * dw_chunks(g, pairs, passes) * 28 * cin * cout floats, at most
+// (DW_PARTIALS + pairs) * 28 * cin * cout.
+constexpr int DW_PARTIALS = 148;
+int dw_chunks(const Grid &g, int pairs, int passes);
+void conv3_dw(const Grid &g, int cin, int cout, int pairs, int passes, const __nv_bfloat16 *in,
+              const __nv_bfloat16 *dy, float *part, float scale, bool more, float *accw, float *accb, float *gw,
+              float *gb, cudaStream_t st);
+// A network's layers: channels, where the FP32 weights start in the parameters and the BF16 ones
+// in their arrays.
+constexpr int LAYERS_MOST = 31;
+struct LayerTable {
+  int layers;
+  int cin[LAYERS_MOST], cout[LAYERS_MOST];
+  int64_t param[LAYERS_MOST], weight[LAYERS_MOST];
+};
+// BF16 weights w and, for the input gradients, wt[26 - tap][cin][cout] = w[tap][cout][cin], of
+// every layer.
+void refresh(const LayerTable &t, const float *p, __nv_bfloat16 *w, __nv_bfloat16 *wt, cudaStream_t st);
 
 // 2x2x2 average (sum / 8) onto the coarse grid gc (ceil halves); C = 32.
-void pool(const Grid &gf, const Grid &gc, const __nv_bfloat16 *fine, __nv_bfloat16 *coarse, cudaStream_t st);
+void pool(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *fine, __nv_bfloat16 *coarse, cudaStream_t st);
 // fine = coarse(x/2, y/2, z/2) + skip; C = 32.
-void up_add(const Grid &gf, const Grid &gc, const __nv_bfloat16 *coarse, const __nv_bfloat16 *skip,
+void up_add(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *coarse, const __nv_bfloat16 *skip,
             __nv_bfloat16 *fine, cudaStream_t st);
 // The adjoints, times the leaky ReLU's derivative at `mask` (1 where mask > 0, else 0.05):
 // coarse = sum of the 8 children of dfine (nearest upsampling); fine = dcoarse(parent) / 8 + dskip
 // (average pooling plus the skip path).
-void up_adjoint(const Grid &gf, const Grid &gc, const __nv_bfloat16 *dfine, const __nv_bfloat16 *mask,
+void up_adjoint(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *dfine, const __nv_bfloat16 *mask,
                 __nv_bfloat16 *dcoarse, cudaStream_t st);
-void pool_adjoint(const Grid &gf, const Grid &gc, const __nv_bfloat16 *dcoarse, const __nv_bfloat16 *dskip,
+void pool_adjoint(const Grid &gf, const Grid &gc, int batch, const __nv_bfloat16 *dcoarse, const __nv_bfloat16 *dskip,
                   const __nv_bfloat16 *mask, __nv_bfloat16 *dfine, cudaStream_t st);
 
-// Between the equations' vectors and the grid: the 16 input channels of voxel v are
-// (r_x, r_y, r_z) * scale[0] at the node's free DOFs (0 where held), feat[v] (a fixed feature:
-// the node's log Young's modulus), and zeros. eq[3 v + a] is the equation of DOF a of node v, -1
-// when held. Out: z[eq] = y[v][a] * scale[1].
-void scatter_input(const Grid &g, const int64_t *eq, const double *r, const float *feat, const double *scale,
-                   __nv_bfloat16 *x, cudaStream_t st);
-void gather_output(const Grid &g, const int64_t *eq, const __nv_bfloat16 *y, const double *scale, double *z,
-                   cudaStream_t st);
-// dy[v][a] = dz[eq[3v + a]] * scale (a < 3; the other 13 channels zero), BF16.
-void scatter_grad(const Grid &g, const int64_t *eq, const double *dz, const double *scale, __nv_bfloat16 *dy,
-                  cudaStream_t st);
+// Between the equations' vectors and the grids of `pairs` vectors (column q at q * ld), `per` passes
+// each with their own scales (scale[2 p], scale[2 p + 1] of pass p): the 16 input channels of voxel
+// v are (r_x, r_y, r_z) * scale[2 p] at the node's free DOFs (0 where held), feat[v] (a fixed
+// feature: the node's log Young's modulus), and zeros. eq[3 v + a] is the equation of DOF a of
+// node v, -1 when held. Out: z[eq] = the sum over the vector's passes of y[v][a] * scale[2 p + 1],
+// on top of z when `add`.
+void scatter_input(const Grid &g, int pairs, int per, const int64_t *eq, const double *r, int64_t ld,
+                   const float *feat, const double *scale, __nv_bfloat16 *x, cudaStream_t st);
+void gather_output(const Grid &g, int pairs, int per, const int64_t *eq, const __nv_bfloat16 *y, const double *scale,
+                   double *z, int64_t ld, bool add, cudaStream_t st);
+// dy[v][a] = dz[eq[3v + a]] * scale[2 p + 1] (a < 3; the other 13 channels zero), BF16.
+void scatter_grad(const Grid &g, int pairs, int per, const int64_t *eq, const double *dz, int64_t ld,
+                  const double *scale, __nv_bfloat16 *dy, cudaStream_t st);
 
 // Adam on n FP32 parameters: m = b1 m + (1 - b1) g, v = b2 v + (1 - b2) g^2,
 // p -= lr (m / (1 - b1^t)) / (sqrt(v / (1 - b2^t)) + eps).
@@ -69,18 +87,35 @@ void adam(int64_t n, float *p, const float *g, float *m, float *v, float lr, flo
 // (partials per CTA, then one CTA), so results are the same on every run.
 void dots(int64_t n, int pairs, const double *const *a, const double *const *b, double *partial, double *out,
           cudaStream_t st);
-// y += alpha[0] * x (alpha on the device, sign s: y += s alpha x)
-void axpy_dev(int64_t n, const double *alpha, double sign, const double *x, double *y, cudaStream_t st);
-// p = z - sum_j beta_j p_j with beta_j = num[j] / den[slot[j]] (device scalars), q = A p done by
-// the caller
+// An iteration of flexible CG. Sums are taken in a fixed order and left in device scalars by the
+// kernel that forms them; `part` holds (1 + MAX_KEPT) x FCG_CTAS partials and *ticket is zero
+// between launches.
+constexpr int MAX_KEPT = 8, FCG_CTAS = 148 * 8;
+struct FcgStep {
+  int64_t n;
+  int update;                    // x += alpha p, r -= alpha q with alpha = alpha[0] / alpha[1] (0 when alpha[1] is 0)
+  const double *alpha, *p, *q;
+  double *x, *r;
+  double *z;                     // null: no preconditioner here; else z = B r, inv B's blocks (null: z = r)
+  const double *inv;
+  int kept;                      // zq[j] = z . qj[j], j < kept
+  const double *qj[MAX_KEPT];
+  double *zq, *rr;               // *rr = r . r
+  double *part;
+  int *ticket;
+};
+void fcg_step(const FcgStep &a, cudaStream_t st);
+// p = z - sum_j beta_j p_j with beta_j = num[j] / den[slot[j]] (device scalars); p may be one of the
+// p_j
 void fcg_direction(int64_t n, int m, const double *z, const double *const *pj, const int *slot, const double *num,
                    const double *den, double *p, cudaStream_t st);
-// alpha = s[0] / s[1] (0 when s[1] is 0), *den = s[1], x += alpha p, r -= alpha q
-void fcg_update(int64_t n, const double *s, double *den, const double *p, const double *q, double *x, double *r,
-                cudaStream_t st);
-// The norms' scalars for the input scaling of the network: s[0] = sqrt(n) / ||r||,
-// s[1] = ||r|| / (sqrt(n) kref); nrm2 = ||r||^2 from dots.
-void input_scales(int64_t n, const double *nrm2, double kref, double *s, cudaStream_t st);
+// q = A p (A by rows), sums[0] = p . r, sums[1] = *den = p . q
+void fcg_product(int64_t n, const int64_t *ptr, const int32_t *idx, const double *val, const double *p,
+                 const double *r, double *q, double *sums, double *den, double *part, int *ticket, cudaStream_t st);
+// The passes' scales of `pairs` vectors from their nrm2 = ||r||^2 (dots): s[2 p] = sqrt(n) / ||r||,
+// s[2 p + 1] = ||r|| / (sqrt(n) kref); with per = 2 (the odd network) the pass on r halves its
+// output scale and the pass on -r has both negated.
+void input_scales(int64_t n, int pairs, int per, const double *nrm2, double kref, double *s, cudaStream_t st);
 
 }  // namespace unet
 }  // namespace fc

@@ -33,16 +33,26 @@ __global__ void bf16_to_f32_kernel(int64_t n, const bf16 *__restrict__ a, float 
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     b[i] = __bfloat162float(a[i]);
 }
+// The vectors of a group of pairs: blockIdx.y is the pair, its column `ld` past the last.
 // d = z - e
-__global__ void sub_kernel(int64_t n, const double *__restrict__ z, const double *__restrict__ e, double *__restrict__ d) {
+__global__ void sub_kernel(int64_t n, const double *__restrict__ z, const double *__restrict__ e, int64_t ld,
+                           double *__restrict__ d) {
+  z += blockIdx.y * n, d += blockIdx.y * n, e += blockIdx.y * ld;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     d[i] = z[i] - e[i];
 }
-// d *= 2 / s[1]; loss = s[0] / s[1] (s = {d.d, e.e}, or {d.Kd, e.r} in the energy norm)
-__global__ void loss_grad_kernel(int64_t n, const double *__restrict__ s, double *__restrict__ d, double *loss) {
-  const double ee = s[1] > 0.0 ? s[1] : 1.0;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && loss) *loss = s[0] / ee;
+// d *= 2 / den; loss = num / den (num, den = d.d, e.e, or d.Kd, e.r in the energy norm); the
+// pairs' losses are added in order onto *loss (onto zero for the first of all)
+__global__ void loss_grad_kernel(int64_t n, const double *__restrict__ num, const double *__restrict__ den,
+                                 double *__restrict__ d, double *loss, int first) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && loss) {
+    double sum = first ? 0.0 : *loss;
+    for (int q = 0; q < (int)gridDim.y; ++q) sum += num[q] / (den[q] > 0.0 ? den[q] : 1.0);
+    *loss = sum;
+  }
+  const double ee = den[blockIdx.y] > 0.0 ? den[blockIdx.y] : 1.0;
   const double c = 2.0 / ee;
+  d += blockIdx.y * n;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     d[i] *= c;
 }
@@ -94,35 +104,19 @@ __global__ void block_jacobi_kernel(int64_t nodes, const int64_t *__restrict__ p
     o[8] = (a[0][0] * a[1][1] - a[0][1] * a[1][0]) * d;
   }
 }
-// z += B r, B the nodal block-Jacobi inverse
-__global__ void block_jacobi_add_kernel(int64_t nodes, const double *__restrict__ inv, const double *__restrict__ r,
-                                        double *__restrict__ z) {
+// z = B r, B the nodal block-Jacobi inverse; blockIdx.y the vector
+__global__ void block_jacobi_apply_kernel(int64_t nodes, const double *__restrict__ inv, const double *__restrict__ r,
+                                          int64_t ld, double *__restrict__ z) {
+  r += blockIdx.y * ld, z += blockIdx.y * 3 * nodes;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nodes; k += (int64_t)gridDim.x * blockDim.x) {
     const double *o = inv + 9 * k;
     const double r0 = r[3 * k], r1 = r[3 * k + 1], r2 = r[3 * k + 2];
-    z[3 * k] += o[0] * r0 + o[1] * r1 + o[2] * r2;
-    z[3 * k + 1] += o[3] * r0 + o[4] * r1 + o[5] * r2;
-    z[3 * k + 2] += o[6] * r0 + o[7] * r1 + o[8] * r2;
+    z[3 * k] = o[0] * r0 + o[1] * r1 + o[2] * r2;
+    z[3 * k + 1] = o[3] * r0 + o[4] * r1 + o[5] * r2;
+    z[3 * k + 2] = o[6] * r0 + o[7] * r1 + o[8] * r2;
   }
 }
-// acc = first ? g s : acc + g s (FP32 gradients of a minibatch)
-__global__ void accumulate_kernel(int64_t n, const float *__restrict__ g, float s, bool first, float *__restrict__ acc) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    acc[i] = first ? g[i] * s : acc[i] + g[i] * s;
-}
-__global__ void add_scalar_kernel(const double *__restrict__ a, double *__restrict__ acc, bool first) {
-  acc[0] = first ? a[0] : acc[0] + a[0];
-}
 
-// the odd network's two passes: P = (s0, s1 / 2), M = (-s0, -s1 / 2) from s = (s0, s1)
-__global__ void odd_scales_kernel(const double *__restrict__ s, double *__restrict__ P, double *__restrict__ M) {
-  P[0] = s[0], P[1] = 0.5 * s[1];
-  M[0] = -s[0], M[1] = -0.5 * s[1];
-}
-__global__ void add_kernel(int64_t n, const double *__restrict__ a, double *__restrict__ z) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    z[i] += a[i];
-}
 __global__ void add_f32_kernel(int64_t n, const float *__restrict__ a, float *__restrict__ z) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     z[i] += a[i];
@@ -145,17 +139,19 @@ struct fc_unet {
   int64_t w_off[MAX_LAYERS], b_off[MAX_LAYERS], wb_off[MAX_LAYERS];
   int64_t params = 0, wcount = 0;
   DeviceBuf p, grad, m, v;   // FP32 parameters, gradients and Adam moments
-  DeviceBuf gacc;            // a minibatch's summed gradients
+  DeviceBuf gacc;            // a minibatch's mean gradient
   DeviceBuf wb, wt;          // BF16 weights and their flipped transposes
   DeviceBuf eq, feat;
   // activations (BF16, channels last), per level: the (pooled) input, the two convolutions of the
   // way down (s = the skip), the way up: u = upsampled + skip, its two convolutions b, d
-  DeviceBuf x, y, pin[MAX_LEVELS], a[MAX_LEVELS], s[MAX_LEVELS], u[MAX_LEVELS], b[MAX_LEVELS], d[MAX_LEVELS];
+  bf16 *x = nullptr, *y = nullptr, *pin[MAX_LEVELS] = {}, *a[MAX_LEVELS] = {}, *s[MAX_LEVELS] = {},
+       *u[MAX_LEVELS] = {}, *b[MAX_LEVELS] = {}, *d[MAX_LEVELS] = {};
   // gradients per level
-  DeviceBuf dy, ga[MAX_LEVELS], gb[MAX_LEVELS], gs[MAX_LEVELS];
+  bf16 *dy = nullptr, *ga[MAX_LEVELS] = {}, *gb[MAX_LEVELS] = {}, *gs[MAX_LEVELS] = {};
+  DeviceBuf arena;           // all of them
   DeviceBuf part;            // weight-gradient partials
   DeviceBuf scal, dotpart;   // device scalars: [0,1] input scales, [2..] dots; dot partials
-  DeviceBuf tz, td, tf;      // training: network output and its difference; FP32 grid copies
+  DeviceBuf tz, td;          // training, a column per pair of a group: the output, its difference
   DeviceBuf bj;              // nodal block-Jacobi inverses (9 doubles a node), added to the output
   bool has_bj = false;
   bool net_on = true;         // false: the preconditioner is the block-Jacobi part alone
@@ -163,7 +159,9 @@ struct fc_unet {
   // odd: M(r) = B r + (net(r) - net(-r)) / 2, so that M(-r) = -M(r) and M(0) = 0 (a part of the
   // output that does not depend on r, from the biases and the modulus channel, cancels)
   bool odd = true;
-  DeviceBuf tz2, gtmp;        // the second pass's output and gradients
+  int cap = 0, pairs_cap = 0;  // passes the activations hold, pairs tz and td hold
+  DeviceBuf gtmp;              // one pass's gradients, where a pair's two do not fit together
+  fc::unet::LayerTable table{};
   int64_t last_net_iterations = 0, last_dropped = 0;
   bool weights_stale = true;
   std::mutex lock;
@@ -173,162 +171,250 @@ namespace {
 
 bf16 *B(const DeviceBuf &b) { return b.as<bf16>(); }
 
-cudaError_t alloc_bf16(DeviceBuf &b, const Grid &g, int c) { return b.alloc(sizeof(bf16) * (size_t)g.voxels() * c); }
+// A group of pairs runs through the network side by side, a pass each (two with the odd form): at
+// most PAIRS_MOST pairs, and activations of at most WORKSPACE_MOST bytes beside a pair's own. The
+// sizes are kept in the handle for the next group.
+constexpr int PAIRS_MOST = 8;
+constexpr size_t WORKSPACE_MOST = (size_t)2 << 30;
+// the device scalars: the passes' scales, then a value per pair each
+constexpr int S_SCALES = 64, S_NRM = 96, S_NUM = 104, S_DEN = 112, S_COUNT = 128;
 
-// BF16 copies of the weights (and the flipped ones for the input gradients) after a change.
+// The activations and gradients of `passes` passes, in one allocation (two dozen of them took a
+// millisecond); the weight gradients' partials with the first.
+bool alloc_passes(fc_unet *u, int passes) {
+  u->cap = 0;
+  const size_t part = (size_t)(fc::unet::DW_PARTIALS + PAIRS_MOST) * 28 * C * C;
+  if (!u->part.p && u->part.alloc(sizeof(float) * part) != cudaSuccess) return false;
+  for (int round = 0; round < 2; ++round) {  // sizes, then places
+    bf16 *base = u->arena.as<bf16>();
+    size_t at = 0;
+    auto take = [&](bf16 *&p, const Grid &g, int c) {
+      p = base + at;
+      at += ((size_t)g.voxels() * c * passes + 127) / 128 * 128;
+    };
+    take(u->x, u->g[0], CIO);
+    take(u->y, u->g[0], CIO);
+    take(u->dy, u->g[0], CIO);
+    for (int lv = 0; lv < u->levels; ++lv) {
+      const Grid &g = u->g[lv];
+      for (bf16 **b : {&u->a[lv], &u->s[lv], &u->ga[lv], &u->gb[lv]}) take(*b, g, C);
+      if (lv > 0) take(u->pin[lv], g, C);
+      if (lv < u->levels - 1)
+        for (bf16 **b : {&u->u[lv], &u->b[lv], &u->d[lv], &u->gs[lv]}) take(*b, g, C);
+    }
+    if (round == 0 && u->arena.alloc(sizeof(bf16) * at) != cudaSuccess) return false;
+  }
+  u->cap = passes;
+  return true;
+}
+
+// Room for `pairs` pairs of `per` passes, or for as many as there is memory for: returns how many
+// passes run together (at least one; a pair's two then run after one another), 0 when there is
+// no room at all.
+int want_passes(fc_unet *u, int pairs, int per) {
+  size_t pass = 0;
+  for (int lv = 0; lv < u->levels; ++lv) pass += sizeof(bf16) * (size_t)u->g[lv].voxels() * C * 9;
+  int want = per * std::min(pairs, PAIRS_MOST);
+  while (want > per && pass * want > WORKSPACE_MOST) want -= per;
+  if (u->cap >= want) return want;
+  cudaStreamSynchronize(u->stream);
+  for (int p = want; p >= 1; p = p > per ? p - per : p - 1)
+    if (alloc_passes(u, p)) return p;
+  return 0;
+}
+
+bool want_pairs(fc_unet *u, int pairs) {
+  if (u->pairs_cap >= pairs) return true;
+  cudaStreamSynchronize(u->stream);
+  u->pairs_cap = 0;
+  if (u->tz.alloc(sizeof(double) * (size_t)u->n * pairs) != cudaSuccess ||
+      u->td.alloc(sizeof(double) * (size_t)u->n * pairs) != cudaSuccess)
+    return false;
+  u->pairs_cap = pairs;
+  return true;
+}
+
+// BF16 copies of the weights (and the flipped ones for the input gradients) after a change: before
+// a kernel that is not a convolution, which reads them before the kernel ahead of it is done.
 void refresh_weights(fc_unet *u) {
   if (!u->weights_stale) return;
-  cudaStream_t st = u->stream;
-  for (int l = 0; l < u->layers; ++l) {
-    const int64_t nw = (int64_t)27 * u->lcin[l] * u->lcout[l];
-    fc::unet::to_bf16(nw, u->p.as<float>() + u->w_off[l], B(u->wb) + u->wb_off[l], st);
-    fc::unet::flip_weights(u->lcin[l], u->lcout[l], B(u->wb) + u->wb_off[l], B(u->wt) + u->wb_off[l], st);
-  }
+  fc::unet::refresh(u->table, u->p.as<float>(), B(u->wb), B(u->wt), u->stream);
   u->weights_stale = false;
 }
 
 const Grid &G(const fc_unet *u, int level) { return u->g[level]; }
 
-void conv(fc_unet *u, int l, const DeviceBuf &in, DeviceBuf &out, bool relu) {
-  fc::unet::conv3(G(u, u->llevel[l]), u->lcin[l], u->lcout[l], B(in), B(u->wb) + u->wb_off[l],
-                  u->p.as<float>() + u->b_off[l], relu, nullptr, B(out), u->stream);
+void conv(fc_unet *u, int passes, int l, const bf16 *in, bf16 *out, bool relu) {
+  fc::unet::conv3(G(u, u->llevel[l]), passes, u->lcin[l], u->lcout[l], in, B(u->wb) + u->wb_off[l],
+                  u->p.as<float>() + u->b_off[l], relu, nullptr, out, u->stream);
 }
 // the input gradient of layer l from its output gradient: conv with the flipped weights, then
 // the ReLU mask of the layer's input (mask null: no ReLU there)
-void conv_t(fc_unet *u, int l, const DeviceBuf &dout, const DeviceBuf *mask, DeviceBuf &din) {
-  fc::unet::conv3(G(u, u->llevel[l]), u->lcout[l], u->lcin[l], B(dout), B(u->wt) + u->wb_off[l], nullptr, false,
-                  mask ? B(*mask) : nullptr, B(din), u->stream);
+void conv_t(fc_unet *u, int passes, int l, const bf16 *dout, const bf16 *mask, bf16 *din) {
+  fc::unet::conv3(G(u, u->llevel[l]), passes, u->lcout[l], u->lcin[l], dout, B(u->wt) + u->wb_off[l], nullptr,
+                  false, mask, din, u->stream);
 }
-void conv_dw(fc_unet *u, int l, const DeviceBuf &in, const DeviceBuf &dout) {
-  fc::unet::conv3_dw(G(u, u->llevel[l]), u->lcin[l], u->lcout[l], B(in), B(dout), u->part.as<float>(),
-                     u->grad.as<float>() + u->w_off[l], u->grad.as<float>() + u->b_off[l], u->stream);
+
+// What backward() does with the parameters' gradients of the pairs it is given: the last pair's
+// lands in u->grad, `scale` times each pair's is added to u->gacc when `acc` (from zero unless
+// `more`).
+struct Gradients {
+  int pairs, per;
+  bool acc;
+  float scale;
+  bool more;
+};
+void conv_dw(fc_unet *u, const Gradients &gr, int l, const bf16 *in, const bf16 *dout) {
+  float *acc = gr.acc ? u->gacc.as<float>() : nullptr, *grad = u->grad.as<float>();
+  fc::unet::conv3_dw(G(u, u->llevel[l]), u->lcin[l], u->lcout[l], gr.pairs, gr.per, in, dout,
+                     u->part.as<float>(), gr.scale, gr.more, acc ? acc + u->w_off[l] : nullptr,
+                     acc ? acc + u->b_off[l] : nullptr, grad + u->w_off[l], grad + u->b_off[l], u->stream);
 }
 
 // the level's input on the way down: x at the top, the pooled skip of the level above below it
-const DeviceBuf &input_of(const fc_unet *u, int lv) { return lv == 0 ? u->x : u->pin[lv]; }
+const bf16 *input_of(const fc_unet *u, int lv) { return lv == 0 ? u->x : u->pin[lv]; }
 // what the level returns upwards: the bottom's second convolution, or the way up's last one
-const DeviceBuf &low_of(const fc_unet *u, int lv) { return lv == u->levels - 1 ? u->s[lv] : u->d[lv]; }
-DeviceBuf &low_of(fc_unet *u, int lv) { return lv == u->levels - 1 ? u->s[lv] : u->d[lv]; }
+bf16 *low_of(const fc_unet *u, int lv) { return lv == u->levels - 1 ? u->s[lv] : u->d[lv]; }
 
-// y = net(x): per level on the way down two convolutions (the second's output is the skip) and a
-// 2x2x2 average pooling, two at the bottom, per level on the way up nearest upsampling plus the
-// skip and two convolutions, then the output convolution (layers in this order).
-void forward(fc_unet *u) {
-  refresh_weights(u);
+// y = net(x) for `P` passes: per level on the way down two convolutions (the second's output is the
+// skip) and a 2x2x2 average pooling, two at the bottom, per level on the way up nearest upsampling
+// plus the skip and two convolutions, then the output convolution (layers in this order).
+void forward(fc_unet *u, int P) {
   cudaStream_t st = u->stream;
   const int D = u->levels;
   int l = 0;
   for (int lv = 0; lv < D; ++lv) {
-    conv(u, l++, input_of(u, lv), u->a[lv], true);
-    conv(u, l++, u->a[lv], u->s[lv], true);
-    if (lv < D - 1) fc::unet::pool(u->g[lv], u->g[lv + 1], B(u->s[lv]), B(u->pin[lv + 1]), st);
+    conv(u, P, l++, input_of(u, lv), u->a[lv], true);
+    conv(u, P, l++, u->a[lv], u->s[lv], true);
+    if (lv < D - 1) fc::unet::pool(u->g[lv], u->g[lv + 1], P, u->s[lv], u->pin[lv + 1], st);
   }
   for (int lv = D - 2; lv >= 0; --lv) {
-    fc::unet::up_add(u->g[lv], u->g[lv + 1], B(low_of(u, lv + 1)), B(u->s[lv]), B(u->u[lv]), st);
-    conv(u, l++, u->u[lv], u->b[lv], true);
-    conv(u, l++, u->b[lv], u->d[lv], true);
+    fc::unet::up_add(u->g[lv], u->g[lv + 1], P, low_of(u, lv + 1), u->s[lv], u->u[lv], st);
+    conv(u, P, l++, u->u[lv], u->b[lv], true);
+    conv(u, P, l++, u->b[lv], u->d[lv], true);
   }
-  conv(u, l, low_of(u, 0), u->y, false);
+  conv(u, P, l, low_of(u, 0), u->y, false);
 }
 
 // parameters' gradients from dL/dy (in u->dy), after forward() on the same input
-void backward(fc_unet *u) {
+void backward(fc_unet *u, const Gradients &gr) {
   cudaStream_t st = u->stream;
-  const int D = u->levels;
+  const int D = u->levels, P = gr.pairs * gr.per;
   int l = u->layers - 1;
-  conv_dw(u, l, low_of(u, 0), u->dy);
-  conv_t(u, l, u->dy, &low_of(u, 0), u->ga[0]);  // dL/d(top output), through its activation
+  conv_dw(u, gr, l, low_of(u, 0), u->dy);
+  conv_t(u, P, l, u->dy, low_of(u, 0), u->ga[0]);  // dL/d(top output), through its activation
   for (int lv = 0; lv < D - 1; ++lv) {  // the way up, from the top level to the coarsest
     l -= 2;
-    conv_dw(u, l + 1, u->b[lv], u->ga[lv]);
-    conv_t(u, l + 1, u->ga[lv], &u->b[lv], u->gb[lv]);
-    conv_dw(u, l, u->u[lv], u->gb[lv]);
-    conv_t(u, l, u->gb[lv], nullptr, u->gs[lv]);  // dL/du: to the skip and, upsampled, below
-    fc::unet::up_adjoint(u->g[lv], u->g[lv + 1], B(u->gs[lv]), B(low_of(u, lv + 1)), B(u->ga[lv + 1]), st);
+    conv_dw(u, gr, l + 1, u->b[lv], u->ga[lv]);
+    conv_t(u, P, l + 1, u->ga[lv], u->b[lv], u->gb[lv]);
+    conv_dw(u, gr, l, u->u[lv], u->gb[lv]);
+    conv_t(u, P, l, u->gb[lv], nullptr, u->gs[lv]);  // dL/du: to the skip and, upsampled, below
+    fc::unet::up_adjoint(u->g[lv], u->g[lv + 1], P, u->gs[lv], low_of(u, lv + 1), u->ga[lv + 1], st);
   }
   for (int lv = D - 1; lv >= 0; --lv) {  // the way down, from the bottom up
     l -= 2;
-    conv_dw(u, l + 1, u->a[lv], u->ga[lv]);
-    conv_t(u, l + 1, u->ga[lv], &u->a[lv], u->gb[lv]);
-    conv_dw(u, l, input_of(u, lv), u->gb[lv]);
+    conv_dw(u, gr, l + 1, u->a[lv], u->ga[lv]);
+    conv_t(u, P, l + 1, u->ga[lv], u->a[lv], u->gb[lv]);
+    conv_dw(u, gr, l, input_of(u, lv), u->gb[lv]);
     if (lv == 0) break;
-    conv_t(u, l, u->gb[lv], nullptr, u->ga[lv]);  // dL/d(pooled input)
-    fc::unet::pool_adjoint(u->g[lv - 1], u->g[lv], B(u->ga[lv]), B(u->gs[lv - 1]), B(u->s[lv - 1]),
-                           B(u->ga[lv - 1]), st);  // dL/d(skip of the level above), masked
+    conv_t(u, P, l, u->gb[lv], nullptr, u->ga[lv]);  // dL/d(pooled input)
+    fc::unet::pool_adjoint(u->g[lv - 1], u->g[lv], P, u->ga[lv], u->gs[lv - 1], u->s[lv - 1],
+                           u->ga[lv - 1], st);  // dL/d(skip of the level above), masked
   }
 }
 
 double *scal(fc_unet *u, int k) { return u->scal.as<double>() + k; }
 
-// z = M(r) on u's stream. The odd network runs twice, on +r then on -r (the second pass's
-// activations stay for a backward pass: scales at scal 12..13, the first's at 10..11).
-void apply(fc_unet *u, const double *r, double *z) {
+// out[q] = a_q . b_q for the columns q of a group of pairs
+void pair_dots(fc_unet *u, int pairs, const double *a, int64_t lda, const double *b, int64_t ldb, double *out) {
+  const double *pa[PAIRS_MOST], *pb[PAIRS_MOST];
+  for (int q = 0; q < pairs; ++q) pa[q] = a + q * lda, pb[q] = b + q * ldb;
+  fc::unet::dots(u->n, pairs, pa, pb, u->dotpart.as<double>(), out, u->stream);
+}
+
+int passes_per_pair(const fc_unet *u) { return u->odd ? 2 : 1; }
+
+// The network's passes [p0, p0 + count) of the group's pairs, forward: their input grids, the pass.
+// A range of whole pairs, or one pass of a pair (count 1).
+void forward_passes(fc_unet *u, const double *r, int64_t ld, int p0, int count) {
+  const int per = passes_per_pair(u), pairs = std::max(1, count / per), each = count / pairs;
+  fc::unet::scatter_input(u->g[0], pairs, each, u->eq.as<int64_t>(), r + p0 / per * ld, ld, u->feat.as<float>(),
+                          scal(u, S_SCALES + 2 * p0), u->x, u->stream);
+  forward(u, count);
+}
+
+// z_q = M(r_q) for the group's pairs (z contiguous), `together` passes at a time.
+void apply(fc_unet *u, int pairs, const double *r, int64_t ld, double *z, int together) {
   cudaStream_t st = u->stream;
-  const double *a[1] = {r}, *b[1] = {r};
-  const int64_t *eq = u->eq.as<int64_t>();
-  fc::unet::dots(u->n, 1, a, b, u->dotpart.as<double>(), scal(u, 2), st);
-  fc::unet::input_scales(u->n, scal(u, 2), u->kref, scal(u, 0), st);
-  cudaMemsetAsync(z, 0, sizeof(double) * (size_t)u->n, st);
-  if (u->odd) {
-    odd_scales_kernel<<<1, 1, 0, st>>>(scal(u, 0), scal(u, 10), scal(u, 12));
-    fc::unet::scatter_input(u->g[0], eq, r, u->feat.as<float>(), scal(u, 10), B(u->x), st);
-    forward(u);
-    fc::unet::gather_output(u->g[0], eq, B(u->y), scal(u, 10), z, st);
-    double *z2 = u->tz2.as<double>();
-    cudaMemsetAsync(z2, 0, sizeof(double) * (size_t)u->n, st);
-    fc::unet::scatter_input(u->g[0], eq, r, u->feat.as<float>(), scal(u, 12), B(u->x), st);
-    forward(u);
-    fc::unet::gather_output(u->g[0], eq, B(u->y), scal(u, 12), z2, st);
-    add_kernel<<<blocks(u->n), 256, 0, st>>>(u->n, z2, z);
-  } else {
-    fc::unet::scatter_input(u->g[0], eq, r, u->feat.as<float>(), scal(u, 0), B(u->x), st);
-    forward(u);
-    fc::unet::gather_output(u->g[0], eq, B(u->y), scal(u, 0), z, st);
+  const int per = passes_per_pair(u);
+  refresh_weights(u);
+  pair_dots(u, pairs, r, ld, r, ld, scal(u, S_NRM));
+  fc::unet::input_scales(u->n, pairs, per, scal(u, S_NRM), u->kref, scal(u, S_SCALES), st);
+  if (u->has_bj)
+    block_jacobi_apply_kernel<<<dim3(blocks(u->n / 3), pairs), 256, 0, st>>>(u->n / 3, u->bj.as<double>(), r, ld, z);
+  else
+    cudaMemsetAsync(z, 0, sizeof(double) * (size_t)u->n * pairs, st);
+  for (int p0 = 0, count; p0 < per * pairs; p0 += count) {
+    count = std::min(per * pairs - p0, together);
+    forward_passes(u, r, ld, p0, count);
+    const int whole = std::max(1, count / per);
+    fc::unet::gather_output(u->g[0], whole, count / whole, u->eq.as<int64_t>(), u->y,
+                            scal(u, S_SCALES + 2 * p0), z + p0 / per * u->n, u->n, u->has_bj || p0 % per != 0, st);
   }
-  if (u->has_bj) block_jacobi_add_kernel<<<blocks(u->n / 3), 256, 0, st>>>(u->n / 3, u->bj.as<double>(), r, z);
 }
 
 // z = B r alone (the network left out)
 void apply_jacobi(fc_unet *u, const double *r, double *z) {
-  cudaMemsetAsync(z, 0, sizeof(double) * (size_t)u->n, u->stream);
-  block_jacobi_add_kernel<<<blocks(u->n / 3), 256, 0, u->stream>>>(u->n / 3, u->bj.as<double>(), r, z);
+  block_jacobi_apply_kernel<<<blocks(u->n / 3), 256, 0, u->stream>>>(u->n / 3, u->bj.as<double>(), r, u->n, z);
 }
 
-// The loss of the pair (r, e) and its gradient into u->grad (forward and backward of the network).
-void pair_gradient(fc_unet *u, const double *d_r, const double *d_e, const int64_t *d_ptr, const int32_t *d_idx,
-                   const double *d_val, double *d_loss) {
+// The losses of `count` pairs (r_q, e_q) added into *d_loss, the last pair's gradient into u->grad,
+// and with `acc` their mean into u->gacc (forward and backward of the network, in groups of pairs).
+// False when there is no memory for one pass.
+bool pair_gradients(fc_unet *u, const double *d_r, const double *d_e, int count, int64_t ld, const int64_t *d_ptr,
+                    const int32_t *d_idx, const double *d_val, double *d_loss, bool acc) {
   cudaStream_t st = u->stream;
+  const int per = passes_per_pair(u);
+  const int together = want_passes(u, count, per);
+  const int most = std::max(1, together / per);
+  if (together == 0 || !want_pairs(u, std::min(count, most))) return false;
   double *z = u->tz.as<double>(), *d = u->td.as<double>();
-  apply(u, d_r, z);
-  sub_kernel<<<blocks(u->n), 256, 0, st>>>(u->n, z, d_e, d);
-  if (d_ptr) {
-    // energy norm: loss = d.Kd / e.r (e.r = e.K e), dL/dz = 2 Kd / e.r
-    fc::launch_spmv(u->n, d_ptr, d_idx, d_val, d, u->n, z, u->n, 1, st);
-    const double *a[2] = {d, d_e}, *b[2] = {z, d_r};
-    fc::unet::dots(u->n, 2, a, b, u->dotpart.as<double>(), scal(u, 4), st);
-    loss_grad_kernel<<<blocks(u->n), 256, 0, st>>>(u->n, scal(u, 4), z, d_loss);
-    d = z;
-  } else {
-    const double *a[2] = {d, d_e}, *b[2] = {d, d_e};
-    fc::unet::dots(u->n, 2, a, b, u->dotpart.as<double>(), scal(u, 4), st);
-    loss_grad_kernel<<<blocks(u->n), 256, 0, st>>>(u->n, scal(u, 4), d, d_loss);
-  }
   const int64_t *eq = u->eq.as<int64_t>();
-  if (!u->odd) {
-    fc::unet::scatter_grad(u->g[0], eq, d, scal(u, 0), B(u->dy), st);
-    backward(u);
-    return;
+  for (int q0 = 0; q0 < count; q0 += most) {
+    const int g = std::min(most, count - q0);
+    const double *r = d_r + q0 * ld, *e = d_e + q0 * ld;
+    apply(u, g, r, ld, z, together);
+    sub_kernel<<<dim3(blocks(u->n), g), 256, 0, st>>>(u->n, z, e, ld, d);
+    double *grad = d;
+    if (d_ptr) {
+      // energy norm: loss = d.Kd / e.r (e.r = e.K e), dL/dz = 2 Kd / e.r
+      fc::launch_spmv(u->n, d_ptr, d_idx, d_val, d, u->n, z, u->n, g, st);
+      pair_dots(u, g, d, u->n, z, u->n, scal(u, S_NUM));
+      pair_dots(u, g, e, ld, r, ld, scal(u, S_DEN));
+      grad = z;
+    } else {
+      pair_dots(u, g, d, u->n, d, u->n, scal(u, S_NUM));
+      pair_dots(u, g, e, ld, e, ld, scal(u, S_DEN));
+    }
+    loss_grad_kernel<<<dim3(blocks(u->n), g), 256, 0, st>>>(u->n, scal(u, S_NUM), scal(u, S_DEN), grad, d_loss,
+                                                            q0 == 0);
+    const float scale = 1.f / (float)count;
+    if (together >= per) {
+      fc::unet::scatter_grad(u->g[0], g, per, eq, grad, u->n, scal(u, S_SCALES), u->dy, st);
+      backward(u, {g, per, acc, scale, q0 > 0});
+      continue;
+    }
+    // room for one pass only: the second pass's activations are live, its gradient first and kept
+    // aside; then the first pass again, forward and backward, and the two added
+    fc::unet::scatter_grad(u->g[0], 1, 1, eq, grad, u->n, scal(u, S_SCALES + 2), u->dy, st);
+    backward(u, {1, 1, acc, scale, q0 > 0});
+    cudaMemcpyAsync(u->gtmp.p, u->grad.p, sizeof(float) * (size_t)u->params, cudaMemcpyDeviceToDevice, st);
+    forward_passes(u, r, ld, 0, 1);
+    fc::unet::scatter_grad(u->g[0], 1, 1, eq, grad, u->n, scal(u, S_SCALES), u->dy, st);
+    backward(u, {1, 1, acc, scale, true});
+    add_f32_kernel<<<blocks(u->params), 256, 0, st>>>(u->params, u->gtmp.as<float>(), u->grad.as<float>());
   }
-  // the second pass (-r) is the one whose activations are live: its gradients first, kept aside;
-  // then the first pass (+r) again, forward and backward, and the two added
-  fc::unet::scatter_grad(u->g[0], eq, d, scal(u, 12), B(u->dy), st);
-  backward(u);
-  cudaMemcpyAsync(u->gtmp.p, u->grad.p, sizeof(float) * (size_t)u->params, cudaMemcpyDeviceToDevice, st);
-  fc::unet::scatter_input(u->g[0], eq, d_r, u->feat.as<float>(), scal(u, 10), B(u->x), st);
-  forward(u);
-  fc::unet::scatter_grad(u->g[0], eq, d, scal(u, 10), B(u->dy), st);
-  backward(u);
-  add_f32_kernel<<<blocks(u->params), 256, 0, st>>>(u->params, u->gtmp.as<float>(), u->grad.as<float>());
+  return true;
 }
 
 int cuda_fail(fc_status *st, cudaError_t e, const char *where) {
@@ -367,7 +453,6 @@ int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const i
   u->lcin[L] = C, u->lcout[L] = CIO, u->llevel[L++] = 0;
   u->layers = L;
   int64_t off = 0, woff = 0;
-  size_t part = 8192;
   for (int l = 0; l < L; ++l) {
     const int64_t nw = (int64_t)27 * u->lcin[l] * u->lcout[l];
     u->w_off[l] = off;
@@ -376,8 +461,10 @@ int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const i
     off += u->lcout[l];
     u->wb_off[l] = woff;
     woff += nw;
-    part = std::max(part, (size_t)fc::unet::dw_chunks(u->g[u->llevel[l]]) * (size_t)nw);
+    u->table.cin[l] = u->lcin[l], u->table.cout[l] = u->lcout[l];
+    u->table.param[l] = u->w_off[l], u->table.weight[l] = u->wb_off[l];
   }
+  u->table.layers = L;
   u->params = off;
   u->wcount = woff;
   const int64_t nodes = u->g[0].voxels();
@@ -394,21 +481,10 @@ int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const i
             u->gacc.alloc(sizeof(float) * off) == cudaSuccess &&
             u->wb.alloc(sizeof(bf16) * woff) == cudaSuccess && u->wt.alloc(sizeof(bf16) * woff) == cudaSuccess &&
             u->eq.alloc(sizeof(int64_t) * 3 * nodes) == cudaSuccess &&
-            u->feat.alloc(sizeof(float) * nodes) == cudaSuccess && u->part.alloc(sizeof(float) * part) == cudaSuccess &&
-            u->scal.alloc(sizeof(double) * 64) == cudaSuccess &&
-            u->dotpart.alloc(sizeof(double) * 8 * 512) == cudaSuccess &&
-            u->tz.alloc(sizeof(double) * n) == cudaSuccess && u->td.alloc(sizeof(double) * n) == cudaSuccess &&
-            u->tz2.alloc(sizeof(double) * n) == cudaSuccess && u->gtmp.alloc(sizeof(float) * off) == cudaSuccess;
-  ok = ok && alloc_bf16(u->x, u->g[0], CIO) == cudaSuccess && alloc_bf16(u->y, u->g[0], CIO) == cudaSuccess &&
-       alloc_bf16(u->dy, u->g[0], CIO) == cudaSuccess;
-  for (int lv = 0; lv < levels && ok; ++lv) {
-    const Grid &g = u->g[lv];
-    for (DeviceBuf *b : {&u->a[lv], &u->s[lv], &u->ga[lv], &u->gb[lv]}) ok = ok && alloc_bf16(*b, g, C) == cudaSuccess;
-    if (lv > 0) ok = ok && alloc_bf16(u->pin[lv], g, C) == cudaSuccess;
-    if (lv < levels - 1)
-      for (DeviceBuf *b : {&u->u[lv], &u->b[lv], &u->d[lv], &u->gs[lv]}) ok = ok && alloc_bf16(*b, g, C) == cudaSuccess;
-  }
-  ok = ok && u->tf.alloc(sizeof(float) * (size_t)u->g[0].voxels() * CIO) == cudaSuccess;
+            u->feat.alloc(sizeof(float) * nodes) == cudaSuccess &&
+            u->scal.alloc(sizeof(double) * S_COUNT) == cudaSuccess &&
+            u->dotpart.alloc(sizeof(double) * 8 * 512) == cudaSuccess && want_pairs(u, 1) &&
+            u->gtmp.alloc(sizeof(float) * off) == cudaSuccess && want_passes(u, 1, passes_per_pair(u)) > 0;
   if (!ok) {
     delete u;
     set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for the network");
@@ -532,9 +608,10 @@ int fc_unet_forward_grid(fc_unet *u, const float *d_x, float *d_y) {
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   const int64_t nv = u->g[0].voxels() * CIO;
-  f32_to_bf16_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, d_x, B(u->x));
-  forward(u);
-  bf16_to_f32_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, B(u->y), d_y);
+  refresh_weights(u);
+  f32_to_bf16_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, d_x, u->x);
+  forward(u, 1);
+  bf16_to_f32_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, u->y, d_y);
   const cudaError_t e = cudaStreamSynchronize(u->stream);
   return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? FC_OK : FC_CUDA_ERROR;
 }
@@ -544,8 +621,8 @@ int fc_unet_backward_grid(fc_unet *u, const float *d_dy) {
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   const int64_t nv = u->g[0].voxels() * CIO;
-  f32_to_bf16_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, d_dy, B(u->dy));
-  backward(u);
+  f32_to_bf16_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, d_dy, u->dy);
+  backward(u, {1, 1, false, 1.f, false});
   const cudaError_t e = cudaStreamSynchronize(u->stream);
   return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? FC_OK : FC_CUDA_ERROR;
 }
@@ -554,9 +631,11 @@ int fc_unet_apply(fc_unet *u, const double *d_r, double *d_z) {
   if (!u || !d_r || !d_z) return FC_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
-  if (u->net_on)
-    apply(u, d_r, d_z);
-  else
+  if (u->net_on) {
+    const int together = want_passes(u, 1, passes_per_pair(u));
+    if (together == 0) return FC_OUT_OF_MEMORY;
+    apply(u, 1, d_r, u->n, d_z, together);
+  } else
     apply_jacobi(u, d_r, d_z);
   return cudaGetLastError() == cudaSuccess ? FC_OK : FC_CUDA_ERROR;
 }
@@ -566,7 +645,7 @@ int fc_unet_train_step(fc_unet *u, const double *d_r, const double *d_e, const i
   if (!u || !d_r || !d_e || step < 1 || (d_ptr && (!d_idx || !d_val))) return FC_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
-  pair_gradient(u, d_r, d_e, d_ptr, d_idx, d_val, d_loss);
+  if (!pair_gradients(u, d_r, d_e, 1, u->n, d_ptr, d_idx, d_val, d_loss, false)) return FC_OUT_OF_MEMORY;
   fc::unet::adam(u->params, u->p.as<float>(), u->grad.as<float>(), u->m.as<float>(), u->v.as<float>(), lr, 0.9f,
                  0.999f, 1e-8f, step, u->stream);
   u->weights_stale = true;
@@ -581,13 +660,7 @@ int fc_unet_train_batch(fc_unet *u, const double *d_r, const double *d_e, int32_
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   cudaStream_t st = u->stream;
-  double *one = scal(u, 8);
-  for (int32_t q = 0; q < count; ++q) {
-    pair_gradient(u, d_r + (int64_t)q * ld, d_e + (int64_t)q * ld, d_ptr, d_idx, d_val, one);
-    accumulate_kernel<<<blocks(u->params), 256, 0, st>>>(u->params, u->grad.as<float>(), 1.f / (float)count, q == 0,
-                                                         u->gacc.as<float>());
-    if (d_loss) add_scalar_kernel<<<1, 1, 0, st>>>(one, d_loss, q == 0);
-  }
+  if (!pair_gradients(u, d_r, d_e, count, ld, d_ptr, d_idx, d_val, d_loss, true)) return FC_OUT_OF_MEMORY;
   fc::unet::adam(u->params, u->p.as<float>(), u->gacc.as<float>(), u->m.as<float>(), u->v.as<float>(), lr, 0.9f,
                  0.999f, 1e-8f, step, st);
   u->weights_stale = true;
@@ -610,20 +683,28 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     cudaSetDevice(net->device);
   }
   cudaStream_t st = net ? net->stream : nullptr;
+  const int together = net ? want_passes(net, 1, passes_per_pair(net)) : 0;
+  if (net && together == 0) {
+    set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for the network");
+    return FC_OUT_OF_MEMORY;
+  }
   // vectors: r, z, q and the ring of `keep` directions p_j and A p_j
   DeviceBuf vec, sc, part;
   const int ring = keep;
   if (vec.alloc(sizeof(double) * (size_t)n * (3 + 2 * ring)) != cudaSuccess ||
-      sc.alloc(sizeof(double) * 64) != cudaSuccess || part.alloc(sizeof(double) * 8 * 512) != cudaSuccess) {
+      sc.alloc(sizeof(double) * 64) != cudaSuccess ||
+      part.alloc(sizeof(double) * (1 + fc::unet::MAX_KEPT) * fc::unet::FCG_CTAS) != cudaSuccess) {
     set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for FCG");
     return FC_OUT_OF_MEMORY;
   }
   double *r = vec.as<double>(), *z = r + n, *tmp = z + n;
   std::vector<double *> P(ring), Q(ring);
   for (int j = 0; j < ring; ++j) P[j] = tmp + n * (1 + 2 * j), Q[j] = P[j] + n;
-  // [0] b.b [1] r.r [2] p.r [3] p.q [5] b - A x squared [8..8+ring) z.q_j [16..16+ring) p_j.q_j
-  // [32..32+CHECK) the last iterations' r.r
+  // [0] b.b [1] r.r [2] p.r [3] p.q [5] b - A x squared [6] a start's r.r [8..8+ring) z.q_j [16..16+ring) p_j.q_j
+  // [32..32+CHECK) the last iterations' r.r [48] the sums' ticket
   double *s = sc.as<double>();
+  int *ticket = reinterpret_cast<int *>(s + 48);
+  cudaMemsetAsync(ticket, 0, sizeof(double), st);
   cudaMemsetAsync(d_x, 0, sizeof(double) * n, st);
   copy_kernel<<<blocks(n), 256, 0, st>>>(n, d_b, r);
   {
@@ -656,45 +737,47 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
   constexpr int CHECK = 8;
   int since = 0;
   double ring_rr[CHECK];
+  // the kept directions' slots, the most recent first, at iteration `it` with `have` stored
+  auto kept = [&](int at, int have, int *slot) {
+    for (int j = 0; j < have; ++j) slot[j] = (at - 1 - j) % ring;
+    return have;
+  };
+  // z = M(r) and its products with the kept directions, for iteration `at`; with `update` the last
+  // direction's step on x and r first (rr: where r.r goes). The network's z is formed apart.
+  auto step = [&](bool update, int at, int have, double *rr_at) {
+    const bool jacobi = net && net->has_bj;
+    fc::unet::FcgStep a{};
+    a.n = n, a.update = update ? 1 : 0, a.alpha = s + 2, a.x = d_x, a.r = r, a.rr = rr_at, a.zq = s + 8;
+    if (update) a.p = P[(at - 1) % ring], a.q = Q[(at - 1) % ring];
+    a.part = part.as<double>(), a.ticket = ticket;
+    int slot[fc::unet::MAX_KEPT];
+    if (!use_net) {
+      a.z = z, a.inv = jacobi ? net->bj.as<double>() : nullptr;
+      a.kept = kept(at, have, slot);
+      for (int j = 0; j < a.kept; ++j) a.qj[j] = Q[slot[j]];
+    }
+    fc::unet::fcg_step(a, st);
+  };
+  bool have_z = false;
   while (!converged && it < max_iter) {
-    // z = M(r)
-    if (use_net)
-      apply(net, r, z);
-    else if (net && net->has_bj)
-      apply_jacobi(net, r, z);
-    else
-      copy_kernel<<<blocks(n), 256, 0, st>>>(n, r, z);
-    // p = z - sum_j (z.q_j / p_j.q_j) p_j over the stored directions (the denominators were kept
-    // in s + 16 + slot when each direction was made)
     double *p = P[it % ring], *q = Q[it % ring];
-    const int m = std::min(stored, ring);
-    std::vector<const double *> pj, qj, zz;
-    std::vector<int> slot;
-    for (int j = 0; j < m; ++j) {
-      const int k = (it - 1 - j) % ring;  // the most recent first
-      if (k < 0) continue;
-      slot.push_back(k);
-      pj.push_back(P[k]);
-      qj.push_back(Q[k]);
-      zz.push_back(z);
+    int slot[fc::unet::MAX_KEPT];
+    const int m = kept(it, stored, slot);
+    const double *pj[fc::unet::MAX_KEPT], *qj[fc::unet::MAX_KEPT], *zz[fc::unet::MAX_KEPT];
+    for (int j = 0; j < m; ++j) pj[j] = P[slot[j]], qj[j] = Q[slot[j]], zz[j] = z;
+    if (use_net) {
+      apply(net, 1, r, n, z, together);
+      if (m > 0) fc::unet::dots(n, m, zz, qj, part.as<double>(), s + 8, st);
+    } else if (!have_z) {
+      step(false, it, m, s + 6);
     }
-    if (!slot.empty()) {
-      fc::unet::dots(n, (int)slot.size(), zz.data(), qj.data(), part.as<double>(), s + 8, st);
-      fc::unet::fcg_direction(n, (int)slot.size(), z, pj.data(), slot.data(), s + 8, s + 16, p, st);
-    } else {
-      copy_kernel<<<blocks(n), 256, 0, st>>>(n, z, p);
-    }
-    fc::launch_spmv(n, d_ptr, d_idx, d_val, p, n, q, n, 1, st);
-    {
-      const double *a[2] = {p, p}, *b[2] = {r, q};
-      fc::unet::dots(n, 2, a, b, part.as<double>(), s + 2, st);
-    }
-    // alpha = p.r / p.q (kept as this direction's denominator), x += alpha p, r -= alpha q
-    fc::unet::fcg_update(n, s + 2, s + 16 + (it % ring), p, q, d_x, r, st);
-    {
-      const double *a[1] = {r}, *b[1] = {r};
-      fc::unet::dots(n, 1, a, b, part.as<double>(), s + 32 + (it % CHECK), st);
-    }
+    // p = z - sum_j (z.q_j / p_j.q_j) p_j over the stored directions (the denominators were kept
+    // in s + 16 + slot when each direction was made); q = A p, p.r, p.q
+    fc::unet::fcg_direction(n, m, z, pj, slot, s + 8, s + 16, p, st);
+    fc::unet::fcg_product(n, d_ptr, d_idx, d_val, p, r, q, s + 2, s + 16 + (it % ring), part.as<double>(), ticket, st);
+    // alpha = p.r / p.q, x += alpha p, r -= alpha q, and the next iteration's z
+    step(true, it + 1, std::min(stored + 1, ring), s + 32 + (it % CHECK));
+    have_z = !use_net;
     ++it;
     stored = std::min(stored + 1, ring);
     if (++since < CHECK && it < max_iter) continue;
@@ -728,6 +811,7 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
       residual_from_kernel<<<blocks(n), 256, 0, st>>>(n, d_b, tmp);
       copy_kernel<<<blocks(n), 256, 0, st>>>(n, tmp, r);
       stored = 0;
+      have_z = false;
     }
     if (converged && replacements < MAX_REPLACEMENTS) {
       // the recurrence says converged: check b - A x itself; when rounding has let the two drift
@@ -743,6 +827,7 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
       if (!(tr <= target)) {
         copy_kernel<<<blocks(n), 256, 0, st>>>(n, tmp, r);
         stored = 0;
+        have_z = false;
         converged = false;
         ++replacements;
       }
