@@ -45,7 +45,7 @@ int fail_status(fc_status *st, const Failure &f) {
 }
 
 enum Kind {
-  K_ASSEMBLE, K_PANEL, K_RETIRED_2, K_GEMM, K_SOLVE_ASSEMBLE, K_RETIRED_5, K_SOLVE_FWD, K_SOLVE_BWD,
+  K_ASSEMBLE, K_PANEL, K_INVERSE, K_GEMM, K_SOLVE_ASSEMBLE, K_RETIRED_5, K_SOLVE_FWD, K_SOLVE_BWD,
   K_SOLVE_DAG_FWD, K_SOLVE_DAG_BWD,
   K_GEMM_MIXED,  // A in the factor's storage type, B and C FP64
   K_GEMM_F64,    // FP64 throughout (the diagonal blocks' inverses)
@@ -105,7 +105,7 @@ struct fc_chol {
   DeviceBuf d_ir_sc;                     // the refinement's SpMV: row-major copies of x and y
   bool refine_pcg = true;                // refinement by preconditioned CG (else plain refinement)
   bool tc = true;                        // FP32 updates on tcgen05 (FC_TF32_MMA_SYNC=1: on mma.sync)
-  DeviceBuf d_asm, d_ranges, d_panel, d_gemm;
+  DeviceBuf d_asm, d_ranges, d_panel, d_inv, d_gemm;
   // the mixed-precision factor's tcgen05 update products: packed operands (reused level after
   // level), their pack and tile tasks, and one TMA tensor map per supernode
   DeviceBuf d_pack, d_pack_t, d_tc_t, d_maps;
@@ -451,7 +451,8 @@ struct MapSpec {
 constexpr int OUTER_PANELS = 4;
 
 void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::vector<fc::AssembleTask> &asm_t,
-                 std::vector<int4> &ranges, std::vector<fc::PanelTask> &panel_t, std::vector<fc::GemmTask> &gemm_t,
+                 std::vector<int4> &ranges, std::vector<fc::PanelTask> &panel_t,
+                 std::vector<fc::InverseTask> &inv_t, std::vector<fc::GemmTask> &gemm_t,
                  std::vector<fc::PackTask> &pack_t, std::vector<fc::TcTask> &tc_t, std::vector<MapSpec> &maps) {
   auto Lp = [&](int64_t off) { return arena_at(h->d_L, h, off); };
   auto Up = [&](int64_t off) { return arena_at(h->d_U, h, off); };
@@ -508,6 +509,7 @@ void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::v
         pre_asm = (int)h->program.size() - 1;
       }
     }
+    const int64_t io = (int64_t)inv_t.size();
     int P = 0;
     for (int64_t s : S) P = std::max(P, (h->width[s] + NB - 1) / NB);
     // Two-level blocking: panels are grouped in outer blocks of OUTER_PANELS. A panel's update of
@@ -569,10 +571,12 @@ void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::v
         const int64_t ioff = ib + in + in * bw;
         // every CTA of the panel stores its share of the factored block and its inverse (keep:
         // the panel's CTA count, pad: this CTA's place among them)
-        if (c1 >= m) panel_t.push_back({(int32_t)s, c0, c1, m, m, 1, doff, ioff, bw, 0});
+        const int64_t lo = h->loff[s], col = h->first[s] + c0;
+        if (c1 >= m) panel_t.push_back({m, c0, c1, m, m, 1, 0, bw, lo, doff, ioff, col});
         const int nrt = (m - c1 + fc::PANEL_ROWS - 1) / fc::PANEL_ROWS;
         for (int r0 = c1, q = 0; r0 < m; r0 += fc::PANEL_ROWS, ++q)
-          panel_t.push_back({(int32_t)s, c0, c1, r0, std::min(m, r0 + fc::PANEL_ROWS), nrt, doff, ioff, bw, q});
+          panel_t.push_back({m, c0, c1, r0, std::min(m, r0 + fc::PANEL_ROWS), nrt, q, bw, lo, doff, ioff, col});
+        if (c1 - c0 > 8) inv_t.push_back({doff, ioff, c1 - c0, bw});  // narrower: by the panel itself
         const int bs = p / OP * OP * NB, be = std::min(w, bs + OP * NB);  // this panel's block
         if (c1 < be) tiles(s, c1, be, c0, c1, gemm_t);                     // within the block
         if (c1 == be && be < w) {                                         // past the block
@@ -636,6 +640,14 @@ void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::v
     int panels_done = -1;
     for (int q = (int)h->program.size() - 1; q >= 0 && panels_done < 0; --q)
       if (h->program[q].lane == 0) panels_done = q;
+    if ((int64_t)inv_t.size() > io) {
+      push(h->program, K_INVERSE, io, (int64_t)inv_t.size() - io, (int)l);
+      h->program.back().lane = 2;
+      if (panels_done >= 0) {
+        h->program.back().dep = panels_done;
+        h->program[panels_done].record = true;
+      }
+    }
     for (int hh = NB; hh < fc::SB; hh *= 2) {
       std::vector<fc::GemmTask> first, second;
       inverse_doubling(h, S, h->d_T.as<double>(), hh, &first, &second);
@@ -643,11 +655,7 @@ void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::v
       int64_t go = (int64_t)gemm_t.size();
       gemm_t.insert(gemm_t.end(), first.begin(), first.end());
       push(h->program, K_GEMM_MIXED, go, (int64_t)first.size(), (int)l);
-      h->program.back().lane = 2;
-      if (hh == NB && panels_done >= 0) {
-        h->program.back().dep = panels_done;
-        h->program[panels_done].record = true;
-      }
+      h->program.back().lane = 2;  // after the panels' inverses, on the same lane
       go = (int64_t)gemm_t.size();
       gemm_t.insert(gemm_t.end(), second.begin(), second.end());
       push(h->program, K_GEMM_F64, go, (int64_t)second.size(), (int)l);
@@ -746,11 +754,12 @@ int plan_factor_upload(fc_chol *h, fc_status *st) {
   std::vector<fc::AssembleTask> asm_t;
   std::vector<int4> ranges;
   std::vector<fc::PanelTask> panel_t;
+  std::vector<fc::InverseTask> inv_t;
   std::vector<fc::GemmTask> gemm_t;
   std::vector<fc::PackTask> pack_t;
   std::vector<fc::TcTask> tc_t;
   std::vector<MapSpec> specs;
-  plan_factor(h, lv, asm_t, ranges, panel_t, gemm_t, pack_t, tc_t, specs);
+  plan_factor(h, lv, asm_t, ranges, panel_t, inv_t, gemm_t, pack_t, tc_t, specs);
   h->gemm_tasks = (int64_t)(gemm_t.size() + tc_t.size());
   h->gemm_flops_factor = 0;
   for (const auto &g : gemm_t) h->gemm_flops_factor += task_flops(g);
@@ -821,7 +830,7 @@ int plan_factor_upload(fc_chol *h, fc_status *st) {
     }
   }
   if ((e = upload(h->d_asm, asm_t, stream)) != cudaSuccess || (e = upload(h->d_ranges, ranges, stream)) != cudaSuccess ||
-      (e = upload(h->d_panel, panel_t, stream)) != cudaSuccess ||
+      (e = upload(h->d_panel, panel_t, stream)) != cudaSuccess || (e = upload(h->d_inv, inv_t, stream)) != cudaSuccess ||
       (e = upload(h->d_gemm, gemm_t, stream)) != cudaSuccess)
     return cuda_fail(st, e, "upload of the plan");
   if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(st, e, "plan upload");
@@ -1430,6 +1439,7 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
         fc::launch_panel(t, h->fp32, d_val, h->d_panel.as<fc::PanelTask>() + l.off, l.count,
                          h->d_status.as<fc::DeviceStatus>(), l.width, st);
         break;
+      case K_INVERSE: fc::launch_inverse(t, h->d_inv.as<fc::InverseTask>() + l.off, l.count, st); break;
       case K_GEMM: fc::launch_gemm(h->d_gemm.as<fc::GemmTask>() + l.off, l.count, gk, st); break;
       case K_PACK_TC: fc::launch_pack_tc(t, h->d_pack_t.as<fc::PackTask>() + l.off, h->d_pack.as<float>(), l.count, st); break;
       case K_GEMM_TC:

@@ -196,148 +196,296 @@ __global__ void scale_kernel(int64_t n, const int64_t *__restrict__ diag_src, co
   scale[j] = d > 0.0 ? 1.0 / sqrt(d) : 1.0;
 }
 
-// ---- panel: factor the diagonal block, invert it, solve the rows below --------------------------
-// The block (pw <= 64 columns) is factored in FP64 in shared memory by strips of 8 columns; the
-// pivot test is the reference's (cholesky.rs:1162-1165): not (d > PIVOT_TOLERANCE |A_jj|) or not
+// ---- panel: factor the diagonal block, solve the rows below ---------------------------------------
+// The block (pw <= 64 columns) and up to PANEL_ROWS rows below it lie in shared memory as one tall
+// panel, factored in FP64 right-looking by strips of 8 columns. Warp 0 carries the chain: it brings
+// the next strip's rows of the block up to date with the strip before (two rows a lane, from shared
+// memory), factors it (pivots and multipliers broadcast by shuffles) and goes on. The other warps
+// follow a strip behind: they solve the strip's columns of the rows below (a row a thread, forward
+// substitution with the 8 x 8 triangle) and store them, and apply the strip to the columns past the
+// next one, of the block (8 x 8 DMMA tiles) and of the rows below (16 x 8). So the rows below end
+// with the block, one barrier a strip, and nothing waits for the block's inverse, which only the
+// solve reads (inverse_kernel, beside the following launches). Bound by the chain of dependent FP64
+// steps. Before, with the inverse formed here and the rows multiplied by it, a 64-column panel of
+// 128 rows took 42 us (16 of them the block, 7.5 the inverse, 9.5 the rows); the panels of a box of
+// 23 x 17 x 19 elements took 31.6 us on average, now 22.
+// The pivot test is the reference's (cholesky.rs:1162-1165): not (d > PIVOT_TOLERANCE |A_jj|) or not
 // finite fails, and the smallest failing column (postorder) is kept in the status word. A failed
-// pivot makes NaNs and nothing else: no index depends on a value. The inverse comes from 8 x 8
-// diagonal blocks and block forward substitution; the rows below are X = B L^-T on the FP64
-// tensor pipe. L may be stored in FP32 (widened on load, rounded on store); the diagonal arena
-// stays FP64.
-constexpr int PANEL_THREADS = 128;
+// pivot makes NaNs and nothing else: no index depends on a value. L may be stored in FP32 (widened
+// on load, rounded on store); the diagonal arena stays FP64. A panel at most 8 columns wide (most
+// supernodes) is inverted here as well, by warp 0 while the rows below end.
+constexpr int PANEL_THREADS = 256, PANEL_THREADS_NARROW = 128;
+constexpr int PANEL_ALD = 68, PANEL_BLD = PANEL_ROWS + 4;  // a warp's fragment reads fall in distinct banks
 // Shared memory of a panel launch whose widest panel is padded to p8 columns (a multiple of 8).
-template <class T>
 __host__ __device__ constexpr size_t panel_smem(int p8) {
-  return sizeof(double) * (p8 * (65 + TS) + 1024 + 128) + sizeof(T) * p8 * tile_stride<T>();
+  return sizeof(double) * ((size_t)p8 * (PANEL_ALD + PANEL_BLD) + 128);
 }
 
-template <class T>
-__global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(Tree t, const double *__restrict__ val,
-                                                              const PanelTask *__restrict__ tasks,
-                                                              DeviceStatus *status, int p8max) {
+// 1 / sqrt(a) on the panel's chain: the hardware's estimate (good to 2^-20 at least) and two Newton
+// steps y += y (1 - a y^2) / 2 (the error squares each time), eight dependent operations; the tails of
+// the exponent range take the library's function. An a that is not positive gives a NaN or an
+// infinity, which the pivot test refuses.
+__device__ __forceinline__ double inverse_root(double a) {
+  if (!(a > 1e-280 && a < 1e280)) return rsqrt(a);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const double e = fma(-a * y, y, 1.0);
+    y = fma(0.5 * y, e, y);
+  }
+  return y;
+}
+
+template <class T, int THREADS>
+__global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__restrict__ val,
+                                                        const PanelTask *__restrict__ tasks, DeviceStatus *status,
+                                                        int p8max) {
+  constexpr int WORKERS = THREADS / 32 - 1;  // warps besides warp 0
   extern __shared__ double sm[];
-  double *inv = sm;                 // inv[k * TS + i] = Linv(i, k) (p8max rows)
-  double *a = inv + p8max * TS;     // factor, column-major, ld 65 (p8max columns)
-  double *tt = a + p8max * 65;      // scratch of the inversion's products (<= 1024 doubles)
-  T *bt2 = reinterpret_cast<T *>(a);  // after the factor is stored: the second row tile (a and tt)
-  double *dg = tt + 1024;           // the matrix's own diagonal entries of the panel's columns
-  double *dv = dg + 64;             // the pivots' reciprocals
-  T *bt = reinterpret_cast<T *>(dv + 64);  // rows below: bt[k * S + r] = L(r0 + r, c0 + k)
+  double *a = sm;                        // the block, column-major
+  double *b = a + p8max * PANEL_ALD;     // the rows below: b[c * PANEL_BLD + i] = L(r0 + i, c0 + c)
+  double *dg = b + p8max * PANEL_BLD;    // the matrix's own diagonal entries of the panel's columns
+  double *dv = dg + 64;                  // the pivots' reciprocals
+  __shared__ double piv[64];             // the pivots, for the test at the end
   __shared__ int fail;
   const PanelTask task = tasks[blockIdx.x];
-  const int s = task.s;
-  const int64_t m = t.height[s], f = t.first[s];
-  T *Ls = static_cast<T *>(t.L) + t.loff[s];
+  const int64_t m = task.m;
+  T *Ls = static_cast<T *>(t.L) + task.loff;
   const int c0 = task.c0, pw = task.c1 - task.c0, rows = task.r1 - task.r0;
-  const int nb8 = (pw + 7) >> 3, P8 = 8 * nb8, K4 = (pw + 3) & ~3;
+  const int nb8 = (pw + 7) >> 3, P8 = 8 * nb8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) fail = pw;
-  // the block's lower triangle (identity past pw, so the padded block inverts to the same leading
-  // pw x pw inverse) and the first row tile in flight first, then the matrix's own diagonal
-  // entries (two dependent loads each) while those land
-  if (rows > 0) load_tile<T>(bt, Ls + task.r0 + (int64_t)c0 * m, 1, m, min(rows, 64), pw, K4);
+  // the block's lower triangle (identity past pw: the padding factors as the identity) and the rows
+  // below in flight first, then the matrix's own diagonal entries (two dependent loads each)
   if (sizeof(T) == 8) {
-    for (int c = warp; c < P8; c += PANEL_THREADS / 32)
+    for (int c = warp; c < P8; c += THREADS / 32)
       for (int r = lane; r < P8; r += 32) {
         if (r < pw && c < pw && r >= c)
-          cp_async8(&a[c * 65 + r], Ls + (c0 + r) + (int64_t)(c0 + c) * m, 8);
+          cp_async8(&a[c * PANEL_ALD + r], Ls + (c0 + r) + (int64_t)(c0 + c) * m, 8);
         else
-          a[c * 65 + r] = (double)(r == c);
+          a[c * PANEL_ALD + r] = (double)(r == c);
       }
+    for (int c = warp; c < pw; c += THREADS / 32)
+      for (int i = lane; i < rows; i += 32)
+        cp_async8(&b[c * PANEL_BLD + i], Ls + task.r0 + i + (int64_t)(c0 + c) * m, 8);
   } else {
-    // FP32 panels: every load of the thread in flight before the widening stores
-    float v[16][2];
+    // FP32 panels are widened as they are stored: a thread's loads of four columns in flight
+    for (int cb = warp; cb < P8; cb += 4 * (THREADS / 32)) {
+      float v[4][2 + PANEL_ROWS / 32];
 #pragma unroll
-    for (int ci = 0; ci < 16; ++ci)
+      for (int q = 0; q < 4; ++q) {
+        const int c = cb + q * (THREADS / 32);
 #pragma unroll
-      for (int ri = 0; ri < 2; ++ri) {
-        const int c = warp + 4 * ci, r = lane + 32 * ri;
-        v[ci][ri] = r < pw && c < pw && r >= c ? (float)Ls[(c0 + r) + (int64_t)(c0 + c) * m] : (float)(r == c);
+        for (int k = 0; k < 2; ++k) {
+          const int r = lane + 32 * k;
+          v[q][k] = r < pw && c < pw && r >= c ? (float)Ls[(c0 + r) + (int64_t)(c0 + c) * m] : (float)(r == c);
+        }
+#pragma unroll
+        for (int k = 0; k < PANEL_ROWS / 32; ++k) {
+          const int i = lane + 32 * k;
+          v[q][2 + k] = c < pw && i < rows ? (float)Ls[task.r0 + i + (int64_t)(c0 + c) * m] : 0.f;
+        }
       }
 #pragma unroll
-    for (int ci = 0; ci < 16; ++ci)
+      for (int q = 0; q < 4; ++q) {
+        const int c = cb + q * (THREADS / 32);
+        if (c >= P8) continue;
 #pragma unroll
-      for (int ri = 0; ri < 2; ++ri) {
-        const int c = warp + 4 * ci, r = lane + 32 * ri;
-        if (c < P8 && r < P8) a[c * 65 + r] = (double)v[ci][ri];
+        for (int k = 0; k < 2; ++k)
+          if (lane + 32 * k < P8) a[c * PANEL_ALD + lane + 32 * k] = (double)v[q][k];
+#pragma unroll
+        for (int k = 0; k < PANEL_ROWS / 32; ++k) b[c * PANEL_BLD + lane + 32 * k] = (double)v[q][2 + k];
       }
+    }
   }
   cp_async_commit();
-  for (int c = tid; c < pw; c += PANEL_THREADS) {
-    const int64_t j = f + c0 + c, ds = t.diag_src[j];
+  for (int c = tid; c < pw; c += THREADS) {
+    const int64_t j = task.col + c, ds = t.diag_src[j];
     const double d = ds >= 0 ? val[ds] : 0.0;
     dg[c] = t.scale ? d * t.scale[j] * t.scale[j] : d;
   }
-  for (int e = tid; e < P8 * TS; e += PANEL_THREADS) inv[e] = 0.0;
   cp_async_wait<0>();
   __syncthreads();
-  // right-looking by strips of 8 columns with look-ahead: warp 0 factors a strip (two rows a
-  // lane, pivots and multipliers broadcast by shuffles); then all warps update the next strip's
-  // columns, and warp 0 factors that strip while warps 1-3 update the rest of the trailing lower
-  // triangle (DMMA, a rank-8 update per 8 x 8 block); padding past pw factors as the identity
-  auto factor_strip = [&](int B) {
-    const int o = 8 * B;
-    const int r0 = o + lane, r1 = o + 32 + lane;
-    double s0[8], s1[8];
+  const int g = lane >> 2, tg = lane & 3;
+  for (int B = 0; B <= nb8; ++B) {
+    if (warp == 0) {
+      if (B < nb8) {
+        const int o = 8 * B, r0 = o + lane, r1 = o + 32 + lane;
+        double s0[8], s1[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      s0[k] = r0 < P8 ? a[(o + k) * 65 + r0] : 0.0;
-      s1[k] = r1 < P8 ? a[(o + k) * 65 + r1] : 0.0;
-    }
+        for (int k = 0; k < 8; ++k) {
+          s0[k] = r0 < P8 ? a[(o + k) * PANEL_ALD + r0] : 0.0;
+          s1[k] = r1 < P8 ? a[(o + k) * PANEL_ALD + r1] : 0.0;
+        }
+        if (B > 0) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double acc = __shfl_sync(0xffffffffu, s0[j], j);
-      const double rd = rsqrt(acc);
-      const double d = acc * rd;
-      if (lane == j) {
-        s0[j] = d;
-        dv[o + j] = rd;
-        if (o + j < pw && (!(acc > PIVOT_TOLERANCE * fabs(dg[o + j])) || !isfinite(acc)) && fail == pw) fail = o + j;
-      } else if (lane > j) {
-        s0[j] *= rd;
+          for (int kk = 0; kk < 8; ++kk) {
+            const double *col = a + (o - 8 + kk) * PANEL_ALD;
+            const double l0 = r0 < P8 ? col[r0] : 0.0, l1 = r1 < P8 ? col[r1] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const double lk = col[o + k];
+              s0[k] -= l0 * lk;
+              s1[k] -= l1 * lk;
+            }
+          }
+        }
+        // the multipliers are broadcast before they are scaled, beside the root: the chain of a column
+        // is the pivot's shuffle, its root, a product and an update
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const double acc = __shfl_sync(0xffffffffu, s0[j], j);
+          double lk[8];
+#pragma unroll
+          for (int k = j + 1; k < 8; ++k) lk[k] = __shfl_sync(0xffffffffu, s0[j], k);
+          const double rd = inverse_root(acc);
+          if (lane == 0) piv[o + j] = acc, dv[o + j] = rd;
+          if (lane >= j) s0[j] *= rd;  // the pivot's own row: acc rd = sqrt(acc)
+          s1[j] *= rd;
+#pragma unroll
+          for (int k = j + 1; k < 8; ++k) {
+            const double l = lk[k] * rd;
+            if (lane > j) s0[k] -= s0[j] * l;
+            s1[k] -= s1[j] * l;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (r0 < P8) a[(o + k) * PANEL_ALD + r0] = s0[k];
+          if (r1 < P8) a[(o + k) * PANEL_ALD + r1] = s1[k];
+        }
+      } else if (pw <= 8 && task.part == 0) {
+        // the 8 x 8 inverse, a column a lane
+        double *Ip = t.Dinv + task.ioff, *Dp = t.D + task.doff + pw * pw;
+        if (lane < pw) {
+          double y[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            y[i] = 0.0;
+            if (i >= lane) {
+              double sum = i == lane ? 1.0 : 0.0;
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (k >= lane && k < i) sum -= a[k * PANEL_ALD + i] * y[k];
+              y[i] = sum * dv[i];
+            }
+            if (i < pw) {
+              Dp[lane * pw + i] = y[i];
+              Ip[(int64_t)lane * task.ild + i] = y[i];
+            }
+          }
+        }
       }
-      s1[j] *= rd;
+    } else if (B > 0) {
+      const int o = 8 * (B - 1), wt = tid - 32, ww = warp - 1;
+      // the strip's columns of the rows below
+      T *dst = Ls + task.r0 + (int64_t)(c0 + o) * m;
+      for (int i = wt; i < rows; i += 32 * WORKERS) {
+        double x[8];
 #pragma unroll
-      for (int k = j + 1; k < 8; ++k) {
-        const double lk = __shfl_sync(0xffffffffu, s0[j], k);
-        if (lane > j) s0[k] -= s0[j] * lk;
-        s1[k] -= s1[j] * lk;
+        for (int k = 0; k < 8; ++k) x[k] = b[(o + k) * PANEL_BLD + i];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          x[k] *= dv[o + k];
+#pragma unroll
+          for (int j = k + 1; j < 8; ++j) x[j] -= x[k] * a[(o + k) * PANEL_ALD + o + j];
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          b[(o + k) * PANEL_BLD + i] = x[k];
+          if (o + k < pw) dst[i + (int64_t)k * m] = T(x[k]);
+        }
+      }
+      // the block's columns past the next strip: 8 x 8 tiles (I, J), I >= J
+      int q = 0;
+      for (int J = o + 16; J < P8; J += 8)
+        for (int I = J; I < P8; I += 8, ++q) {
+          if (q % WORKERS != ww) continue;
+          double c[2] = {0.0, 0.0};
+          dmma(c, a[(o + tg) * PANEL_ALD + I + g], a[(o + tg) * PANEL_ALD + J + g]);
+          dmma(c, a[(o + 4 + tg) * PANEL_ALD + I + g], a[(o + 4 + tg) * PANEL_ALD + J + g]);
+          a[(J + 2 * tg) * PANEL_ALD + I + g] -= c[0];
+          a[(J + 2 * tg + 1) * PANEL_ALD + I + g] -= c[1];
+        }
+      // the rows below's columns past the strip, once every worker's rows are solved
+      if (B < nb8 && rows > 0) {
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * WORKERS) : "memory");
+        const int groups = (rows + 15) >> 4, strips = nb8 - B, items = groups * strips;
+        for (int it = ww; it < items; it += 2 * WORKERS) {
+          // two 16 x 8 tiles at a time, their loads before their stores
+          double c[2][4];
+          int i0[2], J[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int e = min(it + u * WORKERS, items - 1);
+            i0[u] = 16 * (e / strips), J[u] = o + 8 + 8 * (e % strips);
+            double av[4], bv[2];
+            av[0] = b[(o + tg) * PANEL_BLD + i0[u] + g], av[1] = b[(o + tg) * PANEL_BLD + i0[u] + g + 8];
+            av[2] = b[(o + tg + 4) * PANEL_BLD + i0[u] + g], av[3] = b[(o + tg + 4) * PANEL_BLD + i0[u] + g + 8];
+            bv[0] = -a[(o + tg) * PANEL_ALD + J[u] + g], bv[1] = -a[(o + tg + 4) * PANEL_ALD + J[u] + g];
+            c[u][0] = b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g], c[u][1] = b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g];
+            c[u][2] = b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g + 8];
+            c[u][3] = b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g + 8];
+            dmma16(c[u], av, bv);
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            if (it + u * WORKERS >= items) continue;
+            b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g] = c[u][0], b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g] = c[u][1];
+            b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g + 8] = c[u][2];
+            b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g + 8] = c[u][3];
+          }
+        }
       }
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (r0 < P8) a[(o + k) * 65 + r0] = s0[k];
-      if (r1 < P8) a[(o + k) * 65 + r1] = s1[k];
-    }
-  };
-  // the rank-8 update by strip B of the 8 x 8 block (I, J) (I >= J > B)
-  auto update_tile = [&](int B, int I, int J) {
-    const int o = 8 * B, g = lane >> 2, tg = lane & 3;
-    double c[2] = {0.0, 0.0};
-    dmma(c, a[(o + tg) * 65 + I + g], a[(o + tg) * 65 + J + g]);
-    dmma(c, a[(o + 4 + tg) * 65 + I + g], a[(o + 4 + tg) * 65 + J + g]);
-    a[(J + 2 * tg) * 65 + I + g] -= c[0];
-    a[(J + 2 * tg + 1) * 65 + I + g] -= c[1];
-  };
-  if (warp == 0) factor_strip(0);
-  __syncthreads();
-  for (int B = 0; B < nb8; ++B) {
-    if (B + 1 < nb8) {
-      // the next strip's block column, all warps
-      for (int qi = B + 1 + warp; qi < nb8; qi += PANEL_THREADS / 32) update_tile(B, 8 * qi, 8 * (B + 1));
-      __syncthreads();
-      if (warp == 0) {
-        factor_strip(B + 1);
-      } else {
-        int q = 0;
-        for (int qj = B + 2; qj < nb8; ++qj)
-          for (int qi = qj; qi < nb8; ++qi, ++q)
-            if (q % 3 == warp - 1) update_tile(B, 8 * qi, 8 * qj);
-      }
-      __syncthreads();
-    }
+    __syncthreads();
   }
-  // inverse: the diagonal 8 x 8 blocks (a column each) ...
+  // this CTA's columns of the factored block (the panel's CTAs share the stores)
+  double *Dp = t.D + task.doff;
+  for (int c = task.part * (THREADS / 32) + warp; c < pw; c += task.keep * (THREADS / 32))
+    for (int r = lane; r < pw; r += 32) Dp[c * pw + r] = r >= c ? a[c * PANEL_ALD + r] : 0.0;
+  // the pivot test, every column's at once (a column after a failed one fails too)
+  if (task.part == 0) {
+    if (tid < pw && (!(piv[tid] > PIVOT_TOLERANCE * fabs(dg[tid])) || !isfinite(piv[tid]))) atomicMin(&fail, tid);
+    __syncthreads();
+  }
+  if (tid == 0 && task.part == 0 && fail < pw)
+    atomicMin(&status->failed_column, (unsigned long long)(task.col + fail));
+}
+
+// The inverse of a panel's factored block (more than 8 columns), from the diagonal arena: its 8 x 8
+// diagonal blocks a column a thread, then by doubling (h = 8, 16, 32): neighbouring inverses A^-1,
+// C^-1 of h columns give the inverse of [[A, 0], [B, C]], whose lower-left block is
+// -C^-1 (B A^-1); both products on DMMA, 8 x 8 output tiles round-robin over the warps, T = B A^-1 in
+// the scratch. Only the solve and the inverses' doubling read it, so it runs beside the levels
+// that follow.
+constexpr int INVERSE_THREADS = 128;
+constexpr size_t INVERSE_SMEM = sizeof(double) * (64 * 65 + 64 * TS + 1024 + 64);
+
+__global__ void __launch_bounds__(INVERSE_THREADS) inverse_kernel(Tree t, const InverseTask *__restrict__ tasks) {
+  extern __shared__ double sm[];
+  double *inv = sm;              // inv[k * TS + i] = Linv(i, k)
+  double *a = inv + 64 * TS;     // factor, column-major, ld 65
+  double *tt = a + 64 * 65;      // scratch of the products (<= 1024 doubles)
+  double *dv = tt + 1024;        // the diagonal's reciprocals
+  const InverseTask task = tasks[blockIdx.x];
+  const int pw = task.pw, P8 = (pw + 7) / 8 * 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double *Dp = t.D + task.doff, *Ip = t.Dinv + task.ioff;
+  for (int c = warp; c < P8; c += INVERSE_THREADS / 32)
+    for (int r = lane; r < P8; r += 32) {
+      if (r < pw && c < pw && r >= c)
+        cp_async8(&a[c * 65 + r], Dp + c * pw + r, 8);
+      else
+        a[c * 65 + r] = (double)(r == c);
+    }
+  cp_async_commit();
+  for (int e = tid; e < P8 * TS; e += INVERSE_THREADS) inv[e] = 0.0;
+  cp_async_wait<0>();
+  __syncthreads();
+  if (tid < P8) dv[tid] = 1.0 / a[tid * 65 + tid];
+  __syncthreads();
   if (tid < P8) {
     const int B = tid >> 3, j = tid & 7, o = 8 * B;
     double y[8];
@@ -356,9 +504,6 @@ __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(Tree t, const doub
     }
   }
   __syncthreads();
-  // ... then by doubling (h = 8, 16, 32): neighbouring inverses A^-1, C^-1 of h columns give the
-  // inverse of [[A, 0], [B, C]], whose lower-left block is -C^-1 (B A^-1); both products on DMMA,
-  // 8 x 8 output tiles round-robin over the warps, T = B A^-1 in the scratch
   for (int h = 8; h < P8; h *= 2) {
     int tile = 0;
     for (int a0 = 0; a0 + h < P8; a0 += 2 * h) {
@@ -393,48 +538,11 @@ __global__ void __launch_bounds__(PANEL_THREADS) panel_kernel(Tree t, const doub
     }
     __syncthreads();
   }
-  {
-    // this CTA's columns of the factored block and its inverse (the panel's CTAs share the stores)
-    double *Dp = t.D + task.doff, *Ip = t.Dinv + task.ioff;
-    const int nw = PANEL_THREADS / 32;
-    for (int c = task.part * nw + warp; c < pw; c += task.keep * nw)
-      for (int r = lane; r < pw; r += 32) {
-        Dp[c * pw + r] = r >= c ? a[c * 65 + r] : 0.0;
-        Dp[pw * pw + c * pw + r] = inv[c * TS + r];
-        Ip[(int64_t)c * task.ild + r] = r >= c ? inv[c * TS + r] : 0.0;
-      }
-    if (tid == 0 && task.part == 0 && fail < pw)
-      atomicMin(&status->failed_column, (unsigned long long)(f + c0 + fail));
-  }
-  // the rows below, 64 at a time: the first 64 loaded with the block, the next 64 into the factor's
-  // and the scratch's space (free once the factor is stored) while the first are solved, any
-  // further ones one after another
-  if (rows > 64) {
-    __syncthreads();  // every thread is done with a and tt
-    load_tile<T>(bt2, Ls + task.r0 + 64 + (int64_t)c0 * m, 1, m, min(64, rows - 64), pw, K4);
-    cp_async_commit();
-  }
-  for (int rr = 0; rr < rows; rr += 64) {
-    const int nrr = min(64, rows - rr);
-    const T *tile = rr == 64 ? bt2 : bt;
-    if (rr == 64) {
-      cp_async_wait<0>();
-      __syncthreads();
-    } else if (rr > 64) {
-      __syncthreads();  // the previous rows' tile is read
-      load_tile<T>(bt, Ls + task.r0 + rr + (int64_t)c0 * m, 1, m, nrr, pw, K4);
-      cp_async_commit();
-      cp_async_wait<0>();
-      __syncthreads();
+  for (int c = warp; c < pw; c += INVERSE_THREADS / 32)
+    for (int r = lane; r < pw; r += 32) {
+      Dp[pw * pw + c * pw + r] = inv[c * TS + r];
+      Ip[(int64_t)c * task.ild + r] = r >= c ? inv[c * TS + r] : 0.0;
     }
-    double acc[4][4][2];
-    zero_acc(acc);
-    mma_tiles<T>(tile, inv, K4, acc);
-    T *dst = Ls + task.r0 + rr + (int64_t)c0 * m;
-    each_acc(acc, [&](int i, int c, double v) {
-      if (i < nrr && c < pw) dst[i + (int64_t)c * m] = T(v);
-    });
-  }
 }
 
 // ---- tiled C -= A B^T on the FP64 tensor pipe ---------------------------------------------------
@@ -1543,8 +1651,9 @@ void set_smem(K kernel, size_t bytes) {
 void configure_kernels() {
   static bool done = false;
   if (done) return;
-  set_smem(panel_kernel<double>, panel_smem<double>(64));
-  set_smem(panel_kernel<float>, panel_smem<float>(64));
+  set_smem(panel_kernel<double, PANEL_THREADS>, panel_smem(64));
+  set_smem(panel_kernel<float, PANEL_THREADS>, panel_smem(64));
+  set_smem(inverse_kernel, INVERSE_SMEM);
   set_smem(gemm_kernel<double>, gemm_smem<double>());
   set_smem(gemm_kernel<float>, gemm_smem<float>());
   set_smem(gemm_cluster_kernel<double>, gemm_smem<double>());
@@ -1581,10 +1690,22 @@ void launch_panel(const Tree &t, bool fp32, const double *upper_val, const Panel
                   DeviceStatus *status, int p8max, cudaStream_t st) {
   if (count <= 0) return;
   configure_kernels();
-  if (fp32)
-    panel_kernel<float><<<count, PANEL_THREADS, panel_smem<float>(p8max), st>>>(t, upper_val, tasks, status, p8max);
+  // a launch of narrow panels (the bottom levels' thousands) in CTAs of four warps
+  const size_t smem = panel_smem(p8max);
+  if (p8max <= 16 && fp32)
+    panel_kernel<float, PANEL_THREADS_NARROW><<<count, PANEL_THREADS_NARROW, smem, st>>>(t, upper_val, tasks, status, p8max);
+  else if (p8max <= 16)
+    panel_kernel<double, PANEL_THREADS_NARROW><<<count, PANEL_THREADS_NARROW, smem, st>>>(t, upper_val, tasks, status, p8max);
+  else if (fp32)
+    panel_kernel<float, PANEL_THREADS><<<count, PANEL_THREADS, smem, st>>>(t, upper_val, tasks, status, p8max);
   else
-    panel_kernel<double><<<count, PANEL_THREADS, panel_smem<double>(p8max), st>>>(t, upper_val, tasks, status, p8max);
+    panel_kernel<double, PANEL_THREADS><<<count, PANEL_THREADS, smem, st>>>(t, upper_val, tasks, status, p8max);
+}
+
+void launch_inverse(const Tree &t, const InverseTask *tasks, int count, cudaStream_t st) {
+  if (count <= 0) return;
+  configure_kernels();
+  inverse_kernel<<<count, INVERSE_THREADS, INVERSE_SMEM, st>>>(t, tasks);
 }
 
 // A launch of `count` CTAs, as a programmatic dependent of the stream's previous kernel when pdl.

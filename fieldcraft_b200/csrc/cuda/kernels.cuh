@@ -101,17 +101,22 @@ struct AssembleTask {
   int64_t loff, uoff;    // the supernode's L and update-matrix offsets
   int32_t m, w, k0, pad;  // its height and width; its first child's place in the kid lists
 };
-// Panel [c0, c1) of supernode s: factor its diagonal block, invert it, and solve the rows
-// [r0, r1) below it (r0 >= c1; an empty range for a task that only keeps the block). Every task of
-// the panel factors the block itself (no CTA waits on another) and writes its share of the factored
-// block and its inverse (to the diagonal arena at `doff` and to Dinv at `ioff`); part 0 reports the
-// pivots.
+// Panel [c0, c1) of a supernode (height m, panel at loff in the L arena, first column `col` in
+// postorder): factor its diagonal block and solve the rows [r0, r1) below it (r0 >= c1; an empty
+// range for a task that only keeps the block). Every task of the panel factors the block itself (no
+// CTA waits on another) and writes its share of the factored block to the diagonal arena at `doff`;
+// part 0 reports the pivots and, for a panel of at most 8 columns, writes the block's inverse (to
+// the diagonal arena and to Dinv at `ioff`, leading dimension ild).
 struct PanelTask {
-  int32_t s, c0, c1, r0, r1;
-  int32_t keep;  // the panel's CTA count: each stores columns part, part + keep, ... (times 4 warps)
-  int64_t doff;  // of the factored block and its inverse
-  int64_t ioff;  // where the block's inverse goes in Dinv (leading dimension ild)
-  int32_t ild, part;
+  int32_t m, c0, c1, r0, r1;
+  int32_t keep;  // the panel's CTA count: each stores columns part, part + keep, ... (times its warps)
+  int32_t part, ild;
+  int64_t loff, doff, ioff, col;
+};
+// The inverse of a panel's factored block (pw columns, more than 8): both as above.
+struct InverseTask {
+  int64_t doff, ioff;
+  int32_t pw, ild;
 };
 // C(i, j) -= sum_k A(i, k) B(j, k) for i < M, j < N, k < K, strided operands. Flags: 1 touches
 // i >= j only (a diagonal tile of a symmetric matrix); 2 stores C = -sum instead of subtracting;
@@ -278,6 +283,7 @@ void launch_assemble(const Tree &t, bool fp32, const double *upper_val, const As
 // p8max: the widest panel of the launch, rounded up to a multiple of 8 (sizes shared memory).
 void launch_panel(const Tree &t, bool fp32, const double *upper_val, const PanelTask *tasks, int count,
                   DeviceStatus *status, int p8max, cudaStream_t st);
+void launch_inverse(const Tree &t, const InverseTask *tasks, int count, cudaStream_t st);
 // part and counters: the partial sums and counters of split tasks (flag 8), null when there are none.
 void launch_gemm(const GemmTask *tasks, int count, GemmKind kind, cudaStream_t st, double *part = nullptr,
                  int32_t *counters = nullptr);

@@ -252,8 +252,8 @@ int64_t fc_chol_trace_read(fc_chol *h, int64_t *out, int64_t cap);
 /* Per-launch timing with CUDA events on the handle's stream (no reference counterpart: the
  * measurement hook of the benchmark). enable != 0 starts recording; fc_chol_profile_read waits for
  * the stream and returns, per launch kind, the summed milliseconds and the launch count (arrays of
- * `kinds` entries), then clears them. Kinds: 0 front assembly, 1 panel (factor,
- * invert and solve below a diagonal block), 3 GEMM of the factor, 10 and 11 the two GEMMs of a
+ * `kinds` entries), then clears them. Kinds: 0 front assembly, 1 panel (factor a diagonal block and
+ * solve below it), 2 the inverses of the diagonal blocks, 3 GEMM of the factor, 10 and 11 the two GEMMs of a
  * doubling step of the diagonal-block inverses, 12 the tcgen05 GEMM of the mixed-precision factor
  * and 15 the packing of its operands; 16 the LDL^T factor's pivoted panel steps, 17 its W21, 18 its
  * D split and unit lower block inverses;
