@@ -25,6 +25,7 @@
 #include "cuda/kernels.cuh"
 #include "cuda/ldlt_launch.cuh"
 #include "device_buf.hpp"
+#include "host/amalgamate.hpp"
 #include "host/ldlt_fold.hpp"
 #include "host/symbolic.hpp"
 
@@ -82,7 +83,12 @@ struct fc_chol {
   bool own_stream = false;
   int64_t n = 0, ns = 0, entries = 0, nnz = 0, levels = 0;
   double flops = 0;
-  std::vector<int64_t> first, perm, loff, uoff, rows_off, toff, doff;
+  std::vector<int64_t> first, perm, loff, uoff, rows_off, doff;
+  // the reference's own structure, for what a caller sees of it (fc_chol_values, a failed column's
+  // name, the supernodes' count): its supernodes, columns and rows, and each column's place here
+  std::vector<int64_t> ref_first, ref_rptr, ref_perm;
+  std::vector<int32_t> ref_rows, ref_place;
+  int64_t ref_ns = 0;
   std::vector<int64_t> ioff;  // where each supernode's diagonal-block inverses start in Dinv
   int64_t i_len = 0, t_len = 0;
   std::vector<int32_t> width, height, rows;
@@ -97,7 +103,7 @@ struct fc_chol {
   // device
   DeviceBuf d_first, d_width, d_height, d_rows_off, d_rows, d_loff, d_uoff, d_kid_ptr, d_kids, d_rel_off, d_rel;
   DeviceBuf d_kid_meta;
-  DeviceBuf d_a_ptr, d_a_src, d_a_dst, d_diag_src, d_L, d_U, d_D, d_perm, d_val, d_status, d_toff, d_doff;
+  DeviceBuf d_a_ptr, d_a_src, d_a_dst, d_diag_src, d_L, d_U, d_D, d_perm, d_val, d_status, d_doff, d_column;
   DeviceBuf d_a_row, d_a_col, d_scale;   // mixed precision only
   DeviceBuf d_Dinv, d_T;                 // diagonal-block inverses; the doubling's products
   DeviceBuf d_ir_r, d_ir_d, d_ir_sum;    // iterative refinement workspace
@@ -1053,17 +1059,27 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
   return FC_OK;
 }
 
-int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
-  const int64_t ns = sym.ns, n = sym.n;
+// The handle's structure, plans and device memory. merge: on the merged supernodes (host/
+// amalgamate.hpp); the LDL^T factor always keeps the reference's, whose columns bound its pivots.
+int build(fc_chol *h, const fc::Symbolic &ref, bool merge, fc_status *st) {
+  const fc::Amalgamated sym = fc::amalgamate(ref, merge);
+  const int64_t ns = sym.ns, n = ref.n;
   h->n = n;
   h->ns = ns;
-  h->entries = sym.entries;
+  h->entries = ref.entries;
   h->fp32 = h->precision == FC_PRECISION_FP32_IR;
   h->ldlt = h->precision == FC_PRECISION_LDLT;
   h->esize = h->fp32 ? sizeof(float) : sizeof(double);
-  h->nnz = (int64_t)sym.upper_idx.size();
+  h->nnz = (int64_t)ref.upper_idx.size();
   h->first = sym.first;
-  h->perm = sym.perm;
+  h->perm.resize(n);
+  for (int64_t j = 0; j < n; ++j) h->perm[j] = ref.perm[sym.column[j]];
+  h->ref_ns = ref.ns;
+  h->ref_first = ref.first;
+  h->ref_rptr = ref.rptr;
+  h->ref_rows = ref.rows;
+  h->ref_perm = ref.perm;
+  h->ref_place = sym.place;
   h->rows.assign(sym.rows.begin(), sym.rows.end());
   h->rows_off.assign(sym.rptr.begin(), sym.rptr.end() - (ns ? 1 : 0));
   if (ns == 0) h->rows_off.clear();
@@ -1071,11 +1087,12 @@ int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
   h->height.resize(ns);
   h->loff.resize(ns);
   h->uoff.resize(ns);
-  h->toff.resize(ns);
   h->doff.resize(ns);
   h->ioff.resize(ns);
-  int64_t lsum = 0, usum = 0, tsum = 0, dsum = 0, isum = 0;
+  int64_t lsum = 0, usum = 0, dsum = 0, isum = 0;
   double flops = 0;
+  for (int64_t s = 0; s < ref.ns; ++s)
+    for (int64_t c = 0; c < ref.width(s); ++c) flops += (double)(ref.height(s) - c) * (double)(ref.height(s) - c);
   for (int64_t s = 0; s < ns; ++s) {
     const int64_t m = sym.height(s), w = sym.width(s), u = m - w;
     if (m * w > INT32_MAX) {
@@ -1086,10 +1103,8 @@ int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
     h->width[s] = (int32_t)w;
     h->height[s] = (int32_t)m;
     h->loff[s] = lsum;
-    h->toff[s] = tsum;
     lsum += m * w;
     usum += u * u;
-    tsum += fc::trapezoid(m, w);
     h->doff[s] = dsum;
     h->ioff[s] = isum;
     for (int64_t b = 0; b * fc::SB < w; ++b) {
@@ -1100,7 +1115,6 @@ int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
       const int64_t full = w / fc::NB, last = w % fc::NB;
       dsum += 2 * (int64_t)fc::NB * fc::NB * full + 2 * last * last;
     }
-    for (int64_t c = 0; c < w; ++c) flops += (double)(m - c) * (double)(m - c);
   }
   h->l_len = lsum;
   h->u_len = usum;
@@ -1142,12 +1156,15 @@ int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
   for (int64_t s = 0; s < ns; ++s)
     for (int64_t j = sym.first[s]; j < sym.first[s + 1]; ++j) snode[j] = s;
   std::vector<int64_t> a_ptr(n + 1, 0), a_src(h->nnz), a_dst(h->nnz), diag_src(n, -1);
-  for (int64_t e = 0; e < h->nnz; ++e) ++a_ptr[sym.ccol[e] + 1];
+  // an entry's row and column here (a row is an ancestor of its column, so it stays below)
+  auto row_of = [&](int64_t e) { return (int64_t)sym.place[ref.crow[e]]; };
+  auto col_of = [&](int64_t e) { return (int64_t)sym.place[ref.ccol[e]]; };
+  for (int64_t e = 0; e < h->nnz; ++e) ++a_ptr[col_of(e) + 1];
   for (int64_t j = 0; j < n; ++j) a_ptr[j + 1] += a_ptr[j];
   {
     std::vector<int64_t> at(a_ptr.begin(), a_ptr.end() - 1);
     for (int64_t e = 0; e < h->nnz; ++e) {
-      const int64_t r = sym.crow[e], c = sym.ccol[e];
+      const int64_t r = row_of(e), c = col_of(e);
       const int64_t s = snode[c];
       const int32_t *sr = sym.rows.data() + sym.rptr[s];
       const int64_t m = sym.height(s);
@@ -1231,13 +1248,13 @@ int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
   UP(h->d_a_dst, a_dst);
   UP(h->d_diag_src, diag_src);
   UP(h->d_perm, h->perm);
-  UP(h->d_toff, h->toff);
+  UP(h->d_column, sym.column);
   UP(h->d_doff, h->doff);
   if (h->fp32 || h->ldlt) {
     std::vector<int32_t> a_row(h->nnz), a_col(h->nnz);
     for (int64_t q = 0; q < h->nnz; ++q) {
-      a_row[q] = sym.crow[a_src[q]];
-      a_col[q] = sym.ccol[a_src[q]];
+      a_row[q] = (int32_t)row_of(a_src[q]);
+      a_col[q] = (int32_t)col_of(a_src[q]);
     }
     UP(h->d_a_row, a_row);
     UP(h->d_a_col, a_col);
@@ -1274,6 +1291,7 @@ int build(fc_chol *h, const fc::Symbolic &sym, fc_status *st) {
   t.a_dst = h->d_a_dst.as<int64_t>();
   t.diag_src = h->d_diag_src.as<int64_t>();
   t.doff = h->d_doff.as<int64_t>();
+  t.column = h->d_column.as<int32_t>();
   t.a_row = h->d_a_row.as<int32_t>();
   t.a_col = h->d_a_col.as<int32_t>();
   t.scale = h->fp32 ? h->d_scale.as<double>() : nullptr;
@@ -1483,7 +1501,7 @@ int read_status(fc_chol *h, fc_status *st) {
   }
   if (ds.failed_column != ULLONG_MAX) {
     const int64_t col = (int64_t)ds.failed_column;
-    const int64_t orig = col < h->n ? h->perm[col] : col;
+    const int64_t orig = col < h->n ? h->ref_perm[col] : col;
     set_status(st, FC_NOT_POSITIVE_DEFINITE, orig, 0, 0, "the pivot is not positive (relative to the diagonal)");
     return FC_NOT_POSITIVE_DEFINITE;
   }
@@ -1621,13 +1639,14 @@ struct SplitPush {
   }
 };
 
-void solve_tasks(const fc_chol *h, int R, double *x, double *x2, double *v, SolvePlan &p) {
+// split = false: no product is split over K (no partial tiles).
+void solve_tasks(const fc_chol *h, int R, double *x, double *x2, double *v, SolvePlan &p, bool split = true) {
   std::vector<std::vector<int64_t>> lv(h->levels);
   for (int64_t s = 0; s < h->ns; ++s) lv[h->level[s]].push_back(s);
   const std::vector<int64_t> &voff = p.voff;
   std::vector<fc::RowTask> &rows = p.rows;
   std::vector<fc::GemmTask> &gemm = p.gemm;
-  SplitPush sp{p, 2 * prop_sms(h->device), h->solve_cluster};
+  SplitPush sp{p, split ? 2 * prop_sms(h->device) : 0, h->solve_cluster};
   const size_t es = h->esize;
   p.psum = 0, p.scount = 0;
   std::vector<Launch> &fwd = p.fwd, &bwd = p.bwd;
@@ -2528,6 +2547,22 @@ int fc_test_ldlt_fold(int64_t n, int64_t ns, const int64_t *first, const int64_t
   return 0;
 }
 
+// Not part of the public ABI: the merged supernodes (host/amalgamate.cpp) of an analysis, for tests.
+// sizes[2] receives their count and the length of their rows; the arrays (null to size only) are
+// Amalgamated's.
+int fc_test_amalgamate(const fc_symbolic *sym, int merge, int64_t *sizes, int32_t *place, int64_t *first, int64_t *rptr,
+                       int32_t *rows, int64_t *sparent) {
+  const fc::Amalgamated a = fc::amalgamate(sym->s, merge != 0);
+  sizes[0] = a.ns, sizes[1] = (int64_t)a.rows.size();
+  if (!place) return 0;
+  std::copy(a.place.begin(), a.place.end(), place);
+  std::copy(a.first.begin(), a.first.end(), first);
+  std::copy(a.rptr.begin(), a.rptr.end(), rptr);
+  std::copy(a.rows.begin(), a.rows.end(), rows);
+  std::copy(a.sparent.begin(), a.sparent.end(), sparent);
+  return 0;
+}
+
 int fc_symbolic_analyse(int64_t n, const int64_t *ptr, const int32_t *idx, uint64_t max_entries, fc_symbolic **out,
                         fc_status *status) {
   if (!out || n < 0 || (n > 0 && (!ptr || !idx))) {
@@ -2741,35 +2776,34 @@ int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **
   *out = nullptr;
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return cuda_fail(status, e, "cudaSetDevice");
-  fc_chol *h = nullptr;
-  try {
-    h = new fc_chol();
-  } catch (const std::bad_alloc &) {
-    set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "host memory");
-    return FC_OUT_OF_MEMORY;
-  }
-  h->device = device;
-  h->precision = precision;
-  {
-    const char *env = std::getenv("FC_NO_GRAPHS");
-    h->graphs = !(env && env[0] == '1');
-    const char *mma_sync = std::getenv("FC_TF32_MMA_SYNC");
-    h->tc = !(mma_sync && mma_sync[0] == '1');
-    const char *persistent = std::getenv("FC_SOLVE_PERSISTENT");
-    h->dag = persistent && persistent[0] == '1' && precision != FC_PRECISION_LDLT;
-  }
   fc::configure_kernels();
-  if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess) {
-    delete h;
-    return cuda_fail(status, e, "cudaStreamCreate");
-  }
-  h->own_stream = true;
-  int rc;
-  try {
-    rc = build(h, sym->s, status);
-  } catch (const std::bad_alloc &) {
-    rc = FC_OUT_OF_MEMORY;
-    set_status(status, rc, -1, sym->s.entries, 0, "host memory for the plan");
+  fc_chol *h = nullptr;
+  auto make = [&](bool merge) -> int {
+    try {
+      h = new fc_chol();
+      h->device = device;
+      h->precision = precision;
+      const char *env = std::getenv("FC_NO_GRAPHS");
+      h->graphs = !(env && env[0] == '1');
+      const char *mma_sync = std::getenv("FC_TF32_MMA_SYNC");
+      h->tc = !(mma_sync && mma_sync[0] == '1');
+      const char *persistent = std::getenv("FC_SOLVE_PERSISTENT");
+      h->dag = persistent && persistent[0] == '1' && precision != FC_PRECISION_LDLT;
+      if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
+        return cuda_fail(status, e, "cudaStreamCreate");
+      h->own_stream = true;
+      return build(h, sym->s, merge, status);
+    } catch (const std::bad_alloc &) {
+      set_status(status, FC_OUT_OF_MEMORY, -1, sym->s.entries, 0, "host memory for the plan");
+      return FC_OUT_OF_MEMORY;
+    }
+  };
+  int rc = make(precision != FC_PRECISION_LDLT);
+  if (rc == FC_OUT_OF_MEMORY && precision != FC_PRECISION_LDLT) {
+    // the merged supernodes' arenas hold a little more: try the reference's own
+    fc_chol_destroy(h);
+    h = nullptr;
+    rc = make(false);
   }
   if (rc != FC_OK) {
     fc_chol_destroy(h);
@@ -3011,20 +3045,31 @@ int fc_chol_solve_device_noalloc(fc_chol *h, double *d_b, int32_t nrhs, int64_t 
     return FC_INVALID_ARGUMENT;
   };
   if (at_voff > FC_NOALLOC_SCRATCH_BYTES) return too_large(at_voff);
-  solve_tasks(h, R, reinterpret_cast<double *>(base + at_x), reinterpret_cast<double *>(base + at_x2),
-              reinterpret_cast<double *>(base + at_v), p);
-  const size_t at_rows = at_voff + align256(sizeof(int64_t) * p.voff.size());
-  const size_t at_ranges = at_rows + align256(sizeof(fc::RowTask) * p.rows.size());
-  const size_t at_panels = at_ranges + align256(sizeof(int2) * p.ranges.size());
-  const size_t at_gemm = at_panels + align256(sizeof(fc::SolveTask) * p.panels.size());
-  const size_t at_part = at_gemm + align256(sizeof(fc::GemmTask) * p.gemm.size());
-  const size_t at_thin = at_part + align256(sizeof(double) * (size_t)p.psum);
-  const size_t at_tranges = at_thin + align256(sizeof(fc::ThinTask) * p.thin.size());
-  const size_t at_tbwd = at_tranges + align256(sizeof(int4) * p.tranges.size());
-  const size_t at_tpart = at_tbwd + align256(sizeof(fc::ThinBwdTask) * p.tbwd.size());
-  const size_t at_tcount = at_tpart + align256(sizeof(double) * (size_t)p.tpart);
-  const size_t counters = (size_t)std::max<int64_t>(p.tcount + p.scount, 1);
-  const size_t need = at_tcount + sizeof(int32_t) * counters;
+  size_t at_rows, at_ranges, at_panels, at_gemm, at_part, at_thin, at_tranges, at_tbwd, at_tpart, at_tcount, counters,
+      need;
+  auto lay_out = [&](bool split) {
+    solve_tasks(h, R, reinterpret_cast<double *>(base + at_x), reinterpret_cast<double *>(base + at_x2),
+                reinterpret_cast<double *>(base + at_v), p, split);
+    at_rows = at_voff + align256(sizeof(int64_t) * p.voff.size());
+    at_ranges = at_rows + align256(sizeof(fc::RowTask) * p.rows.size());
+    at_panels = at_ranges + align256(sizeof(int2) * p.ranges.size());
+    at_gemm = at_panels + align256(sizeof(fc::SolveTask) * p.panels.size());
+    at_part = at_gemm + align256(sizeof(fc::GemmTask) * p.gemm.size());
+    at_thin = at_part + align256(sizeof(double) * (size_t)p.psum);
+    at_tranges = at_thin + align256(sizeof(fc::ThinTask) * p.thin.size());
+    at_tbwd = at_tranges + align256(sizeof(int4) * p.tranges.size());
+    at_tpart = at_tbwd + align256(sizeof(fc::ThinBwdTask) * p.tbwd.size());
+    at_tcount = at_tpart + align256(sizeof(double) * (size_t)p.tpart);
+    counters = (size_t)std::max<int64_t>(p.tcount + p.scount, 1);
+    need = at_tcount + sizeof(int32_t) * counters;
+  };
+  lay_out(true);
+  if (need > FC_NOALLOC_SCRATCH_BYTES) {
+    // without the split products' partial tiles (32 KB a chunk, whatever R is)
+    p = SolvePlan();
+    solve_offsets(h, R, p);
+    lay_out(false);
+  }
   if (need > FC_NOALLOC_SCRATCH_BYTES) return too_large(need);
   // Every region is written before it is read in this call: the task lists and offsets here, x by
   // the permutation, x2 by the forward panels, each update vector's rows zeroed by its assembly
@@ -3308,8 +3353,28 @@ int fc_chol_values(fc_chol *h, double *dst, fc_status *status) {
     set_status(status, FC_OUT_OF_MEMORY, -1, h->entries, 0, "device memory for the copy");
     return FC_OUT_OF_MEMORY;
   }
-  fc::launch_pack_trapezoids(h->tree, h->fp32, h->ns, h->d_toff.as<int64_t>(), tmp.as<double>(), h->stream);
-  cudaError_t e = cudaMemcpyAsync(dst, tmp.p, sizeof(double) * h->entries, cudaMemcpyDeviceToHost, h->stream);
+  // the reference's supernodes in their own layout, each column looked up in the supernode here that
+  // holds it
+  DeviceBuf d_first, d_rptr, d_rows, d_place, d_toff, d_snode;
+  std::vector<int64_t> toff(h->ref_ns);
+  std::vector<int32_t> snode(h->n);
+  for (int64_t s = 0, at = 0; s < h->ref_ns; ++s) {
+    toff[s] = at;
+    at += fc::trapezoid(h->ref_rptr[s + 1] - h->ref_rptr[s], h->ref_first[s + 1] - h->ref_first[s]);
+  }
+  for (int64_t s = 0; s < h->ns; ++s)
+    for (int64_t j = h->first[s]; j < h->first[s + 1]; ++j) snode[j] = (int32_t)s;
+  cudaError_t e = cudaSuccess;
+  if ((e = upload(d_first, h->ref_first, h->stream)) != cudaSuccess || (e = upload(d_rptr, h->ref_rptr, h->stream)) != cudaSuccess ||
+      (e = upload(d_rows, h->ref_rows, h->stream)) != cudaSuccess || (e = upload(d_place, h->ref_place, h->stream)) != cudaSuccess ||
+      (e = upload(d_toff, toff, h->stream)) != cudaSuccess || (e = upload(d_snode, snode, h->stream)) != cudaSuccess) {
+    set_status(status, FC_OUT_OF_MEMORY, -1, h->entries, 0, "device memory for the copy");
+    return FC_OUT_OF_MEMORY;
+  }
+  const fc::ReferenceLayout layout{h->ref_ns, d_first.as<int64_t>(), d_rptr.as<int64_t>(), d_rows.as<int32_t>(),
+                                   d_place.as<int32_t>(), d_toff.as<int64_t>(), d_snode.as<int32_t>()};
+  fc::launch_pack_trapezoids(h->tree, h->fp32, layout, tmp.as<double>(), h->stream);
+  e = cudaMemcpyAsync(dst, tmp.p, sizeof(double) * h->entries, cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return cuda_fail(status, e, "values");
   set_status(status, FC_OK);
@@ -3370,7 +3435,7 @@ int64_t fc_chol_stat(const fc_chol *h, int what) {
     case 1: return (int64_t)h->program.size();
     case 2: return h->l_len * 8;
     case 3: return h->u_len * 8;
-    case 4: return h->ns;
+    case 4: return h->ref_ns;
     case 5: return (int64_t)h->flops;
     case 6: return h->gemm_tasks;
     case 7: return h->last_factor_launches;

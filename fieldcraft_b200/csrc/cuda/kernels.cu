@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
     __syncthreads();
   }
   if (tid == 0 && task.part == 0 && fail < pw)
-    atomicMin(&status->failed_column, (unsigned long long)(task.col + fail));
+    atomicMin(&status->failed_column, (unsigned long long)t.column[task.col + fail]);
 }
 
 // The inverse of a panel's factored block (more than 8 columns), from the diagonal arena: its 8 x 8
@@ -1621,22 +1621,34 @@ __global__ void __launch_bounds__(256) sumsq_kernel(int64_t n, int64_t ld, const
   if (threadIdx.x == 0) out[blockIdx.x] = part[0];
 }
 
-// The factor in the reference's packed trapezoids; an FP32 factor of S A S is brought back to A's
-// (L(A) = S^-1 L(S A S), row by row).
+// The factor in the reference's packed trapezoids, a reference supernode a CTA: a column's rows are
+// looked up among the rows of the supernode here that holds it (a merged one holds more, explicit
+// zeros besides). An FP32 factor of S A S is brought back to A's (L(A) = S^-1 L(S A S), row by row).
 template <class T>
-__global__ void pack_kernel(Tree t, const int64_t *__restrict__ toff, double *__restrict__ dst) {
-  const int s = blockIdx.x;
-  const int64_t m = t.height[s], w = t.width[s];
-  const T *Ls = static_cast<const T *>(t.L) + t.loff[s];
-  const int32_t *rows = t.rows + t.rows_off[s];
-  double *d = dst + toff[s];
+__global__ void pack_kernel(Tree t, ReferenceLayout ref, double *__restrict__ dst) {
+  const int64_t s = blockIdx.x, f = ref.first[s], w = ref.first[s + 1] - f, m = ref.rptr[s + 1] - ref.rptr[s];
+  const int32_t *rows = ref.rows + ref.rptr[s];
+  double *d = dst + ref.toff[s];
   for (int64_t c = 0; c < w; ++c) {
     const int64_t start = c * m - c * (c > 0 ? c - 1 : 0) / 2;
-    const int64_t p = c / NB, c0 = p * NB, c1 = c0 + NB < w ? c0 + NB : w, pw = c1 - c0;
-    const double *Dp = t.D + t.doff[s] + 2 * (int64_t)NB * NB * p;
+    const int64_t j = ref.place[f + c], g = ref.snode[j], gm = t.height[g], gw = t.width[g], gc = j - t.first[g];
+    const T *Ls = static_cast<const T *>(t.L) + t.loff[g];
+    const int32_t *grows = t.rows + t.rows_off[g];
+    const int64_t p = gc / NB, c0 = p * NB, c1 = c0 + NB < gw ? c0 + NB : gw, pw = c1 - c0;
+    const double *Dp = t.D + t.doff[g] + 2 * (int64_t)NB * NB * p;
     for (int64_t r = c + threadIdx.x; r < m; r += blockDim.x) {
-      const double v = r < c1 ? Dp[(c - c0) * pw + (r - c0)] : (double)Ls[r + c * m];
-      d[start + r - c] = t.scale ? v / t.scale[rows[r]] : v;
+      const int32_t row = ref.place[rows[r]];
+      int64_t lo = gc, hi = gm;  // the first row at or past `row`
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) / 2;
+        if (grows[mid] < row)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      if (lo >= gm || grows[lo] != row) continue;  // every row of the reference's is there
+      const double v = lo < c1 ? Dp[(gc - c0) * pw + (lo - c0)] : (double)Ls[lo + gc * gm];
+      d[start + r - c] = t.scale ? v / t.scale[row] : v;
     }
   }
 }
@@ -1896,12 +1908,12 @@ void launch_sumsq(int64_t n, int R, int64_t ld, const double *v, double *out, cu
   if (R > 0) sumsq_kernel<<<R, 256, 0, st>>>(n, ld, v, out);
 }
 
-void launch_pack_trapezoids(const Tree &t, bool fp32, int64_t ns, const int64_t *toff, double *dst, cudaStream_t st) {
-  if (ns <= 0) return;
+void launch_pack_trapezoids(const Tree &t, bool fp32, const ReferenceLayout &ref, double *dst, cudaStream_t st) {
+  if (ref.ns <= 0) return;
   if (fp32)
-    pack_kernel<float><<<(unsigned)ns, 128, 0, st>>>(t, toff, dst);
+    pack_kernel<float><<<(unsigned)ref.ns, 128, 0, st>>>(t, ref, dst);
   else
-    pack_kernel<double><<<(unsigned)ns, 128, 0, st>>>(t, toff, dst);
+    pack_kernel<double><<<(unsigned)ref.ns, 128, 0, st>>>(t, ref, dst);
 }
 
 }  // namespace fc

@@ -77,6 +77,7 @@ struct Tree {
   const int64_t *diag_src;  // [n] upper-entry index of A(j, j), -1 if absent
   const int64_t *doff;      // [ns] diagonal arena: panel p of s keeps its factored block and its
                             // inverse (pw x pw each, column-major) at doff[s] + 2 NB NB p
+  const int32_t *column;    // [n] the reference's postordered column of each (names a failed pivot)
   const int32_t *a_row;     // mixed precision: each input entry's postordered row and column
   const int32_t *a_col;
   const double *scale;      // mixed precision: S = diag(A)^-1/2 (postorder); null in FP64
@@ -338,7 +339,16 @@ constexpr int SPMV_ROWS_MIN_R = 4;
 void launch_spmv(int64_t n, const int64_t *ptr, const int32_t *idx, const double *val, const double *x, int64_t ldx,
                  double *y, int64_t ldy, int R, cudaStream_t st, double *scratch = nullptr);
 // Copies the L panels out into the reference's packed trapezoids (dst offsets per supernode).
-void launch_pack_trapezoids(const Tree &t, bool fp32, int64_t ns, const int64_t *toff, double *dst,
-                            cudaStream_t st);
+// The reference's layout of the factor: its supernodes' columns and rows (postordered), place[j] the
+// column here of postordered column j, toff where each supernode's packed trapezoid starts, and
+// snode[] the supernode here of each column here.
+struct ReferenceLayout {
+  int64_t ns;
+  const int64_t *first, *rptr;
+  const int32_t *rows, *place;
+  const int64_t *toff;
+  const int32_t *snode;
+};
+void launch_pack_trapezoids(const Tree &t, bool fp32, const ReferenceLayout &ref, double *dst, cudaStream_t st);
 
 }  // namespace fc
