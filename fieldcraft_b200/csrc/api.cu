@@ -25,6 +25,7 @@
 #include "cuda/kernels.cuh"
 #include "cuda/ldlt_launch.cuh"
 #include "device_buf.hpp"
+#include "scratch.hpp"
 #include "host/amalgamate.hpp"
 #include "host/ldlt_fold.hpp"
 #include "host/symbolic.hpp"
@@ -81,6 +82,7 @@ struct fc_chol {
   size_t esize = 8;    // bytes of an entry of L / U
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  std::unique_ptr<fc::host::ScratchUser> scratch_user;
   int64_t n = 0, ns = 0, entries = 0, nnz = 0, levels = 0;
   double flops = 0;
   std::vector<int64_t> first, perm, loff, uoff, rows_off, doff;
@@ -2783,6 +2785,7 @@ int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **
       h = new fc_chol();
       h->device = device;
       h->precision = precision;
+      h->scratch_user = std::make_unique<fc::host::ScratchUser>(device);
       const char *env = std::getenv("FC_NO_GRAPHS");
       h->graphs = !(env && env[0] == '1');
       const char *mma_sync = std::getenv("FC_TF32_MMA_SYNC");
@@ -3138,7 +3141,7 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
   const size_t block = sizeof(double) * (size_t)n * R;
   const bool pcg = h->refine_pcg;
   auto need = [&](DeviceBuf &b, size_t bytes) { return b.bytes >= bytes || b.alloc(bytes) == cudaSuccess; };
-  if (!need(h->d_ir_r, block) || !need(h->d_ir_d, block) || !need(h->d_ir_sum, 6 * sizeof(double) * R) ||
+  if (!need(h->d_ir_r, block) || !need(h->d_ir_d, block) || !need(h->d_ir_sum, (6 + fc::COLUMN_PARTS) * sizeof(double) * R) ||
       !need(h->d_ir_sc, 2 * block) ||
       (pcg && (!need(h->d_ir_p, block) || !need(h->d_ir_q, block) || !need(h->d_ir_t, block) ||
                !need(h->d_ir_done, sizeof(int) * R)))) {
@@ -3147,7 +3150,9 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
   }
   cudaStream_t st = h->stream;
   double *r = h->d_ir_r.as<double>(), *z = h->d_ir_d.as<double>(), *sums = h->d_ir_sum.as<double>();
-  // sums: [0, R) residual norms^2, [R, 2R) ||b||^2, [2R, 3R) r.z, [3R, 4R) r.z new, [4R, 5R) p.q
+  // sums: [0, R) residual norms^2, [R, 2R) ||b||^2, [2R, 3R) r.z, [3R, 4R) r.z new, [4R, 5R) p.q, from
+  // 6R the column sums' partials
+  double *parts = sums + 6 * R;
   std::vector<double> host(2 * R), rel(R, 0.0);
   std::vector<int> done(R, 0);
   cudaError_t e = cudaSuccess;
@@ -3158,7 +3163,7 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
       e = cudaMemcpyAsync(r + (int64_t)j * n, d_b + (int64_t)j * ld, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
   }
   if (e != cudaSuccess) return cuda_fail(status, e, "refinement set-up");
-  fc::launch_sumsq(n, R, n, r, sums + R, st);
+  fc::launch_coldot(n, R, r, n, r, n, sums + R, parts, st);
   e = cudaMemcpyAsync(host.data() + R, sums + R, sizeof(double) * R, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(status, e, "refinement set-up");
@@ -3166,7 +3171,7 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
   auto check = [&](double *t) -> int {
     fc::launch_spmv(n, d_ptr, d_idx, d_val, d_x, ld, t, n, R, st, h->d_ir_sc.as<double>());
     fc::launch_residual(n, R, d_b, ld, t, n, st);
-    fc::launch_sumsq(n, R, n, t, sums, st);
+    fc::launch_coldot(n, R, t, n, t, n, sums, parts, st);
     cudaError_t e2 = cudaMemcpyAsync(host.data(), sums, 2 * sizeof(double) * R, cudaMemcpyDeviceToHost, st);
     if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(st);
     if (e2 == cudaSuccess) e2 = cudaGetLastError();
@@ -3210,12 +3215,12 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
     if ((rc = enqueue_solve(h, z, R, n, status)) != FC_OK) return rc;
     ++it;
     cudaMemcpyAsync(p, z, block, cudaMemcpyDeviceToDevice, st);
-    fc::launch_coldot(n, R, r, n, z, n, rz, st);
+    fc::launch_coldot(n, R, r, n, z, n, rz, parts, st);
     cudaMemsetAsync(d_done, 0, sizeof(int) * R, st);
     // the recurrence's residual r (one norm per column, read each iteration) says when to look
     // at the true residual; only the true residual decides convergence and which columns stop
     auto recurrence_small = [&]() -> int {
-      fc::launch_sumsq(n, R, n, r, sums, st);
+      fc::launch_coldot(n, R, r, n, r, n, sums, parts, st);
       cudaError_t e2 = cudaMemcpyAsync(host.data(), sums, sizeof(double) * R, cudaMemcpyDeviceToHost, st);
       if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(st);
       if (e2 == cudaSuccess) e2 = cudaGetLastError();
@@ -3231,7 +3236,7 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
     };
     for (;;) {
       fc::launch_spmv(n, d_ptr, d_idx, d_val, p, n, q, n, R, st, h->d_ir_sc.as<double>());
-      fc::launch_coldot(n, R, p, n, q, n, pq, st);
+      fc::launch_coldot(n, R, p, n, q, n, pq, parts, st);
       fc::launch_pcg_step(n, R, rz, pq, d_done, p, q, d_x, ld, r, st);
       rc = recurrence_small();
       if (rc == -1) rc = check(t);
@@ -3246,7 +3251,7 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
       if (e != cudaSuccess) return cuda_fail(status, e, "refinement");
       if ((rc = enqueue_solve(h, z, R, n, status)) != FC_OK) return rc;
       ++it;
-      fc::launch_coldot(n, R, r, n, z, n, rz_new, st);
+      fc::launch_coldot(n, R, r, n, z, n, rz_new, parts, st);
       fc::launch_pcg_direction(n, R, rz_new, rz, z, p, st);
       std::swap(rz, rz_new);
     }
@@ -3505,14 +3510,12 @@ int fc_csr_spmv_device(int64_t n, const int64_t *d_ptr, const int32_t *d_idx, co
   if (n < 0 || nrhs < 0 || (n > 0 && (!d_ptr || !d_idx || !d_val || !d_x || !d_y || ld < n))) return FC_INVALID_ARGUMENT;
   const cudaStream_t st = (cudaStream_t)stream;
   // several right-hand sides: through row-major copies in stream-ordered scratch (freed in order)
-  double *scratch = nullptr;
-  if (n > 0 && nrhs >= fc::SPMV_ROWS_MIN_R &&
-      cudaMallocAsync(reinterpret_cast<void **>(&scratch), sizeof(double) * 2 * (size_t)n * nrhs, st) != cudaSuccess) {
-    cudaGetLastError();
-    scratch = nullptr;
+  if (n > 0 && nrhs >= fc::SPMV_ROWS_MIN_R) {
+    fc::host::Scratch scratch(sizeof(double) * 2 * (size_t)n * nrhs, st);
+    fc::launch_spmv(n, d_ptr, d_idx, d_val, d_x, ld, d_y, ld, nrhs, st, static_cast<double *>(scratch.p));
+  } else {
+    fc::launch_spmv(n, d_ptr, d_idx, d_val, d_x, ld, d_y, ld, nrhs, st, nullptr);
   }
-  fc::launch_spmv(n, d_ptr, d_idx, d_val, d_x, ld, d_y, ld, nrhs, st, scratch);
-  if (scratch) cudaFreeAsync(scratch, st);
   return cudaGetLastError() == cudaSuccess ? FC_OK : FC_CUDA_ERROR;
 }
 

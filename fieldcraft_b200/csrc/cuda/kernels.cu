@@ -1562,21 +1562,34 @@ __global__ void update_kernel(int64_t n, int R, const double *__restrict__ d, in
 }
 
 // Preconditioned CG on column-major n x R blocks, one independent recurrence per column, every
-// scalar on the device: out[j] = sum_i a(i, j) b(i, j) (one CTA a column, a fixed tree order).
+// scalar on the device: out[j] = sum_i a(i, j) b(i, j), by COLUMN_PARTS ranges of rows a column and
+// then their sums, both by a fixed tree. (One CTA a column took 147 us for 16 columns of 155 000
+// rows, 40 MB at a quarter of a TB/s.)
+__device__ __forceinline__ double tree_sum(double s) {
+  __shared__ double part[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  double sum = 0.0;
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) sum += part[w];
+  return sum;
+}
 __global__ void __launch_bounds__(256) coldot_kernel(int64_t n, const double *__restrict__ a, int64_t lda,
                                                      const double *__restrict__ b, int64_t ldb,
-                                                     double *__restrict__ out) {
-  __shared__ double part[256];
-  const double *ca = a + blockIdx.x * lda, *cb = b + blockIdx.x * ldb;
+                                                     double *__restrict__ parts) {
+  const int64_t j = blockIdx.x / COLUMN_PARTS, p = blockIdx.x % COLUMN_PARTS;
+  const double *ca = a + j * lda, *cb = b + j * ldb;
+  const int64_t per = (n + COLUMN_PARTS - 1) / COLUMN_PARTS, i1 = min(n, (p + 1) * per);
   double s = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += ca[i] * cb[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) part[threadIdx.x] += part[threadIdx.x + h];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = part[0];
+#pragma unroll 4
+  for (int64_t i = p * per + threadIdx.x; i < i1; i += blockDim.x) s += ca[i] * cb[i];
+  s = tree_sum(s);
+  if (threadIdx.x == 0) parts[blockIdx.x] = s;
+}
+__global__ void __launch_bounds__(COLUMN_PARTS) colsum_kernel(const double *__restrict__ parts, double *__restrict__ out) {
+  const double s = tree_sum(parts[(int64_t)blockIdx.x * COLUMN_PARTS + threadIdx.x]);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 // alpha_j = rz[j] / pq[j]; x_j += alpha_j p_j; r_j -= alpha_j q_j (columns with done[j] set keep x, r).
@@ -1603,22 +1616,6 @@ __global__ void pcg_direction_kernel(int64_t n, int R, const double *__restrict_
     const double beta = rz_old[j] != 0.0 ? rz_new[j] / rz_old[j] : 0.0;
     p[e] = z[e] + beta * p[e];
   }
-}
-
-// out[j] = sum_i v(i, j)^2 for each column j (one CTA a column, a fixed tree order).
-__global__ void __launch_bounds__(256) sumsq_kernel(int64_t n, int64_t ld, const double *__restrict__ v,
-                                                    double *__restrict__ out) {
-  __shared__ double part[256];
-  const double *col = v + blockIdx.x * ld;
-  double s = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += col[i] * col[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) part[threadIdx.x] += part[threadIdx.x + h];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = part[0];
 }
 
 // The factor in the reference's packed trapezoids, a reference supernode a CTA: a column's rows are
@@ -1883,9 +1880,10 @@ void launch_update(int64_t n, int R, const double *d, int64_t ldd, double *x, in
 }
 
 void launch_coldot(int64_t n, int R, const double *a, int64_t lda, const double *b, int64_t ldb, double *out,
-                   cudaStream_t st) {
+                   double *parts, cudaStream_t st) {
   if (n <= 0 || R <= 0) return;
-  coldot_kernel<<<R, 256, 0, st>>>(n, a, lda, b, ldb, out);
+  coldot_kernel<<<(unsigned)R * COLUMN_PARTS, 256, 0, st>>>(n, a, lda, b, ldb, parts);
+  colsum_kernel<<<R, COLUMN_PARTS, 0, st>>>(parts, out);
 }
 
 void launch_pcg_step(int64_t n, int R, const double *rz, const double *pq, const int *done, const double *p,
@@ -1902,10 +1900,6 @@ void launch_pcg_direction(int64_t n, int R, const double *rz_new, const double *
   if (total <= 0) return;
   pcg_direction_kernel<<<(int)std::min<int64_t>((total + 255) / 256, 148 * 16), 256, 0, st>>>(n, R, rz_new, rz_old, z,
                                                                                               p);
-}
-
-void launch_sumsq(int64_t n, int R, int64_t ld, const double *v, double *out, cudaStream_t st) {
-  if (R > 0) sumsq_kernel<<<R, 256, 0, st>>>(n, ld, v, out);
 }
 
 void launch_pack_trapezoids(const Tree &t, bool fp32, const ReferenceLayout &ref, double *dst, cudaStream_t st) {

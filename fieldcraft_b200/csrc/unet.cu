@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <random>
 #include <string>
@@ -13,6 +14,7 @@
 #include "cuda/kernels.cuh"
 #include "cuda/unet_kernels.cuh"
 #include "device_buf.hpp"
+#include "scratch.hpp"
 
 using fc::host::DeviceBuf;
 using fc::host::set_status;
@@ -164,6 +166,7 @@ struct fc_unet {
   fc::unet::LayerTable table{};
   int64_t last_net_iterations = 0, last_dropped = 0;
   bool weights_stale = true;
+  std::unique_ptr<fc::host::ScratchUser> scratch_user;
   std::mutex lock;
 };
 
@@ -439,6 +442,7 @@ int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const i
   if (e != cudaSuccess) return cuda_fail(status, e, "device");
   fc_unet *u = new fc_unet();
   u->device = device;
+  u->scratch_user = std::make_unique<fc::host::ScratchUser>(device);
   u->n = n;
   u->kref = kref;
   u->levels = levels;
@@ -689,27 +693,26 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     return FC_OUT_OF_MEMORY;
   }
   // vectors: r, z, q and the ring of `keep` directions p_j and A p_j
-  DeviceBuf vec, sc, part;
   const int ring = keep;
-  if (vec.alloc(sizeof(double) * (size_t)n * (3 + 2 * ring)) != cudaSuccess ||
-      sc.alloc(sizeof(double) * 64) != cudaSuccess ||
-      part.alloc(sizeof(double) * (1 + fc::unet::MAX_KEPT) * fc::unet::FCG_CTAS) != cudaSuccess) {
+  constexpr size_t SCALARS = 64, PARTS = (1 + fc::unet::MAX_KEPT) * fc::unet::FCG_CTAS;
+  fc::host::Scratch scratch(sizeof(double) * (SCALARS + PARTS + (size_t)n * (3 + 2 * ring)), st);
+  if (!scratch.p) {
     set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for FCG");
     return FC_OUT_OF_MEMORY;
   }
-  double *r = vec.as<double>(), *z = r + n, *tmp = z + n;
+  double *const s = static_cast<double *>(scratch.p), *const part = s + SCALARS;
+  double *r = part + PARTS, *z = r + n, *tmp = z + n;
   std::vector<double *> P(ring), Q(ring);
   for (int j = 0; j < ring; ++j) P[j] = tmp + n * (1 + 2 * j), Q[j] = P[j] + n;
   // [0] b.b [1] r.r [2] p.r [3] p.q [5] b - A x squared [6] a start's r.r [8..8+ring) z.q_j [16..16+ring) p_j.q_j
   // [32..32+CHECK) the last iterations' r.r [48] the sums' ticket
-  double *s = sc.as<double>();
   int *ticket = reinterpret_cast<int *>(s + 48);
   cudaMemsetAsync(ticket, 0, sizeof(double), st);
   cudaMemsetAsync(d_x, 0, sizeof(double) * n, st);
   copy_kernel<<<blocks(n), 256, 0, st>>>(n, d_b, r);
   {
     const double *a[1] = {d_b}, *b[1] = {d_b};
-    fc::unet::dots(n, 1, a, b, part.as<double>(), s + 0, st);
+    fc::unet::dots(n, 1, a, b, part, s + 0, st);
   }
   double bb = 0.0, rr = 0.0;
   cudaMemcpyAsync(&bb, s, sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -749,7 +752,7 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     fc::unet::FcgStep a{};
     a.n = n, a.update = update ? 1 : 0, a.alpha = s + 2, a.x = d_x, a.r = r, a.rr = rr_at, a.zq = s + 8;
     if (update) a.p = P[(at - 1) % ring], a.q = Q[(at - 1) % ring];
-    a.part = part.as<double>(), a.ticket = ticket;
+    a.part = part, a.ticket = ticket;
     int slot[fc::unet::MAX_KEPT];
     if (!use_net) {
       a.z = z, a.inv = jacobi ? net->bj.as<double>() : nullptr;
@@ -767,14 +770,14 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     for (int j = 0; j < m; ++j) pj[j] = P[slot[j]], qj[j] = Q[slot[j]], zz[j] = z;
     if (use_net) {
       apply(net, 1, r, n, z, together);
-      if (m > 0) fc::unet::dots(n, m, zz, qj, part.as<double>(), s + 8, st);
+      if (m > 0) fc::unet::dots(n, m, zz, qj, part, s + 8, st);
     } else if (!have_z) {
       step(false, it, m, s + 6);
     }
     // p = z - sum_j (z.q_j / p_j.q_j) p_j over the stored directions (the denominators were kept
     // in s + 16 + slot when each direction was made); q = A p, p.r, p.q
     fc::unet::fcg_direction(n, m, z, pj, slot, s + 8, s + 16, p, st);
-    fc::unet::fcg_product(n, d_ptr, d_idx, d_val, p, r, q, s + 2, s + 16 + (it % ring), part.as<double>(), ticket, st);
+    fc::unet::fcg_product(n, d_ptr, d_idx, d_val, p, r, q, s + 2, s + 16 + (it % ring), part, ticket, st);
     // alpha = p.r / p.q, x += alpha p, r -= alpha q, and the next iteration's z
     step(true, it + 1, std::min(stored + 1, ring), s + 32 + (it % CHECK));
     have_z = !use_net;
@@ -819,7 +822,7 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
       fc::launch_spmv(n, d_ptr, d_idx, d_val, d_x, n, tmp, n, 1, st);
       residual_from_kernel<<<blocks(n), 256, 0, st>>>(n, d_b, tmp);
       const double *a[1] = {tmp}, *b2[1] = {tmp};
-      fc::unet::dots(n, 1, a, b2, part.as<double>(), s + 5, st);
+      fc::unet::dots(n, 1, a, b2, part, s + 5, st);
       double tr = 0.0;
       cudaMemcpyAsync(&tr, s + 5, sizeof(double), cudaMemcpyDeviceToHost, st);
       e = cudaStreamSynchronize(st);
@@ -839,7 +842,7 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     fc::launch_spmv(n, d_ptr, d_idx, d_val, d_x, n, r, n, 1, st);
     residual_inplace_kernel<<<blocks(n), 256, 0, st>>>(n, d_b, r);
     const double *a[1] = {r}, *b[1] = {r};
-    fc::unet::dots(n, 1, a, b, part.as<double>(), s + 1, st);
+    fc::unet::dots(n, 1, a, b, part, s + 1, st);
     cudaMemcpyAsync(&rr, s + 1, sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
     return bb > 0.0 ? std::sqrt(rr / bb) : std::sqrt(rr);
