@@ -201,47 +201,52 @@ __global__ void scale_kernel(int64_t n, const int64_t *__restrict__ diag_src, co
 // panel, factored in FP64 right-looking by strips of 8 columns. Warp 0 carries the chain: it brings
 // the next strip's rows of the block up to date with the strip before (two rows a lane, from shared
 // memory), factors it (pivots and multipliers broadcast by shuffles) and goes on. The other warps
-// follow a strip behind: they solve the strip's columns of the rows below (a row a thread, forward
-// substitution with the 8 x 8 triangle) and store them, and apply the strip to the columns past the
-// next one, of the block (8 x 8 DMMA tiles) and of the rows below (16 x 8). So the rows below end
-// with the block, one barrier a strip, and nothing waits for the block's inverse, which only the
-// solve reads (inverse_kernel, beside the following launches). Bound by the chain of dependent FP64
-// steps. Before, with the inverse formed here and the rows multiplied by it, a 64-column panel of
-// 128 rows took 42 us (16 of them the block, 7.5 the inverse, 9.5 the rows); the panels of a box of
-// 23 x 17 x 19 elements took 31.6 us on average, now 22.
+// follow a strip behind: eight of them take 16 of the rows below each, solve the strip's columns of
+// them (a row a lane, forward substitution with the 8 x 8 triangle), store them and bring their later
+// columns up to date (16 x 8 DMMA tiles), with no barrier between; three apply the strip to the
+// block's columns past the next strip (8 x 8 tiles). So the rows below end with the block, one
+// barrier a strip, and nothing waits for the block's inverse, which only the solve reads
+// (inverse_kernel, beside the following launches). Bound by the chain of dependent FP64 steps, some
+// 35 cycles each: the warps that share warp 0's scheduler are the ones with the short tiles, and the
+// matrix's own diagonal, which the pivot test needs, is loaded while the first strip is factored.
+// With the inverse formed here and the rows multiplied by it, a 64-column panel of 128 rows took 42
+// us; with the rows' solve and update a barrier apart over seven warps and a longer root 23, of which
+// 4 were the loads, 1.6 a strip's factors and 2 to 5 the first strips' rows; now about 19.
 // The pivot test is the reference's (cholesky.rs:1162-1165): not (d > PIVOT_TOLERANCE |A_jj|) or not
 // finite fails, and the smallest failing column (postorder) is kept in the status word. A failed
 // pivot makes NaNs and nothing else: no index depends on a value. L may be stored in FP32 (widened
-// on load, rounded on store); the diagonal arena stays FP64. A panel at most 8 columns wide (most
-// supernodes) is inverted here as well, by warp 0 while the rows below end.
-constexpr int PANEL_THREADS = 256, PANEL_THREADS_NARROW = 128;
+// on load, rounded on store); the diagonal arena stays FP64. A panel at most 8 columns wide is
+// inverted here as well, by warp 0 while the rows below end.
+constexpr int PANEL_THREADS = 384, PANEL_THREADS_NARROW = 128;
 constexpr int PANEL_ALD = 68, PANEL_BLD = PANEL_ROWS + 4;  // a warp's fragment reads fall in distinct banks
 // Shared memory of a panel launch whose widest panel is padded to p8 columns (a multiple of 8).
 __host__ __device__ constexpr size_t panel_smem(int p8) {
   return sizeof(double) * ((size_t)p8 * (PANEL_ALD + PANEL_BLD) + 128);
 }
 
-// 1 / sqrt(a) on the panel's chain: the hardware's estimate (good to 2^-20 at least) and two Newton
-// steps y += y (1 - a y^2) / 2 (the error squares each time), eight dependent operations; the tails of
-// the exponent range take the library's function. An a that is not positive gives a NaN or an
-// infinity, which the pivot test refuses.
-__device__ __forceinline__ double inverse_root(double a) {
-  if (!(a > 1e-280 && a < 1e280)) return rsqrt(a);
+// 1 / sqrt(a) and 1 / a on the panel's chain, from the hardware's estimate y of the root (good to
+// 2^-20 at least): with e = 1 - a y^2, the binomial series y (1 + e / 2 + 3 e^2 / 8) and
+// y^2 (1 + e + e^2) leave errors of e^3, below 2^-56: four dependent operations after the estimate. The
+// tails of the exponent range take the library's function. An a that is not positive gives NaNs or
+// infinities, which the pivot test refuses.
+__device__ __forceinline__ void inverse_root(double a, double &root, double &inverse) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const double e = fma(-a * y, y, 1.0);
-    y = fma(0.5 * y, e, y);
+  const double e = fma(-a * y, y, 1.0), u = y * y;
+  root = fma(y * e, fma(e, 0.375, 0.5), y);
+  inverse = fma(u, fma(e, e, e), u);
+  if (!(a > 1e-280 && a < 1e280)) {
+    root = rsqrt(a);
+    inverse = root * root;
   }
-  return y;
 }
 
 template <class T, int THREADS>
 __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__restrict__ val,
                                                         const PanelTask *__restrict__ tasks, DeviceStatus *status,
                                                         int p8max) {
-  constexpr int WORKERS = THREADS / 32 - 1;  // warps besides warp 0
+  // warp w's part past warp 0's: rows below (a group of 16 at a time), or the block's later columns
+  constexpr int ROW_WARPS = THREADS == PANEL_THREADS ? 8 : 3, BLOCK_WARPS = THREADS / 32 - 1 - ROW_WARPS;
   extern __shared__ double sm[];
   double *a = sm;                        // the block, column-major
   double *b = a + p8max * PANEL_ALD;     // the rows below: b[c * PANEL_BLD + i] = L(r0 + i, c0 + c)
@@ -300,13 +305,19 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
     }
   }
   cp_async_commit();
-  for (int c = tid; c < pw; c += THREADS) {
-    const int64_t j = task.col + c, ds = t.diag_src[j];
-    const double d = ds >= 0 ? val[ds] : 0.0;
-    dg[c] = t.scale ? d * t.scale[j] * t.scale[j] : d;
+  int row_warp = warp - 1, block_warp = -1;
+  if (BLOCK_WARPS > 0) {  // 4, 8 and 11 take the block
+    row_warp = warp < 4 ? warp - 1 : warp < 8 ? warp - 2 : warp - 3;
+    if (warp == 4 || warp == 8 || warp == 11) block_warp = warp == 4 ? 0 : warp == 8 ? 1 : 2, row_warp = -1;
   }
   cp_async_wait<0>();
   __syncthreads();
+  if (task.part == 0 && warp > 0)  // beside the first strip: two dependent loads each
+    for (int c = tid - 32; c < pw; c += THREADS - 32) {
+      const int64_t j = task.col + c, ds = t.diag_src[j];
+      const double d = ds >= 0 ? val[ds] : 0.0;
+      dg[c] = t.scale ? d * t.scale[j] * t.scale[j] : d;
+    }
   const int g = lane >> 2, tg = lane & 3;
   for (int B = 0; B <= nb8; ++B) {
     if (warp == 0) {
@@ -331,24 +342,28 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
             }
           }
         }
-        // the multipliers are broadcast before they are scaled, beside the root: the chain of a column
-        // is the pivot's shuffle, its root, a product and an update
+        // the multipliers are broadcast and multiplied before the root is there: the chain of a
+        // column is the pivot's shuffle, its reciprocal and one update
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const double acc = __shfl_sync(0xffffffffu, s0[j], j);
-          double lk[8];
+          double t0[8], t1[8];
 #pragma unroll
-          for (int k = j + 1; k < 8; ++k) lk[k] = __shfl_sync(0xffffffffu, s0[j], k);
-          const double rd = inverse_root(acc);
+          for (int k = j + 1; k < 8; ++k) {
+            const double lk = __shfl_sync(0xffffffffu, s0[j], k);
+            t0[k] = lane > j ? s0[j] * lk : 0.0;
+            t1[k] = s1[j] * lk;
+          }
+          double rd, rr;
+          inverse_root(acc, rd, rr);
+#pragma unroll
+          for (int k = j + 1; k < 8; ++k) {
+            s0[k] = fma(-t0[k], rr, s0[k]);
+            s1[k] = fma(-t1[k], rr, s1[k]);
+          }
           if (lane == 0) piv[o + j] = acc, dv[o + j] = rd;
           if (lane >= j) s0[j] *= rd;  // the pivot's own row: acc rd = sqrt(acc)
           s1[j] *= rd;
-#pragma unroll
-          for (int k = j + 1; k < 8; ++k) {
-            const double l = lk[k] * rd;
-            if (lane > j) s0[k] -= s0[j] * l;
-            s1[k] -= s1[j] * l;
-          }
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -378,64 +393,67 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
         }
       }
     } else if (B > 0) {
-      const int o = 8 * (B - 1), wt = tid - 32, ww = warp - 1;
-      // the strip's columns of the rows below
+      const int o = 8 * (B - 1);
       T *dst = Ls + task.r0 + (int64_t)(c0 + o) * m;
-      for (int i = wt; i < rows; i += 32 * WORKERS) {
-        double x[8];
+      if (row_warp >= 0) {
+        for (int i0 = 16 * row_warp; i0 < rows; i0 += 16 * ROW_WARPS) {
+          // the strip's columns of these rows
+          if (lane < 16 && i0 + lane < rows) {
+            double x[8];
+            double *bi = b + o * PANEL_BLD + i0 + lane;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) x[k] = b[(o + k) * PANEL_BLD + i];
+            for (int k = 0; k < 8; ++k) x[k] = bi[k * PANEL_BLD];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          x[k] *= dv[o + k];
+            for (int k = 0; k < 8; ++k) {
+              x[k] *= dv[o + k];
 #pragma unroll
-          for (int j = k + 1; j < 8; ++j) x[j] -= x[k] * a[(o + k) * PANEL_ALD + o + j];
+              for (int j = k + 1; j < 8; ++j) x[j] -= x[k] * a[(o + k) * PANEL_ALD + o + j];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              bi[k * PANEL_BLD] = x[k];
+              if (o + k < pw) dst[i0 + lane + (int64_t)k * m] = T(x[k]);
+            }
+          }
+          __syncwarp();
+          // and their later columns
+          double av[4];
+          av[0] = -b[(o + tg) * PANEL_BLD + i0 + g], av[1] = -b[(o + tg) * PANEL_BLD + i0 + g + 8];
+          av[2] = -b[(o + tg + 4) * PANEL_BLD + i0 + g], av[3] = -b[(o + tg + 4) * PANEL_BLD + i0 + g + 8];
+          for (int J = o + 8; J < P8; J += 16) {
+            // two 16 x 8 tiles at a time, their loads before their stores
+            double c[2][4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int j = min(J + 8 * u, P8 - 8);
+              const double bv[2] = {a[(o + tg) * PANEL_ALD + j + g], a[(o + tg + 4) * PANEL_ALD + j + g]};
+              const double *bj = b + (j + 2 * tg) * PANEL_BLD + i0 + g;
+              c[u][0] = bj[0], c[u][1] = bj[PANEL_BLD], c[u][2] = bj[8], c[u][3] = bj[PANEL_BLD + 8];
+              dmma16(c[u], av, bv);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              if (J + 8 * u >= P8) continue;
+              double *bj = b + (J + 8 * u + 2 * tg) * PANEL_BLD + i0 + g;
+              bj[0] = c[u][0], bj[PANEL_BLD] = c[u][1], bj[8] = c[u][2], bj[PANEL_BLD + 8] = c[u][3];
+            }
+          }
         }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          b[(o + k) * PANEL_BLD + i] = x[k];
-          if (o + k < pw) dst[i + (int64_t)k * m] = T(x[k]);
-        }
-      }
-      // the block's columns past the next strip: 8 x 8 tiles (I, J), I >= J
-      int q = 0;
-      for (int J = o + 16; J < P8; J += 8)
-        for (int I = J; I < P8; I += 8, ++q) {
-          if (q % WORKERS != ww) continue;
+      } else {
+        // the block's columns past the next strip: 8 x 8 tiles (I, J), I >= J, down the columns
+        int I = o + 16 + 8 * block_warp, J = o + 16;
+        while (J < P8) {
+          if (I >= P8) {
+            I = J + 8 + (I - P8);
+            J += 8;
+            continue;
+          }
           double c[2] = {0.0, 0.0};
           dmma(c, a[(o + tg) * PANEL_ALD + I + g], a[(o + tg) * PANEL_ALD + J + g]);
           dmma(c, a[(o + 4 + tg) * PANEL_ALD + I + g], a[(o + 4 + tg) * PANEL_ALD + J + g]);
           a[(J + 2 * tg) * PANEL_ALD + I + g] -= c[0];
           a[(J + 2 * tg + 1) * PANEL_ALD + I + g] -= c[1];
-        }
-      // the rows below's columns past the strip, once every worker's rows are solved
-      if (B < nb8 && rows > 0) {
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * WORKERS) : "memory");
-        const int groups = (rows + 15) >> 4, strips = nb8 - B, items = groups * strips;
-        for (int it = ww; it < items; it += 2 * WORKERS) {
-          // two 16 x 8 tiles at a time, their loads before their stores
-          double c[2][4];
-          int i0[2], J[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int e = min(it + u * WORKERS, items - 1);
-            i0[u] = 16 * (e / strips), J[u] = o + 8 + 8 * (e % strips);
-            double av[4], bv[2];
-            av[0] = b[(o + tg) * PANEL_BLD + i0[u] + g], av[1] = b[(o + tg) * PANEL_BLD + i0[u] + g + 8];
-            av[2] = b[(o + tg + 4) * PANEL_BLD + i0[u] + g], av[3] = b[(o + tg + 4) * PANEL_BLD + i0[u] + g + 8];
-            bv[0] = -a[(o + tg) * PANEL_ALD + J[u] + g], bv[1] = -a[(o + tg + 4) * PANEL_ALD + J[u] + g];
-            c[u][0] = b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g], c[u][1] = b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g];
-            c[u][2] = b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g + 8];
-            c[u][3] = b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g + 8];
-            dmma16(c[u], av, bv);
-          }
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            if (it + u * WORKERS >= items) continue;
-            b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g] = c[u][0], b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g] = c[u][1];
-            b[(J[u] + 2 * tg) * PANEL_BLD + i0[u] + g + 8] = c[u][2];
-            b[(J[u] + 2 * tg + 1) * PANEL_BLD + i0[u] + g + 8] = c[u][3];
-          }
+          I += 8 * BLOCK_WARPS;
         }
       }
     }
