@@ -522,72 +522,80 @@ __global__ void __launch_bounds__(256) dot_final_kernel(int ctas, const double *
 }
 
 // ---- an iteration of flexible CG, three launches ------------------------------------------------
-// Each is a programmatic dependent of the one before it (its CTAs are there when that one ends),
-// and the scalars between them are finished by the last CTA of the kernel that sums them. Bound by
-// the latency of three launches and two grid-wide sums: 36 us an iteration on 48 x 48 x 8 elements.
-// As eleven launches, with a second launch for every sum, it took 95 us.
+// Each is a programmatic dependent of the one before it (its CTAs are there when that one ends). Bound
+// by the latency of three launches and by K from L2. As eleven launches, with a second launch for
+// every sum, an iteration on 48 x 48 x 8 elements took 95 us; with each sum finished by the last CTA
+// of the kernel that forms it (a fence, an atomic and another pass at the end of two kernels) 36; with
+// the partials added where they are read 28. 64 threads a CTA in the step: 20 000 nodes are then 306
+// CTAs, two an SM, and not 77.
 constexpr int FCG_THREADS = 256, STEP_THREADS = 64;
 
-// out[k] = the sum over the grid of v[k], k < count: per CTA a fixed tree and the CTAs' partials in
-// a fixed order by the last CTA to finish, all of its threads' loads in flight together (part:
-// count x gridDim.x; *ticket starts and ends zero).
+// The CTA's sums of v[k] into part[k * ctas + blockIdx.x], k < count: a fixed tree.
 template <int K, int THREADS>
-__device__ __forceinline__ void grid_sums(double (&v)[K], int count, double *part, int *ticket, double *const (&out)[K]) {
+__device__ __forceinline__ void cta_partials(double (&v)[K], int count, double *const (&part)[K]) {
   constexpr int WARPS = THREADS / 32;
   __shared__ double s[K][WARPS];
-  __shared__ int last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto cta_sums = [&]() {  // the CTA's sum of v[k] to thread k
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-      if (lane == 0) s[k][warp] = v[k];
-    }
-    __syncthreads();
-    double sum = 0.0;
-    if ((int)threadIdx.x < count) {
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) sum += s[threadIdx.x][w];
-    }
-    return sum;
-  };
-  const double mine = cta_sums();
-  if ((int)threadIdx.x < count) {
-    part[threadIdx.x * gridDim.x + blockIdx.x] = mine;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    double sum = 0.0;
-    if (k < count)
-#pragma unroll 8
-      for (int b = threadIdx.x; b < (int)gridDim.x; b += THREADS) sum += __ldcg(part + k * gridDim.x + b);
-    v[k] = sum;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if (lane == 0) s[k][warp] = v[k];
   }
-  const double total = cta_sums();
+  __syncthreads();
 #pragma unroll
   for (int k = 0; k < K; ++k)
-    if (k < count && (int)threadIdx.x == k) *out[k] = total;
-  if (threadIdx.x == 0) *ticket = 0;
+    if (k < count && (int)threadIdx.x == k) {
+      double sum = 0.0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) sum += s[k][w];
+      part[k][blockIdx.x] = sum;
+    }
 }
 
-// A thread a node (three equations), 64 a CTA (a plate's 20 000 nodes in CTAs of 256 left half the
-// SMs idle): with `update`, x += alpha p and r -= alpha q, alpha = p.r / p.q;
-// then, with `z`, z = B r (inv: B's 3 x 3 blocks; null: z = r) and its products with the kept
-// directions' q_j; always r.r.
+// out[k] (shared) = the sum of part[k * stride + b], b < ctas, k < count, on every CTA the same: warps
+// take sums in turn, each lane every 32nd partial, eight loads in flight.
+template <int THREADS>
+__device__ __forceinline__ void add_partials(const double *part, int64_t stride, int ctas, int count, double *out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k = warp; k < count; k += THREADS / 32) {
+    double sum = 0.0;
+#pragma unroll 8
+    for (int b = lane; b < ctas; b += 32) sum += part[k * stride + b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) out[k] = sum;
+  }
+  __syncthreads();
+}
+
+__host__ __device__ inline int step_ctas(int64_t n) {
+  const int64_t c = ((n + 2) / 3 + STEP_THREADS - 1) / STEP_THREADS;
+  return (int)(c < 1 ? 1 : c > FCG_CTAS ? FCG_CTAS : c);
+}
+// The product's CTAs: every one the same number of rounds of rows.
+__host__ __device__ inline int product_ctas(int64_t n) {
+  constexpr int ROWS = FCG_THREADS / SPMV_LANES;
+  const int64_t groups = (n + ROWS - 1) / ROWS, rounds = (groups + FCG_CTAS - 1) / FCG_CTAS;
+  return groups < 1 ? 1 : (int)((groups + rounds - 1) / rounds);
+}
+
+// A thread a node (three equations), 64 a CTA: with `update`, x += alpha p and r -= alpha q; then, with
+// `z`, z = B r (inv: B's 3 x 3 blocks; null: z = r) and its products with the kept directions' q_j;
+// always r.r.
 __global__ void __launch_bounds__(STEP_THREADS) fcg_step_kernel(FcgStep a) {
+  __shared__ double pr_pq[2];
   pdl_wait();
   pdl_trigger();
   double v[1 + MAX_KEPT];
 #pragma unroll
   for (int k = 0; k <= MAX_KEPT; ++k) v[k] = 0.0;
-  const double alpha = a.update && a.alpha[1] != 0.0 ? a.alpha[0] / a.alpha[1] : 0.0;
+  double alpha = 0.0;
+  if (a.update) {
+    add_partials<STEP_THREADS>(a.product, FCG_CTAS, product_ctas(a.n), 2, pr_pq);
+    alpha = pr_pq[1] != 0.0 ? pr_pq[0] / pr_pq[1] : 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.den = pr_pq[1];
+  }
   const int64_t nodes = (a.n + 2) / 3;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nodes; k += (int64_t)gridDim.x * blockDim.x) {
     double r[3];
@@ -619,19 +627,24 @@ __global__ void __launch_bounds__(STEP_THREADS) fcg_step_kernel(FcgStep a) {
         if (j < a.kept) v[1 + j] += z[c] * a.qj[j][i];
     }
   }
-  double *out[1 + MAX_KEPT];
-  out[0] = a.rr;
+  double *part[1 + MAX_KEPT];
+  part[0] = a.rr;
 #pragma unroll
-  for (int j = 0; j < MAX_KEPT; ++j) out[1 + j] = a.zq + j;
-  grid_sums<1 + MAX_KEPT, STEP_THREADS>(v, 1 + (a.z ? a.kept : 0), a.part, a.ticket, out);
+  for (int j = 0; j < MAX_KEPT; ++j) part[1 + j] = a.zq + (int64_t)j * gridDim.x;
+  cta_partials<1 + MAX_KEPT, STEP_THREADS>(v, 1 + (a.z ? a.kept : 0), part);
 }
 
-// p = z - sum_j beta_j p_j, beta_j = num[j] / den[slot[j]]; p may be one of the p_j (an entry is read
-// before it is written).
 __global__ void __launch_bounds__(FCG_THREADS) fcg_direction_kernel(int64_t n, int m, const double *z, DirPtrs pj,
-                                                                    const double *num, const double *den, double *p) {
+                                                                    const double *num, const double *zq,
+                                                                    const double *den, double *p) {
+  __shared__ double sums[MAX_KEPT];
   pdl_wait();
   pdl_trigger();
+  if (zq && m > 0) {
+    const int ctas = step_ctas(n);
+    add_partials<FCG_THREADS>(zq, ctas, ctas, m, sums);
+    num = sums;
+  }
   double beta[MAX_KEPT];
 #pragma unroll
   for (int j = 0; j < MAX_KEPT; ++j) {
@@ -649,15 +662,13 @@ __global__ void __launch_bounds__(FCG_THREADS) fcg_direction_kernel(int64_t n, i
   }
 }
 
-// q = A p, and p.r, p.q (also into *den).
 __global__ void __launch_bounds__(FCG_THREADS) fcg_product_kernel(int64_t n, const int64_t *__restrict__ ptr,
                                                                   const int32_t *__restrict__ idx,
                                                                   const double *__restrict__ val, const double *p,
-                                                                  const double *r, double *q, double *sums, double *den,
-                                                                  double *part, int *ticket) {
+                                                                  const double *r, double *q, double *sums) {
   pdl_wait();
   pdl_trigger();
-  double v[3] = {0.0, 0.0, 0.0};
+  double v[2] = {0.0, 0.0};
   constexpr int ROWS = FCG_THREADS / SPMV_LANES;
   const int lane = threadIdx.x % SPMV_LANES;
   // every lane of a warp goes round as often as its last row: the sums are taken by shuffles
@@ -672,9 +683,14 @@ __global__ void __launch_bounds__(FCG_THREADS) fcg_product_kernel(int64_t n, con
       v[1] += pr * sum;
     }
   }
-  v[2] = v[1];
-  double *const out[3] = {sums, sums + 1, den};
-  grid_sums<3, FCG_THREADS>(v, 3, part, ticket, out);
+  double *const part[2] = {sums, sums + FCG_CTAS};
+  cta_partials<2, FCG_THREADS>(v, 2, part);
+}
+
+__global__ void __launch_bounds__(FCG_THREADS) fcg_norms_kernel(int count, int ctas, const double *rr, double *out) {
+  __shared__ double sums[8];
+  add_partials<FCG_THREADS>(rr, FCG_CTAS, ctas, count, sums);
+  if ((int)threadIdx.x < count) out[threadIdx.x] = sums[threadIdx.x];
 }
 
 // The passes' scales of pair threadIdx.x from nrm2 = ||r||^2: (sqrt(n) / ||r||, ||r|| / (sqrt(n) kref)),
@@ -832,27 +848,27 @@ static void launch_dependent(void (*kernel)(P...), int64_t grid, int threads, cu
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+int fcg_step_ctas(int64_t n) { return step_ctas(n); }
+
 void fcg_step(const FcgStep &a, cudaStream_t st) {
-  const int64_t nodes = (a.n + 2) / 3;
-  launch_dependent(fcg_step_kernel, std::min<int64_t>((nodes + STEP_THREADS - 1) / STEP_THREADS, FCG_CTAS), STEP_THREADS, st,
-                   a);
+  launch_dependent(fcg_step_kernel, step_ctas(a.n), STEP_THREADS, st, a);
 }
 
 void fcg_direction(int64_t n, int m, const double *z, const double *const *pj, const int *slot, const double *num,
-                   const double *den, double *p, cudaStream_t st) {
+                   const double *zq, const double *den, double *p, cudaStream_t st) {
   DirPtrs dp{};
   for (int j = 0; j < m && j < MAX_KEPT; ++j) dp.p[j] = pj[j], dp.slot[j] = slot[j];
   launch_dependent(fcg_direction_kernel, std::min<int64_t>((n + FCG_THREADS - 1) / FCG_THREADS, FCG_CTAS),
-                   FCG_THREADS, st, n, m, z,
-                   dp, num, den, p);
+                   FCG_THREADS, st, n, m, z, dp, num, zq, den, p);
 }
 
 void fcg_product(int64_t n, const int64_t *ptr, const int32_t *idx, const double *val, const double *p,
-                 const double *r, double *q, double *sums, double *den, double *part, int *ticket, cudaStream_t st) {
-  constexpr int ROWS = FCG_THREADS / SPMV_LANES;
-  launch_dependent(fcg_product_kernel, std::min<int64_t>((n + ROWS - 1) / ROWS, FCG_CTAS), FCG_THREADS, st, n, ptr, idx,
-                   val, p, r,
-                   q, sums, den, part, ticket);
+                 const double *r, double *q, double *sums, cudaStream_t st) {
+  launch_dependent(fcg_product_kernel, product_ctas(n), FCG_THREADS, st, n, ptr, idx, val, p, r, q, sums);
+}
+
+void fcg_norms(int64_t n, int count, const double *rr, double *out, cudaStream_t st) {
+  fcg_norms_kernel<<<1, FCG_THREADS, 0, st>>>(count, step_ctas(n), rr, out);
 }
 
 void input_scales(int64_t n, int pairs, int per, const double *nrm2, double kref, double *s, cudaStream_t st) {

@@ -87,31 +87,35 @@ void adam(int64_t n, float *p, const float *g, float *m, float *v, float lr, flo
 // (partials per CTA, then one CTA), so results are the same on every run.
 void dots(int64_t n, int pairs, const double *const *a, const double *const *b, double *partial, double *out,
           cudaStream_t st);
-// An iteration of flexible CG. Sums are taken in a fixed order and left in device scalars by the
-// kernel that forms them; `part` holds (1 + MAX_KEPT) x FCG_CTAS partials and *ticket is zero
-// between launches.
+// An iteration of flexible CG in three launches. A kernel leaves its sums as one partial a CTA, and
+// the kernel that needs them adds the partials itself, every CTA in the same fixed order: no pass
+// and no last CTA in between.
 constexpr int MAX_KEPT = 8, FCG_CTAS = 148 * 8;
 struct FcgStep {
   int64_t n;
-  int update;                    // x += alpha p, r -= alpha q with alpha = alpha[0] / alpha[1] (0 when alpha[1] is 0)
-  const double *alpha, *p, *q;
+  int update;                    // x += alpha p, r -= alpha q with alpha = p.r / p.q (0 when p.q is 0)
+  const double *product;         // the product's partials (fcg_product)
+  double *den;                   // receives p.q
+  const double *p, *q;
   double *x, *r;
   double *z;                     // null: no preconditioner here; else z = B r, inv B's blocks (null: z = r)
   const double *inv;
-  int kept;                      // zq[j] = z . qj[j], j < kept
+  int kept;                      // partials of z . qj[j], j < kept
   const double *qj[MAX_KEPT];
-  double *zq, *rr;               // *rr = r . r
-  double *part;
-  int *ticket;
+  double *zq;                    // kept x fcg_step_ctas(n) partials
+  double *rr;                    // fcg_step_ctas(n) partials of r . r
 };
+int fcg_step_ctas(int64_t n);
 void fcg_step(const FcgStep &a, cudaStream_t st);
-// p = z - sum_j beta_j p_j with beta_j = num[j] / den[slot[j]] (device scalars); p may be one of the
-// p_j
+// p = z - sum_j beta_j p_j with beta_j = (z . q_j) / den[slot[j]], the numerators given as device
+// scalars (num) or as fcg_step's partials (zq); p may be one of the p_j
 void fcg_direction(int64_t n, int m, const double *z, const double *const *pj, const int *slot, const double *num,
-                   const double *den, double *p, cudaStream_t st);
-// q = A p (A by rows), sums[0] = p . r, sums[1] = *den = p . q
+                   const double *zq, const double *den, double *p, cudaStream_t st);
+// q = A p (A by rows); the partials of p . r, then of p . q, in `sums` (2 x FCG_CTAS doubles)
 void fcg_product(int64_t n, const int64_t *ptr, const int32_t *idx, const double *val, const double *p,
-                 const double *r, double *q, double *sums, double *den, double *part, int *ticket, cudaStream_t st);
+                 const double *r, double *q, double *sums, cudaStream_t st);
+// out[k] = the sum of the partials of r . r at rr + k * FCG_CTAS, k < count
+void fcg_norms(int64_t n, int count, const double *rr, double *out, cudaStream_t st);
 // The passes' scales of `pairs` vectors from their nrm2 = ||r||^2 (dots): s[2 p] = sqrt(n) / ||r||,
 // s[2 p + 1] = ||r|| / (sqrt(n) kref); with per = 2 (the odd network) the pass on r halves its
 // output scale and the pass on -r has both negated.

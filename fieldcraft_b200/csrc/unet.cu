@@ -694,7 +694,9 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
   }
   // vectors: r, z, q and the ring of `keep` directions p_j and A p_j
   const int ring = keep;
-  constexpr size_t SCALARS = 64, PARTS = (1 + fc::unet::MAX_KEPT) * fc::unet::FCG_CTAS;
+  constexpr int CHECK = 8;
+  static_assert(8 * 296 <= 2 * fc::unet::FCG_CTAS, "the dots write over p.r and p.q at most");
+  constexpr size_t SCALARS = 64, PARTS = (size_t)(2 + fc::unet::MAX_KEPT + CHECK + 1) * fc::unet::FCG_CTAS;
   fc::host::Scratch scratch(sizeof(double) * (SCALARS + PARTS + (size_t)n * (3 + 2 * ring)), st);
   if (!scratch.p) {
     set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for FCG");
@@ -704,10 +706,11 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
   double *r = part + PARTS, *z = r + n, *tmp = z + n;
   std::vector<double *> P(ring), Q(ring);
   for (int j = 0; j < ring; ++j) P[j] = tmp + n * (1 + 2 * j), Q[j] = P[j] + n;
-  // [0] b.b [1] r.r [2] p.r [3] p.q [5] b - A x squared [6] a start's r.r [8..8+ring) z.q_j [16..16+ring) p_j.q_j
-  // [32..32+CHECK) the last iterations' r.r [48] the sums' ticket
-  int *ticket = reinterpret_cast<int *>(s + 48);
-  cudaMemsetAsync(ticket, 0, sizeof(double), st);
+  // [0] b.b [1] r.r [5] b - A x squared [8..8+ring) z.q_j with the network [16..16+ring) p_j.q_j
+  // [32..32+CHECK) the last iterations' r.r; part: the dots' partials, and flexible CG's: p.r and p.q,
+  // z.q_j, and r.r of CHECK iterations and of a start
+  double *const part_pq = part, *const part_zq = part + 2 * fc::unet::FCG_CTAS,
+               *const part_rr = part_zq + fc::unet::MAX_KEPT * fc::unet::FCG_CTAS;
   cudaMemsetAsync(d_x, 0, sizeof(double) * n, st);
   copy_kernel<<<blocks(n), 256, 0, st>>>(n, d_b, r);
   {
@@ -737,7 +740,6 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
   // ||r||^2 of each iteration lands in a ring of device scalars (s + 32 + it % CHECK); the host
   // reads them every CHECK iterations (one synchronisation per CHECK iterations), then decides on
   // convergence, the safeguard and a residual replacement in iteration order.
-  constexpr int CHECK = 8;
   int since = 0;
   double ring_rr[CHECK];
   // the kept directions' slots, the most recent first, at iteration `it` with `have` stored
@@ -746,13 +748,14 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     return have;
   };
   // z = M(r) and its products with the kept directions, for iteration `at`; with `update` the last
-  // direction's step on x and r first (rr: where r.r goes). The network's z is formed apart.
-  auto step = [&](bool update, int at, int have, double *rr_at) {
+  // direction's step on x and r first (rr_slot: where r.r's partials go). The network's z is formed
+  // apart.
+  auto step = [&](bool update, int at, int have, int rr_slot) {
     const bool jacobi = net && net->has_bj;
     fc::unet::FcgStep a{};
-    a.n = n, a.update = update ? 1 : 0, a.alpha = s + 2, a.x = d_x, a.r = r, a.rr = rr_at, a.zq = s + 8;
-    if (update) a.p = P[(at - 1) % ring], a.q = Q[(at - 1) % ring];
-    a.part = part, a.ticket = ticket;
+    a.n = n, a.update = update ? 1 : 0, a.product = part_pq, a.x = d_x, a.r = r, a.zq = part_zq;
+    a.rr = part_rr + (int64_t)rr_slot * fc::unet::FCG_CTAS;
+    if (update) a.p = P[(at - 1) % ring], a.q = Q[(at - 1) % ring], a.den = s + 16 + (at - 1) % ring;
     int slot[fc::unet::MAX_KEPT];
     if (!use_net) {
       a.z = z, a.inv = jacobi ? net->bj.as<double>() : nullptr;
@@ -772,18 +775,19 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
       apply(net, 1, r, n, z, together);
       if (m > 0) fc::unet::dots(n, m, zz, qj, part, s + 8, st);
     } else if (!have_z) {
-      step(false, it, m, s + 6);
+      step(false, it, m, CHECK);
     }
     // p = z - sum_j (z.q_j / p_j.q_j) p_j over the stored directions (the denominators were kept
     // in s + 16 + slot when each direction was made); q = A p, p.r, p.q
-    fc::unet::fcg_direction(n, m, z, pj, slot, s + 8, s + 16, p, st);
-    fc::unet::fcg_product(n, d_ptr, d_idx, d_val, p, r, q, s + 2, s + 16 + (it % ring), part, ticket, st);
+    fc::unet::fcg_direction(n, m, z, pj, slot, s + 8, use_net ? nullptr : part_zq, s + 16, p, st);
+    fc::unet::fcg_product(n, d_ptr, d_idx, d_val, p, r, q, part_pq, st);
     // alpha = p.r / p.q, x += alpha p, r -= alpha q, and the next iteration's z
-    step(true, it + 1, std::min(stored + 1, ring), s + 32 + (it % CHECK));
+    step(true, it + 1, std::min(stored + 1, ring), it % CHECK);
     have_z = !use_net;
     ++it;
     stored = std::min(stored + 1, ring);
     if (++since < CHECK && it < max_iter) continue;
+    fc::unet::fcg_norms(n, CHECK, part_rr, s + 32, st);
     cudaMemcpyAsync(ring_rr, s + 32, sizeof(double) * CHECK, cudaMemcpyDeviceToHost, st);
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(status, e, "FCG");
