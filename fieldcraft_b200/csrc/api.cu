@@ -64,7 +64,8 @@ struct Launch {
   int64_t off;
   int count;
   int level;  // the level of the supernodal tree the launch belongs to (cancellation points)
-  int width;  // panel launches: the widest panel, padded (sizes the kernel's shared memory)
+  int width;  // panel launches: the widest panel, padded (sizes the kernel's shared memory); LDL^T's: the
+              // most own columns a front has left
   // the factorisation runs on three streams (lanes): lane 0 the chain of panels and what needs
   // them, lane 1 the updates of columns past the next outer block (beside the next panels), lane 2
   // the diagonal blocks' inverses (needed by the solve only); `dep` is a launch on another lane
@@ -72,6 +73,7 @@ struct Launch {
   int lane = 0;
   int dep = -1;
   bool record = false;
+  int rows = 0;  // LDL^T's panel launches: the tallest front
 };
 
 }  // namespace
@@ -894,7 +896,7 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
       h->d_lscale.alloc(sizeof(double) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
       h->d_lorder.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
       h->d_lpivots.alloc((size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
-      h->d_lpos.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(h->ns, 1)) != cudaSuccess ||
+      h->d_lpos.alloc(sizeof(int32_t) * 2 * (size_t)std::max<int64_t>(h->ns, 1)) != cudaSuccess ||
       h->d_ltwos.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(h->ns, 1)) != cudaSuccess ||
       h->d_lfailed.alloc(sizeof(unsigned long long)) != cudaSuccess ||
       h->d_ldd.alloc(sizeof(double) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess ||
@@ -955,12 +957,12 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
     }
     for (int p = 0; p < P; ++p) {
       const int64_t po = (int64_t)pan_t.size(), go = (int64_t)gemm_t.size();
-      int tallest = 0;
+      int tallest = 0, widest = 0;
       for (size_t q = 0; q < S.size(); ++q) {
         const int64_t s = S[q];
         const int m = h->height[s], w = h->width[s];
         if (p * L::PANEL >= w) continue;
-        tallest = std::max(tallest, m);
+        tallest = std::max(tallest, m), widest = std::max(widest, w - p * L::PANEL);
         const int earliest = (p + 1) * L::PANEL;
         const int64_t slots = earliest < w ? L::update_tiles(m, w, earliest) : 0;
         L::PanelTask t{};
@@ -974,7 +976,8 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
           gemm_t.push_back(fc::GemmTask{});  // empty until the panel step writes it
         }
       }
-      push(h->program, K_LDLT_PANEL, po, (int64_t)pan_t.size() - po, (int)l, tallest);
+      push(h->program, K_LDLT_PANEL, po, (int64_t)pan_t.size() - po, (int)l, widest);
+      if ((int64_t)pan_t.size() > po) h->program.back().rows = tallest;
       push(h->program, K_GEMM, go, (int64_t)gemm_t.size() - go, (int)l);
     }
     const int64_t ao = (int64_t)aft_t.size();
@@ -1472,8 +1475,8 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
         break;
       case K_GEMM_F64: fc::launch_gemm(h->d_gemm.as<fc::GemmTask>() + l.off, l.count, fc::GemmKind::F64, st); break;
       case K_LDLT_PANEL:
-        fc::ldlt::launch_panel(h->d_lpanel.as<fc::ldlt::PanelTask>() + l.off, l.count, l.width, h->d_lpos.as<int32_t>(),
-                               h->d_ltwos.as<int32_t>(), h->d_lfailed.as<unsigned long long>(), st);
+        fc::ldlt::launch_panel(h->d_lpanel.as<fc::ldlt::PanelTask>() + l.off, l.count, l.rows, l.width,
+                               h->d_lpos.as<int32_t>(), h->d_lpos.as<int32_t>() + h->ns, h->d_ltwos.as<int32_t>(), h->d_lfailed.as<unsigned long long>(), st);
         break;
       case K_LDLT_AFTER: fc::ldlt::launch_after(h->d_lafter.as<fc::ldlt::AfterTask>() + l.off, l.count, st); break;
       case K_LDLT_INVERSE: fc::ldlt::launch_inverse(h->d_linv.as<fc::ldlt::InverseTask>() + l.off, l.count, st); break;

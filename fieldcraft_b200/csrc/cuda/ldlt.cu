@@ -1,7 +1,8 @@
 // The device LDL^T's pivoted panel step (ldlt_panel.cuh on CUDA threads): one CTA per front of
-// a level, each taking its next panel from where the previous one ended. The source of the
-// panel is the one the CPU emulation checks against the oracle bit for bit; this file gives it
-// the device's block (threads, __syncthreads) and its per-supernode state.
+// a level on its own rows, each taking its next panel from where the previous one ended, then the
+// rows below spread over the GPU. The source of the first is the one the CPU emulation checks
+// against the oracle bit for bit; this file gives it the device's block (threads, __syncthreads)
+// and its per-supernode state.
 #include <cstdint>
 
 #include "cuda/ldlt_launch.cuh"
@@ -15,16 +16,18 @@ struct DeviceBlock {
   __device__ void sync() { __syncthreads(); }
 };
 
-// Per supernode s: pos[s] is where its next panel starts (w when done), twos[s] counts its 2 x 2
-// pivots. A singular column lowers *failed to its postorder index (the first failing column in
+// Per supernode s: pos[s] is where its next panel starts (w when done), from[s] where the last one
+// did (pos[s] when there was none), twos[s] counts its 2 x 2 pivots. A singular column lowers *failed to its postorder index (the first failing column in
 // postorder is the one reported) and ends the supernode. After the panel the CTA writes the
 // update of the later own columns as GEMM tasks (C -= L_panel W^T on the lower tiles, for the
 // launch that follows); the slots it does not need stay empty (M = N = K = 0: no work).
 __global__ void __launch_bounds__(MAX_THREADS) ldlt_panel_kernel(const PanelTask *__restrict__ tasks,
                                                                  int32_t *__restrict__ pos,
+                                                                 int32_t *__restrict__ from,
                                                                  int32_t *__restrict__ twos,
                                                                  unsigned long long *__restrict__ failed) {
-  __shared__ Shared sh;
+  extern __shared__ __align__(16) unsigned char panel_sm[];
+  Shared &sh = *reinterpret_cast<Shared *>(panel_sm);
   const PanelTask &task = tasks[blockIdx.x];
   const Front &f = task.front;
   const int c0 = pos[task.s];
@@ -34,7 +37,7 @@ __global__ void __launch_bounds__(MAX_THREADS) ldlt_panel_kernel(const PanelTask
     DeviceBlock blk;
     int made = 0;
     end = c0;
-    const int singular = panel(blk, sh, f, c0, &end, &made);
+    const int singular = panel_own(blk, sh, f, c0, &end, &made);
     if (singular >= 0) {
       if (threadIdx.x == 0) {
         atomicMin(failed, (unsigned long long)(task.first + singular));
@@ -43,7 +46,6 @@ __global__ void __launch_bounds__(MAX_THREADS) ldlt_panel_kernel(const PanelTask
       end = f.w;
     } else {
       ok = true;
-      panel_w(blk, f, c0, end);
       if (threadIdx.x == 0) twos[task.s] += made;
     }
   }
@@ -67,8 +69,91 @@ __global__ void __launch_bounds__(MAX_THREADS) ldlt_panel_kernel(const PanelTask
     }
     task.slots[q] = g;
   }
-  if (!ok) return;
-  if (threadIdx.x == 0) pos[task.s] = end;
+  if (threadIdx.x == 0) {
+    from[task.s] = ok ? c0 : end;
+    if (ok) pos[task.s] = end;
+  }
+}
+
+// After it: L of the rows below the own columns, and L D of the own rows past the panel (the update's
+// coefficients). Eight threads a row, thread t of them the columns t, t + 8, ... in registers: as soon
+// as a column's entry is divided the later ones take its product, so a row is a chain of 64 divisions
+// and not of 2 000 subtractions, and its entries see panel_below's operations in panel_below's order.
+constexpr int BELOW_ROWS = 32, BELOW_THREADS = 8 * BELOW_ROWS, BELOW_HELD = (PANEL + 8) / 8;
+__global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTask *__restrict__ tasks,
+                                                                   const int32_t *__restrict__ pos,
+                                                                   const int32_t *__restrict__ from) {
+  __shared__ double coef[PANEL + 1][8 * BELOW_HELD];  // L D at (row j, column q) of the panel's block: [q][j]
+  __shared__ double d[PANEL + 1], e[PANEL + 1];
+  __shared__ int8_t kind[PANEL + 1];
+  const PanelTask &task = tasks[blockIdx.x];
+  const Front f = task.front;
+  const int c0 = from[task.s], c1 = pos[task.s], kw = c1 - c0;
+  const int64_t r0 = c0 + (int64_t)blockIdx.y * BELOW_ROWS;
+  if (kw <= 0 || r0 >= f.m || r0 + BELOW_ROWS <= c1) return;
+  for (int k = threadIdx.x; k < kw; k += BELOW_THREADS) {
+    d[k] = at(f, c0 + k, c0 + k);
+    kind[k] = f.pivots[c0 + k];
+    e[k] = kind[k] == PIVOT_FIRST ? at(f, c0 + k + 1, c0 + k) : 0.0;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 7;
+  const int64_t r = r0 + (threadIdx.x >> 3);
+  // times_d for any row past the panel's columns q
+  auto product = [&](int64_t row, int q) {
+    const double x = at(f, row, c0 + q);
+    if (kind[q] == PIVOT_FIRST) return add(mul(x, d[q]), mul(at(f, row, c0 + q + 1), e[q]));
+    if (kind[q] == PIVOT_SECOND) return add(mul(at(f, row, c0 + q - 1), e[q - 1]), mul(x, d[q]));
+    return mul(x, d[q]);
+  };
+  if (r >= c1 && r < f.w)
+    for (int q = lane; q < kw; q += 8) f.W[(r - c1) + q * f.ld_w] = product(r, q);
+  if (r0 + BELOW_ROWS <= f.w) return;
+  // the panel's block below the pivots (no entry of a 2 x 2 pivot's own is read)
+  for (int x = threadIdx.x; x < (PANEL + 1) * 8 * BELOW_HELD; x += BELOW_THREADS) {
+    const int q = x / (8 * BELOW_HELD), j = x % (8 * BELOW_HELD);
+    coef[q][j] = j < kw && q < j && !(kind[q] == PIVOT_FIRST && j == q + 1) ? product(c0 + j, q) : 0.0;
+  }
+  __syncthreads();
+  const bool mine = r >= f.w && r < f.m;
+  double g[BELOW_HELD];
+#pragma unroll
+  for (int t = 0; t < BELOW_HELD; ++t) g[t] = mine && 8 * t + lane < kw ? at(f, r, c0 + 8 * t + lane) : 0.0;
+#pragma unroll
+  for (int t = 0; t < BELOW_HELD; ++t) {
+    for (int o = 0; o < 8 && 8 * t + o < kw; ++o) {
+      const int k = 8 * t + o;
+      if (kind[k] == PIVOT_SECOND) continue;
+      const double x = __shfl_sync(0xffffffffu, g[t], o, 8);
+      if (kind[k] == PIVOT_FIRST) {
+        double y = __shfl_sync(0xffffffffu, g[t], (o + 1) & 7, 8);
+        if (t + 1 < BELOW_HELD) {
+          const double z = __shfl_sync(0xffffffffu, g[t + 1 < BELOW_HELD ? t + 1 : t], 0, 8);
+          if (o == 7) y = z;
+        }
+        const double d11 = d[k], d21 = e[k], d22 = d[k + 1], det = sub(mul(d11, d22), mul(d21, d21));
+        const double l0 = sub(mul(x, d22), mul(y, d21)) / det, l1 = sub(mul(y, d11), mul(x, d21)) / det;
+#pragma unroll
+        for (int u = t; u < BELOW_HELD; ++u) {
+          const int j = 8 * u + lane;
+          if (j > k + 1) g[u] = sub(sub(g[u], mul(l0, coef[k][j])), mul(l1, coef[k + 1][j]));
+          if (j == k) g[u] = l0;
+          if (j == k + 1) g[u] = l1;
+        }
+      } else {
+        const double l = x / d[k];
+#pragma unroll
+        for (int u = t; u < BELOW_HELD; ++u) {
+          const int j = 8 * u + lane;
+          if (j > k) g[u] = sub(g[u], mul(l, coef[k][j]));
+          if (j == k) g[u] = l;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < BELOW_HELD; ++t)
+    if (mine && 8 * t + lane < kw) at(f, r, c0 + 8 * t + lane) = g[t];
 }
 
 __global__ void __launch_bounds__(W21_ROWS) ldlt_after_kernel(const AfterTask *__restrict__ tasks) {
@@ -167,13 +252,19 @@ void launch_fold(int64_t n, const int32_t *local, const int32_t *order, const in
   if (rows_len > 0) ldlt_rows_kernel<<<grid_for(rows_len, 256), 256, 0, st>>>(rows_len, rows, own, rows_out);
 }
 
-// A thread a row up to 1024: a column step is a chain of loads and barriers (bound by their latency,
-// about 2.6 us a column). With 256 threads a top front's rows went round the block six times a step
-// and one thread formed L D from global memory: 90 ms of panels for 16 x 14 x 13 elements, now 12.
-void launch_panel(const PanelTask *tasks, int count, int tallest, int32_t *pos, int32_t *twos,
-                  unsigned long long *failed, cudaStream_t st) {
-  const int threads = tallest >= MAX_THREADS ? MAX_THREADS : tallest <= 64 ? 64 : (tallest + 31) / 32 * 32;
-  if (count > 0) ldlt_panel_kernel<<<count, threads, 0, st>>>(tasks, pos, twos, failed);
+// A thread an own row up to 1024: a column step is a chain of loads and barriers, bound by their
+// latency, and the rows below would make it longer (they are most of a front's rows, and a CTA has one
+// SM's FP64 units): they come after it, all of a level's together. Panels of 16 x 14 x 13 elements:
+// 12.1 ms on all rows with each column formed when it is looked at (3.3 us a column on the longest
+// chain); 7.5 and 2.3 for the rows below.
+void launch_panel(const PanelTask *tasks, int count, int tallest, int widest, int32_t *pos, int32_t *from,
+                  int32_t *twos, unsigned long long *failed, cudaStream_t st) {
+  if (count <= 0) return;
+  const int threads = widest >= MAX_THREADS ? MAX_THREADS : widest <= 64 ? 64 : (widest + 31) / 32 * 32;
+  cudaFuncSetAttribute(ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
+  ldlt_panel_kernel<<<count, threads, sizeof(Shared), st>>>(tasks, pos, from, twos, failed);
+  const dim3 grid(count, (tallest + BELOW_ROWS - 1) / BELOW_ROWS);
+  ldlt_below_kernel<<<grid, BELOW_THREADS, 0, st>>>(tasks, pos, from);
 }
 
 void launch_after(const AfterTask *tasks, int count, cudaStream_t st) {

@@ -43,9 +43,10 @@ struct InverseTask {
 };
 
 void launch_inverse(const InverseTask *tasks, int count, cudaStream_t st);
-// `tallest`: the largest m of the launch's fronts (sizes its CTAs).
-void launch_panel(const PanelTask *tasks, int count, int tallest, int32_t *pos, int32_t *twos, unsigned long long *failed,
-                  cudaStream_t st);
+// `tallest`, `widest`: the largest m and w of the launch's fronts (they size its grid and its CTAs);
+// pos, from, twos: a number a supernode (see the kernel).
+void launch_panel(const PanelTask *tasks, int count, int tallest, int widest, int32_t *pos, int32_t *from,
+                  int32_t *twos, unsigned long long *failed, cudaStream_t st);
 void launch_after(const AfterTask *tasks, int count, cudaStream_t st);
 void launch_scale(int64_t nnz, const int64_t *a_src, const int32_t *a_row, const int32_t *a_col, const double *val,
                   unsigned long long *scale_bits, cudaStream_t st);

@@ -18,11 +18,16 @@
 #define FC_LDLT_FN __device__ __forceinline__
 #define FC_LDLT_HD __host__ __device__ __forceinline__  // arithmetic the host plan shares
 #define FC_LDLT_ONCE __device__ __forceinline__
+#define FC_LDLT_UNROLL _Pragma("unroll")
 #else
 #include <cmath>
 #define FC_LDLT_FN inline
 #define FC_LDLT_HD inline
 #define FC_LDLT_ONCE __attribute__((noinline, noclone))  // its barrier stays one call site
+#define FC_LDLT_UNROLL
+#endif
+#ifndef FC_LDLT_HELD_ROWS
+#define FC_LDLT_HELD_ROWS 1024
 #endif
 
 namespace fc {
@@ -33,6 +38,8 @@ constexpr int ROOK_STEPS = 64;                // ldlt.rs:81
 constexpr int PANEL = 64;                     // cholesky.rs:54
 constexpr double PIVOT_TOLERANCE = 1e-10;     // cholesky.rs:48
 constexpr int MAX_THREADS = 1024;
+// Columns held up to date ahead of the search, and the own rows there is room for (see panel_own).
+constexpr int HELD = 8, HELD_ROWS = FC_LDLT_HELD_ROWS;
 constexpr int8_t PIVOT_ONE = 0, PIVOT_FIRST = 1, PIVOT_SECOND = 2;
 
 #if defined(__CUDACC__)
@@ -71,6 +78,10 @@ struct Shared {
   double d[PANEL + 1];     // D's diagonal at the panel's factored columns
   double e[PANEL + 1];     // its subdiagonal at the first column of a 2 x 2 pivot
   int8_t kind[PANEL + 1];  // PIVOT_ONE / PIVOT_FIRST / PIVOT_SECOND
+  double rows[HELD][PANEL];       // rows of L D for the columns to hold
+  double next[HELD];              // L D of the newest column at the held columns' rows
+  double held[HELD][HELD_ROWS];   // the held columns, own rows from the panel's start
+  double ab[2][HELD_ROWS];        // Front's a and b, own rows from the panel's start
 #if defined(__CUDACC__)
   double best_v[32];  // a warp each
   int best_i[32];
@@ -143,7 +154,7 @@ FC_LDLT_ONCE bool block_best(Block &blk, Shared &sh, double bv, int bi, int bn, 
   return bn == 0;
 }
 
-// Column c (local, >= k) of the part still to factor, rows [k, m), into out: the front's entries
+// Column c (local, >= k) of the part still to factor, own rows [k, w), into out: the front's entries
 // less the products with the panel's factored columns [c0, k) (Block::current, ldlt.rs:173-192),
 // a row a thread, 16 columns' loads in flight; and the largest magnitude of it over [lo, w) except
 // row `skip`, with the lowest such index (largest, ldlt.rs:145-163; lo when all are zero). Returns
@@ -157,7 +168,7 @@ FC_LDLT_FN bool current(Block &blk, Shared &sh, const Front &f, int c0, int k, i
   blk.sync();
   double bv = 0.0;
   int bi = lo, bn = 0;
-  for (int64_t r = k + blk.tid(); r < f.m; r += blk.size()) {
+  for (int r = k + blk.tid(); r < f.w; r += blk.size()) {
     double v = r >= c ? at(f, r, c) : at(f, c, r);
     const double *L = &at(f, r, c0);
     int q = 0;
@@ -177,17 +188,77 @@ FC_LDLT_FN bool current(Block &blk, Shared &sh, const Front &f, int c0, int k, i
 #endif
     for (; q < len; ++q) v = sub(v, mul(L[q * f.m], sh.row[q]));
     out[r] = v;
-    if (r >= lo && r < f.w && r != skip) {
+    if (r >= lo && r != skip) {
       const double x = magnitude(v);
       if (not_a_number(x)) {
         bn = 1;
       } else if (x > bv) {
         bv = x;
-        bi = (int)r;
+        bi = r;
       }
     }
   }
   return block_best(blk, sh, bv, bi, bn, lo, f.w, index, value);
+}
+
+// The columns [k, k + count), count <= COUNT, into sh.held: their own rows less the products with the
+// panel's factored columns [c0, k), each entry's in order, the columns side by side (one column's
+// subtractions are a chain, 64 at most). Row r is always held by the same thread.
+template <int COUNT, class Block>
+FC_LDLT_FN void hold(Block &blk, Shared &sh, const Front &f, int c0, int k, int count) {
+  const int len = k - c0;
+  for (int e = blk.tid(); e < COUNT * PANEL; e += blk.size()) {
+    const int j = e / PANEL, q = e % PANEL;
+    if (q < len) sh.rows[j][q] = j < count ? times_d(sh, f, c0, k + j, q) : 0.0;
+  }
+  blk.sync();
+  for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
+    if (r < k) continue;
+    double v[COUNT];
+    FC_LDLT_UNROLL
+    for (int j = 0; j < COUNT; ++j) v[j] = j < count && r >= k + j ? at(f, r, k + j) : 0.0;
+    const double *L = &at(f, r, c0);
+    int q = 0;
+    for (; q + 8 <= len; q += 8) {
+      double l[8];
+      FC_LDLT_UNROLL
+      for (int t = 0; t < 8; ++t) l[t] = L[(q + t) * f.m];
+      FC_LDLT_UNROLL
+      for (int t = 0; t < 8; ++t)
+        FC_LDLT_UNROLL
+        for (int j = 0; j < COUNT; ++j) v[j] = sub(v[j], mul(l[t], sh.rows[j][q + t]));
+    }
+    for (; q < len; ++q) {
+      const double l = L[q * f.m];
+      FC_LDLT_UNROLL
+      for (int j = 0; j < COUNT; ++j) v[j] = sub(v[j], mul(l, sh.rows[j][q]));
+    }
+    FC_LDLT_UNROLL
+    for (int j = 0; j < COUNT; ++j)
+      if (j < count) sh.held[j][r - c0] = v[j];
+  }
+}
+
+// current() for the held column k = base + j: into out, and the largest below the diagonal.
+template <class Block>
+FC_LDLT_FN bool held_column(Block &blk, Shared &sh, const Front &f, int c0, int k, int base, double *out, int &index,
+                            double &value) {
+  double bv = 0.0;
+  int bi = k + 1, bn = 0;
+  for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
+    if (r < k) continue;
+    const double v = sh.held[k - base][r - c0];
+    out[r] = v;
+    const double x = magnitude(v);
+    if (r == k) continue;
+    if (not_a_number(x)) {
+      bn = 1;
+    } else if (x > bv) {
+      bv = x;
+      bi = r;
+    }
+  }
+  return block_best(blk, sh, bv, bi, bn, k + 1, f.w, index, value);
 }
 
 // Symmetric interchange of local columns p and q (both at pivot positions >= k) in the front,
@@ -216,7 +287,7 @@ FC_LDLT_FN void interchange(Block &blk, const Front &f, int p, int q, double *a,
 template <class Block>
 FC_LDLT_FN void one(Block &blk, Shared &sh, const Front &f, int c0, int k, const double *col) {
   const double d = col[k];
-  for (int64_t r = k + 1 + blk.tid(); r < f.m; r += blk.size()) at(f, r, k) = col[r] / d;
+  for (int r = k + 1 + blk.tid(); r < f.w; r += blk.size()) at(f, r, k) = col[r] / d;
   if (blk.tid() == 0) {
     at(f, k, k) = d;
     f.pivots[k] = PIVOT_ONE;
@@ -226,13 +297,42 @@ FC_LDLT_FN void one(Block &blk, Shared &sh, const Front &f, int c0, int k, const
   blk.sync();
 }
 
+// The same for the held column k, which stayed in its place: the held columns after it, [k + 1, stop),
+// take its product.
+template <class Block>
+FC_LDLT_FN void one_held(Block &blk, Shared &sh, const Front &f, int c0, int k, int base, int stop, double *col) {
+  const double d = col[k];
+  for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
+    if (r <= k) continue;
+    const double l = col[r] / d;
+    at(f, r, k) = l;
+    col[r] = l;
+    if (r < stop) sh.next[r - base] = mul(l, d);
+  }
+  if (blk.tid() == 0) {
+    at(f, k, k) = d;
+    f.pivots[k] = PIVOT_ONE;
+    sh.d[k - c0] = d;
+    sh.kind[k - c0] = PIVOT_ONE;
+  }
+  blk.sync();
+  for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
+    if (r <= k) continue;
+    const double l = col[r];
+    for (int j = k + 1; j < stop; ++j) {
+      double &v = sh.held[j - base][r - c0];
+      v = sub(v, mul(l, sh.next[j - base]));
+    }
+  }
+}
+
 // A 2 x 2 pivot at k, k + 1 from the current columns a (k) and b (k + 1) (Block::two,
 // ldlt.rs:223-248).
 template <class Block>
 FC_LDLT_FN void two(Block &blk, Shared &sh, const Front &f, int c0, int k, const double *a, const double *b) {
   const double d11 = a[k], d21 = a[k + 1], d22 = b[k + 1];
   const double det = sub(mul(d11, d22), mul(d21, d21));
-  for (int64_t r = k + 2 + blk.tid(); r < f.m; r += blk.size()) {
+  for (int r = k + 2 + blk.tid(); r < f.w; r += blk.size()) {
     const double x = a[r], y = b[r];
     at(f, r, k) = sub(mul(x, d22), mul(y, d21)) / det;
     at(f, r, k + 1) = sub(mul(y, d11), mul(x, d21)) / det;
@@ -252,20 +352,42 @@ FC_LDLT_FN void two(Block &blk, Shared &sh, const Front &f, int c0, int k, const
   blk.sync();
 }
 
-// The panel from column c0 (Block::panel, ldlt.rs:250-335). Returns -1, or the own column (the
-// structure's order) found singular; *end receives where the panel ended and *twos the 2 x 2
-// pivots it made. Every thread returns the same.
+// The panel from column c0 on the own rows (Block::panel, ldlt.rs:250-335): its pivots, L of the rows
+// [c0, w), and the interchanges of all rows. Returns -1, or the own column (the structure's order) found
+// singular; *end receives where the panel ended and *twos the 2 x 2 pivots it made. Every thread returns
+// the same.
+//
+// The next HELD columns are kept up to date in `held`, so that a column which is a pivot where it stands
+// (the usual one) is there when its turn comes: formed when it is looked at, its chain of up to 64
+// subtractions and the loads for it were most of a column's time. An interchange may move any of them:
+// the columns after it are formed anew, first two of them, then four, then HELD.
 template <class Block>
-FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_out, int *twos) {
+FC_LDLT_FN int panel_own(Block &blk, Shared &sh, const Front &f, int c0, int *end_out, int *twos) {
   const int w = f.w;
   const int end = c0 + PANEL < w ? c0 + PANEL : w;
-  double *a = f.a, *b = f.b;
-  int k = c0;
+  const bool holds = w - c0 <= HELD_ROWS;
+  double *a = holds ? sh.ab[0] - c0 : f.a, *b = holds ? sh.ab[1] - c0 : f.b;
+  int k = c0, base = c0, stop = c0, ahead = HELD;
   *twos = 0;
   while (k < end) {
     int r0;
     double omega_k;
-    const bool numbers = current(blk, sh, f, c0, k, k, a, k + 1, -1, r0, omega_k);
+    bool numbers;
+    if (holds) {
+      if (k >= stop) {
+        const int count = end - k < ahead ? end - k : ahead;
+        if (count > 4)
+          hold<8>(blk, sh, f, c0, k, count);
+        else if (count > 2)
+          hold<4>(blk, sh, f, c0, k, count);
+        else
+          hold<2>(blk, sh, f, c0, k, count);
+        base = k, stop = k + count, ahead = HELD < 2 * ahead ? HELD : 2 * ahead;
+      }
+      numbers = held_column(blk, sh, f, c0, k, base, a, r0, omega_k);
+    } else {
+      numbers = current(blk, sh, f, c0, k, k, a, k + 1, -1, r0, omega_k);
+    }
     const double akk = magnitude(a[k]);
     if (!finite(akk) || !numbers || !finite(omega_k)) return f.order[k];
     bool pair = false;
@@ -301,7 +423,12 @@ FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_ou
     if (!pair) {
       interchange(blk, f, k, p, a, b);
       if (!(magnitude(a[k]) > PIVOT_TOLERANCE * f.scale[f.order[k]])) return f.order[k];
-      one(blk, sh, f, c0, k, a);
+      if (holds && p == k) {
+        one_held(blk, sh, f, c0, k, base, stop, a);
+      } else {
+        one(blk, sh, f, c0, k, a);
+        stop = k, ahead = 2;
+      }
       k += 1;
     } else {
       // i to k, then r to k + 1 (r was at k if i took its place)
@@ -313,11 +440,47 @@ FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_ou
       if (!(offdiagonal > PIVOT_TOLERANCE * size)) return f.order[k];
       two(blk, sh, f, c0, k, a, b);
       *twos += 1;
+      stop = k, ahead = 2;
       k += 2;
     }
   }
   *end_out = k;
   return -1;
+}
+
+// L of the rows [max(r0, w), r1) over the panel's columns [c0, c1), from panel_own's pivots (sh.d, e and
+// kind): each row's entries by themselves, with the operations and the order of one(), two() and
+// current(). (The device's kernel, which keeps a row in registers, is in ldlt.cu.)
+template <class Block>
+FC_LDLT_FN void panel_below(Block &blk, const Shared &sh, const Front &f, int c0, int c1, int64_t r0, int64_t r1) {
+  for (int64_t r = (r0 > f.w ? r0 : f.w) + blk.tid(); r < r1; r += blk.size()) {
+    auto value = [&](int k, int len) {
+      double v = at(f, r, c0 + k);
+      for (int q = 0; q < len; ++q) v = sub(v, mul(at(f, r, c0 + q), times_d(sh, f, c0, c0 + k, q)));
+      return v;
+    };
+    for (int k = 0; k < c1 - c0; ++k) {
+      const double x = value(k, k);
+      if (sh.kind[k] == PIVOT_FIRST) {
+        const double y = value(k + 1, k), d11 = sh.d[k], d21 = sh.e[k], d22 = sh.d[k + 1];
+        const double det = sub(mul(d11, d22), mul(d21, d21));
+        at(f, r, c0 + k) = sub(mul(x, d22), mul(y, d21)) / det;
+        at(f, r, c0 + k + 1) = sub(mul(y, d11), mul(x, d21)) / det;
+        ++k;
+      } else {
+        at(f, r, c0 + k) = x / sh.d[k];
+      }
+    }
+  }
+  blk.sync();
+}
+
+// Both: the whole panel on one block.
+template <class Block>
+FC_LDLT_FN int panel(Block &blk, Shared &sh, const Front &f, int c0, int *end_out, int *twos) {
+  const int singular = panel_own(blk, sh, f, c0, end_out, twos);
+  if (singular < 0) panel_below(blk, sh, f, c0, *end_out, f.w, f.m);
+  return singular;
 }
 
 // W = L D for the rows [c1, w) over the panel's columns [c0, c1): the coefficients of the update
