@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 LENGTHS = [0, 1, 2, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 80, 81, 82, 112, 113, 200]
 
 
-@pytest.mark.parametrize("nrhs", [1, 2, 3, 4, 5, 8, 9, 64, 65])
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65])
 def test_rows_of_every_length(cuda, nrhs):
     torch = cuda
     rng = np.random.default_rng(nrhs)
