@@ -1441,50 +1441,53 @@ __global__ void permute_out_kernel(const int64_t *__restrict__ perm, int64_t n, 
   }
 }
 
-// y = A x with x and y row-major (n x R: a row's right-hand sides contiguous): one warp per row and
-// block of 64 right-hand sides, two a lane, the row's entries in order (index and value the same
-// for the whole warp, the x row of each entry read as 512 contiguous bytes; four entries in
-// flight). Each output is one thread's sum over the row in entry order, whatever R is.
+// y = A x with x and y row-major (n x R: a row's right-hand sides contiguous): LANES lanes a row and
+// block of LANES COLS right-hand sides, COLS a lane, the row's entries in order (index and value the
+// same for the row's lanes, the x row of each entry read as contiguous bytes; AHEAD entries in flight).
+// Each output is one thread's sum over the row in entry order, whatever R is. Bound by the reads of x
+// from L2 and by the instructions of a warp, so a row has no more lanes than columns (a warp a row and
+// two columns a lane at every R took 271 us for 10.4 M entries and R = 16, this 125).
+template <int LANES, int COLS, int AHEAD>
 __global__ void __launch_bounds__(256) spmv_rows_kernel(int64_t n, const int64_t *__restrict__ ptr,
                                                         const int32_t *__restrict__ idx,
                                                         const double *__restrict__ val,
                                                         const double *__restrict__ x, double *__restrict__ y, int R) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x % LANES;
+  const int64_t row = blockIdx.x * (int64_t)(256 / LANES) + threadIdx.x / LANES;
   if (row >= n) return;
-  const int ja = blockIdx.y * 64 + lane, jb = ja + 32;
-  const bool oka = ja < R, okb = jb < R;
-  double a0 = 0.0, a1 = 0.0;
+  const int j0 = blockIdx.y * (LANES * COLS) + lane;
+  double sum[COLS];
+  bool on[COLS];
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) sum[c] = 0.0, on[c] = j0 + c * LANES < R;
   const int64_t e1 = ptr[row + 1];
   int64_t e = ptr[row];
-  for (; e + 3 < e1; e += 4) {
-    int c[4];
-    double v[4], xa[4], xb[4];
+  for (; e + AHEAD <= e1; e += AHEAD) {
+    int col[AHEAD];
+    double v[AHEAD], xs[AHEAD][COLS];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      c[q] = idx[e + q];
-      v[q] = val[e + q];
+    for (int q = 0; q < AHEAD; ++q) col[q] = idx[e + q], v[q] = val[e + q];
+#pragma unroll
+    for (int q = 0; q < AHEAD; ++q) {
+      const double *xr = x + (int64_t)col[q] * R + j0;
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) xs[q][c] = on[c] ? xr[c * LANES] : 0.0;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double *xr = x + (int64_t)c[q] * R;
-      xa[q] = oka ? xr[ja] : 0.0;
-      xb[q] = okb ? xr[jb] : 0.0;
-    }
+    for (int q = 0; q < AHEAD; ++q)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      a0 = fma(v[q], xa[q], a0);
-      a1 = fma(v[q], xb[q], a1);
-    }
+      for (int c = 0; c < COLS; ++c) sum[c] = fma(v[q], xs[q][c], sum[c]);
   }
   for (; e < e1; ++e) {
     const double v = val[e];
-    const double *xr = x + (int64_t)idx[e] * R;
-    if (oka) a0 = fma(v, xr[ja], a0);
-    if (okb) a1 = fma(v, xr[jb], a1);
+    const double *xr = x + (int64_t)idx[e] * R + j0;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+      if (on[c]) sum[c] = fma(v, xr[c * LANES], sum[c]);
   }
-  if (oka) y[row * R + ja] = a0;
-  if (okb) y[row * R + jb] = a1;
+#pragma unroll
+  for (int c = 0; c < COLS; ++c)
+    if (on[c]) y[row * R + j0 + c * LANES] = sum[c];
 }
 
 // dst (n x R row-major) <- src (column-major, leading dimension ld), and back: 32 x 32 tiles
@@ -1883,8 +1886,19 @@ void launch_spmv(int64_t n, const int64_t *ptr, const int32_t *idx, const double
     double *xr = scratch, *yr = scratch + n * R;
     const dim3 tgrid((unsigned)((n + 31) / 32), (unsigned)((R + 31) / 32));
     to_rows_kernel<<<tgrid, 256, 0, st>>>(n, R, x, ldx, xr);
-    spmv_rows_kernel<<<dim3((unsigned)((n + 7) / 8), (unsigned)((R + 63) / 64)), 256, 0, st>>>(n, ptr, idx, val, xr,
-                                                                                              yr, R);
+    auto rows = [&](auto kernel, int lanes, int cols) {
+      const int64_t per = 256 / lanes;
+      const dim3 grid((unsigned)((n + per - 1) / per), (unsigned)((R + cols - 1) / cols));
+      kernel<<<grid, 256, 0, st>>>(n, ptr, idx, val, xr, yr, R);
+    };
+    if (R <= 8)
+      rows(spmv_rows_kernel<8, 1, 8>, 8, 8);
+    else if (R <= 16)
+      rows(spmv_rows_kernel<16, 1, 8>, 16, 16);
+    else if (R <= 32)
+      rows(spmv_rows_kernel<32, 1, 8>, 32, 32);
+    else
+      rows(spmv_rows_kernel<32, 2, 4>, 32, 64);
     to_cols_kernel<<<tgrid, 256, 0, st>>>(n, R, yr, y, ldy);
     return;
   }
