@@ -20,10 +20,10 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 constexpr float SLOPE = 0.05f;  // leaky ReLU: x for x > 0, SLOPE x otherwise
 __device__ __forceinline__ float gate(float mask) { return mask > 0.f ? 1.f : SLOPE; }
-constexpr int TX = 8, TY = 8;            // a weight gradient's tile: 8 x 8 voxels of a z plane
-constexpr int HX = TX + 2, HY = TY + 2;  // its input halo, with a plane more on either side in z
-constexpr int HV_DW = HX * HY * 3;
-constexpr int DW_THREADS = 9 * 32;
+// A weight gradient's tile: tx x ty voxels of a z plane, DW_VOXELS at most (DwTile); with the input's
+// halo, a plane more on either side in z too, DW_HALO voxels at most.
+constexpr int DW_VOXELS = 128, DW_HALO = 560;
+__host__ __device__ constexpr int dw_threads(int cout) { return 9 * (cout / 16) * 32; }
 // A convolution's CTA: twelve warps of one or two groups of 16 voxels, so that a tile is 384 voxels at
 // most (ConvTile), and the most voxels of a tile with its halo: two of them and the weights in 227 KB.
 constexpr int CONV_WARPS = 12, CONV_THREADS = 32 * CONV_WARPS;
@@ -66,18 +66,21 @@ __host__ __device__ constexpr size_t conv_smem(int buffers, int halo) {
   return sizeof(bf16) * cstride(CIN) * ((size_t)27 * COUT + (size_t)buffers * halo);
 }
 
-// The halo of a tile (planes [z - 1, z - 1 + PLANES) of one grid of the batch) into shared memory,
-// zero outside the grid.
-template <int CIN, int PLANES, int THREADS>
-__device__ __forceinline__ void load_halo(bf16 *ts, const Grid &g, const bf16 *in, int x0, int y0, int z) {
+// The halo of the tile at (x0, y0, z0), hx x hy x planes voxels from one before each, into shared
+// memory, zero outside the grid: a row of hx voxels a warp at a time.
+template <int CIN, int WARPS>
+__device__ __forceinline__ void load_halo(bf16 *ts, const Grid &g, const bf16 *in, int x0, int y0, int z0, int hx,
+                                          int hy, int planes) {
   constexpr int CS = cstride(CIN);
-  for (int e = threadIdx.x; e < HX * HY * PLANES * (CIN / 8); e += THREADS) {
-    const int hv = e / (CIN / 8), c8 = e % (CIN / 8);
-    const int hx = hv % HX, hy = (hv / HX) % HY, hz = hv / (HX * HY);
-    const int gx = x0 + hx - 1, gy = y0 + hy - 1, gz = z + hz - 1;
-    const bool ok = gx >= 0 && gx < g.X && gy >= 0 && gy < g.Y && gz >= 0 && gz < g.Z;
-    const int64_t v = ok ? ((int64_t)gz * g.Y + gy) * g.X + gx : 0;
-    cp16(ts + hv * CS + c8 * 8, in + v * CIN + c8 * 8, ok);
+  for (int row = threadIdx.x >> 5; row < hy * planes; row += WARPS) {
+    const int gy = y0 - 1 + row % hy, gz = z0 - 1 + row / hy;
+    const bool in_grid = gy >= 0 && gy < g.Y && gz >= 0 && gz < g.Z;
+    const int64_t v = in_grid ? ((int64_t)gz * g.Y + gy) * g.X : 0;
+    for (int e = threadIdx.x & 31; e < hx * (CIN / 8); e += 32) {
+      const int x = e / (CIN / 8), c8 = e % (CIN / 8), gx = x0 - 1 + x;
+      const bool ok = in_grid && gx >= 0 && gx < g.X;
+      cp16(ts + (row * hx + x) * CS + c8 * 8, in + (ok ? (v + gx) * CIN + c8 * 8 : 0), ok);
+    }
   }
 }
 
@@ -160,21 +163,10 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
             ntz = (g.Z + tile.tz - 1) / tile.tz;
   const int ntiles = ntx * nty * ntz;
   const int64_t total = (int64_t)ntiles * batch, voxels = g.voxels();
-  // a halo row (hx voxels) a warp at a time, zero outside the grid
   auto load = [&](int64_t t, bf16 *ts) {
     const int i = (int)(t % ntiles);
-    const bf16 *src = in + t / ntiles * voxels * CIN;
-    const int x0 = i % ntx * tile.tx - 1, y0 = i / ntx % nty * tile.ty - 1, z0 = i / (ntx * nty) * tile.tz - 1;
-    for (int row = warp; row < hy * (tile.tz + 2); row += CONV_WARPS) {
-      const int gy = y0 + row % hy, gz = z0 + row / hy;
-      const bool in_grid = gy >= 0 && gy < g.Y && gz >= 0 && gz < g.Z;
-      const int64_t v = in_grid ? ((int64_t)gz * g.Y + gy) * g.X : 0;
-      for (int e = lane; e < hx * (CIN / 8); e += 32) {
-        const int x = e / (CIN / 8), c8 = e % (CIN / 8), gx = x0 + x;
-        const bool ok = in_grid && gx >= 0 && gx < g.X;
-        cp16(ts + (row * hx + x) * CS + c8 * 8, src + (ok ? (v + gx) * CIN + c8 * 8 : 0), ok);
-      }
-    }
+    load_halo<CIN, CONV_WARPS>(ts, g, in + t / ntiles * voxels * CIN, i % ntx * tile.tx, i / ntx % nty * tile.ty,
+                               i / (ntx * nty) * tile.tz, hx, hy, tile.tz + 2);
   };
   pdl_wait();
   pdl_trigger();
@@ -222,55 +214,59 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
 }
 
 // Weight gradient: CTA blockIdx.x takes a chunk of one pair's tiles (a pair: `passes` grids of the
-// batch, whose gradients add), warp w the three taps along x at (dy, dz) = (w % 3 - 1, w / 3 - 1),
-// each the GEMM dW_tap (COUT x CIN) += dY^T (COUT x voxels) X_tap (voxels x CIN), both operands
-// read transposed by ldmatrix.trans from channels-last tiles and dY's fragments shared by the
-// three. Warp 4 also multiplies dY^T by ones: the bias gradient. A chunk's partial is 28 blocks of
-// COUT x CIN floats, the taps' and one whose first COUT are the bias's. The next tile's copies are
-// in flight while a tile is multiplied (16 passes on a 33 x 33 x 9 grid: 53 us, with one buffer 56). A
-// warp a tap, seven CTAs a chunk, read every tile seven times; a pass at a time, its 8 us launch was
-// latency, 16 of them 131 us.
+// batch, whose gradients add), warp w sixteen output channels (w / 9) of the three taps along x at
+// (dy, dz) = (w % 9 % 3 - 1, w % 9 / 3 - 1), each the GEMM dW_tap (COUT x CIN) += dY^T (COUT x voxels)
+// X_tap (voxels x CIN), both operands read transposed by ldmatrix.trans from channels-last tiles and
+// dY's fragments shared by the three. The fifth warp of each nine also multiplies dY^T by ones: the bias
+// gradient. A chunk's partial is 28 blocks of COUT x CIN floats, the taps' and one whose first COUT are
+// the bias's. A tile's voxels, x fastest, are taken 16 by 16 wherever they lie in it, so a tile fits the
+// grid (8 x 8 voxels: on a 33 x 33 plane a third of the products were outside it); past its last one dY
+// is zero. The next tile's copies are in flight while a tile is multiplied. Nine warps with all the
+// channels, 100 accumulators a thread, left one of the four schedulers three warps and the others two:
+// 16 passes on a 33 x 33 x 9 grid took 53 us with both, 30 so. Bound by the fragments' shared-memory
+// reads and the tensor pipe.
+struct DwTile {
+  int tx, ty, tiles;  // tiles: of one pair, all its passes
+};
 template <int CIN, int COUT>
 __host__ __device__ constexpr size_t dw_smem() {
-  return 2 * sizeof(bf16) * ((size_t)HV_DW * cstride(CIN) + (size_t)TX * TY * cstride(COUT));
+  return 2 * sizeof(bf16) * ((size_t)DW_HALO * cstride(CIN) + (size_t)DW_VOXELS * cstride(COUT));
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(DW_THREADS) conv3_dw_kernel(Grid g, int passes, int chunks,
-                                                              const bf16 *__restrict__ in,
-                                                              const bf16 *__restrict__ dy, float *__restrict__ part) {
-  constexpr int CS = cstride(CIN), DS = cstride(COUT);
+__global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTile tile, int chunks,
+                                                                   const bf16 *__restrict__ in,
+                                                                   const bf16 *__restrict__ dy,
+                                                                   float *__restrict__ part, int passes) {
+  constexpr int CS = cstride(CIN), DS = cstride(COUT), THREADS = dw_threads(COUT);
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int BUFFER = HV_DW * CS + TX * TY * DS;
+  constexpr int BUFFER = DW_HALO * CS + DW_VOXELS * DS;
   bf16 *buffers = reinterpret_cast<bf16 *>(smem);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ int place[DW_VOXELS];  // where a voxel of the tile lies in its halo
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, unit = warp % 9, mt = warp / 9;
   const int gq = lane >> 2, tg = lane & 3, q = lane >> 3, r = lane & 7;
-  const int dyo = warp % 3 - 1, dz = warp / 3 - 1;
-  const int ntx = (g.X + TX - 1) / TX, nty = (g.Y + TY - 1) / TY;
+  const int hx = tile.tx + 2, hy = tile.ty + 2, here = tile.tx * tile.ty, steps = (here + 15) / 16;
+  const int ntx = (g.X + tile.tx - 1) / tile.tx, nty = (g.Y + tile.ty - 1) / tile.ty;
   const int ntiles = ntx * nty * g.Z;
   const int pair = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
   const int64_t total = (int64_t)ntiles * passes, per = (total + chunks - 1) / chunks, voxels = g.voxels();
-  float acc[3][COUT / 16][CIN / 8][4];
-  float sum[COUT / 16][4];
-#pragma unroll
-  for (int mt = 0; mt < COUT / 16; ++mt) {
-    sum[mt][0] = sum[mt][1] = sum[mt][2] = sum[mt][3] = 0.f;
-#pragma unroll
-    for (int t = 0; t < 3; ++t)
-#pragma unroll
-      for (int nt = 0; nt < CIN / 8; ++nt) acc[t][mt][nt][0] = acc[t][mt][nt][1] = acc[t][mt][nt][2] = acc[t][mt][nt][3] = 0.f;
-  }
   const int64_t t0 = chunk * per, t1 = min(total, t0 + per);
+  for (int m = tid; m < DW_VOXELS; m += THREADS) place[m] = m < here ? (m / tile.tx * hx + m % tile.tx) * CS : 0;
+  float acc[3][CIN / 8][4], sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+#pragma unroll
+    for (int nt = 0; nt < CIN / 8; ++nt) acc[t][nt][0] = acc[t][nt][1] = acc[t][nt][2] = acc[t][nt][3] = 0.f;
   auto load = [&](int64_t t) {
-    bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + HV_DW * CS;
-    const int tile = (int)(t % ntiles);
+    bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + DW_HALO * CS;
+    const int i = (int)(t % ntiles);
     const int64_t base = ((int64_t)pair * passes + t / ntiles) * voxels;
-    const int x0 = (tile % ntx) * TX, y0 = ((tile / ntx) % nty) * TY, z = tile / (ntx * nty);
-    load_halo<CIN, 3, DW_THREADS>(ts, g, in + base * CIN, x0, y0, z);
-    for (int e = tid; e < TX * TY * (COUT / 8); e += DW_THREADS) {
+    const int x0 = i % ntx * tile.tx, y0 = i / ntx % nty * tile.ty, z = i / (ntx * nty);
+    load_halo<CIN, THREADS / 32>(ts, g, in + base * CIN, x0, y0, z, hx, hy, 3);
+    for (int e = tid; e < 16 * steps * (COUT / 8); e += THREADS) {
       const int m = e / (COUT / 8), c8 = e % (COUT / 8);
-      const int gx = x0 + m % TX, gy = y0 + m / TX;
-      const bool ok = gx < g.X && gy < g.Y;
+      const int gx = x0 + m % tile.tx, gy = y0 + m / tile.tx;
+      const bool ok = m < here && gx < g.X && gy < g.Y;
       const int64_t v = base + (ok ? ((int64_t)z * g.Y + gy) * g.X + gx : 0);
       cp16(ds + m * DS + c8 * 8, dy + v * COUT + c8 * 8, ok);
     }
@@ -282,54 +278,41 @@ __global__ void __launch_bounds__(DW_THREADS) conv3_dw_kernel(Grid g, int passes
     commit();
     asm volatile("cp.async.wait_group 1;\n" ::);
     __syncthreads();
-    const bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + HV_DW * CS;
+    const bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + DW_HALO * CS;
+    const bf16 *rows = ts + (unit / 3 * hy + unit % 3) * hx * CS + (q >> 1) * 8;
+#pragma unroll 2
+    for (int ks = 0; ks < steps; ++ks) {
+      uint32_t a[4];  // rows: voxel ks 16 + (q >> 1) 8 + r; columns: channel
+      ldsm_x4_t(a, ds + (ks * 16 + (q >> 1) * 8 + r) * DS + mt * 16 + (q & 1) * 8);
+      if (unit == 4) mma_bf16(sum, a, 0x3f803f80u, 0x3f803f80u);  // ones
+      const bf16 *brow = rows + place[ks * 16 + (q & 1) * 8 + r];  // B row: the voxel, shifted by the tap
 #pragma unroll
-    for (int ks = 0; ks < TX * TY / 16; ++ks) {
-      uint32_t a[COUT / 16][4];
-#pragma unroll
-      for (int mt = 0; mt < COUT / 16; ++mt)  // rows: voxel ks 16 + (q >> 1) 8 + r; columns: channel
-        ldsm_x4_t(a[mt], ds + (ks * 16 + (q >> 1) * 8 + r) * DS + mt * 16 + (q & 1) * 8);
-      if (warp == 4) {
-#pragma unroll
-        for (int mt = 0; mt < COUT / 16; ++mt) mma_bf16(sum[mt], a[mt], 0x3f803f80u, 0x3f803f80u);  // ones
-      }
-      const int k = ks * 16 + (q & 1) * 8 + r;  // B row: voxel k of the tile, shifted by the tap
-#pragma unroll
-      for (int dx = 0; dx < 3; ++dx) {
-        const bf16 *brow = ts + (((1 + dz) * HY + (1 + k / TX + dyo)) * HX + (k % TX + dx)) * CS;
+      for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
         for (int np = 0; np < CIN / 16; ++np) {
           uint32_t b[4];
-          ldsm_x4_t(b, brow + (2 * np + (q >> 1)) * 8);
-#pragma unroll
-          for (int mt = 0; mt < COUT / 16; ++mt) {
-            mma_bf16(acc[dx][mt][2 * np], a[mt], b[0], b[1]);
-            mma_bf16(acc[dx][mt][2 * np + 1], a[mt], b[2], b[3]);
-          }
+          ldsm_x4_t(b, brow + dx * CS + np * 16);
+          mma_bf16(acc[dx][2 * np], a, b[0], b[1]);
+          mma_bf16(acc[dx][2 * np + 1], a, b[2], b[3]);
         }
-      }
     }
     __syncthreads();
   }
   float *chunk_part = part + (int64_t)blockIdx.x * 28 * COUT * CIN;
 #pragma unroll
   for (int dx = 0; dx < 3; ++dx) {
-    float *dst = chunk_part + (3 * warp + dx) * COUT * CIN;  // tap dx + 3 (dy + 3 dz)
+    float *dst = chunk_part + (3 * unit + dx) * COUT * CIN;  // tap dx + 3 (dy + 3 dz)
 #pragma unroll
-    for (int mt = 0; mt < COUT / 16; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < CIN / 8; ++nt) {
-        const int co = mt * 16 + gq, ci = nt * 8 + 2 * tg;
-        *reinterpret_cast<float2 *>(dst + co * CIN + ci) = make_float2(acc[dx][mt][nt][0], acc[dx][mt][nt][1]);
-        *reinterpret_cast<float2 *>(dst + (co + 8) * CIN + ci) = make_float2(acc[dx][mt][nt][2], acc[dx][mt][nt][3]);
-      }
-  }
-  if (warp == 4 && tg == 0)
-#pragma unroll
-    for (int mt = 0; mt < COUT / 16; ++mt) {
-      chunk_part[27 * COUT * CIN + mt * 16 + gq] = sum[mt][0];
-      chunk_part[27 * COUT * CIN + mt * 16 + gq + 8] = sum[mt][2];
+    for (int nt = 0; nt < CIN / 8; ++nt) {
+      const int co = mt * 16 + gq, ci = nt * 8 + 2 * tg;
+      *reinterpret_cast<float2 *>(dst + co * CIN + ci) = make_float2(acc[dx][nt][0], acc[dx][nt][1]);
+      *reinterpret_cast<float2 *>(dst + (co + 8) * CIN + ci) = make_float2(acc[dx][nt][2], acc[dx][nt][3]);
     }
+  }
+  if (unit == 4 && tg == 0) {
+    chunk_part[27 * COUT * CIN + mt * 16 + gq] = sum[0];
+    chunk_part[27 * COUT * CIN + mt * 16 + gq + 8] = sum[2];
+  }
 }
 
 // The chunks' partials of each pair added in a fixed order (8 threads an element take every eighth
@@ -773,6 +756,17 @@ __global__ void input_scales_kernel(int64_t n, const double *__restrict__ nrm2, 
 
 int grid_for(int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>((work + 255) / 256, 148 * 8)); }
 
+// The sides of n voxels cut in equal parts, the last one shorter: `most` at most, 3 at least.
+int sides(int n, int most, int (&out)[64]) {
+  int count = 0;
+  for (int parts = (n + most - 1) / most; parts <= n && count < 64; ++parts) {
+    const int side = (n + parts - 1) / parts;
+    if (count > 0 && side < 3) break;
+    if (count == 0 || out[count - 1] != side) out[count++] = side;
+  }
+  return count;
+}
+
 // The tile of a convolution over `batch` grids: the sides divide the grid's evenly, and of those the
 // one with the least work for the busiest SM, in groups of 16 voxels: its rounds of tiles, each its
 // groups (six at least, a lone group being latency) and about one and a half for its barriers and
@@ -780,15 +774,6 @@ int grid_for(int64_t work) { return (int)std::max<int64_t>(1, std::min<int64_t>(
 ConvTile conv_tile(const Grid &g, int batch, int sms) {
   ConvTile best{};
   double least = 0.0;
-  auto sides = [](int n, int most, int (&out)[64]) {
-    int count = 0;
-    for (int parts = (n + most - 1) / most; parts <= n && count < 64; ++parts) {
-      const int side = (n + parts - 1) / parts;
-      if (count > 0 && side < 3) break;
-      if (count == 0 || out[count - 1] != side) out[count++] = side;
-    }
-    return count;
-  };
   int xs[64], ys[64], zs[64];
   const int nx = sides(g.X, 24, xs), ny = sides(g.Y, 24, ys), nz = sides(g.Z, 16, zs);
   for (int k = 0; k < nz; ++k)
@@ -841,6 +826,38 @@ void conv3_launch(const Grid &g, int batch, const bf16 *in, const bf16 *w, const
   cudaLaunchKernelEx(&cfg, conv3_kernel<CIN, COUT>, g, batch, tile, in, w, bias, relu ? 1 : 0, mask, out);
 }
 
+// About one chunk an SM over all pairs (18 warps of 110 registers a thread: one CTA an SM).
+int chunks_of(int64_t tiles, int pairs) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (DW_PARTIALS + pairs - 1) / pairs));
+}
+
+// A weight gradient's tile: the one with the least steps of 16 voxels in its longest chunk, a tile's
+// barriers about a step.
+DwTile dw_tile(const Grid &g, int pairs, int passes) {
+  struct Known {
+    int X, Y, Z, pairs, passes;
+    DwTile tile;
+  };
+  static thread_local Known known[32] = {};
+  Known &k = known[(uint32_t)(g.X * 31 + g.Y * 17 + g.Z * 7 + pairs * 3 + passes) % 32];
+  if (k.X == g.X && k.Y == g.Y && k.Z == g.Z && k.pairs == pairs && k.passes == passes) return k.tile;
+  DwTile best{};
+  double least = 0.0;
+  int xs[64], ys[64];
+  const int nx = sides(g.X, 24, xs), ny = sides(g.Y, 24, ys);
+  for (int j = 0; j < ny; ++j)
+    for (int i = 0; i < nx; ++i) {
+      const int tx = xs[i], ty = ys[j];
+      if (tx * ty > DW_VOXELS || (tx + 2) * (ty + 2) * 3 > DW_HALO) continue;
+      const int64_t tiles = (int64_t)passes * ((g.X + tx - 1) / tx) * ((g.Y + ty - 1) / ty) * g.Z;
+      const int chunks = chunks_of(tiles, pairs);
+      const double cost = (double)((tiles + chunks - 1) / chunks) * ((tx * ty + 15) / 16 + 1.0);
+      if (best.tx == 0 || cost < least) least = cost, best = DwTile{tx, ty, (int)tiles};
+    }
+  k = Known{g.X, g.Y, g.Z, pairs, passes, best};
+  return best;
+}
+
 template <int CIN, int COUT>
 void dw_launch(const Grid &g, int pairs, int passes, const bf16 *in, const bf16 *dy, float *part, float scale,
                bool more, float *accw, float *accb, float *gw, float *gb, cudaStream_t st) {
@@ -849,8 +866,9 @@ void dw_launch(const Grid &g, int pairs, int passes, const bf16 *in, const bf16 
       cudaFuncSetAttribute(conv3_dw_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
       cudaSuccess;
   (void)configured;
-  const int chunks = dw_chunks(g, pairs, passes);
-  conv3_dw_kernel<CIN, COUT><<<pairs * chunks, DW_THREADS, smem, st>>>(g, passes, chunks, in, dy, part);
+  const DwTile tile = dw_tile(g, pairs, passes);
+  const int chunks = chunks_of(tile.tiles, pairs);
+  conv3_dw_kernel<CIN, COUT><<<pairs * chunks, dw_threads(COUT), smem, st>>>(g, tile, chunks, in, dy, part, passes);
   const int elements = 27 * CIN * COUT + COUT;
   dw_reduce_kernel<<<(elements + REDUCE_ELEMENTS - 1) / REDUCE_ELEMENTS, REDUCE_WAYS * REDUCE_ELEMENTS, 0, st>>>(
       pairs, chunks, 27 * CIN * COUT, COUT, (int64_t)28 * CIN * COUT, part, scale, more ? 1 : 0, accw, accb, gw, gb);
@@ -870,11 +888,7 @@ void conv3(const Grid &g, int batch, int cin, int cout, const __nv_bfloat16 *in,
     conv3_launch<16, 16>(g, batch, in, w, bias, relu, mask, out, st);
 }
 
-// About one chunk an SM over all pairs (9 warps and 100 accumulators a thread: one CTA an SM).
-int dw_chunks(const Grid &g, int pairs, int passes) {
-  const int64_t tiles = (int64_t)passes * ((g.X + TX - 1) / TX) * ((g.Y + TY - 1) / TY) * g.Z;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (DW_PARTIALS + pairs - 1) / pairs));
-}
+int dw_chunks(const Grid &g, int pairs, int passes) { return chunks_of(dw_tile(g, pairs, passes).tiles, pairs); }
 
 void conv3_dw(const Grid &g, int cin, int cout, int pairs, int passes, const __nv_bfloat16 *in,
               const __nv_bfloat16 *dy, float *part, float scale, bool more, float *accw, float *accb, float *gw,
