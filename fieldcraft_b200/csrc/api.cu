@@ -750,6 +750,30 @@ void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::v
   join();
 }
 
+// The events of the program's launches that others wait for, and the lanes' streams.
+int create_lanes(fc_chol *h, fc_status *st) {
+  cudaError_t e = cudaSuccess;
+  for (cudaEvent_t ev : h->lane_events)
+    if (ev) cudaEventDestroy(ev);
+  h->lane_events.assign(h->program.size(), nullptr);
+  for (size_t q = 0; q < h->program.size(); ++q)
+    if (h->program[q].record && (e = cudaEventCreateWithFlags(&h->lane_events[q], cudaEventDisableTiming)) != cudaSuccess)
+      return cuda_fail(st, e, "lane events");
+  // lane 0 (the panels' chain, on the critical path) at the highest priority, lane 1 (the long
+  // updates beside it) at the lowest: a free SM takes the next panel's CTAs before more updates
+  int least = 0, greatest = 0;
+  cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  if (!h->side && ((e = cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, least)) != cudaSuccess ||
+                   (e = cudaStreamCreateWithPriority(&h->hi, cudaStreamNonBlocking, greatest)) != cudaSuccess ||
+                   (e = cudaStreamCreateWithPriority(&h->side2, cudaStreamNonBlocking, least)) != cudaSuccess ||
+                   (e = cudaEventCreateWithFlags(&h->join2_event, cudaEventDisableTiming)) != cudaSuccess ||
+                   (e = cudaEventCreateWithFlags(&h->fork_event, cudaEventDisableTiming)) != cudaSuccess ||
+                   (e = cudaEventCreateWithFlags(&h->join_event, cudaEventDisableTiming)) != cudaSuccess ||
+                   (e = cudaEventCreateWithFlags(&h->hi_join_event, cudaEventDisableTiming)) != cudaSuccess))
+    return cuda_fail(st, e, "lane stream");
+  return FC_OK;
+}
+
 // The factorisation's launch program and task arrays (again after an option changes the kernels'
 // tiles), uploaded; the captured factor graph is dropped.
 int plan_factor_upload(fc_chol *h, fc_status *st) {
@@ -844,32 +868,15 @@ int plan_factor_upload(fc_chol *h, fc_status *st) {
       (e = upload(h->d_gemm, gemm_t, stream)) != cudaSuccess)
     return cuda_fail(st, e, "upload of the plan");
   if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(st, e, "plan upload");
-  for (cudaEvent_t ev : h->lane_events)
-    if (ev) cudaEventDestroy(ev);
-  h->lane_events.assign(h->program.size(), nullptr);
-  for (size_t q = 0; q < h->program.size(); ++q)
-    if (h->program[q].record && (e = cudaEventCreateWithFlags(&h->lane_events[q], cudaEventDisableTiming)) != cudaSuccess)
-      return cuda_fail(st, e, "lane events");
-  // lane 0 (the panels' chain, on the critical path) at the highest priority, lane 1 (the long
-  // updates beside it) at the lowest: a free SM takes the next panel's CTAs before more updates
-  int least = 0, greatest = 0;
-  cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  if (!h->side && ((e = cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, least)) != cudaSuccess ||
-                   (e = cudaStreamCreateWithPriority(&h->hi, cudaStreamNonBlocking, greatest)) != cudaSuccess ||
-                   (e = cudaStreamCreateWithPriority(&h->side2, cudaStreamNonBlocking, least)) != cudaSuccess ||
-                   (e = cudaEventCreateWithFlags(&h->join2_event, cudaEventDisableTiming)) != cudaSuccess ||
-                   (e = cudaEventCreateWithFlags(&h->fork_event, cudaEventDisableTiming)) != cudaSuccess ||
-                   (e = cudaEventCreateWithFlags(&h->join_event, cudaEventDisableTiming)) != cudaSuccess ||
-                   (e = cudaEventCreateWithFlags(&h->hi_join_event, cudaEventDisableTiming)) != cudaSuccess))
-    return cuda_fail(st, e, "lane stream");
-  return FC_OK;
+  return create_lanes(h, st);
 }
 
-// The symmetric indefinite factor's program (FC_PRECISION_LDLT, one stream), per level: the
+// The symmetric indefinite factor's program (FC_PRECISION_LDLT), per level: the
 // fronts' assembly; ceil(w / 64) pivoted panel steps, each followed by the GEMM of the update
 // tasks the panel step wrote (slots sized for the earliest panel end, the rest left empty);
-// W21 = L21 D and D out of the fronts; the update matrices -L21 W21^T; the children's entries in
-// them. The panels' scratch (two columns and W per front) and W21 are reused level after level.
+// W21 = L21 D; the update matrices -L21 W21^T; the children's entries in them; and beside these and
+// the levels above (lane 2) D out of the fronts and the diagonal blocks' inverses. The panels'
+// scratch (two columns and W per front) and W21 are reused level after level.
 int plan_ldlt_upload(fc_chol *h, fc_status *st) {
   namespace L = fc::ldlt;
   if (h->factor_graph) {
@@ -1007,7 +1014,12 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
         inv_t.push_back(t);
       }
     }
+    // beside the levels above, from here on: only the solve reads the inverses, and nothing above
+    // reads a front's own block again
+    h->program.back().record = true;
+    const int ready = (int)h->program.size() - 1;
     push(h->program, K_LDLT_INVERSE, io, (int64_t)inv_t.size() - io, (int)l);
+    h->program.back().lane = 2, h->program.back().dep = ready;
     for (int hh = fc::NB; hh < fc::SB; hh *= 2) {
       std::vector<fc::GemmTask> first_t, second_t;
       inverse_doubling(h, S, h->d_T.as<double>(), hh, &first_t, &second_t);
@@ -1015,9 +1027,11 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
       int64_t d0 = (int64_t)gemm_t.size();
       gemm_t.insert(gemm_t.end(), first_t.begin(), first_t.end());
       push(h->program, K_GEMM_MIXED, d0, (int64_t)first_t.size(), (int)l);
+      h->program.back().lane = 2;
       d0 = (int64_t)gemm_t.size();
       gemm_t.insert(gemm_t.end(), second_t.begin(), second_t.end());
       push(h->program, K_GEMM_F64, d0, (int64_t)second_t.size(), (int)l);
+      h->program.back().lane = 2;
     }
     // the update matrices: U = -L21 W21^T (lower tiles)
     const int64_t go = (int64_t)gemm_t.size();
@@ -1055,9 +1069,7 @@ int plan_ldlt_upload(fc_chol *h, fc_status *st) {
       (e = upload(h->d_linv, inv_t, stream)) != cudaSuccess)
     return cuda_fail(st, e, "upload of the LDL^T plan");
   if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return cuda_fail(st, e, "plan upload");
-  for (cudaEvent_t ev : h->lane_events)
-    if (ev) cudaEventDestroy(ev);
-  h->lane_events.assign(h->program.size(), nullptr);
+  if (const int rc = create_lanes(h, st); rc != FC_OK) return rc;
   h->stree = h->tree;
   h->stree.rows = h->d_lsrows.as<int32_t>();
   h->stree.own = h->d_lown.as<int32_t>();
@@ -1484,13 +1496,13 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
     if (lanes && l.record) cudaEventRecord(h->lane_events[li], st);
     ++launches;
   }
+  join();
   if (h->ldlt) {
     fc::ldlt::launch_fold(h->n, h->d_llocal.as<int32_t>(), h->d_lorder.as<int32_t>(), h->d_perm.as<int64_t>(),
                           h->d_lown.as<int32_t>(), h->d_lsperm.as<int64_t>(), (int64_t)h->rows.size(),
                           h->d_rows.as<int32_t>(), h->d_lsrows.as<int32_t>(), user);
     h->ldlt_ready = true;
   }
-  join();
   h->last_factor_launches = launches;
   return FC_OK;
 }

@@ -1446,7 +1446,7 @@ __global__ void permute_out_kernel(const int64_t *__restrict__ perm, int64_t n, 
 // same for the row's lanes, the x row of each entry read as contiguous bytes; AHEAD entries in flight).
 // Each output is one thread's sum over the row in entry order, whatever R is. Bound by the reads of x
 // from L2 and by the instructions of a warp, so a row has no more lanes than columns (a warp a row and
-// two columns a lane at every R took 271 us for 10.4 M entries and R = 16, this 125).
+// two columns a lane at every R took 271 us for 10.4 M entries and R = 16, this 142).
 template <int LANES, int COLS, int AHEAD>
 __global__ void __launch_bounds__(256) spmv_rows_kernel(int64_t n, const int64_t *__restrict__ ptr,
                                                         const int32_t *__restrict__ idx,

@@ -156,10 +156,23 @@ __global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTa
     if (mine && 8 * t + lane < kw) at(f, r, c0 + 8 * t + lane) = g[t];
 }
 
-__global__ void __launch_bounds__(W21_ROWS) ldlt_after_kernel(const AfterTask *__restrict__ tasks) {
+// front_w21 with an element a thread at a time, eight threads a row (a thread a row, each column's
+// loads waiting for the one before: 29 us a launch).
+__global__ void __launch_bounds__(8 * W21_ROWS) ldlt_after_kernel(const AfterTask *__restrict__ tasks) {
   const AfterTask &task = tasks[blockIdx.x];
-  DeviceBlock blk;
-  front_w21(blk, task.front, task.w21, task.front.m - task.front.w, task.r0, task.r1);
+  const Front f = task.front;
+  const int64_t r = task.r0 + threadIdx.x % W21_ROWS, ld = f.m - f.w;
+  if (r >= task.r1) return;
+  double *__restrict__ out = task.w21 + (r - f.w);
+#pragma unroll 4
+  for (int k = threadIdx.x / W21_ROWS; k < f.w; k += 8) {
+    const int8_t kind = f.pivots[k];
+    const double x = at(f, r, k), d = at(f, k, k);
+    double v = mul(x, d);
+    if (kind == PIVOT_FIRST) v = add(v, mul(at(f, r, k + 1), at(f, k + 1, k)));
+    if (kind == PIVOT_SECOND) v = add(mul(at(f, r, k - 1), at(f, k, k - 1)), v);
+    out[k * ld] = v;
+  }
 }
 
 // y <- D^-1 y between the solve's forward and backward passes: n unknowns in postorder, R
@@ -268,7 +281,7 @@ void launch_panel(const PanelTask *tasks, int count, int tallest, int widest, in
 }
 
 void launch_after(const AfterTask *tasks, int count, cudaStream_t st) {
-  if (count > 0) ldlt_after_kernel<<<count, W21_ROWS, 0, st>>>(tasks);
+  if (count > 0) ldlt_after_kernel<<<count, 8 * W21_ROWS, 0, st>>>(tasks);
 }
 
 void launch_scale(int64_t nnz, const int64_t *a_src, const int32_t *a_row, const int32_t *a_col, const double *val,

@@ -24,7 +24,7 @@ struct PanelTask {
 
 // After a level's panels: rows [r0, r1) of a front's W21 = L21 D into w21 (leading dimension
 // m - w, for the update-matrix GEMM). A CTA takes W21_ROWS rows.
-constexpr int W21_ROWS = 64;
+constexpr int W21_ROWS = 32;
 struct AfterTask {
   Front front;
   double *w21;

@@ -116,16 +116,16 @@ FC_LDLT_FN double times_d(const Shared &sh, const Front &f, int c0, int c, int q
 template <class Block>
 FC_LDLT_ONCE bool block_best(Block &blk, Shared &sh, double bv, int bi, int bn, int lo, int none, int &index,
                              double &value) {
-  auto better = [](double x, int i, double y, int j) { return x > y || (x == y && i < j); };
 #if defined(__CUDACC__)
   const int lane = blk.tid() & 31, warps = (blk.size() + 31) >> 5;
+  // Magnitudes order as their bits do: the warp's largest in three integer reductions (the two
+  // halves' largest, then the lowest index that has both) instead of five rounds of FP64 comparisons.
   auto warp_best = [&]() {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double x = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int i = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (better(x, i, bv, bi)) bv = x, bi = i;
-    }
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(bv);
+    const unsigned high = (unsigned)(bits >> 32), top = __reduce_max_sync(0xffffffffu, high);
+    const unsigned low = high == top ? (unsigned)bits : 0u, below = __reduce_max_sync(0xffffffffu, low);
+    bi = __reduce_min_sync(0xffffffffu, high == top && low == below ? bi : 0x7fffffff);
+    bv = __longlong_as_double((long long)((unsigned long long)top << 32 | below));
     bn = __any_sync(0xffffffffu, bn);
   };
   warp_best();
@@ -140,6 +140,7 @@ FC_LDLT_ONCE bool block_best(Block &blk, Shared &sh, double bv, int bi, int bn, 
   bn = lane < warps ? sh.nan[lane] : 0;
   warp_best();
 #else
+  auto better = [](double x, int i, double y, int j) { return x > y || (x == y && i < j); };
   sh.best_v[blk.tid()] = bv;
   sh.best_i[blk.tid()] = bi;
   sh.nan[blk.tid()] = bn;
@@ -373,6 +374,7 @@ FC_LDLT_FN int panel_own(Block &blk, Shared &sh, const Front &f, int c0, int *en
     int r0;
     double omega_k;
     bool numbers;
+    const double limit = PIVOT_TOLERANCE * f.scale[f.order[k]];  // column k's, read while it is looked at
     if (holds) {
       if (k >= stop) {
         const int count = end - k < ahead ? end - k : ahead;
@@ -422,7 +424,7 @@ FC_LDLT_FN int panel_own(Block &blk, Shared &sh, const Front &f, int c0, int *en
     }
     if (!pair) {
       interchange(blk, f, k, p, a, b);
-      if (!(magnitude(a[k]) > PIVOT_TOLERANCE * f.scale[f.order[k]])) return f.order[k];
+      if (!(magnitude(a[k]) > (p == k ? limit : PIVOT_TOLERANCE * f.scale[f.order[k]]))) return f.order[k];
       if (holds && p == k) {
         one_held(blk, sh, f, c0, k, base, stop, a);
       } else {
