@@ -21,7 +21,8 @@ struct DeviceBlock {
 // postorder is the one reported) and ends the supernode. After the panel the CTA writes the
 // update of the later own columns as GEMM tasks (C -= L_panel W^T on the lower tiles, for the
 // launch that follows); the slots it does not need stay empty (M = N = K = 0: no work).
-__global__ void __launch_bounds__(MAX_THREADS) ldlt_panel_kernel(const PanelTask *__restrict__ tasks,
+constexpr int PANEL_THREADS = 512;
+__global__ void __launch_bounds__(PANEL_THREADS) ldlt_panel_kernel(const PanelTask *__restrict__ tasks,
                                                                  int32_t *__restrict__ pos,
                                                                  int32_t *__restrict__ from,
                                                                  int32_t *__restrict__ twos,
@@ -265,7 +266,7 @@ void launch_fold(int64_t n, const int32_t *local, const int32_t *order, const in
   if (rows_len > 0) ldlt_rows_kernel<<<grid_for(rows_len, 256), 256, 0, st>>>(rows_len, rows, own, rows_out);
 }
 
-// A thread an own row up to 1024: a column step is a chain of loads and barriers, bound by their
+// A thread an own row up to 512: a column step is a chain of loads and barriers, bound by their
 // latency, and the rows below would make it longer (they are most of a front's rows, and a CTA has one
 // SM's FP64 units): they come after it, all of a level's together. Panels of 16 x 14 x 13 elements:
 // 12.1 ms on all rows with each column formed when it is looked at (3.3 us a column on the longest
@@ -273,7 +274,7 @@ void launch_fold(int64_t n, const int32_t *local, const int32_t *order, const in
 void launch_panel(const PanelTask *tasks, int count, int tallest, int widest, int32_t *pos, int32_t *from,
                   int32_t *twos, unsigned long long *failed, cudaStream_t st) {
   if (count <= 0) return;
-  const int threads = widest >= MAX_THREADS ? MAX_THREADS : widest <= 64 ? 64 : (widest + 31) / 32 * 32;
+  const int threads = widest >= PANEL_THREADS ? PANEL_THREADS : widest <= 64 ? 64 : (widest + 31) / 32 * 32;
   cudaFuncSetAttribute(ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
   ldlt_panel_kernel<<<count, threads, sizeof(Shared), st>>>(tasks, pos, from, twos, failed);
   const dim3 grid(count, (tallest + BELOW_ROWS - 1) / BELOW_ROWS);

@@ -78,7 +78,7 @@ struct Shared {
   double d[PANEL + 1];     // D's diagonal at the panel's factored columns
   double e[PANEL + 1];     // its subdiagonal at the first column of a 2 x 2 pivot
   int8_t kind[PANEL + 1];  // PIVOT_ONE / PIVOT_FIRST / PIVOT_SECOND
-  double rows[HELD][PANEL];       // rows of L D for the columns to hold
+  alignas(16) double rows[PANEL][HELD];  // rows of L D for the columns to hold: [column of L][row]
   double next[HELD];              // L D of the newest column at the held columns' rows
   double held[HELD][HELD_ROWS];   // the held columns, own rows from the panel's start
   double ab[2][HELD_ROWS];        // Front's a and b, own rows from the panel's start
@@ -209,8 +209,8 @@ template <int COUNT, class Block>
 FC_LDLT_FN void hold(Block &blk, Shared &sh, const Front &f, int c0, int k, int count) {
   const int len = k - c0;
   for (int e = blk.tid(); e < COUNT * PANEL; e += blk.size()) {
-    const int j = e / PANEL, q = e % PANEL;
-    if (q < len) sh.rows[j][q] = j < count ? times_d(sh, f, c0, k + j, q) : 0.0;
+    const int j = e % COUNT, q = e / COUNT;
+    if (q < len) sh.rows[q][j] = j < count ? times_d(sh, f, c0, k + j, q) : 0.0;
   }
   blk.sync();
   for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
@@ -220,19 +220,22 @@ FC_LDLT_FN void hold(Block &blk, Shared &sh, const Front &f, int c0, int k, int 
     for (int j = 0; j < COUNT; ++j) v[j] = j < count && r >= k + j ? at(f, r, k + j) : 0.0;
     const double *L = &at(f, r, c0);
     int q = 0;
-    for (; q + 8 <= len; q += 8) {
-      double l[8];
+    for (; q + 16 <= len; q += 16) {
+      double l[16];
       FC_LDLT_UNROLL
-      for (int t = 0; t < 8; ++t) l[t] = L[(q + t) * f.m];
+      for (int t = 0; t < 16; ++t) l[t] = L[(q + t) * f.m];
       FC_LDLT_UNROLL
-      for (int t = 0; t < 8; ++t)
+      for (int t = 0; t < 16; ++t)
         FC_LDLT_UNROLL
-        for (int j = 0; j < COUNT; ++j) v[j] = sub(v[j], mul(l[t], sh.rows[j][q + t]));
+        for (int j = 0; j < COUNT; ++j) v[j] = sub(v[j], mul(l[t], sh.rows[q + t][j]));
     }
+#if defined(__CUDACC__)
+#pragma unroll 4
+#endif
     for (; q < len; ++q) {
       const double l = L[q * f.m];
       FC_LDLT_UNROLL
-      for (int j = 0; j < COUNT; ++j) v[j] = sub(v[j], mul(l, sh.rows[j][q]));
+      for (int j = 0; j < COUNT; ++j) v[j] = sub(v[j], mul(l, sh.rows[q][j]));
     }
     FC_LDLT_UNROLL
     for (int j = 0; j < COUNT; ++j)
