@@ -122,13 +122,14 @@ __device__ __noinline__ void dense_block(double lambda, double mu, const double 
 // point, and each block goes with its mirror image to the matrix in shared memory, which is stored
 // as it lies. The terms with a structural zero of B or D add exactly nothing while everything is
 // finite and are left out; an element whose D or gradients are not finite takes them all
-// (dense_block). Bound by FP64 arithmetic and the 4.6 KB an element stores: 0.28 ms for 48 x 40 x 36
-// elements (318 MB, 1.1 TB/s). With entry_kernel and the kernels below, K, reactions and stresses of
-// that box take 0.67 ms; with one thread an element, a row, a DOF and an element each, their matrices
+// (dense_block). Bound by FP64 arithmetic and the 4.6 KB an element stores: 0.19 ms for 48 x 40 x 36
+// elements (318 MB, 1.7 TB/s) with four blocks an SM, one's gradients beside another's products (0.28
+// with two at the compiler's 128 registers a thread, 0.22 with three; five spill: 0.21). With
+// entry_kernel and the kernels below, K, reactions and stresses of that box take 0.59 ms; with one thread an element, a row, a DOF and an element each, their matrices
 // accumulated in global memory, they took 6.1 ms.
 constexpr int ELEMENTS = 6, ELEMENT_THREADS = 36 * ELEMENTS;
 
-__global__ void __launch_bounds__(ELEMENT_THREADS) element_kernel(fc::assembly::Box box, int64_t elements,
+__global__ void __launch_bounds__(ELEMENT_THREADS, 4) element_kernel(fc::assembly::Box box, int64_t elements,
                                                                   const double *__restrict__ young, double nu,
                                                                   double *__restrict__ ke, int *__restrict__ bad) {
   __shared__ double grad[ELEMENTS][8][8][3];
