@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTa
                                                                    const int32_t *__restrict__ from) {
   __shared__ double coef[PANEL + 1][8 * BELOW_HELD];  // L D at (row j, column q) of the panel's block: [q][j]
   __shared__ double d[PANEL + 1], e[PANEL + 1];
+  __shared__ double by[PANEL + 1], inv[PANEL + 1];  // what a pivot's columns are divided by, and its reciprocal
   __shared__ int8_t kind[PANEL + 1];
   const PanelTask &task = tasks[blockIdx.x];
   const Front f = task.front;
@@ -98,6 +99,10 @@ __global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTa
     e[k] = kind[k] == PIVOT_FIRST ? at(f, c0 + k + 1, c0 + k) : 0.0;
   }
   __syncthreads();
+  for (int k = threadIdx.x; k < kw; k += BELOW_THREADS) {
+    by[k] = kind[k] == PIVOT_FIRST ? sub(mul(d[k], d[k + 1]), mul(e[k], e[k])) : d[k];
+    inv[k] = reciprocal(by[k]);
+  }
   const int lane = threadIdx.x & 7;
   const int64_t r = r0 + (threadIdx.x >> 3);
   // times_d for any row past the panel's columns q
@@ -109,17 +114,25 @@ __global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTa
   };
   if (r >= c1 && r < f.w)
     for (int q = lane; q < kw; q += 8) f.W[(r - c1) + q * f.ld_w] = product(r, q);
-  if (r0 + BELOW_ROWS <= f.w) return;
-  // the panel's block below the pivots (no entry of a 2 x 2 pivot's own is read)
-  for (int x = threadIdx.x; x < (PANEL + 1) * 8 * BELOW_HELD; x += BELOW_THREADS) {
-    const int q = x / (8 * BELOW_HELD), j = x % (8 * BELOW_HELD);
-    coef[q][j] = j < kw && q < j && !(kind[q] == PIVOT_FIRST && j == q + 1) ? product(c0 + j, q) : 0.0;
-  }
-  __syncthreads();
+  if (r0 + BELOW_ROWS <= f.w || f.m == f.w) return;
   const bool mine = r >= f.w && r < f.m;
   double g[BELOW_HELD];
 #pragma unroll
   for (int t = 0; t < BELOW_HELD; ++t) g[t] = mine && 8 * t + lane < kw ? at(f, r, c0 + 8 * t + lane) : 0.0;
+  // the panel's block below the pivots (no entry of a 2 x 2 pivot's own is read), six loads at a time
+  constexpr int ENTRIES = (PANEL + 1) * 8 * BELOW_HELD, TOGETHER = 6;
+  for (int x0 = threadIdx.x; x0 < ENTRIES; x0 += TOGETHER * BELOW_THREADS) {
+    double v[TOGETHER];
+#pragma unroll
+    for (int u = 0; u < TOGETHER; ++u) {
+      const int x = x0 + u * BELOW_THREADS, q = x / (8 * BELOW_HELD), j = x % (8 * BELOW_HELD);
+      v[u] = j < kw && q < j && !(kind[q] == PIVOT_FIRST && j == q + 1) ? product(c0 + j, q) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < TOGETHER; ++u)
+      if (x0 + u * BELOW_THREADS < ENTRIES) (&coef[0][0])[x0 + u * BELOW_THREADS] = v[u];
+  }
+  __syncthreads();
 #pragma unroll
   for (int t = 0; t < BELOW_HELD; ++t) {
     for (int o = 0; o < 8 && 8 * t + o < kw; ++o) {
@@ -132,8 +145,9 @@ __global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTa
           const double z = __shfl_sync(0xffffffffu, g[t + 1 < BELOW_HELD ? t + 1 : t], 0, 8);
           if (o == 7) y = z;
         }
-        const double d11 = d[k], d21 = e[k], d22 = d[k + 1], det = sub(mul(d11, d22), mul(d21, d21));
-        const double l0 = sub(mul(x, d22), mul(y, d21)) / det, l1 = sub(mul(y, d11), mul(x, d21)) / det;
+        const double d11 = d[k], d21 = e[k], d22 = d[k + 1];
+        const double l0 = quotient(sub(mul(x, d22), mul(y, d21)), by[k], inv[k]);
+        const double l1 = quotient(sub(mul(y, d11), mul(x, d21)), by[k], inv[k]);
 #pragma unroll
         for (int u = t; u < BELOW_HELD; ++u) {
           const int j = 8 * u + lane;
@@ -142,7 +156,7 @@ __global__ void __launch_bounds__(BELOW_THREADS) ldlt_below_kernel(const PanelTa
           if (j == k + 1) g[u] = l1;
         }
       } else {
-        const double l = x / d[k];
+        const double l = quotient(x, by[k], inv[k]);
 #pragma unroll
         for (int u = t; u < BELOW_HELD; ++u) {
           const int j = 8 * u + lane;
@@ -270,7 +284,8 @@ void launch_fold(int64_t n, const int32_t *local, const int32_t *order, const in
 // latency, and the rows below would make it longer (they are most of a front's rows, and a CTA has one
 // SM's FP64 units): they come after it, all of a level's together. Panels of 16 x 14 x 13 elements:
 // 12.1 ms on all rows with each column formed when it is looked at (3.3 us a column on the longest
-// chain); 7.5 and 2.3 for the rows below.
+// chain); 7.5 and 2.3 for the rows below with eight columns held ahead; 5.2 and 1.5 with their
+// coefficients side by side and zeros kept from the division's slow way.
 void launch_panel(const PanelTask *tasks, int count, int tallest, int widest, int32_t *pos, int32_t *from,
                   int32_t *twos, unsigned long long *failed, cudaStream_t st) {
   if (count <= 0) return;

@@ -21,6 +21,7 @@
 #define FC_LDLT_UNROLL _Pragma("unroll")
 #else
 #include <cmath>
+#include <cstring>
 #define FC_LDLT_FN inline
 #define FC_LDLT_HD inline
 #define FC_LDLT_ONCE __attribute__((noinline, noclone))  // its barrier stays one call site
@@ -46,6 +47,7 @@ constexpr int8_t PIVOT_ONE = 0, PIVOT_FIRST = 1, PIVOT_SECOND = 2;
 FC_LDLT_FN double mul(double a, double b) { return __dmul_rn(a, b); }
 FC_LDLT_FN double add(double a, double b) { return __dadd_rn(a, b); }
 FC_LDLT_FN double sub(double a, double b) { return __dsub_rn(a, b); }
+FC_LDLT_FN double fused(double a, double b, double c) { return __fma_rn(a, b, c); }
 FC_LDLT_FN double magnitude(double x) { return fabs(x); }
 FC_LDLT_FN bool finite(double x) { return isfinite(x); }
 FC_LDLT_FN bool not_a_number(double x) { return isnan(x); }
@@ -53,10 +55,40 @@ FC_LDLT_FN bool not_a_number(double x) { return isnan(x); }
 FC_LDLT_FN double mul(double a, double b) { return a * b; }
 FC_LDLT_FN double add(double a, double b) { return a + b; }
 FC_LDLT_FN double sub(double a, double b) { return a - b; }
+FC_LDLT_FN double fused(double a, double b, double c) { return std::fma(a, b, c); }
 FC_LDLT_FN double magnitude(double x) { return std::fabs(x); }
 FC_LDLT_FN bool finite(double x) { return std::isfinite(x); }
 FC_LDLT_FN bool not_a_number(double x) { return std::isnan(x); }
 #endif
+
+// x / d, correctly rounded, for many x and one d, from y = reciprocal(d) (Markstein, IBM J. Res. Dev. 34,
+// 1990: with y the correctly rounded 1 / d and q within a unit of x / d in the last place, q plus the
+// exact remainder x - q d times y rounds to x / d; one such step brings x y that close, the second ends
+// it). Five dependent operations in place of a division's. Not for a significand of all ones (the
+// theorem's exception) nor where a step could leave the normal range: there the division itself.
+FC_LDLT_FN double reciprocal(double d) {
+  const double size = magnitude(d), most = 2.037035976334486e90;  // 2^300
+  if (!(size < most && size > 1.0 / most)) return 0.0;
+#if defined(__CUDACC__)
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(d);
+#else
+  unsigned long long bits;
+  std::memcpy(&bits, &d, sizeof(bits));
+#endif
+  return (bits << 12) == 0xfffffffffffff000ull ? 0.0 : 1.0 / d;
+}
+FC_LDLT_FN double quotient(double x, double d, double y) {
+  const double size = magnitude(x), most = 4.149515568880993e180;  // 2^600
+  if (!(y != 0.0 && size < most && (size > 1.0 / most || size == 0.0))) return x / d;
+  const double first = mul(x, y);
+  double q = fused(fused(-first, d, x), y, first);
+  q = fused(fused(-q, d, x), y, q);
+  return size == 0.0 ? first : q;  // (the zero's sign)
+}
+
+// x / d for a finite d other than zero: a zero's quotient apart, which the division takes its slow way
+// for (a front has many, and one lane's is its warp's).
+FC_LDLT_FN double divided(double x, double d) { return x == 0.0 ? mul(x, d) : x / d; }
 
 // One front and its per-column state.
 struct Front {
@@ -291,7 +323,7 @@ FC_LDLT_FN void interchange(Block &blk, const Front &f, int p, int q, double *a,
 template <class Block>
 FC_LDLT_FN void one(Block &blk, Shared &sh, const Front &f, int c0, int k, const double *col) {
   const double d = col[k];
-  for (int r = k + 1 + blk.tid(); r < f.w; r += blk.size()) at(f, r, k) = col[r] / d;
+  for (int r = k + 1 + blk.tid(); r < f.w; r += blk.size()) at(f, r, k) = divided(col[r], d);
   if (blk.tid() == 0) {
     at(f, k, k) = d;
     f.pivots[k] = PIVOT_ONE;
@@ -308,7 +340,7 @@ FC_LDLT_FN void one_held(Block &blk, Shared &sh, const Front &f, int c0, int k, 
   const double d = col[k];
   for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
     if (r <= k) continue;
-    const double l = col[r] / d;
+    const double l = divided(col[r], d);
     at(f, r, k) = l;
     col[r] = l;
     if (r < stop) sh.next[r - base] = mul(l, d);
@@ -323,10 +355,12 @@ FC_LDLT_FN void one_held(Block &blk, Shared &sh, const Front &f, int c0, int k, 
   for (int r = c0 + blk.tid(); r < f.w; r += blk.size()) {
     if (r <= k) continue;
     const double l = col[r];
-    for (int j = k + 1; j < stop; ++j) {
-      double &v = sh.held[j - base][r - c0];
-      v = sub(v, mul(l, sh.next[j - base]));
-    }
+    double v[HELD], y[HELD];  // every load before the stores: one after the other they are a chain
+    FC_LDLT_UNROLL
+    for (int j = 0; j < HELD; ++j) v[j] = sh.held[j][r - c0], y[j] = sh.next[j];
+    FC_LDLT_UNROLL
+    for (int j = 0; j < HELD; ++j)
+      if (j > k - base && j < stop - base) sh.held[j][r - c0] = sub(v[j], mul(l, y[j]));
   }
 }
 
@@ -468,12 +502,12 @@ FC_LDLT_FN void panel_below(Block &blk, const Shared &sh, const Front &f, int c0
       const double x = value(k, k);
       if (sh.kind[k] == PIVOT_FIRST) {
         const double y = value(k + 1, k), d11 = sh.d[k], d21 = sh.e[k], d22 = sh.d[k + 1];
-        const double det = sub(mul(d11, d22), mul(d21, d21));
-        at(f, r, c0 + k) = sub(mul(x, d22), mul(y, d21)) / det;
-        at(f, r, c0 + k + 1) = sub(mul(y, d11), mul(x, d21)) / det;
+        const double det = sub(mul(d11, d22), mul(d21, d21)), inv = reciprocal(det);
+        at(f, r, c0 + k) = quotient(sub(mul(x, d22), mul(y, d21)), det, inv);
+        at(f, r, c0 + k + 1) = quotient(sub(mul(y, d11), mul(x, d21)), det, inv);
         ++k;
       } else {
-        at(f, r, c0 + k) = x / sh.d[k];
+        at(f, r, c0 + k) = quotient(x, sh.d[k], reciprocal(sh.d[k]));
       }
     }
   }
