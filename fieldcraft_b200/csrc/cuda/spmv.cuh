@@ -14,13 +14,11 @@ constexpr int SPMV_LANES = 16;
 // sum over the row's entries of val * x[idx], on every lane of the row's group: six entries a lane in
 // flight (a whole 81-entry row at once: the chain is then row pointer, entries, x, whatever the
 // row), the lanes' sums by a butterfly. Every lane of the warp calls it; a row with ok false is empty.
-__device__ __forceinline__ double spmv_row(bool ok, int64_t row, const int64_t *__restrict__ ptr,
-                                           const int32_t *__restrict__ idx, const double *__restrict__ val,
-                                           const double *x, int lane) {
+__device__ __forceinline__ double spmv_entries(int64_t e0, int64_t e1, const int32_t *__restrict__ idx,
+                                               const double *__restrict__ val, const double *x, int lane) {
   constexpr int FLIGHT = 6;
-  const int64_t e1 = ok ? ptr[row + 1] : 0;
   double sum = 0.0;
-  for (int64_t e = ok ? ptr[row] + lane : 0; e < e1; e += FLIGHT * SPMV_LANES) {
+  for (int64_t e = e0 + lane; e < e1; e += FLIGHT * SPMV_LANES) {
     int32_t c[FLIGHT];
     double v[FLIGHT], xv[FLIGHT];
 #pragma unroll
@@ -38,6 +36,11 @@ __device__ __forceinline__ double spmv_row(bool ok, int64_t row, const int64_t *
 #pragma unroll
   for (int o = SPMV_LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, SPMV_LANES);
   return sum;
+}
+__device__ __forceinline__ double spmv_row(bool ok, int64_t row, const int64_t *__restrict__ ptr,
+                                           const int32_t *__restrict__ idx, const double *__restrict__ val,
+                                           const double *x, int lane) {
+  return spmv_entries(ok ? ptr[row] : 0, ok ? ptr[row + 1] : 0, idx, val, x, lane);
 }
 
 }  // namespace fc
