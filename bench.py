@@ -35,7 +35,7 @@ METRIC = "s to rel-res 1e-10: FP32+IR & NN-FCG vs FP64 GPU Cholesky; TFLOP/s, GB
 UNIT = "s"
 N_EL, NRHS, SEED = 48, 64, 2024
 # profile kinds (fc_chol_profile_read) and their names
-KERNEL_KINDS = [(0, "assemble"), (1, "panel"), (3, "gemm"), (12, "gemm_tcgen05"), (15, "pack_tcgen05"),
+KERNEL_KINDS = [(0, "assemble"), (1, "panel"), (2, "panel_inverse"), (3, "gemm"), (12, "gemm_tcgen05"), (15, "pack_tcgen05"),
                 (10, "inverse_products"),
                 (11, "inverse_blocks"),
                 (19, "solve_gemm"), (20, "solve_assemble"),
