@@ -35,7 +35,8 @@ METRIC = "s to rel-res 1e-10: FP32+IR & NN-FCG vs FP64 GPU Cholesky; TFLOP/s, GB
 UNIT = "s"
 N_EL, NRHS, SEED = 48, 64, 2024
 # profile kinds (fc_chol_profile_read) and their names
-KERNEL_KINDS = [(0, "assemble"), (1, "panel"), (2, "panel_inverse"), (3, "gemm"), (12, "gemm_tcgen05"), (15, "pack_tcgen05"),
+KERNEL_KINDS = [(0, "assemble"), (1, "panel"), (2, "panel_inverse"), (3, "gemm"), (12, "gemm_tcgen05"),
+                (15, "pack_tcgen05"),
                 (10, "inverse_products"),
                 (11, "inverse_blocks"),
                 (19, "solve_gemm"), (20, "solve_assemble"),
@@ -814,16 +815,7 @@ def assembly_bytes(f) -> float:
     """The front assembly's algorithmic bytes per factorisation (FP64 entries): every value of A
     read once, every child's update-matrix entry (lower triangle) read once, every front entry
     (the L trapezoid and the update matrix's lower triangle) written once."""
-    from fieldcraft_b200.cholesky import Symbolic  # noqa: F401
-    a = f.symbolic.arrays()
-    w = np.diff(a["first"]).astype(np.float64)
-    m = np.diff(a["rptr"]).astype(np.float64)
-    u = m - w
-    lower_u = u * (u + 1) / 2
-    trap = w * m - w * (w - 1) / 2
-    has_parent = u > 0
-    nnz_upper = float(a["nnz"]) if "nnz" in a else float(a["slot"].size)
-    return 8.0 * (nnz_upper + lower_u[has_parent].sum() + trap.sum() + lower_u.sum())
+    return 8.0 * f.stat(16)
 
 
 def roofline_table(p, f, ms_k, cnt_k, gemm_flops, dgemm, solve_graph_ms, spmv_ms, R, hbm):

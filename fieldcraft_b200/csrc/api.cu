@@ -1488,7 +1488,8 @@ int enqueue_factor_direct(fc_chol *h, const double *d_val, const volatile int32_
       case K_GEMM_F64: fc::launch_gemm(h->d_gemm.as<fc::GemmTask>() + l.off, l.count, fc::GemmKind::F64, st); break;
       case K_LDLT_PANEL:
         fc::ldlt::launch_panel(h->d_lpanel.as<fc::ldlt::PanelTask>() + l.off, l.count, l.rows, l.width,
-                               h->d_lpos.as<int32_t>(), h->d_lpos.as<int32_t>() + h->ns, h->d_ltwos.as<int32_t>(), h->d_lfailed.as<unsigned long long>(), st);
+                               h->d_lpos.as<int32_t>(), h->d_lpos.as<int32_t>() + h->ns, h->d_ltwos.as<int32_t>(),
+                               h->d_lfailed.as<unsigned long long>(), st);
         break;
       case K_LDLT_AFTER: fc::ldlt::launch_after(h->d_lafter.as<fc::ldlt::AfterTask>() + l.off, l.count, st); break;
       case K_LDLT_INVERSE: fc::ldlt::launch_inverse(h->d_linv.as<fc::ldlt::InverseTask>() + l.off, l.count, st); break;
@@ -3467,6 +3468,14 @@ int64_t fc_chol_stat(const fc_chol *h, int what) {
     case 13: return h->dag ? h->dag_fwd : 0;
     case 14: return h->dag ? h->dag_bwd : 0;
     case 15: return (int64_t)h->gemm_flops_updates;
+    case 16: {
+      int64_t values = h->nnz;
+      for (int64_t s = 0; s < h->ns; ++s) {
+        const int64_t w = h->width[s], u = h->height[s] - w, lower = u * (u + 1) / 2;
+        values += w * h->height[s] - w * (w - 1) / 2 + 2 * lower;
+      }
+      return values;
+    }
   }
   return -1;
 }

@@ -623,8 +623,8 @@ __host__ __device__ inline int step_ctas(int64_t n) {
 }
 // The product's CTAs, all resident at once, every one the same number of rounds of rows: a CTA's partial
 // sums follow its last round, and a second wave of CTAs started its rounds after the first one's end
-// (1 184 CTAs, 740 of them resident: 30.4 us an iteration from a cold L2; four an SM 28.6, five 29.0, six
-// with fewer registers 30.1).
+// (912 CTAs, 740 of them resident: 32.2 us an iteration on 48 x 48 x 8 elements; four an SM 30.3, five
+// 30.7, six with fewer registers 31.9).
 constexpr int PRODUCT_PER_SM = 4;
 __host__ __device__ inline int product_ctas(int64_t n) {
   constexpr int ROWS = FCG_THREADS / SPMV_LANES;

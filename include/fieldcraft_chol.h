@@ -186,13 +186,14 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
                                 int32_t max_iter, double *relres, int32_t *iterations, fc_status *status);
 
 /* Plan statistics: 0 levels, 1 launches of the factor, 2 bytes of L on device, 3 bytes of the
- * update matrices, 4 supernodes, 5 factor flops (sum of column counts squared), 6 GEMM tasks,
+ * update matrices, 4 supernodes (the analysis'), 5 factor flops (sum of column counts squared), 6 GEMM tasks,
  * 7 kernels launched by the last factorisation, 8 kernels launched by the last solve, 9 flops of
  * the factor's GEMM tasks, 10 flops of the last solve plan's GEMM tasks, 11 the ordinal among the
  * factor's GEMM launches of the one with the most flops, 12 the same among the launches whose
  * tasks all have K <= 64 (the panels' updates of later columns), 13 and 14 the tasks of the
  * persistent solve's forward and backward lists, 15 flops of the factor's update GEMM launches
- * alone (9 without the diagonal blocks' inverse doubling). */
+ * alone (9 without the diagonal blocks' inverse doubling), 16 values that the front assembly reads
+ * and writes at least (A's, each update matrix's lower triangle both ways, the fronts' columns). */
 int64_t fc_chol_stat(const fc_chol *h, int what);
 
 /* Execution options of a handle (no reference counterpart). Each takes effect from the next solve.
