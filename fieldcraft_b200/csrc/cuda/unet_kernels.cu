@@ -127,7 +127,8 @@ __device__ __forceinline__ void conv_groups(float (&acc)[2][COUT / 8][4], const 
 // are read for four MMAs, with two four for eight. In tiles of 8 x 8 x 2, one group a warp, 39% of the
 // MMAs on a 33 x 33 x 9 grid fell outside it (16 passes: 33 us, with tiles that fit 23). The passes of a
 // batch run side by side: alone, a pass on a plate's grid has about one tile an SM and a launch is mostly
-// the weights' load.
+// the weights' load, which with one CTA an SM no longer runs beside the launch before (an application on
+// 65 x 65 x 9 nodes 0.172 ms, 0.155 with two CTAs an SM; a training step on eight pairs 1.67 ms against 1.88).
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
     conv3_kernel(Grid g, int batch, ConvTile tile, const bf16 *__restrict__ in, const bf16 *__restrict__ w,
