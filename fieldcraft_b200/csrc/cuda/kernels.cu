@@ -224,20 +224,27 @@ __host__ __device__ constexpr size_t panel_smem(int p8) {
   return sizeof(double) * ((size_t)p8 * (PANEL_ALD + PANEL_BLD) + 128);
 }
 
-// 1 / sqrt(a) and 1 / a on the panel's chain, from the hardware's estimate y of the root (good to
+// 2^E and 2^-E for the exponent E of a, both kept in the normal range.
+__device__ __forceinline__ void exponent_scales(double a, double &up, double &down) {
+  const int e = min(max(__double2hiint(a) >> 20 & 0x7ff, 1), 2045);
+  up = __hiloint2double(e << 20, 0);
+  down = __hiloint2double((2046 - e) << 20, 0);
+}
+
+// 1 / sqrt(a) and up / a on the panel's chain, from the hardware's estimate y of the root (good to
 // 2^-20 at least): with e = 1 - a y^2, the binomial series y (1 + e / 2 + 3 e^2 / 8) and
 // y^2 (1 + e + e^2) leave errors of e^3, below 2^-56: four dependent operations after the estimate. The
 // tails of the exponent range take the library's function. An a that is not positive gives NaNs or
 // infinities, which the pivot test refuses.
-__device__ __forceinline__ void inverse_root(double a, double &root, double &inverse) {
+__device__ __forceinline__ void inverse_root(double a, double up, double &root, double &inverse) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a * y, y, 1.0), u = y * y;
+  const double e = fma(-a * y, y, 1.0), u = y * up * y;
   root = fma(y * e, fma(e, 0.375, 0.5), y);
   inverse = fma(u, fma(e, e, e), u);
   if (!(a > 1e-280 && a < 1e280)) {
     root = rsqrt(a);
-    inverse = root * root;
+    inverse = root * up * root;
   }
 }
 
@@ -343,19 +350,23 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
           }
         }
         // the multipliers are broadcast and multiplied before the root is there: the chain of a
-        // column is the pivot's shuffle, its reciprocal and one update
+        // column is the pivot's shuffle, its reciprocal and one update. Two entries' product has the
+        // pivot's size and not their own, and leaves the range where they are far from 1: one of
+        // them is brought to the pivot's exponent first, exactly, and the reciprocal back
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const double acc = __shfl_sync(0xffffffffu, s0[j], j);
-          double t0[8], t1[8];
+          double up, down, t0[8], t1[8];
+          exponent_scales(acc, up, down);
+          const double m0 = s0[j] * down, m1 = s1[j] * down;
 #pragma unroll
           for (int k = j + 1; k < 8; ++k) {
             const double lk = __shfl_sync(0xffffffffu, s0[j], k);
-            t0[k] = lane > j ? s0[j] * lk : 0.0;
-            t1[k] = s1[j] * lk;
+            t0[k] = lane > j ? m0 * lk : 0.0;
+            t1[k] = m1 * lk;
           }
           double rd, rr;
-          inverse_root(acc, rd, rr);
+          inverse_root(acc, up, rd, rr);
 #pragma unroll
           for (int k = j + 1; k < 8; ++k) {
             s0[k] = fma(-t0[k], rr, s0[k]);
