@@ -2565,6 +2565,12 @@ int fc_test_ldlt_fold(int64_t n, int64_t ns, const int64_t *first, const int64_t
   return 0;
 }
 
+// Not part of the public ABI: the panel's root and reciprocal on device arrays, for tests.
+int fc_test_inverse_root(int64_t n, const double *d_a, double *d_up, double *d_root, double *d_inverse) {
+  fc::launch_inverse_root(n, d_a, d_up, d_root, d_inverse, nullptr);
+  return cudaDeviceSynchronize() == cudaSuccess ? 0 : -1;
+}
+
 // Not part of the public ABI: the merged supernodes (host/amalgamate.cpp) of an analysis, for tests.
 // sizes[2] receives their count and the length of their rows; the arrays (null to size only) are
 // Amalgamated's.

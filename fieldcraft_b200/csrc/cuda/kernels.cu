@@ -231,9 +231,10 @@ __device__ __forceinline__ void exponent_scales(double a, double &up, double &do
   down = __hiloint2double((2046 - e) << 20, 0);
 }
 
-// 1 / sqrt(a) and up / a on the panel's chain, from the hardware's estimate y of the root (good to
-// 2^-20 at least): with e = 1 - a y^2, the binomial series y (1 + e / 2 + 3 e^2 / 8) and
-// y^2 (1 + e + e^2) leave errors of e^3, below 2^-56: four dependent operations after the estimate. The
+// 1 / sqrt(a) and up / a on the panel's chain, from the hardware's estimate y of the root (whose low 32
+// bits are zero: within 2^-20): with e = 1 - a y^2, at most 2^-19, the binomial series
+// y (1 + e / 2 + 3 e^2 / 8) and y^2 (1 + e + e^2) leave 5 e^3 / 16 and e^3, below 2^-58 and 2^-57 of the
+// results, and their roundings 3 and 6 times 2^-54: four dependent operations after the estimate. The
 // tails of the exponent range take the library's function. An a that is not positive gives NaNs or
 // infinities, which the pivot test refuses.
 __device__ __forceinline__ void inverse_root(double a, double up, double &root, double &inverse) {
@@ -572,6 +573,16 @@ __global__ void __launch_bounds__(INVERSE_THREADS) inverse_kernel(Tree t, const 
       Dp[pw * pw + c * pw + r] = inv[c * TS + r];
       Ip[(int64_t)c * task.ild + r] = r >= c ? inv[c * TS + r] : 0.0;
     }
+}
+
+__global__ void inverse_root_kernel(int64_t n, const double *__restrict__ a, double *__restrict__ up,
+                                    double *__restrict__ root, double *__restrict__ inverse) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double u, down, r, v;
+  exponent_scales(a[i], u, down);
+  inverse_root(a[i], u, r, v);
+  up[i] = u, root[i] = r, inverse[i] = v;
 }
 
 // ---- tiled C -= A B^T on the FP64 tensor pipe ---------------------------------------------------
@@ -1756,6 +1767,10 @@ void launch_panel(const Tree &t, bool fp32, const double *upper_val, const Panel
     panel_kernel<float, PANEL_THREADS><<<count, PANEL_THREADS, smem, st>>>(t, upper_val, tasks, status, p8max);
   else
     panel_kernel<double, PANEL_THREADS><<<count, PANEL_THREADS, smem, st>>>(t, upper_val, tasks, status, p8max);
+}
+
+void launch_inverse_root(int64_t n, const double *a, double *up, double *root, double *inverse, cudaStream_t st) {
+  if (n > 0) inverse_root_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, a, up, root, inverse);
 }
 
 void launch_inverse(const Tree &t, const InverseTask *tasks, int count, cudaStream_t st) {

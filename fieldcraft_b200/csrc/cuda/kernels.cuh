@@ -285,6 +285,8 @@ void launch_assemble(const Tree &t, bool fp32, const double *upper_val, const As
 void launch_panel(const Tree &t, bool fp32, const double *upper_val, const PanelTask *tasks, int count,
                   DeviceStatus *status, int p8max, cudaStream_t st);
 void launch_inverse(const Tree &t, const InverseTask *tasks, int count, cudaStream_t st);
+// For tests: the panel's root and reciprocal of each a (1 / sqrt(a), up / a and up, a power of two near a).
+void launch_inverse_root(int64_t n, const double *a, double *up, double *root, double *inverse, cudaStream_t st);
 // part and counters: the partial sums and counters of split tasks (flag 8), null when there are none.
 void launch_gemm(const GemmTask *tasks, int count, GemmKind kind, cudaStream_t st, double *part = nullptr,
                  int32_t *counters = nullptr);
