@@ -2544,6 +2544,39 @@ cudaError_t noalloc_scratch(int device, unsigned char **base) {
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// The no-allocation solve's layout in the scratch: x | x2 | v | voff | row tasks | child ranges | panel
+// tasks | GEMM tasks | split partial tiles | thin forward tasks | their child ranges | thin backward
+// tasks | their partial sums | the counters (thin, then split). split = false: without the split
+// products' partial tiles (32 KB a chunk, whatever R is).
+struct NoallocLayout {
+  size_t x = 0, x2, v, voff, rows, ranges, panels, gemm, part, thin, tranges, tbwd, tpart, tcount, counters, need;
+};
+NoallocLayout noalloc_plan(const fc_chol *h, int R, unsigned char *base, bool split, SolvePlan &p) {
+  NoallocLayout at;
+  p = SolvePlan();
+  solve_offsets(h, R, p);
+  const size_t vec = align256(sizeof(double) * (size_t)h->n * R);
+  at.x2 = vec, at.v = 2 * vec;
+  at.voff = at.v + align256(sizeof(double) * (size_t)p.vsum);
+  at.need = at.voff;
+  if (at.need > FC_NOALLOC_SCRATCH_BYTES) return at;  // no use in planning the tasks
+  solve_tasks(h, R, reinterpret_cast<double *>(base + at.x), reinterpret_cast<double *>(base + at.x2),
+              reinterpret_cast<double *>(base + at.v), p, split);
+  at.rows = at.voff + align256(sizeof(int64_t) * p.voff.size());
+  at.ranges = at.rows + align256(sizeof(fc::RowTask) * p.rows.size());
+  at.panels = at.ranges + align256(sizeof(int2) * p.ranges.size());
+  at.gemm = at.panels + align256(sizeof(fc::SolveTask) * p.panels.size());
+  at.part = at.gemm + align256(sizeof(fc::GemmTask) * p.gemm.size());
+  at.thin = at.part + align256(sizeof(double) * (size_t)p.psum);
+  at.tranges = at.thin + align256(sizeof(fc::ThinTask) * p.thin.size());
+  at.tbwd = at.tranges + align256(sizeof(int4) * p.tranges.size());
+  at.tpart = at.tbwd + align256(sizeof(fc::ThinBwdTask) * p.tbwd.size());
+  at.tcount = at.tpart + align256(sizeof(double) * (size_t)p.tpart);
+  at.counters = (size_t)std::max<int64_t>(p.tcount + p.scount, 1);
+  at.need = at.tcount + sizeof(int32_t) * at.counters;
+  return at;
+}
+
 }  // namespace
 
 extern "C" {
@@ -2569,6 +2602,17 @@ int fc_test_ldlt_fold(int64_t n, int64_t ns, const int64_t *first, const int64_t
 int fc_test_inverse_root(int64_t n, const double *d_a, double *d_up, double *d_root, double *d_inverse) {
   fc::launch_inverse_root(n, d_a, d_up, d_root, d_inverse, nullptr);
   return cudaDeviceSynchronize() == cudaSuccess ? 0 : -1;
+}
+
+// Not part of the public ABI, for tests: the scratch that the no-allocation solve of nrhs vectors would
+// need, with its long products split or not (at least that much where it is over the limit).
+int64_t fc_test_noalloc_need(fc_chol *h, int32_t nrhs, int split) {
+  std::lock_guard<std::mutex> g(h->lock);
+  unsigned char *base = nullptr;
+  cudaSetDevice(h->device);
+  if (noalloc_scratch(h->device, &base) != cudaSuccess) return -1;
+  SolvePlan p;
+  return (int64_t)noalloc_plan(h, nrhs, base, split != 0, p).need;
 }
 
 // Not part of the public ABI: the merged supernodes (host/amalgamate.cpp) of an analysis, for tests.
@@ -2791,7 +2835,10 @@ int fc_symbolic_import(const fc_symbolic_arrays *in, fc_symbolic **out, fc_statu
   return FC_OK;
 }
 
-int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **out, fc_status *status) {
+// A handle planned on the merged supernodes (merge) or on the reference's own. `refused`: how many plans
+// to give up as if there were no memory for them (for tests).
+static int create(const fc_symbolic *sym, int precision, int device, bool merge, int refused, fc_chol **out,
+                  fc_status *status) {
   if (!sym || !out ||
       (precision != FC_PRECISION_FP64 && precision != FC_PRECISION_FP32_IR && precision != FC_PRECISION_LDLT)) {
     set_status(status, FC_INVALID_ARGUMENT, -1, 0, 0, "null argument or unknown precision");
@@ -2802,7 +2849,7 @@ int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **
   if (e != cudaSuccess) return cuda_fail(status, e, "cudaSetDevice");
   fc::configure_kernels();
   fc_chol *h = nullptr;
-  auto make = [&](bool merge) -> int {
+  auto make = [&](bool merged) -> int {
     try {
       h = new fc_chol();
       h->device = device;
@@ -2817,15 +2864,21 @@ int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **
       if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
         return cuda_fail(status, e, "cudaStreamCreate");
       h->own_stream = true;
-      return build(h, sym->s, merge, status);
+      const int rc = build(h, sym->s, merged, status);
+      if (rc == FC_OK && refused-- > 0) {
+        set_status(status, FC_OUT_OF_MEMORY, -1, sym->s.entries, 0, "device memory");
+        return FC_OUT_OF_MEMORY;
+      }
+      return rc;
     } catch (const std::bad_alloc &) {
       set_status(status, FC_OUT_OF_MEMORY, -1, sym->s.entries, 0, "host memory for the plan");
       return FC_OUT_OF_MEMORY;
     }
   };
-  int rc = make(precision != FC_PRECISION_LDLT);
-  if (rc == FC_OUT_OF_MEMORY && precision != FC_PRECISION_LDLT) {
-    // the merged supernodes' arenas hold a little more: try the reference's own
+  int rc = make(merge);
+  if (merge && (rc == FC_OUT_OF_MEMORY || rc == FC_CUDA_ERROR)) {
+    // the merged supernodes' arenas may hold a little more (a plan's upload that finds no memory is
+    // FC_CUDA_ERROR): try the reference's own
     fc_chol_destroy(h);
     h = nullptr;
     rc = make(false);
@@ -2837,6 +2890,17 @@ int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **
   *out = h;
   set_status(status, FC_OK);
   return FC_OK;
+}
+
+int fc_chol_create(const fc_symbolic *sym, int precision, int device, fc_chol **out, fc_status *status) {
+  return create(sym, precision, device, precision != FC_PRECISION_LDLT, 0, out, status);
+}
+
+// Not part of the public ABI, for tests: a handle on the merged supernodes or on the reference's own, and
+// one whose first `refused` plans find no memory.
+int fc_test_chol_create(const fc_symbolic *sym, int precision, int device, int merge, int refused, fc_chol **out,
+                        fc_status *status) {
+  return create(sym, precision, device, merge != 0, refused, out, status);
 }
 
 void fc_chol_destroy(fc_chol *h) {
@@ -3054,48 +3118,16 @@ int fc_chol_solve_device_noalloc(fc_chol *h, double *d_b, int32_t nrhs, int64_t 
   cudaError_t e = noalloc_scratch(h->device, &base);
   if (e != cudaSuccess) return cuda_fail(status, e, "cudaGetSymbolAddress of the solve scratch");
   const int R = nrhs;
-  // Layout in the scratch: x | x2 | v | voff | row tasks | child ranges | panel tasks | GEMM tasks
-  // | split partial tiles | thin forward tasks | their child ranges | thin backward tasks | their
-  // partial sums | the counters (thin, then split).
   SolvePlan p;
-  solve_offsets(h, R, p);
-  const size_t vec = align256(sizeof(double) * (size_t)h->n * R);
-  const size_t at_x = 0, at_x2 = vec, at_v = 2 * vec;
-  const size_t at_voff = at_v + align256(sizeof(double) * (size_t)p.vsum);
-  auto too_large = [&](size_t need) {
+  NoallocLayout at = noalloc_plan(h, R, base, true, p);
+  if (at.need > FC_NOALLOC_SCRATCH_BYTES) at = noalloc_plan(h, R, base, false, p);
+  if (at.need > FC_NOALLOC_SCRATCH_BYTES) {
     char msg[160];
-    std::snprintf(msg, sizeof(msg), "the solve needs %zu bytes of scratch; the no-allocation limit is %zu",
-                  need, (size_t)FC_NOALLOC_SCRATCH_BYTES);
+    std::snprintf(msg, sizeof(msg), "the solve needs %zu bytes of scratch; the no-allocation limit is %zu", at.need,
+                  (size_t)FC_NOALLOC_SCRATCH_BYTES);
     set_status(status, FC_INVALID_ARGUMENT, -1, 0, 0, msg);
     return FC_INVALID_ARGUMENT;
-  };
-  if (at_voff > FC_NOALLOC_SCRATCH_BYTES) return too_large(at_voff);
-  size_t at_rows, at_ranges, at_panels, at_gemm, at_part, at_thin, at_tranges, at_tbwd, at_tpart, at_tcount, counters,
-      need;
-  auto lay_out = [&](bool split) {
-    solve_tasks(h, R, reinterpret_cast<double *>(base + at_x), reinterpret_cast<double *>(base + at_x2),
-                reinterpret_cast<double *>(base + at_v), p, split);
-    at_rows = at_voff + align256(sizeof(int64_t) * p.voff.size());
-    at_ranges = at_rows + align256(sizeof(fc::RowTask) * p.rows.size());
-    at_panels = at_ranges + align256(sizeof(int2) * p.ranges.size());
-    at_gemm = at_panels + align256(sizeof(fc::SolveTask) * p.panels.size());
-    at_part = at_gemm + align256(sizeof(fc::GemmTask) * p.gemm.size());
-    at_thin = at_part + align256(sizeof(double) * (size_t)p.psum);
-    at_tranges = at_thin + align256(sizeof(fc::ThinTask) * p.thin.size());
-    at_tbwd = at_tranges + align256(sizeof(int4) * p.tranges.size());
-    at_tpart = at_tbwd + align256(sizeof(fc::ThinBwdTask) * p.tbwd.size());
-    at_tcount = at_tpart + align256(sizeof(double) * (size_t)p.tpart);
-    counters = (size_t)std::max<int64_t>(p.tcount + p.scount, 1);
-    need = at_tcount + sizeof(int32_t) * counters;
-  };
-  lay_out(true);
-  if (need > FC_NOALLOC_SCRATCH_BYTES) {
-    // without the split products' partial tiles (32 KB a chunk, whatever R is)
-    p = SolvePlan();
-    solve_offsets(h, R, p);
-    lay_out(false);
   }
-  if (need > FC_NOALLOC_SCRATCH_BYTES) return too_large(need);
   // Every region is written before it is read in this call: the task lists and offsets here, x by
   // the permutation, x2 by the forward panels, each update vector's rows zeroed by its assembly
   // (or stored whole by a thin forward tile), each partial tile stored by its chunk before the
@@ -3103,28 +3135,28 @@ int fc_chol_solve_device_noalloc(fc_chol *h, double *d_b, int32_t nrhs, int64_t 
   auto put = [&](size_t at, const void *src, size_t bytes) {
     if (bytes && e == cudaSuccess) e = cudaMemcpyAsync(base + at, src, bytes, cudaMemcpyHostToDevice, h->stream);
   };
-  put(at_voff, p.voff.data(), sizeof(int64_t) * p.voff.size());
-  put(at_rows, p.rows.data(), sizeof(fc::RowTask) * p.rows.size());
-  put(at_ranges, p.ranges.data(), sizeof(int2) * p.ranges.size());
-  put(at_panels, p.panels.data(), sizeof(fc::SolveTask) * p.panels.size());
-  put(at_gemm, p.gemm.data(), sizeof(fc::GemmTask) * p.gemm.size());
-  put(at_thin, p.thin.data(), sizeof(fc::ThinTask) * p.thin.size());
-  put(at_tranges, p.tranges.data(), sizeof(int4) * p.tranges.size());
-  put(at_tbwd, p.tbwd.data(), sizeof(fc::ThinBwdTask) * p.tbwd.size());
-  if (e == cudaSuccess) e = cudaMemsetAsync(base + at_tcount, 0, sizeof(int32_t) * counters, h->stream);
+  put(at.voff, p.voff.data(), sizeof(int64_t) * p.voff.size());
+  put(at.rows, p.rows.data(), sizeof(fc::RowTask) * p.rows.size());
+  put(at.ranges, p.ranges.data(), sizeof(int2) * p.ranges.size());
+  put(at.panels, p.panels.data(), sizeof(fc::SolveTask) * p.panels.size());
+  put(at.gemm, p.gemm.data(), sizeof(fc::GemmTask) * p.gemm.size());
+  put(at.thin, p.thin.data(), sizeof(fc::ThinTask) * p.thin.size());
+  put(at.tranges, p.tranges.data(), sizeof(int4) * p.tranges.size());
+  put(at.tbwd, p.tbwd.data(), sizeof(fc::ThinBwdTask) * p.tbwd.size());
+  if (e == cudaSuccess) e = cudaMemsetAsync(base + at.tcount, 0, sizeof(int32_t) * at.counters, h->stream);
   if (e != cudaSuccess) return cuda_fail(status, e, "copy of the solve plan into the scratch");
-  const SolveBuffers b{reinterpret_cast<double *>(base + at_x), reinterpret_cast<double *>(base + at_x2),
-                       reinterpret_cast<double *>(base + at_v), reinterpret_cast<const int64_t *>(base + at_voff),
-                       reinterpret_cast<const fc::RowTask *>(base + at_rows),
-                       reinterpret_cast<const int2 *>(base + at_ranges),
-                       reinterpret_cast<const fc::SolveTask *>(base + at_panels),
-                       reinterpret_cast<const fc::GemmTask *>(base + at_gemm),
-                       reinterpret_cast<double *>(base + at_part),
-                       reinterpret_cast<const fc::ThinTask *>(base + at_thin),
-                       reinterpret_cast<const int4 *>(base + at_tranges),
-                       reinterpret_cast<const fc::ThinBwdTask *>(base + at_tbwd),
-                       reinterpret_cast<double *>(base + at_tpart),
-                       reinterpret_cast<int32_t *>(base + at_tcount),
+  const SolveBuffers b{reinterpret_cast<double *>(base + at.x), reinterpret_cast<double *>(base + at.x2),
+                       reinterpret_cast<double *>(base + at.v), reinterpret_cast<const int64_t *>(base + at.voff),
+                       reinterpret_cast<const fc::RowTask *>(base + at.rows),
+                       reinterpret_cast<const int2 *>(base + at.ranges),
+                       reinterpret_cast<const fc::SolveTask *>(base + at.panels),
+                       reinterpret_cast<const fc::GemmTask *>(base + at.gemm),
+                       reinterpret_cast<double *>(base + at.part),
+                       reinterpret_cast<const fc::ThinTask *>(base + at.thin),
+                       reinterpret_cast<const int4 *>(base + at.tranges),
+                       reinterpret_cast<const fc::ThinBwdTask *>(base + at.tbwd),
+                       reinterpret_cast<double *>(base + at.tpart),
+                       reinterpret_cast<int32_t *>(base + at.tcount),
                        p.lg};
   int64_t launches = 0;
   fc::launch_permute_in(h->d_perm.as<int64_t>(), h->n, d_b, ld, b.x, R, h->tree.scale, h->stream);

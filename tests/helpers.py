@@ -279,3 +279,20 @@ def hex_pattern(n: int, sigma: float, nested_dissection) -> Csr:
                         value = 0.01 * ((v + w) % 3)
                     rows[3 * place[v] + a].append((3 * place[w] + b, value))
     return rows_to_csr(rows)
+
+
+def factor_on(sym, merge: bool, precision: int = 0, refused: int = 0):
+    """A Factor whose handle is planned on the merged supernodes or on the analysis' own (what
+    fc_chol_create falls back to); its first `refused` plans find no memory."""
+    import ctypes as C
+
+    from fieldcraft_b200 import Factor, _lib
+    from fieldcraft_b200._lib import Status
+    from fieldcraft_b200.cholesky import raise_for
+
+    st, h = Status(), C.c_void_p()
+    _lib.load().fc_test_chol_create(sym.handle, precision, 0, int(merge), refused, C.byref(h), C.byref(st))
+    raise_for(st)
+    f = Factor.__new__(Factor)
+    f.handle, f.n, f.symbolic = h, sym.n, sym
+    return f
