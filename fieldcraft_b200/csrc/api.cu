@@ -2598,6 +2598,19 @@ int fc_test_ldlt_fold(int64_t n, int64_t ns, const int64_t *first, const int64_t
   return 0;
 }
 
+// Not part of the public ABI, for tests: the LDL^T solve's maps as the last factorisation left them on the
+// device (ldlt::launch_fold): own[n], perm[n] and the row lists.
+int fc_test_ldlt_maps(fc_chol *h, int32_t *own, int64_t *perm, int32_t *rows) {
+  if (!h->ldlt || !h->ldlt_ready || cudaStreamSynchronize(h->stream) != cudaSuccess) return -1;
+  auto get = [](void *dst, const DeviceBuf &src, size_t bytes) {
+    return bytes == 0 || cudaMemcpy(dst, src.p, bytes, cudaMemcpyDeviceToHost) == cudaSuccess;
+  };
+  return get(own, h->d_lown, sizeof(int32_t) * (size_t)h->n) && get(perm, h->d_lsperm, sizeof(int64_t) * (size_t)h->n) &&
+                 get(rows, h->d_lsrows, sizeof(int32_t) * h->rows.size())
+             ? 0
+             : -1;
+}
+
 // Not part of the public ABI: the panel's root and reciprocal on device arrays, for tests.
 int fc_test_inverse_root(int64_t n, const double *d_a, double *d_up, double *d_root, double *d_inverse) {
   fc::launch_inverse_root(n, d_a, d_up, d_root, d_inverse, nullptr);
