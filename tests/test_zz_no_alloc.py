@@ -13,6 +13,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
+import helpers as H
 from fieldcraft_b200 import FP32_IR, FP64, Factor, Symbolic, _lib, problems
 from fieldcraft_b200._lib import Status
 
@@ -66,17 +67,23 @@ def test_no_alloc_solve_matches_the_ordinary_solve(cuda):
     fc.close()
 
 
+@pytest.mark.parametrize("merge", [True, False], ids=["merged", "own"])
 @pytest.mark.parametrize("precision", [FP64, FP32_IR], ids=["fp64", "fp32_ir"])
-def test_no_alloc_solve_with_split_products(cuda, precision):
+def test_no_alloc_solve_with_split_products(cuda, precision, merge):
     """The 16^3 block: its top separator (867 columns) makes the solve split long products in
-    chunks that the last CTA adds (partials and counters in the scratch), and its thin
-    supernodes with more than 128 rows below sum their backward steps in chunks the same way.
-    With the FP64 factor and with the mixed-precision one (a 4-byte L); two calls in a row."""
+    chunks that the last CTA adds (partials and counters in the scratch), and on the analysis' own
+    supernodes the thin ones with more than 128 rows below sum their backward steps in chunks the
+    same way. With the FP64 factor and with the mixed-precision one (a 4-byte L); two calls in a row."""
     torch = cuda
     lib = _lib.load()
     p = problems.lognormal_block(16, nrhs=5)
     up = p.upper()
-    f = Factor(Symbolic(up, 2**62), precision=precision)
+    sym = Symbolic(up, 2**62)
+    f = H.factor_on(sym, merge, precision)
+    s = sym.arrays()
+    width, below = np.diff(s["first"]), np.diff(s["rptr"]) - np.diff(s["first"])
+    assert width.max() > 512  # the split products
+    assert merge or np.any((width <= 8) & (below > 128))
     f.factor(up.val)
     b = column_major(torch, p.rhs)
     ref = ordinary(lib, f, b, 5, p.n)
