@@ -22,7 +22,7 @@ constexpr float SLOPE = 0.05f;  // leaky ReLU: x for x > 0, SLOPE x otherwise
 __device__ __forceinline__ float gate(float mask) { return mask > 0.f ? 1.f : SLOPE; }
 // A weight gradient's tile: tx x ty voxels of a z plane, DW_VOXELS at most (DwTile); with the input's
 // halo, a plane more on either side in z too, DW_HALO voxels at most.
-constexpr int DW_VOXELS = 128, DW_HALO = 560;
+constexpr int DW_VOXELS = 128, DW_HALO = 560, DW_TOGETHER = 4;
 __host__ __device__ constexpr int dw_threads(int cout) { return 9 * (cout / 16) * 32; }
 // A convolution's CTA: twelve warps of one or two groups of 16 voxels, so that a tile is 384 voxels at
 // most (ConvTile), and the most voxels of a tile with its halo: two of them and the weights in 227 KB.
@@ -224,8 +224,12 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
 // grid (8 x 8 voxels: on a 33 x 33 plane a third of the products were outside it); past its last one dY
 // is zero. The next tile's copies are in flight while a tile is multiplied. Nine warps with all the
 // channels, 100 accumulators a thread, left one of the four schedulers three warps and the others two:
-// 16 passes on a 33 x 33 x 9 grid took 53 us with both, 30 so. Bound by the fragments' shared-memory
-// reads and the tensor pipe.
+// 16 passes on a 33 x 33 x 9 grid took 53 us with both, 30 so. The tensor pipe truncates what it adds to
+// an accumulator, so its sums leave it every DW_TOGETHER steps (64 voxels) and are added rounded: kept in
+// it over a chunk of 4 100 voxels a gradient was off by 4.7e-6, now by 2e-7 (2-norm, eight pairs on 65 x
+// 65 x 9 nodes). Half of the input channels at a time, so that both sums fit the registers, for an eighth
+// more fragment reads: a training step on eight pairs 1.39 -> 1.41 ms. Bound by the fragments'
+// shared-memory reads and the tensor pipe.
 struct DwTile {
   int tx, ty, tiles;  // tiles: of one pair, all its passes
 };
@@ -253,7 +257,7 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
   const int64_t total = (int64_t)ntiles * passes, per = (total + chunks - 1) / chunks, voxels = g.voxels();
   const int64_t t0 = chunk * per, t1 = min(total, t0 + per);
   for (int m = tid; m < DW_VOXELS; m += THREADS) place[m] = m < here ? (m / tile.tx * hx + m % tile.tx) * CS : 0;
-  float acc[3][CIN / 8][4], sum[4] = {0.f, 0.f, 0.f, 0.f};
+  float acc[3][CIN / 8][4], bias[2] = {0.f, 0.f};
 #pragma unroll
   for (int t = 0; t < 3; ++t)
 #pragma unroll
@@ -281,21 +285,31 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
     __syncthreads();
     const bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + DW_HALO * CS;
     const bf16 *rows = ts + (unit / 3 * hy + unit % 3) * hx * CS + (q >> 1) * 8;
+    for (int k0 = 0; k0 < steps; k0 += DW_TOGETHER) {
+      const int k1 = min(steps, k0 + DW_TOGETHER);
+#pragma unroll
+      for (int np = 0; np < CIN / 16; ++np) {
+        float here[3][2][4] = {}, ones[4] = {};
 #pragma unroll 2
-    for (int ks = 0; ks < steps; ++ks) {
-      uint32_t a[4];  // rows: voxel ks 16 + (q >> 1) 8 + r; columns: channel
-      ldsm_x4_t(a, ds + (ks * 16 + (q >> 1) * 8 + r) * DS + mt * 16 + (q & 1) * 8);
-      if (unit == 4) mma_bf16(sum, a, 0x3f803f80u, 0x3f803f80u);  // ones
-      const bf16 *brow = rows + place[ks * 16 + (q & 1) * 8 + r];  // B row: the voxel, shifted by the tap
+        for (int ks = k0; ks < k1; ++ks) {
+          uint32_t a[4];  // rows: voxel ks 16 + (q >> 1) 8 + r; columns: channel
+          ldsm_x4_t(a, ds + (ks * 16 + (q >> 1) * 8 + r) * DS + mt * 16 + (q & 1) * 8);
+          if (unit == 4 && np == 0) mma_bf16(ones, a, 0x3f803f80u, 0x3f803f80u);
+          const bf16 *brow = rows + place[ks * 16 + (q & 1) * 8 + r] + np * 16;  // B row: the voxel, shifted by the tap
 #pragma unroll
-      for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-        for (int np = 0; np < CIN / 16; ++np) {
-          uint32_t b[4];
-          ldsm_x4_t(b, brow + dx * CS + np * 16);
-          mma_bf16(acc[dx][2 * np], a, b[0], b[1]);
-          mma_bf16(acc[dx][2 * np + 1], a, b[2], b[3]);
+          for (int dx = 0; dx < 3; ++dx) {
+            uint32_t b[4];
+            ldsm_x4_t(b, brow + dx * CS);
+            mma_bf16(here[dx][0], a, b[0], b[1]);
+            mma_bf16(here[dx][1], a, b[2], b[3]);
+          }
         }
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[dx][2 * np + e / 4][e % 4] += here[dx][e / 4][e % 4];
+        if (np == 0) bias[0] += ones[0], bias[1] += ones[2];
+      }
     }
     __syncthreads();
   }
@@ -311,8 +325,8 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
     }
   }
   if (unit == 4 && tg == 0) {
-    chunk_part[27 * COUT * CIN + mt * 16 + gq] = sum[0];
-    chunk_part[27 * COUT * CIN + mt * 16 + gq + 8] = sum[2];
+    chunk_part[27 * COUT * CIN + mt * 16 + gq] = bias[0];
+    chunk_part[27 * COUT * CIN + mt * 16 + gq + 8] = bias[1];
   }
 }
 
@@ -834,7 +848,7 @@ void conv3_launch(const Grid &g, int batch, const bf16 *in, const bf16 *w, const
   cudaLaunchKernelEx(&cfg, conv3_kernel<CIN, COUT>, g, batch, tile, in, w, bias, relu ? 1 : 0, mask, out);
 }
 
-// About one chunk an SM over all pairs (18 warps of 110 registers a thread: one CTA an SM).
+// About one chunk an SM over all pairs (18 warps of 96 registers a thread: one CTA an SM).
 int chunks_of(int64_t tiles, int pairs) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (DW_PARTIALS + pairs - 1) / pairs));
 }

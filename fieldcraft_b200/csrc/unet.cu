@@ -607,6 +607,21 @@ int fc_unet_get_grads(fc_unet *u, float *host) {
              : FC_CUDA_ERROR;
 }
 
+// Not part of the public ABI, for tests: the weight gradient of one layer on device arrays (conv3_dw); in
+// and dy in BF16, pairs * passes grids each; gw and gb receive the sum over the pairs of scale g.
+int fc_test_unet_dw(int32_t X, int32_t Y, int32_t Z, int32_t cin, int32_t cout, int32_t pairs, int32_t passes,
+                    const void *d_in, const void *d_dy, float scale, float *d_gw, float *d_gb) {
+  const Grid g{X, Y, Z};
+  const size_t nw = (size_t)27 * cin * cout;
+  DeviceBuf part, last;
+  if (part.alloc(sizeof(float) * (size_t)pairs * fc::unet::dw_chunks(g, pairs, passes) * 28 * cin * cout) != cudaSuccess ||
+      last.alloc(sizeof(float) * (nw + cout)) != cudaSuccess)
+    return FC_OUT_OF_MEMORY;
+  fc::unet::conv3_dw(g, cin, cout, pairs, passes, static_cast<const bf16 *>(d_in), static_cast<const bf16 *>(d_dy),
+                     part.as<float>(), scale, false, d_gw, d_gb, last.as<float>(), last.as<float>() + nw, nullptr);
+  return cudaDeviceSynchronize() == cudaSuccess ? FC_OK : FC_CUDA_ERROR;
+}
+
 int fc_unet_forward_grid(fc_unet *u, const float *d_x, float *d_y) {
   if (!u || !d_x || !d_y) return FC_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> g(u->lock);
