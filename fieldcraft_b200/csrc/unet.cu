@@ -14,6 +14,7 @@
 #include "cuda/kernels.cuh"
 #include "cuda/unet_kernels.cuh"
 #include "device_buf.hpp"
+#include "host/pass_room.hpp"
 #include "scratch.hpp"
 
 using fc::host::DeviceBuf;
@@ -130,7 +131,19 @@ Grid coarser(const Grid &g) { return Grid{(g.X + 1) / 2, (g.Y + 1) / 2, (g.Z + 1
 
 }  // namespace
 
-struct fc_unet {
+// What a group of passes works in, all in one allocation of its owner's.
+struct Activations {
+  // BF16, channels last, per level: the (pooled) input, the two convolutions of the way down (s =
+  // the skip), the way up: u = upsampled + skip, its two convolutions b, d
+  bf16 *x = nullptr, *y = nullptr, *pin[MAX_LEVELS] = {}, *a[MAX_LEVELS] = {}, *s[MAX_LEVELS] = {},
+       *u[MAX_LEVELS] = {}, *b[MAX_LEVELS] = {}, *d[MAX_LEVELS] = {};
+  // gradients per level
+  bf16 *dy = nullptr, *ga[MAX_LEVELS] = {}, *gb[MAX_LEVELS] = {}, *gs[MAX_LEVELS] = {};
+  // training, a column per pair of a group: the output, its difference
+  double *tz = nullptr, *td = nullptr;
+};
+
+struct fc_unet : Activations {  // those of the call that runs (choose_passes)
   int device = 0;
   cudaStream_t stream = nullptr;
   int64_t n = 0;
@@ -144,16 +157,8 @@ struct fc_unet {
   DeviceBuf gacc;            // a minibatch's mean gradient
   DeviceBuf wb, wt;          // BF16 weights and their flipped transposes
   DeviceBuf eq, feat;
-  // activations (BF16, channels last), per level: the (pooled) input, the two convolutions of the
-  // way down (s = the skip), the way up: u = upsampled + skip, its two convolutions b, d
-  bf16 *x = nullptr, *y = nullptr, *pin[MAX_LEVELS] = {}, *a[MAX_LEVELS] = {}, *s[MAX_LEVELS] = {},
-       *u[MAX_LEVELS] = {}, *b[MAX_LEVELS] = {}, *d[MAX_LEVELS] = {};
-  // gradients per level
-  bf16 *dy = nullptr, *ga[MAX_LEVELS] = {}, *gb[MAX_LEVELS] = {}, *gs[MAX_LEVELS] = {};
-  DeviceBuf arena;           // all of them
   DeviceBuf part;            // weight-gradient partials
   DeviceBuf scal, dotpart;   // device scalars: [0,1] input scales, [2..] dots; dot partials
-  DeviceBuf tz, td;          // training, a column per pair of a group: the output, its difference
   DeviceBuf bj;              // nodal block-Jacobi inverses (9 doubles a node), added to the output
   bool has_bj = false;
   bool net_on = true;         // false: the preconditioner is the block-Jacobi part alone
@@ -161,7 +166,11 @@ struct fc_unet {
   // odd: M(r) = B r + (net(r) - net(-r)) / 2, so that M(-r) = -M(r) and M(0) = 0 (a part of the
   // output that does not depend on r, from the biases and the modulus channel, cancels)
   bool odd = true;
-  int cap = 0, pairs_cap = 0;  // passes the activations hold, pairs tz and td hold
+  // the handle's own activations, made with it and kept to its end, and a larger group's
+  fc::PassRoom room;
+  Activations own, group;
+  DeviceBuf own_mem, group_mem;
+  int most_grown = INT32_MAX;  // larger groups find no memory (for tests)
   DeviceBuf gtmp;              // one pass's gradients, where a pair's two do not fit together
   fc::unet::LayerTable table{};
   int64_t last_net_iterations = 0, last_dropped = 0;
@@ -175,66 +184,80 @@ namespace {
 bf16 *B(const DeviceBuf &b) { return b.as<bf16>(); }
 
 // A group of pairs runs through the network side by side, a pass each (two with the odd form): at
-// most PAIRS_MOST pairs, and activations of at most WORKSPACE_MOST bytes beside a pair's own. The
-// sizes are kept in the handle for the next group.
+// most PAIRS_MOST pairs, and activations of at most WORKSPACE_MOST bytes beside the handle's own.
 constexpr int PAIRS_MOST = 8;
 constexpr size_t WORKSPACE_MOST = (size_t)2 << 30;
 // the device scalars: the passes' scales, then a value per pair each
 constexpr int S_SCALES = 64, S_NRM = 96, S_NUM = 104, S_DEN = 112, S_COUNT = 128;
 
-// The activations and gradients of `passes` passes, in one allocation (two dozen of them took a
-// millisecond); the weight gradients' partials with the first.
-bool alloc_passes(fc_unet *u, int passes) {
-  u->cap = 0;
-  const size_t part = (size_t)(fc::unet::DW_PARTIALS + PAIRS_MOST) * 28 * C * C;
-  if (!u->part.p && u->part.alloc(sizeof(float) * part) != cudaSuccess) return false;
+// The activations and gradients of `passes` passes in `mem`, one allocation (two dozen of them took a
+// millisecond). Null pointers and false when there is no memory for it.
+bool alloc_passes(const fc_unet *u, int passes, DeviceBuf &mem, Activations &out) {
+  const int pairs = std::min(passes, PAIRS_MOST);
   for (int round = 0; round < 2; ++round) {  // sizes, then places
-    bf16 *base = u->arena.as<bf16>();
+    Activations a;
+    unsigned char *base = mem.as<unsigned char>();
     size_t at = 0;
-    auto take = [&](bf16 *&p, const Grid &g, int c) {
-      p = base + at;
-      at += ((size_t)g.voxels() * c * passes + 127) / 128 * 128;
+    auto take = [&](auto *&p, size_t count) {
+      p = reinterpret_cast<std::decay_t<decltype(p)>>(base + at);
+      at += (sizeof(*p) * count + 255) / 256 * 256;
     };
-    take(u->x, u->g[0], CIO);
-    take(u->y, u->g[0], CIO);
-    take(u->dy, u->g[0], CIO);
+    auto grid = [&](bf16 *&p, const Grid &g, int c) { take(p, (size_t)g.voxels() * c * passes); };
+    take(a.tz, (size_t)u->n * pairs);
+    take(a.td, (size_t)u->n * pairs);
+    grid(a.x, u->g[0], CIO);
+    grid(a.y, u->g[0], CIO);
+    grid(a.dy, u->g[0], CIO);
     for (int lv = 0; lv < u->levels; ++lv) {
       const Grid &g = u->g[lv];
-      for (bf16 **b : {&u->a[lv], &u->s[lv], &u->ga[lv], &u->gb[lv]}) take(*b, g, C);
-      if (lv > 0) take(u->pin[lv], g, C);
+      for (bf16 **b : {&a.a[lv], &a.s[lv], &a.ga[lv], &a.gb[lv]}) grid(*b, g, C);
+      if (lv > 0) grid(a.pin[lv], g, C);
       if (lv < u->levels - 1)
-        for (bf16 **b : {&u->u[lv], &u->b[lv], &u->d[lv], &u->gs[lv]}) take(*b, g, C);
+        for (bf16 **b : {&a.u[lv], &a.b[lv], &a.d[lv], &a.gs[lv]}) grid(*b, g, C);
     }
-    if (round == 0 && u->arena.alloc(sizeof(bf16) * at) != cudaSuccess) return false;
+    if (round == 1) {
+      out = a;
+    } else if (mem.alloc(at) != cudaSuccess) {
+      out = Activations();
+      return false;
+    }
   }
-  u->cap = passes;
   return true;
 }
 
-// Room for `pairs` pairs of `per` passes, or for as many as there is memory for: returns how many
-// passes run together (at least one; a pair's two then run after one another), 0 when there is
-// no room at all.
-int want_passes(fc_unet *u, int pairs, int per) {
+// The handle's own: a vector's passes together, or one where they find no memory.
+bool alloc_own(fc_unet *u, int passes) {
+  for (u->room.own = passes; u->room.own > 0; --u->room.own)
+    if (alloc_passes(u, u->room.own, u->own_mem, u->own)) return true;
+  return false;
+}
+
+void use(fc_unet *u, const Activations &a) { static_cast<Activations &>(*u) = a; }
+
+// Room for the passes of `pairs` vectors, or for as many as there is memory for: returns how many run
+// together (at least one; a vector's two then run after one another).
+int choose_passes(fc_unet *u, int pairs, int per) {
   size_t pass = 0;
   for (int lv = 0; lv < u->levels; ++lv) pass += sizeof(bf16) * (size_t)u->g[lv].voxels() * C * 9;
   int want = per * std::min(pairs, PAIRS_MOST);
   while (want > per && pass * want > WORKSPACE_MOST) want -= per;
-  if (u->cap >= want) return want;
-  cudaStreamSynchronize(u->stream);
-  for (int p = want; p >= 1; p = p > per ? p - per : p - 1)
-    if (alloc_passes(u, p)) return p;
-  return 0;
-}
-
-bool want_pairs(fc_unet *u, int pairs) {
-  if (u->pairs_cap >= pairs) return true;
-  cudaStreamSynchronize(u->stream);
-  u->pairs_cap = 0;
-  if (u->tz.alloc(sizeof(double) * (size_t)u->n * pairs) != cudaSuccess ||
-      u->td.alloc(sizeof(double) * (size_t)u->n * pairs) != cudaSuccess)
-    return false;
-  u->pairs_cap = pairs;
-  return true;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (want > u->room.own && cudaStreamIsCapturing(u->stream, &capturing) != cudaSuccess) {
+    cudaGetLastError();
+    capturing = cudaStreamCaptureStatusActive;
+  }
+  const fc::PassRoom::Choice c = u->room.choose(want, per, capturing != cudaStreamCaptureStatusNone, [&](int passes) {
+    // (an allocation is not part of a capture that runs on another stream)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaStreamSynchronize(u->stream);
+    u->group_mem.release();
+    const bool ok = passes <= u->most_grown && alloc_passes(u, passes, u->group_mem, u->group);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return ok;
+  });
+  use(u, c.in_group ? u->group : u->own);
+  return c.passes;
 }
 
 // BF16 copies of the weights (and the flipped ones for the input gradients) after a change: before
@@ -373,15 +396,13 @@ void apply_jacobi(fc_unet *u, const double *r, double *z) {
 
 // The losses of `count` pairs (r_q, e_q) added into *d_loss, the last pair's gradient into u->grad,
 // and with `acc` their mean into u->gacc (forward and backward of the network, in groups of pairs).
-// False when there is no memory for one pass.
-bool pair_gradients(fc_unet *u, const double *d_r, const double *d_e, int count, int64_t ld, const int64_t *d_ptr,
+void pair_gradients(fc_unet *u, const double *d_r, const double *d_e, int count, int64_t ld, const int64_t *d_ptr,
                     const int32_t *d_idx, const double *d_val, double *d_loss, bool acc) {
   cudaStream_t st = u->stream;
   const int per = passes_per_pair(u);
-  const int together = want_passes(u, count, per);
+  const int together = choose_passes(u, count, per);
   const int most = std::max(1, together / per);
-  if (together == 0 || !want_pairs(u, std::min(count, most))) return false;
-  double *z = u->tz.as<double>(), *d = u->td.as<double>();
+  double *z = u->tz, *d = u->td;
   const int64_t *eq = u->eq.as<int64_t>();
   for (int q0 = 0; q0 < count; q0 += most) {
     const int g = std::min(most, count - q0);
@@ -417,7 +438,6 @@ bool pair_gradients(fc_unet *u, const double *d_r, const double *d_e, int count,
     backward(u, {1, 1, acc, scale, true});
     add_f32_kernel<<<blocks(u->params), 256, 0, st>>>(u->params, u->gtmp.as<float>(), u->grad.as<float>());
   }
-  return true;
 }
 
 int cuda_fail(fc_status *st, cudaError_t e, const char *where) {
@@ -487,8 +507,9 @@ int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const i
             u->eq.alloc(sizeof(int64_t) * 3 * nodes) == cudaSuccess &&
             u->feat.alloc(sizeof(float) * nodes) == cudaSuccess &&
             u->scal.alloc(sizeof(double) * S_COUNT) == cudaSuccess &&
-            u->dotpart.alloc(sizeof(double) * 8 * 512) == cudaSuccess && want_pairs(u, 1) &&
-            u->gtmp.alloc(sizeof(float) * off) == cudaSuccess && want_passes(u, 1, passes_per_pair(u)) > 0;
+            u->dotpart.alloc(sizeof(double) * 8 * 512) == cudaSuccess &&
+            u->part.alloc(sizeof(float) * (fc::unet::DW_PARTIALS + PAIRS_MOST) * 28 * C * C) == cudaSuccess &&
+            u->gtmp.alloc(sizeof(float) * off) == cudaSuccess && alloc_own(u, passes_per_pair(u));
   if (!ok) {
     delete u;
     set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for the network");
@@ -607,6 +628,20 @@ int fc_unet_get_grads(fc_unet *u, float *host) {
              : FC_CUDA_ERROR;
 }
 
+// Not part of the public ABI, for tests: the handle's own activations for `own` passes, and no memory for
+// groups of more than `group`. Returns what the own ones hold.
+int fc_test_unet_room(fc_unet *u, int own, int group) {
+  std::lock_guard<std::mutex> g(u->lock);
+  cudaSetDevice(u->device);
+  cudaStreamSynchronize(u->stream);
+  u->group_mem.release();
+  u->room = fc::PassRoom();
+  u->most_grown = group;
+  if (!alloc_own(u, own)) return 0;
+  use(u, u->own);
+  return u->room.own;
+}
+
 // Not part of the public ABI, for tests: the weight gradient of one layer on device arrays (conv3_dw); in
 // and dy in BF16, pairs * passes grids each; gw and gb receive the sum over the pairs of scale g.
 int fc_test_unet_dw(int32_t X, int32_t Y, int32_t Z, int32_t cin, int32_t cout, int32_t pairs, int32_t passes,
@@ -627,6 +662,7 @@ int fc_unet_forward_grid(fc_unet *u, const float *d_x, float *d_y) {
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   const int64_t nv = u->g[0].voxels() * CIO;
+  use(u, u->own);
   refresh_weights(u);
   f32_to_bf16_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, d_x, u->x);
   forward(u, 1);
@@ -640,6 +676,7 @@ int fc_unet_backward_grid(fc_unet *u, const float *d_dy) {
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   const int64_t nv = u->g[0].voxels() * CIO;
+  use(u, u->own);
   f32_to_bf16_kernel<<<blocks(nv), 256, 0, u->stream>>>(nv, d_dy, u->dy);
   backward(u, {1, 1, false, 1.f, false});
   const cudaError_t e = cudaStreamSynchronize(u->stream);
@@ -651,9 +688,7 @@ int fc_unet_apply(fc_unet *u, const double *d_r, double *d_z) {
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   if (u->net_on) {
-    const int together = want_passes(u, 1, passes_per_pair(u));
-    if (together == 0) return FC_OUT_OF_MEMORY;
-    apply(u, 1, d_r, u->n, d_z, together);
+    apply(u, 1, d_r, u->n, d_z, choose_passes(u, 1, passes_per_pair(u)));
   } else
     apply_jacobi(u, d_r, d_z);
   return cudaGetLastError() == cudaSuccess ? FC_OK : FC_CUDA_ERROR;
@@ -664,7 +699,7 @@ int fc_unet_train_step(fc_unet *u, const double *d_r, const double *d_e, const i
   if (!u || !d_r || !d_e || step < 1 || (d_ptr && (!d_idx || !d_val))) return FC_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
-  if (!pair_gradients(u, d_r, d_e, 1, u->n, d_ptr, d_idx, d_val, d_loss, false)) return FC_OUT_OF_MEMORY;
+  pair_gradients(u, d_r, d_e, 1, u->n, d_ptr, d_idx, d_val, d_loss, false);
   fc::unet::adam(u->params, u->p.as<float>(), u->grad.as<float>(), u->m.as<float>(), u->v.as<float>(), lr, 0.9f,
                  0.999f, 1e-8f, step, u->stream);
   u->weights_stale = true;
@@ -679,7 +714,7 @@ int fc_unet_train_batch(fc_unet *u, const double *d_r, const double *d_e, int32_
   std::lock_guard<std::mutex> g(u->lock);
   cudaSetDevice(u->device);
   cudaStream_t st = u->stream;
-  if (!pair_gradients(u, d_r, d_e, count, ld, d_ptr, d_idx, d_val, d_loss, true)) return FC_OUT_OF_MEMORY;
+  pair_gradients(u, d_r, d_e, count, ld, d_ptr, d_idx, d_val, d_loss, true);
   fc::unet::adam(u->params, u->p.as<float>(), u->gacc.as<float>(), u->m.as<float>(), u->v.as<float>(), lr, 0.9f,
                  0.999f, 1e-8f, step, st);
   u->weights_stale = true;
@@ -702,11 +737,7 @@ int fc_fcg_solve(fc_unet *net, fc_chol *fallback, int64_t n, const int64_t *d_pt
     cudaSetDevice(net->device);
   }
   cudaStream_t st = net ? net->stream : nullptr;
-  const int together = net ? want_passes(net, 1, passes_per_pair(net)) : 0;
-  if (net && together == 0) {
-    set_status(status, FC_OUT_OF_MEMORY, -1, 0, 0, "device memory for the network");
-    return FC_OUT_OF_MEMORY;
-  }
+  const int together = net ? choose_passes(net, 1, passes_per_pair(net)) : 0;
   // vectors: r, z, q and the ring of `keep` directions p_j and A p_j
   const int ring = keep;
   constexpr int CHECK = 8;

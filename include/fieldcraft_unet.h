@@ -41,6 +41,12 @@ int fc_unet_create(int32_t nx, int32_t ny, int32_t nz, int64_t n, const int64_t 
 int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const int64_t *eq, const float *feat,
                           double kref, int32_t levels, uint64_t seed, int32_t device, fc_unet **out,
                           fc_status *status);
+/* Memory: a handle holds the activations of one vector's passes (two with the odd form: about 700
+ * bytes a node and pass) from its creation to its end, and from its first minibatch on those of a group
+ * of up to 8 pairs, at most 2 GB. A call that finds no memory for its group runs in smaller ones, and a
+ * size that was refused is not asked for again; no call after creation fails for memory but
+ * fc_unet_set_operator and fc_fcg_solve (vectors of their own). In a stream capture fc_unet_apply and
+ * the training steps use the first room only, which a graph may keep as long as the handle lives. */
 void fc_unet_destroy(fc_unet *net);
 /* K by rows on the device (as fc_csr_spmv_device; the pointers are read here only): adds the
  * nodal block-Jacobi part B r to the preconditioner (equations node by node, three a node: n must
