@@ -198,20 +198,24 @@ __global__ void scale_kernel(int64_t n, const int64_t *__restrict__ diag_src, co
 
 // ---- panel: factor the diagonal block, solve the rows below ---------------------------------------
 // The block (pw <= 64 columns) and up to PANEL_ROWS rows below it lie in shared memory as one tall
-// panel, factored in FP64 right-looking by strips of 8 columns. Warp 0 carries the chain: it brings
-// the next strip's rows of the block up to date with the strip before (two rows a lane, from shared
-// memory), factors it (pivots and multipliers broadcast by shuffles) and goes on. The other warps
-// follow a strip behind: eight of them take 16 of the rows below each, solve the strip's columns of
-// them (a row a lane, forward substitution with the 8 x 8 triangle), store them and bring their later
-// columns up to date (16 x 8 DMMA tiles), with no barrier between; three apply the strip to the
-// block's columns past the next strip (8 x 8 tiles). So the rows below end with the block, one
-// barrier a strip, and nothing waits for the block's inverse, which only the solve reads
-// (inverse_kernel, beside the following launches). Bound by the chain of dependent FP64 steps, some
-// 35 cycles each: the warps that share warp 0's scheduler are the ones with the short tiles, and the
-// matrix's own diagonal, which the pivot test needs, is loaded while the first strip is factored.
-// With the inverse formed here and the rows multiplied by it, a 64-column panel of 128 rows took 42
-// us; with the rows' solve and update a barrier apart over seven warps and a longer root 23, of which
-// 4 were the loads, 1.6 a strip's factors and 2 to 5 the first strips' rows; now about 19.
+// panel, factored in FP64 by strips of 8 columns. Warp 0 carries the chain: it brings the next strip's
+// rows of the block up to date with the strip before (two rows a lane, from shared memory), factors it
+// (pivots and multipliers broadcast by shuffles) and goes on. The other warps follow a strip behind:
+// eight of them take 16 of the rows below each, sum the earlier strips' products for the strip's columns
+// of them (16 x 8 DMMA tiles), solve these (a row a lane, forward substitution with the 8 x 8 triangle)
+// and store them, with no barrier between; three apply the strip to the block's columns past the next
+// strip (8 x 8 tiles). So the rows below end with the block, one barrier a strip, and nothing waits for
+// the block's inverse, which only the solve reads (inverse_kernel, beside the following launches). A
+// strip's products, and below the block all earlier strips', are summed apart and taken from an entry at
+// once: taken one by one they rounded it at its own size up to eight times as often (64-column panels'
+// rows below off by 4.8 x 2^-53 of an entry in the last strip, with this 2.1), and a solve's error was
+// 1.4 times as large; for that a refactorisation of 24 624 unknowns takes 3.14 ms instead of 3.09. Bound
+// by the chain of dependent FP64 steps, some 35 cycles each: the warps that share warp 0's scheduler are
+// the ones with the short tiles, and the matrix's own diagonal, which the pivot test needs, is loaded
+// while the first strip is factored. With the inverse formed here and the rows multiplied by it, a
+// 64-column panel of 128 rows took 42 us; with the rows' solve and update a barrier apart over seven
+// warps and a longer root 23, of which 4 were the loads, 1.6 a strip's factors and 2 to 5 the first
+// strips' rows; now about 20.
 // The pivot test is the reference's (cholesky.rs:1162-1165): not (d > PIVOT_TOLERANCE |A_jj|) or not
 // finite fails, and the smallest failing column (postorder) is kept in the status word. A failed
 // pivot makes NaNs and nothing else: no index depends on a value. L may be stored in FP32 (widened
@@ -338,6 +342,7 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
           s1[k] = r1 < P8 ? a[(o + k) * PANEL_ALD + r1] : 0.0;
         }
         if (B > 0) {
+          double u0[8] = {}, u1[8] = {};
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const double *col = a + (o - 8 + kk) * PANEL_ALD;
@@ -345,10 +350,12 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               const double lk = col[o + k];
-              s0[k] -= l0 * lk;
-              s1[k] -= l1 * lk;
+              u0[k] = fma(l0, lk, u0[k]);
+              u1[k] = fma(l1, lk, u1[k]);
             }
           }
+#pragma unroll
+          for (int k = 0; k < 8; ++k) s0[k] -= u0[k], s1[k] -= u1[k];
         }
         // the multipliers are broadcast and multiplied before the root is there: the chain of a
         // column is the pivot's shuffle, its reciprocal and one update. Two entries' product has the
@@ -409,17 +416,36 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
       T *dst = Ls + task.r0 + (int64_t)(c0 + o) * m;
       if (row_warp >= 0) {
         for (int i0 = 16 * row_warp; i0 < rows; i0 += 16 * ROW_WARPS) {
+          // the earlier strips' part of the strip's columns, summed apart
+          if (o > 0) {
+            double c[2][4] = {};
+            for (int s = 0; s < o; s += 16) {
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                const int k = s + 8 * u;
+                if (k >= o) continue;
+                const double av[4] = {b[(k + tg) * PANEL_BLD + i0 + g], b[(k + tg) * PANEL_BLD + i0 + g + 8],
+                                      b[(k + tg + 4) * PANEL_BLD + i0 + g], b[(k + tg + 4) * PANEL_BLD + i0 + g + 8]};
+                const double bv[2] = {a[(k + tg) * PANEL_ALD + o + g], a[(k + tg + 4) * PANEL_ALD + o + g]};
+                dmma16(c[u], av, bv);
+              }
+            }
+            double *bj = b + (o + 2 * tg) * PANEL_BLD + i0 + g;
+            bj[0] -= c[0][0] + c[1][0], bj[PANEL_BLD] -= c[0][1] + c[1][1];
+            bj[8] -= c[0][2] + c[1][2], bj[PANEL_BLD + 8] -= c[0][3] + c[1][3];
+            __syncwarp();
+          }
           // the strip's columns of these rows
           if (lane < 16 && i0 + lane < rows) {
-            double x[8];
+            double x[8], sum[8] = {};
             double *bi = b + o * PANEL_BLD + i0 + lane;
 #pragma unroll
             for (int k = 0; k < 8; ++k) x[k] = bi[k * PANEL_BLD];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-              x[k] *= dv[o + k];
+              x[k] = (x[k] - sum[k]) * dv[o + k];
 #pragma unroll
-              for (int j = k + 1; j < 8; ++j) x[j] -= x[k] * a[(o + k) * PANEL_ALD + o + j];
+              for (int j = k + 1; j < 8; ++j) sum[j] = fma(x[k], a[(o + k) * PANEL_ALD + o + j], sum[j]);
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -428,28 +454,6 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
             }
           }
           __syncwarp();
-          // and their later columns
-          double av[4];
-          av[0] = -b[(o + tg) * PANEL_BLD + i0 + g], av[1] = -b[(o + tg) * PANEL_BLD + i0 + g + 8];
-          av[2] = -b[(o + tg + 4) * PANEL_BLD + i0 + g], av[3] = -b[(o + tg + 4) * PANEL_BLD + i0 + g + 8];
-          for (int J = o + 8; J < P8; J += 16) {
-            // two 16 x 8 tiles at a time, their loads before their stores
-            double c[2][4];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int j = min(J + 8 * u, P8 - 8);
-              const double bv[2] = {a[(o + tg) * PANEL_ALD + j + g], a[(o + tg + 4) * PANEL_ALD + j + g]};
-              const double *bj = b + (j + 2 * tg) * PANEL_BLD + i0 + g;
-              c[u][0] = bj[0], c[u][1] = bj[PANEL_BLD], c[u][2] = bj[8], c[u][3] = bj[PANEL_BLD + 8];
-              dmma16(c[u], av, bv);
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              if (J + 8 * u >= P8) continue;
-              double *bj = b + (J + 8 * u + 2 * tg) * PANEL_BLD + i0 + g;
-              bj[0] = c[u][0], bj[PANEL_BLD] = c[u][1], bj[8] = c[u][2], bj[PANEL_BLD + 8] = c[u][3];
-            }
-          }
         }
       } else {
         // the block's columns past the next strip: 8 x 8 tiles (I, J), I >= J, down the columns
