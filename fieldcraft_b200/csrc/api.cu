@@ -92,7 +92,7 @@ struct fc_chol {
   // name, the supernodes' count): its supernodes, columns and rows, and each column's place here
   std::vector<int64_t> ref_first, ref_rptr, ref_perm;
   std::vector<int32_t> ref_rows, ref_place;
-  int64_t ref_ns = 0;
+  int64_t ref_ns = 0, ref_levels = 0;
   std::vector<int64_t> ioff;  // where each supernode's diagonal-block inverses start in Dinv
   int64_t i_len = 0, t_len = 0;
   std::vector<int32_t> width, height, rows;
@@ -1092,6 +1092,14 @@ int build(fc_chol *h, const fc::Symbolic &ref, bool merge, fc_status *st) {
   h->perm.resize(n);
   for (int64_t j = 0; j < n; ++j) h->perm[j] = ref.perm[sym.column[j]];
   h->ref_ns = ref.ns;
+  {
+    std::vector<int64_t> height(ref.ns, 1);
+    h->ref_levels = 0;
+    for (int64_t s = 0; s < ref.ns; ++s) {  // children before parents
+      h->ref_levels = std::max(h->ref_levels, height[s]);
+      if (ref.sparent[s] != fc::NONE) height[ref.sparent[s]] = std::max(height[ref.sparent[s]], height[s] + 1);
+    }
+  }
   h->ref_first = ref.first;
   h->ref_rptr = ref.rptr;
   h->ref_rows = ref.rows;
@@ -3503,7 +3511,7 @@ int fc_chol_inertia(fc_chol *h, int64_t *positive, int64_t *negative, int64_t *t
 int64_t fc_chol_stat(const fc_chol *h, int what) {
   if (!h) return -1;
   switch (what) {
-    case 0: return h->levels;
+    case 0: return h->ref_levels;
     case 1: return (int64_t)h->program.size();
     case 2: return h->l_len * 8;
     case 3: return h->u_len * 8;
@@ -3527,6 +3535,8 @@ int64_t fc_chol_stat(const fc_chol *h, int what) {
       }
       return values;
     }
+    case 17: return h->levels;
+    case 18: return h->ns;
   }
   return -1;
 }

@@ -122,8 +122,8 @@ int fc_chol_set_stream(fc_chol *h, void *stream);
 
 /* Symbolic::numeric + Symbolic::factor (cholesky.rs:1392-1416, 1443-1529) from host values:
  * upper_val[nnz] in the order of the analysed UpperColumns. cancel, when not NULL, is read
- * between levels of the supernodal tree (the reference reads its progress between
- * supernodes, :1476-1484): non-zero stops with FC_CANCELLED. Errors: FC_NOT_POSITIVE_DEFINITE
+ * between levels of the plan's supernodal tree (fc_chol_stat 17 of them; the reference reads its
+ * progress between supernodes, :1476-1484): non-zero stops with FC_CANCELLED. Errors: FC_NOT_POSITIVE_DEFINITE
  * with the original column of the first failing pivot in postorder (:1506-1528). */
 int fc_chol_factor(fc_chol *h, const double *upper_val, int64_t nnz, const volatile int32_t *cancel,
                    fc_status *status);
@@ -185,8 +185,10 @@ int fc_chol_refine_solve_device(fc_chol *h, const int64_t *d_ptr, const int32_t 
                                 const double *d_b, double *d_x, int32_t nrhs, int64_t ld, double tol,
                                 int32_t max_iter, double *relres, int32_t *iterations, fc_status *status);
 
-/* Plan statistics: 0 levels, 1 launches of the factor, 2 bytes of L on device, 3 bytes of the
- * update matrices, 4 supernodes (the analysis'), 5 factor flops (sum of column counts squared), 6 GEMM tasks,
+/* Plan statistics: 0 levels and 4 supernodes of the analysis' tree, 17 levels and 18 supernodes of the
+ * plan's (the Cholesky factor runs on merged supernodes, which store some explicit zeros), 1 launches
+ * of the factor, 2 bytes of L on device, 3 bytes of the update matrices, 5 factor flops (sum of the
+ * analysis' column counts squared), 6 GEMM tasks,
  * 7 kernels launched by the last factorisation, 8 kernels launched by the last solve, 9 flops of
  * the factor's GEMM tasks, 10 flops of the last solve plan's GEMM tasks, 11 the ordinal among the
  * factor's GEMM launches of the one with the most flops, 12 the same among the launches whose

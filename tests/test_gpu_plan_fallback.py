@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import helpers as H
-from fieldcraft_b200 import FP32_IR, FP64, Factor, Symbolic, _lib, problems
+from fieldcraft_b200 import FP32_IR, FP64, Factor, LdltFactor, Symbolic, _lib, problems
 from fieldcraft_b200._lib import Status
 from fieldcraft_b200.cholesky import OutOfMemory
 
@@ -34,8 +34,8 @@ def test_a_refused_plan_is_made_on_the_analysis_own_supernodes(cuda, name, preci
     sym = Symbolic(up, 2**62)
     b = np.asfortranarray(np.random.default_rng(2).standard_normal((p.n, 3)))
     merged, own, refused = (H.factor_on(sym, m, precision, k) for m, k in ((True, 0), (False, 0), (True, 1)))
-    assert own.stat(0) > merged.stat(0) and own.stat(1) > merged.stat(1)  # levels, launches
-    assert [refused.stat(k) for k in (0, 1, 2, 3)] == [own.stat(k) for k in (0, 1, 2, 3)]
+    assert all(own.stat(k) > merged.stat(k) for k in (1, 17, 18))  # the plans' launches, levels, supernodes
+    assert [refused.stat(k) for k in (1, 2, 3, 17, 18)] == [own.stat(k) for k in (1, 2, 3, 17, 18)]
     found = []
     for f in (merged, own, refused):
         f.factor(up.val)
@@ -55,6 +55,23 @@ def test_a_refused_plan_is_made_on_the_analysis_own_supernodes(cuda, name, preci
     assert np.array_equal(found[1][0], found[2][0]) and np.array_equal(found[1][1], found[2][1])
     if precision == FP64:  # the values as the parity tests hold them; the FP32 factor's follow its condition
         assert np.max(np.abs(found[0][1] - found[1][1])) <= 1e-11 * np.max(np.abs(found[1][1]))
+
+
+@pytest.mark.parametrize("name", ["block", "beam"])
+def test_the_analysis_levels_and_supernodes_whatever_the_plan(cuda, name):
+    up = {"block": lambda: problems.lognormal_block(9, nrhs=1), "beam": problems.cantilever}[name]().upper()
+    sym = Symbolic(up, 2**62)
+    s = sym.arrays()
+    owner = np.repeat(np.arange(s["ns"]), np.diff(s["first"]))
+    height = np.ones(s["ns"], int)
+    for k in range(s["ns"]):  # children before parents: the parent owns the first row below
+        rows = s["rows"][s["rptr"][k] + s["first"][k + 1] - s["first"][k]:s["rptr"][k + 1]]
+        if rows.size:
+            height[owner[rows[0]]] = max(height[owner[rows[0]]], height[k] + 1)
+    merged, own, ldlt = H.factor_on(sym, True), H.factor_on(sym, False), LdltFactor(sym)
+    for f in (merged, own, ldlt):
+        assert (f.stat(0), f.stat(4)) == (height.max(), s["ns"])
+    assert (own.stat(17), own.stat(18)) == (ldlt.stat(17), ldlt.stat(18)) == (height.max(), s["ns"])
 
 
 def test_no_plan_at_all_is_out_of_memory(cuda):
