@@ -579,8 +579,8 @@ void plan_factor(fc_chol *h, const std::vector<std::vector<int64_t>> &lv, std::v
         int bw;
         const int64_t ib = inv_block(h, s, c0 / fc::SB, bw), in = c0 % fc::SB;
         const int64_t ioff = ib + in + in * bw;
-        // every CTA of the panel stores its share of the factored block and its inverse (keep:
-        // the panel's CTA count, pad: this CTA's place among them)
+        // every CTA of the panel stores its share of the factored block (keep: the panel's CTA count,
+        // part: this CTA's place among them)
         const int64_t lo = h->loff[s], col = h->first[s] + c0;
         if (c1 >= m) panel_t.push_back({m, c0, c1, m, m, 1, 0, bw, lo, doff, ioff, col});
         const int nrt = (m - c1 + fc::PANEL_ROWS - 1) / fc::PANEL_ROWS;

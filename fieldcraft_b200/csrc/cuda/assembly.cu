@@ -125,8 +125,9 @@ __device__ __noinline__ void dense_block(double lambda, double mu, const double 
 // (dense_block). Bound by FP64 arithmetic and the 4.6 KB an element stores: 0.19 ms for 48 x 40 x 36
 // elements (318 MB, 1.7 TB/s) with four blocks an SM, one's gradients beside another's products (0.28
 // with two at the compiler's 128 registers a thread, 0.22 with three; five spill: 0.21). With
-// entry_kernel and the kernels below, K, reactions and stresses of that box take 0.59 ms; with one thread an element, a row, a DOF and an element each, their matrices
-// accumulated in global memory, they took 6.1 ms.
+// entry_kernel and the kernels below, K, reactions and stresses of that box take 0.59 ms; with one
+// thread an element, a row, a DOF and an element each, their matrices accumulated in global memory,
+// they took 6.1 ms.
 constexpr int ELEMENTS = 6, ELEMENT_THREADS = 36 * ELEMENTS;
 
 __global__ void __launch_bounds__(ELEMENT_THREADS, 4) element_kernel(fc::assembly::Box box, int64_t elements,

@@ -935,9 +935,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, STAGES == GEMM_STAGES ? 6 : 2)
   const int bk0 = jfast ? tid / NW : tid % GEMM_KC;
   const int bdk = jfast ? GEMM_THREADS / NW : 0;
   const int bdj = jfast ? 0 : GEMM_THREADS / GEMM_KC;
-  // through the row list, a stage's row numbers are read a stage ahead (the list is the plan's: no
-  // kernel writes it). Read when they are used, a load's latency stood in every stage of the backward
-  // solve's products (one solve of a 64 x 64 x 8 plate: 0.937 ms, with this 0.897)
+  // through the row list, a stage's row numbers are read a stage ahead, the first before pdl_wait: no
+  // kernel of the solve writes the list, and LDL^T's, which the end of its factorisation does, is
+  // complete before the solve's first kernel (the permutation, launched the ordinary way) starts. Read
+  // when they are used, a load's latency stood in every stage of the backward solve's products (one
+  // solve of a 64 x 64 x 8 plate: 0.937 ms, with this 0.897)
   int row[BPER];
   auto load_index = [&](int kb) {
 #pragma unroll

@@ -1,6 +1,9 @@
 // The pivoted panel of the symmetric indefinite LDL^T (crates/solver/src/ldlt.rs:250-335) on one
-// front, written once for a thread block: the device kernel runs it with CUDA threads; the tests
-// run the same source with host threads and a barrier, against the oracle, bit for bit.
+// front, written once for a thread block: the device kernel runs panel_own with CUDA threads; the tests
+// run the same source with host threads and a barrier, against the oracle, bit for bit. What follows a
+// panel (the rows below, W, W21, the rows' order) the device has in forms of its own (ldlt.cu);
+// panel_below, panel, panel_w, front_w21 and permute_rows_below here are the plain statement of it, which
+// the tests complete a front with. split_d, unit_lower_inverse and D^-1 are shared again.
 //
 // The front holds a supernode's own columns: m rows x w columns, column-major with leading
 // dimension m, entries (r, c) with r >= c meaningful. Columns before the panel are final (L below

@@ -3,9 +3,11 @@
 // The reference's fundamental supernodes keep the exact fill pattern; on the device each of them is
 // a front to assemble, a level's launches and an update matrix written and read once. Merging a
 // supernode into its parent stores some explicit zeros and takes the child's update matrix and often
-// a level away. On the 48^3 hex8 block the 36 407 supernodes become under 10 000, the tree 17 levels
-// high at most instead of 93, the update matrices 1.4e9 entries instead of 5.75e9, for about 1 % more
-// entries in L and half a per cent more operations.
+// a level away. On the 48^3 hex8 block the 36 407 supernodes become 5 627, the 93 levels 14, the update
+// matrices' lower triangles 5.7e9 entries 1.3e9, for 1.8 % more entries in L (7.4 % more bytes: the panels
+// are stored as rectangles) and 0.4 % more operations. A solve multiplies by the inverses of wider blocks
+// and sums in another order: its residual is 1.2 times that on the supernodes unmerged, its error 1.15
+// times (geometric means over 48 boxes and plates of 2 000 to 9 000 unknowns).
 #pragma once
 
 #include <cstdint>

@@ -5,8 +5,9 @@ same in most supernodes (the updates run on the FP64 tensor pipe with fused mult
 exact tie in the rook search, common on a uniform grid, may break the other way: another, equally
 valid factor), solutions within 1e-10 of the oracle's and
 solve_many bit for bit the single solves, values unchanged by a solve, singular columns named.
-The panel's source is also checked bit for bit on the CPU (tests/test_ldlt_panel_emulated.py) and
-the solve's structure by tests/test_ldlt_fold.py."""
+The panel's source is also checked bit for bit on the CPU (tests/test_ldlt_panel_emulated.py), its rows
+below on the GPU (tests/test_gpu_ldlt_fronts.py), and the solve's maps against a fold of the pivots into
+the structure (tests/test_gpu_ldlt_maps.py)."""
 import numpy as np
 import pytest
 

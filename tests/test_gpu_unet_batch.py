@@ -1,6 +1,7 @@
 """Minibatches through the network in groups of pairs: a batch's losses and its last pair's gradient
 are those of the pairs run alone, at batches of one, of part of a group, of a whole group and past
-it, on grids whose sides fall on both sides of the 8 x 8 x 2 tiles, with the odd form and without.
+it, on grids of one tile a pass and of several, with fewer tiles in a batch than SMs (one halo buffer, a
+tile a chunk) and with more (two buffers, several tiles a chunk), with the odd form and without.
 
 The forward pass of a pair is the same arithmetic alone or in a batch (the loss agrees to FP64
 rounding); its gradient is summed in other chunks: FP32 sums of N terms in another order differ by
@@ -28,7 +29,7 @@ def network(dims, levels, odd):
 
 
 @pytest.mark.parametrize("dims,levels,odd", [((7, 7, 1), 2, True), ((15, 8, 3), 3, True), ((16, 9, 2), 3, False),
-                                             ((23, 17, 4), 4, True)])
+                                             ((23, 17, 4), 4, True), ((48, 31, 7), 3, True)])
 @pytest.mark.parametrize("count", [1, 3, 8, 11])
 def test_batches_are_their_pairs(cuda, dims, levels, odd, count):
     torch = cuda
