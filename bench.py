@@ -63,9 +63,10 @@ def parse():
     ap.add_argument("--nn-plate", type=int, default=64, metavar="N",
                     help="the headline line's learned preconditioner on an N x N x 8 plate (the config-5 "
                          "workload at N = 128) with on-policy training; 0: on the headline's own K")
-    ap.add_argument("--profile-kernels", choices=["fp32-factor", "unet"], default=None,
-                    help="a short run for a profiler: two FP32 factorisations of the --n-el block, or the "
-                         "U-Net's forward and backward passes on a 64x64x8 plate, twice")
+    ap.add_argument("--profile-kernels", choices=["fp32-factor", "unet", "ldlt", "assembly", "fcg"], default=None,
+                    help="a short run for a profiler: two FP32 factorisations of the --n-el block; the U-Net's "
+                         "forward and backward passes and a minibatch on a 64x64x8 plate; two LDL^T "
+                         "factorisations or assemblies of the --n-el block; 24 iterations of flexible CG")
     ap.add_argument("--ldlt", type=int, default=0, metavar="N_EL",
                     help="instead: the symmetric indefinite LDL^T (factor, inertia and solve of 16 RHS) on the "
                          "N_EL^3 lognormal block shifted by 2%% of its mean diagonal, against the oracle's LDL^T")
@@ -830,7 +831,7 @@ def roofline_table(p, f, ms_k, cnt_k, gemm_flops, dgemm, solve_graph_ms, spmv_ms
     asm_ms = float(ms_k[0])
     solve_b = 2 * entries * 8 + 2 * n * R * 8
     solve_fl = 4 * entries * R
-    spmv_b = (nnz * 12 + (n + 1) * 8 + 2 * n * 8) * R
+    spmv_b = nnz * 12 + (n + 1) * 8 + 2 * n * 8 * R  # K once for all the right-hand sides
     out = {
         "gemm": {"bound": "tensor", "achieved": gemm_flops / (ms_k[3] * 1e-3) / 1e12, "peak": dgemm,
                  "unit": "TFLOP/s", "ms": float(ms_k[3]), "launches": int(cnt_k[3])},
@@ -842,7 +843,7 @@ def roofline_table(p, f, ms_k, cnt_k, gemm_flops, dgemm, solve_graph_ms, spmv_ms
                   "gbs_frac": solve_b / (solve_graph_ms * 1e-3) / 1e9 / hbm_gbs,
                   "algorithmic": f"4 |L| R flops; 2 |L| 8 + 2 n R 8 bytes (R = {R}); timed alone"},
         "spmv": {"bound": "hbm", "achieved": spmv_b / (spmv_ms * 1e-3) / 1e9, "peak": hbm_gbs, "unit": "GB/s",
-                 "ms": spmv_ms, "algorithmic": "(12 nnz + 8 (n+1) + 16 n) bytes per right-hand side"},
+                 "ms": spmv_ms, "algorithmic": f"12 nnz + 8 (n+1) bytes, and 16 n per right-hand side (R = {R})"},
         "panel": {"bound": "latency", "ms": float(ms_k[1]), "launches": int(cnt_k[1])},
         "hbm_peak_source": hbm_src,
     }
@@ -853,8 +854,12 @@ def roofline_table(p, f, ms_k, cnt_k, gemm_flops, dgemm, solve_graph_ms, spmv_ms
 
 def profile_kernels(args, torch, lib):
     """Runs for a profiler (no timing): the FP32 factorisation of the --n-el block twice (the
-    tcgen05 update GEMMs), or the U-Net's forward and backward passes twice."""
+    tcgen05 update GEMMs), the U-Net's forward and backward passes and a minibatch of eight pairs twice,
+    the LDL^T of the --n-el block shifted by 2 % of its mean diagonal twice, the --n-el block's assembly,
+    reactions and stresses twice, or 24 iterations of flexible CG with the block-Jacobi part on a
+    48 x 48 x 8 plate."""
     from fieldcraft_b200 import FP32_IR, Factor, Symbolic, problems
+    from fieldcraft_b200.cholesky import Timeout
     if args.profile_kernels == "fp32-factor":
         p = problems.lognormal_block(args.n_el, nrhs=1, seed=SEED)
         up = p.upper()
@@ -865,15 +870,57 @@ def profile_kernels(args, torch, lib):
         torch.cuda.synchronize()
         f.close()
         print(json.dumps({"profile_kernels": "fp32-factor", "n": p.n}), flush=True)
+    elif args.profile_kernels == "ldlt":
+        from fieldcraft_b200 import LdltFactor, UpperColumns
+        p = problems.lognormal_block(args.n_el, nrhs=1, seed=SEED)
+        csr = p.csr
+        on = csr.idx == np.repeat(np.arange(p.n), np.diff(csr.ptr))
+        csr.val[on] -= 0.02 * csr.val[on].mean()
+        up = UpperColumns.from_symmetric(csr)
+        f = LdltFactor(Symbolic(up, 2**62))
+        for _ in range(2):
+            f.factor(up.val)
+        f.close()
+        print(json.dumps({"profile_kernels": "ldlt", "n": p.n}), flush=True)
+    elif args.profile_kernels == "assembly":
+        n = args.n_el
+        young = 2.1e5 * np.exp(0.5 * np.random.default_rng(SEED).standard_normal(n**3))
+        p = problems.box(n, n, n, 1.0, 1.0, 1.0, young, 0.3, problems.node_grid(n, n, n)[2] == 0)
+        d = problems.DeviceAssembly(p)
+        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+        new = lambda k: torch.empty(k, dtype=torch.float64, device="cuda")  # noqa: E731
+        e, q, u, dofs = dev(young), dev(np.ones(p.n)), new(p.eq.size), p.eq.size
+        for _ in range(2):
+            d.assemble(e, new(p.csr.val.size))
+            d.reactions(q, r=new(dofs), u=u)
+            d.stresses(e, u, new(48 * n**3), new(2 * dofs), new(dofs // 3))
+        torch.cuda.synchronize()
+        d.close()
+        print(json.dumps({"profile_kernels": "assembly", "n": p.n}), flush=True)
+    elif args.profile_kernels == "fcg":
+        from fieldcraft_b200.unet import UNet, fcg
+        p = problems.plate(48, 48, 8, nrhs=1)
+        csr = tuple(torch.from_numpy(a).cuda() for a in (p.csr.ptr, p.csr.idx, p.csr.val))
+        net = UNet(p, seed=0, levels=2, operator=csr)
+        net.enable(False)
+        b = torch.randn(p.n, dtype=torch.float64, device="cuda")
+        try:
+            fcg(csr, b, torch.zeros_like(b), net=net, tol=1e-12, max_iter=24, keep=4)
+        except Timeout:
+            pass  # 24 iterations are what is wanted
+        net.close()
+        print(json.dumps({"profile_kernels": "fcg", "n": p.n}), flush=True)
     else:
         from fieldcraft_b200.unet import UNet
         p = problems.plate(64, 64, 8, nrhs=1)
         net = UNet(p, seed=0, kref=100.0)
         x = torch.randn(net.voxels * 16, device="cuda", dtype=torch.float32)
         y = torch.empty_like(x)
+        r, e = torch.randn((2, 8, p.n), device="cuda", dtype=torch.float64)
         for _ in range(2):
             net.forward_grid(x, y)
             net.backward_grid(x)
+            net.train_batch(r, e, 1e-3, 1)
         torch.cuda.synchronize()
         net.close()
         print(json.dumps({"profile_kernels": "unet", "voxels": net.voxels}), flush=True)
