@@ -214,8 +214,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   }
 }
 
-// Weight gradient: CTA blockIdx.x takes a chunk of one pair's tiles (a pair: `passes` grids of the
-// batch, whose gradients add), warp w sixteen output channels (w / 9) of the three taps along x at
+// Weight gradient: CTA blockIdx.x takes a chunk of one pass's tiles (every pass cut alike, so that what
+// cancels between two passes, as an odd network's output biases do, cancels to the last bit), warp w
+// sixteen output channels (w / 9) of the three taps along x at
 // (dy, dz) = (w % 9 % 3 - 1, w % 9 / 3 - 1), each the GEMM dW_tap (COUT x CIN) += dY^T (COUT x voxels)
 // X_tap (voxels x CIN), both operands read transposed by ldmatrix.trans from channels-last tiles and
 // dY's fragments shared by the three. The fifth warp of each nine also multiplies dY^T by ones: the bias
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
 // more fragment reads: a training step on eight pairs 1.39 -> 1.41 ms. Bound by the fragments'
 // shared-memory reads and the tensor pipe.
 struct DwTile {
-  int tx, ty, tiles;  // tiles: of one pair, all its passes
+  int tx, ty, tiles;  // tiles: of one pass
 };
 template <int CIN, int COUT>
 __host__ __device__ constexpr size_t dw_smem() {
@@ -242,7 +243,7 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTile tile, int chunks,
                                                                    const bf16 *__restrict__ in,
                                                                    const bf16 *__restrict__ dy,
-                                                                   float *__restrict__ part, int passes) {
+                                                                   float *__restrict__ part) {
   constexpr int CS = cstride(CIN), DS = cstride(COUT), THREADS = dw_threads(COUT);
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int BUFFER = DW_HALO * CS + DW_VOXELS * DS;
@@ -253,19 +254,16 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
   const int hx = tile.tx + 2, hy = tile.ty + 2, here = tile.tx * tile.ty, steps = (here + 15) / 16;
   const int ntx = (g.X + tile.tx - 1) / tile.tx, nty = (g.Y + tile.ty - 1) / tile.ty;
   const int ntiles = ntx * nty * g.Z;
-  const int pair = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
-  const int64_t total = (int64_t)ntiles * passes, per = (total + chunks - 1) / chunks, voxels = g.voxels();
-  const int64_t t0 = chunk * per, t1 = min(total, t0 + per);
+  const int per = (ntiles + chunks - 1) / chunks, t0 = blockIdx.x % chunks * per, t1 = min(ntiles, t0 + per);
+  const int64_t base = (int64_t)(blockIdx.x / chunks) * g.voxels();
   for (int m = tid; m < DW_VOXELS; m += THREADS) place[m] = m < here ? (m / tile.tx * hx + m % tile.tx) * CS : 0;
   float acc[3][CIN / 8][4], bias[2] = {0.f, 0.f};
 #pragma unroll
   for (int t = 0; t < 3; ++t)
 #pragma unroll
     for (int nt = 0; nt < CIN / 8; ++nt) acc[t][nt][0] = acc[t][nt][1] = acc[t][nt][2] = acc[t][nt][3] = 0.f;
-  auto load = [&](int64_t t) {
-    bf16 *ts = buffers + ((t - t0) & 1) * BUFFER, *ds = ts + DW_HALO * CS;
-    const int i = (int)(t % ntiles);
-    const int64_t base = ((int64_t)pair * passes + t / ntiles) * voxels;
+  auto load = [&](int i) {
+    bf16 *ts = buffers + ((i - t0) & 1) * BUFFER, *ds = ts + DW_HALO * CS;
     const int x0 = i % ntx * tile.tx, y0 = i / ntx % nty * tile.ty, z = i / (ntx * nty);
     load_halo<CIN, THREADS / 32>(ts, g, in + base * CIN, x0, y0, z, hx, hy, 3);
     for (int e = tid; e < 16 * steps * (COUT / 8); e += THREADS) {
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
   };
   if (t0 < t1) load(t0);
   commit();
-  for (int64_t t = t0; t < t1; ++t) {
+  for (int t = t0; t < t1; ++t) {
     if (t + 1 < t1) load(t + 1);  // into the buffer that the barrier below the last tile freed
     commit();
     asm volatile("cp.async.wait_group 1;\n" ::);
@@ -330,27 +328,27 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
   }
 }
 
-// The chunks' partials of each pair added in a fixed order (8 threads an element take every eighth
-// chunk, then those 8 sums in order), a pair after the other: gw and gb receive the last pair's
-// gradient; accw and accb (null: not kept) the sum of the pairs' gradients times `scale`, added to
-// what they hold when `more`.
-constexpr int REDUCE_WAYS = 8, REDUCE_ELEMENTS = 32, REDUCE_PAIRS = 8;
+// The chunks' partials of each pass added in a fixed order (8 threads an element take every eighth
+// chunk, then those 8 sums in order), a pair's passes after one another and the pairs too: gw and gb
+// receive the last pair's gradient; accw and accb (null: not kept) the sum of the pairs' gradients times
+// `scale`, added to what they hold when `more`.
+constexpr int REDUCE_WAYS = 8, REDUCE_ELEMENTS = 32, REDUCE_GRIDS = 8;
 __global__ void __launch_bounds__(REDUCE_WAYS * REDUCE_ELEMENTS)
-    dw_reduce_kernel(int pairs, int chunks, int weights, int cout, int64_t stride, const float *__restrict__ part,
-                     float scale, int more, float *__restrict__ accw, float *__restrict__ accb, float *__restrict__ gw,
-                     float *__restrict__ gb) {
-  __shared__ float s[REDUCE_PAIRS][REDUCE_WAYS][REDUCE_ELEMENTS];
+    dw_reduce_kernel(int pairs, int passes, int chunks, int weights, int cout, int64_t stride,
+                     const float *__restrict__ part, float scale, int more, float *__restrict__ accw,
+                     float *__restrict__ accb, float *__restrict__ gw, float *__restrict__ gb) {
+  __shared__ float s[REDUCE_GRIDS][REDUCE_WAYS][REDUCE_ELEMENTS];
   const int el = threadIdx.x % REDUCE_ELEMENTS, way = threadIdx.x / REDUCE_ELEMENTS;
-  const int e = blockIdx.x * REDUCE_ELEMENTS + el;
+  const int e = blockIdx.x * REDUCE_ELEMENTS + el, grids = pairs * passes;
   const bool on = e < weights + cout;
   float *acc = accw ? (e < weights ? accw + e : accb + (e - weights)) : nullptr;
   float *grad = e < weights ? gw + e : gb + (e - weights);
   float sum = on && way == 0 && acc && more ? *acc : 0.f, last = 0.f;
-  for (int p0 = 0; p0 < pairs; p0 += REDUCE_PAIRS) {
-    const int np = min(REDUCE_PAIRS, pairs - p0);
+  for (int p0 = 0; p0 < grids; p0 += REDUCE_GRIDS) {
+    const int np = min(REDUCE_GRIDS, grids - p0);
     __syncthreads();
 #pragma unroll
-    for (int p = 0; p < REDUCE_PAIRS; ++p) {  // every pair's loads in flight
+    for (int p = 0; p < REDUCE_GRIDS; ++p) {  // every pass's loads in flight
       float v = 0.f;
       if (on && p < np)
         for (int c = way; c < chunks; c += REDUCE_WAYS) v += part[((int64_t)(p0 + p) * chunks + c) * stride + e];
@@ -359,10 +357,12 @@ __global__ void __launch_bounds__(REDUCE_WAYS * REDUCE_ELEMENTS)
     __syncthreads();
     if (way == 0)
       for (int p = 0; p < np; ++p) {
-        last = 0.f;
+        float v = 0.f;
 #pragma unroll
-        for (int k = 0; k < REDUCE_WAYS; ++k) last += s[p][k][el];
-        sum += last * scale;
+        for (int k = 0; k < REDUCE_WAYS; ++k) v += s[p][k][el];
+        const int pass = (p0 + p) % passes;
+        last = pass == 0 ? v : last + v;
+        if (pass == passes - 1) sum += last * scale;
       }
   }
   if (on && way == 0) {
@@ -848,21 +848,22 @@ void conv3_launch(const Grid &g, int batch, const bf16 *in, const bf16 *w, const
   cudaLaunchKernelEx(&cfg, conv3_kernel<CIN, COUT>, g, batch, tile, in, w, bias, relu ? 1 : 0, mask, out);
 }
 
-// About one chunk an SM over all pairs (18 warps of 96 registers a thread: one CTA an SM).
-int chunks_of(int64_t tiles, int pairs) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (DW_PARTIALS + pairs - 1) / pairs));
+// The chunks of a pass: at most one a CTA over all passes, and a CTA an SM (18 warps of 96 registers a
+// thread), so that they run in one wave.
+int chunks_of(int64_t tiles, int grids) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, DW_PARTIALS / grids));
 }
 
 // A weight gradient's tile: the one with the least steps of 16 voxels in its longest chunk, a tile's
 // barriers about a step.
-DwTile dw_tile(const Grid &g, int pairs, int passes) {
+DwTile dw_tile(const Grid &g, int grids) {
   struct Known {
-    int X, Y, Z, pairs, passes;
+    int X, Y, Z, grids;
     DwTile tile;
   };
   static thread_local Known known[32] = {};
-  Known &k = known[(uint32_t)(g.X * 31 + g.Y * 17 + g.Z * 7 + pairs * 3 + passes) % 32];
-  if (k.X == g.X && k.Y == g.Y && k.Z == g.Z && k.pairs == pairs && k.passes == passes) return k.tile;
+  Known &k = known[(uint32_t)(g.X * 31 + g.Y * 17 + g.Z * 7 + grids) % 32];
+  if (k.X == g.X && k.Y == g.Y && k.Z == g.Z && k.grids == grids) return k.tile;
   DwTile best{};
   double least = 0.0;
   int xs[64], ys[64];
@@ -871,12 +872,12 @@ DwTile dw_tile(const Grid &g, int pairs, int passes) {
     for (int i = 0; i < nx; ++i) {
       const int tx = xs[i], ty = ys[j];
       if (tx * ty > DW_VOXELS || (tx + 2) * (ty + 2) * 3 > DW_HALO) continue;
-      const int64_t tiles = (int64_t)passes * ((g.X + tx - 1) / tx) * ((g.Y + ty - 1) / ty) * g.Z;
-      const int chunks = chunks_of(tiles, pairs);
+      const int64_t tiles = (int64_t)((g.X + tx - 1) / tx) * ((g.Y + ty - 1) / ty) * g.Z;
+      const int chunks = chunks_of(tiles, grids);
       const double cost = (double)((tiles + chunks - 1) / chunks) * ((tx * ty + 15) / 16 + 1.0);
       if (best.tx == 0 || cost < least) least = cost, best = DwTile{tx, ty, (int)tiles};
     }
-  k = Known{g.X, g.Y, g.Z, pairs, passes, best};
+  k = Known{g.X, g.Y, g.Z, grids, best};
   return best;
 }
 
@@ -888,12 +889,13 @@ void dw_launch(const Grid &g, int pairs, int passes, const bf16 *in, const bf16 
       cudaFuncSetAttribute(conv3_dw_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
       cudaSuccess;
   (void)configured;
-  const DwTile tile = dw_tile(g, pairs, passes);
-  const int chunks = chunks_of(tile.tiles, pairs);
-  conv3_dw_kernel<CIN, COUT><<<pairs * chunks, dw_threads(COUT), smem, st>>>(g, tile, chunks, in, dy, part, passes);
+  const int grids = pairs * passes;
+  const DwTile tile = dw_tile(g, grids);
+  const int chunks = chunks_of(tile.tiles, grids);
+  conv3_dw_kernel<CIN, COUT><<<grids * chunks, dw_threads(COUT), smem, st>>>(g, tile, chunks, in, dy, part);
   const int elements = 27 * CIN * COUT + COUT;
   dw_reduce_kernel<<<(elements + REDUCE_ELEMENTS - 1) / REDUCE_ELEMENTS, REDUCE_WAYS * REDUCE_ELEMENTS, 0, st>>>(
-      pairs, chunks, 27 * CIN * COUT, COUT, (int64_t)28 * CIN * COUT, part, scale, more ? 1 : 0, accw, accb, gw, gb);
+      pairs, passes, chunks, 27 * CIN * COUT, COUT, (int64_t)28 * CIN * COUT, part, scale, more ? 1 : 0, accw, accb, gw, gb);
 }
 
 }  // namespace
@@ -910,7 +912,7 @@ void conv3(const Grid &g, int batch, int cin, int cout, const __nv_bfloat16 *in,
     conv3_launch<16, 16>(g, batch, in, w, bias, relu, mask, out, st);
 }
 
-int dw_chunks(const Grid &g, int pairs, int passes) { return chunks_of(dw_tile(g, pairs, passes).tiles, pairs); }
+int dw_chunks(const Grid &g, int grids) { return chunks_of(dw_tile(g, grids).tiles, grids); }
 
 void conv3_dw(const Grid &g, int cin, int cout, int pairs, int passes, const __nv_bfloat16 *in,
               const __nv_bfloat16 *dy, float *part, float scale, bool more, float *accw, float *accb, float *gw,

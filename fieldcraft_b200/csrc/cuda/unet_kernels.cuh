@@ -29,12 +29,12 @@ void conv3(const Grid &g, int batch, int cin, int cout, const __nv_bfloat16 *in,
            const float *bias, bool relu, const __nv_bfloat16 *mask, __nv_bfloat16 *out, cudaStream_t st);
 // Weight gradient of conv3 over `pairs` pairs of `passes` passes each: per pair g_w[tap][cout][cin] =
 // sum over its passes' voxels of dy[v][cout] in[v + tap][cin] and g_b[cout] = sum of dy[v][cout],
-// in chunks of tiles whose partials are added in order. gw and gb receive the last pair's; accw and
-// accb (or null) the sum over the pairs of scale g, on top of what they hold when `more`. part must
-// hold pairs * dw_chunks(g, pairs, passes) * 28 * cin * cout floats, at most
-// (DW_PARTIALS + pairs) * 28 * cin * cout.
+// in chunks of each pass's tiles whose partials are added in order, then the passes. gw and gb receive
+// the last pair's; accw and accb (or null) the sum over the pairs of scale g, on top of what they hold
+// when `more`. part must hold grids * dw_chunks(g, grids) * 28 * cin * cout floats with grids = pairs *
+// passes: at most max(DW_PARTIALS, grids) * 28 * cin * cout.
 constexpr int DW_PARTIALS = 148;
-int dw_chunks(const Grid &g, int pairs, int passes);
+int dw_chunks(const Grid &g, int grids);
 void conv3_dw(const Grid &g, int cin, int cout, int pairs, int passes, const __nv_bfloat16 *in,
               const __nv_bfloat16 *dy, float *part, float scale, bool more, float *accw, float *accb, float *gw,
               float *gb, cudaStream_t st);

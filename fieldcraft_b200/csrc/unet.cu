@@ -508,7 +508,7 @@ int fc_unet_create_levels(int32_t nx, int32_t ny, int32_t nz, int64_t n, const i
             u->feat.alloc(sizeof(float) * nodes) == cudaSuccess &&
             u->scal.alloc(sizeof(double) * S_COUNT) == cudaSuccess &&
             u->dotpart.alloc(sizeof(double) * 8 * 512) == cudaSuccess &&
-            u->part.alloc(sizeof(float) * (fc::unet::DW_PARTIALS + PAIRS_MOST) * 28 * C * C) == cudaSuccess &&
+            u->part.alloc(sizeof(float) * std::max(fc::unet::DW_PARTIALS, 2 * PAIRS_MOST) * 28 * C * C) == cudaSuccess &&
             u->gtmp.alloc(sizeof(float) * off) == cudaSuccess && alloc_own(u, passes_per_pair(u));
   if (!ok) {
     delete u;
@@ -649,7 +649,7 @@ int fc_test_unet_dw(int32_t X, int32_t Y, int32_t Z, int32_t cin, int32_t cout, 
   const Grid g{X, Y, Z};
   const size_t nw = (size_t)27 * cin * cout;
   DeviceBuf part, last;
-  if (part.alloc(sizeof(float) * (size_t)pairs * fc::unet::dw_chunks(g, pairs, passes) * 28 * cin * cout) != cudaSuccess ||
+  if (part.alloc(sizeof(float) * (size_t)pairs * passes * fc::unet::dw_chunks(g, pairs * passes) * 28 * cin * cout) != cudaSuccess ||
       last.alloc(sizeof(float) * (nw + cout)) != cudaSuccess)
     return FC_OUT_OF_MEMORY;
   fc::unet::conv3_dw(g, cin, cout, pairs, passes, static_cast<const bf16 *>(d_in), static_cast<const bf16 *>(d_dy),
