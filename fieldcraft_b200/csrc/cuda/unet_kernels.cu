@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
 // an accumulator, so its sums leave it every DW_TOGETHER steps (64 voxels) and are added rounded: kept in
 // it over a chunk of 4 100 voxels a gradient was off by 4.7e-6, now by 2e-7 (2-norm, eight pairs on 65 x
 // 65 x 9 nodes). Half of the input channels at a time, so that both sums fit the registers, for an eighth
-// more fragment reads: a training step on eight pairs 1.39 -> 1.41 ms. Bound by the fragments'
+// more fragment reads: 63 -> 67 us on 33 x 33 x 9 nodes. Bound by the fragments'
 // shared-memory reads and the tensor pipe.
 struct DwTile {
   int tx, ty, tiles;  // tiles: of one pass
@@ -331,13 +331,14 @@ __global__ void __launch_bounds__(dw_threads(COUT)) conv3_dw_kernel(Grid g, DwTi
 // The chunks' partials of each pass added in a fixed order (8 threads an element take every eighth
 // chunk, then those 8 sums in order), a pair's passes after one another and the pairs too: gw and gb
 // receive the last pair's gradient; accw and accb (null: not kept) the sum of the pairs' gradients times
-// `scale`, added to what they hold when `more`.
-constexpr int REDUCE_WAYS = 8, REDUCE_ELEMENTS = 32, REDUCE_GRIDS = 8;
+// `scale`, added to what they hold when `more`. Bound by the loads' latency: all passes' are in flight at
+// once (16 passes of 9 chunks: 11 us with a cold cache; eight passes at a time, one after another, 24).
+constexpr int REDUCE_WAYS = 8, REDUCE_ELEMENTS = 32, REDUCE_GRIDS = 16;
 __global__ void __launch_bounds__(REDUCE_WAYS * REDUCE_ELEMENTS)
     dw_reduce_kernel(int pairs, int passes, int chunks, int weights, int cout, int64_t stride,
                      const float *__restrict__ part, float scale, int more, float *__restrict__ accw,
                      float *__restrict__ accb, float *__restrict__ gw, float *__restrict__ gb) {
-  __shared__ float s[REDUCE_GRIDS][REDUCE_WAYS][REDUCE_ELEMENTS];
+  __shared__ float s[REDUCE_GRIDS][REDUCE_WAYS][REDUCE_ELEMENTS], total[REDUCE_GRIDS][REDUCE_ELEMENTS];
   const int el = threadIdx.x % REDUCE_ELEMENTS, way = threadIdx.x / REDUCE_ELEMENTS;
   const int e = blockIdx.x * REDUCE_ELEMENTS + el, grids = pairs * passes;
   const bool on = e < weights + cout;
@@ -347,21 +348,33 @@ __global__ void __launch_bounds__(REDUCE_WAYS * REDUCE_ELEMENTS)
   for (int p0 = 0; p0 < grids; p0 += REDUCE_GRIDS) {
     const int np = min(REDUCE_GRIDS, grids - p0);
     __syncthreads();
+    float v[REDUCE_GRIDS];
 #pragma unroll
-    for (int p = 0; p < REDUCE_GRIDS; ++p) {  // every pass's loads in flight
-      float v = 0.f;
-      if (on && p < np)
-        for (int c = way; c < chunks; c += REDUCE_WAYS) v += part[((int64_t)(p0 + p) * chunks + c) * stride + e];
-      s[p][way][el] = v;
+    for (int p = 0; p < REDUCE_GRIDS; ++p) v[p] = 0.f;
+    if (on)
+      for (int c = way; c < chunks; c += REDUCE_WAYS) {
+        float x[REDUCE_GRIDS];  // every pass's loads in flight
+#pragma unroll
+        for (int p = 0; p < REDUCE_GRIDS; ++p)
+          x[p] = p < np ? part[((int64_t)(p0 + p) * chunks + c) * stride + e] : 0.f;
+#pragma unroll
+        for (int p = 0; p < REDUCE_GRIDS; ++p) v[p] += x[p];
+      }
+#pragma unroll
+    for (int p = 0; p < REDUCE_GRIDS; ++p) s[p][way][el] = v[p];
+    __syncthreads();
+    // the ways' sums of a pass, a warp a pass; then the passes
+    for (int p = way; p < np; p += REDUCE_WAYS) {
+      float t = 0.f;
+#pragma unroll
+      for (int k = 0; k < REDUCE_WAYS; ++k) t += s[p][k][el];
+      total[p][el] = t;
     }
     __syncthreads();
     if (way == 0)
       for (int p = 0; p < np; ++p) {
-        float v = 0.f;
-#pragma unroll
-        for (int k = 0; k < REDUCE_WAYS; ++k) v += s[p][k][el];
         const int pass = (p0 + p) % passes;
-        last = pass == 0 ? v : last + v;
+        last = pass == 0 ? total[p][el] : last + total[p][el];
         if (pass == passes - 1) sum += last * scale;
       }
   }
