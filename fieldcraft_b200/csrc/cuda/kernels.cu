@@ -203,13 +203,14 @@ __global__ void scale_kernel(int64_t n, const int64_t *__restrict__ diag_src, co
 // (pivots and multipliers broadcast by shuffles) and goes on. The other warps follow a strip behind:
 // eight of them take 16 of the rows below each, sum the earlier strips' products for the strip's columns
 // of them (16 x 8 DMMA tiles), solve these (a row a lane, forward substitution with the 8 x 8 triangle)
-// and store them, with no barrier between; three apply the strip to the block's columns past the next
-// strip (8 x 8 tiles). So the rows below end with the block, one barrier a strip, and nothing waits for
-// the block's inverse, which only the solve reads (inverse_kernel, beside the following launches). A
-// strip's products, and below the block all earlier strips', are summed apart and taken from an entry at
-// once: taken one by one they rounded it at its own size up to eight times as often (64-column panels'
-// rows below off by 4.8 x 2^-53 of an entry in the last strip, with this 2.1), and a solve's error was
-// 1.4 times as large; for that a refactorisation of 24 624 unknowns takes 3.14 ms instead of 3.09. Bound
+// and store them, with no barrier between; three add the strip's products to the sums of the block's
+// columns past the next strip (8 x 8 tiles). So the rows below end with the block, one barrier a strip,
+// and nothing waits for the block's inverse, which only the solve reads (inverse_kernel, beside the
+// following launches). All earlier strips' products are summed apart, in the block and below it, and
+// taken from an entry at once: taken one by one they rounded it at its own size up to eight times a
+// strip (64-column panels' rows below off by 4.8 x 2^-53 of an entry in the last strip, with this 2.0),
+// and a solve's error was 1.6 times as large; for that a refactorisation of 24 624 unknowns takes 3.15 ms
+// instead of 3.09. Bound
 // by the chain of dependent FP64 steps, some 35 cycles each: the warps that share warp 0's scheduler are
 // the ones with the short tiles, and the matrix's own diagonal, which the pivot test needs, is loaded
 // while the first strip is factored. With the inverse formed here and the rows multiplied by it, a
@@ -225,7 +226,7 @@ constexpr int PANEL_THREADS = 384, PANEL_THREADS_NARROW = 128;
 constexpr int PANEL_ALD = 68, PANEL_BLD = PANEL_ROWS + 4;  // a warp's fragment reads fall in distinct banks
 // Shared memory of a panel launch whose widest panel is padded to p8 columns (a multiple of 8).
 __host__ __device__ constexpr size_t panel_smem(int p8) {
-  return sizeof(double) * ((size_t)p8 * (PANEL_ALD + PANEL_BLD) + 128);
+  return sizeof(double) * ((size_t)p8 * (PANEL_ALD + PANEL_BLD) + 128 + (p8 > 16 ? (size_t)p8 * PANEL_ALD : 0));
 }
 
 // 2^E and 2^-E for the exponent E of a, both kept in the normal range.
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
   double *b = a + p8max * PANEL_ALD;     // the rows below: b[c * PANEL_BLD + i] = L(r0 + i, c0 + c)
   double *dg = b + p8max * PANEL_BLD;    // the matrix's own diagonal entries of the panel's columns
   double *dv = dg + 64;                  // the pivots' reciprocals
+  double *ab = dv + 64;                  // what the strips before the last take from the block's later columns
   __shared__ double piv[64];             // the pivots, for the test at the end
   __shared__ int fail;
   const PanelTask task = tasks[blockIdx.x];
@@ -343,6 +345,12 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
         }
         if (B > 0) {
           double u0[8] = {}, u1[8] = {};
+          if (B > 1)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              u0[k] = r0 < P8 ? ab[(o + k) * PANEL_ALD + r0] : 0.0;
+              u1[k] = r1 < P8 ? ab[(o + k) * PANEL_ALD + r1] : 0.0;
+            }
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const double *col = a + (o - 8 + kk) * PANEL_ALD;
@@ -467,8 +475,9 @@ __global__ void __launch_bounds__(THREADS) panel_kernel(Tree t, const double *__
           double c[2] = {0.0, 0.0};
           dmma(c, a[(o + tg) * PANEL_ALD + I + g], a[(o + tg) * PANEL_ALD + J + g]);
           dmma(c, a[(o + 4 + tg) * PANEL_ALD + I + g], a[(o + 4 + tg) * PANEL_ALD + J + g]);
-          a[(J + 2 * tg) * PANEL_ALD + I + g] -= c[0];
-          a[(J + 2 * tg + 1) * PANEL_ALD + I + g] -= c[1];
+          double *to = ab + (J + 2 * tg) * PANEL_ALD + I + g;
+          to[0] = o > 0 ? to[0] + c[0] : c[0];
+          to[PANEL_ALD] = o > 0 ? to[PANEL_ALD] + c[1] : c[1];
           I += 8 * BLOCK_WARPS;
         }
       }

@@ -6,7 +6,7 @@
 // a level away. On the 48^3 hex8 block the 36 407 supernodes become 5 627, the 93 levels 14, the update
 // matrices' lower triangles 5.7e9 entries 1.3e9, for 1.8 % more entries in L (7.4 % more bytes: the panels
 // are stored as rectangles) and 0.4 % more operations. A solve multiplies by the inverses of wider blocks
-// and sums in another order: its residual is 1.2 times that on the supernodes unmerged, its error 1.15
+// and sums in another order: its residual is 1.18 times that on the supernodes unmerged, its error 1.09
 // times (geometric means over 48 boxes and plates of 2 000 to 9 000 unknowns).
 #pragma once
 

@@ -3,11 +3,12 @@ rest between 1.2 and 1.8: an update takes about 0.002 from an entry, so each ope
 rounds it by up to 2^-53 (uniformly: 2^-53 / sqrt 3 in the root mean square) and A - L L^T counts them.
 
 An entry's division leaves about 1.85 x 2^-53: the root's error of 0.48 twice and the roundings of L's two
-factors, 1.2 in all, times the entries' 1.5. In the panel's block strip B subtracts B sums of eight products
-and up to seven single ones: over its last four strips sqrt((5.5 + 3.5) / 3 + 1.85^2) = 2.5, held to
-2.7 (each product subtracted by itself in the next strip's rows: 2.9). Below the block all the earlier
-strips' products are summed apart, and the strip's own: sqrt(2 / 3 + 1.85^2) = 2.0, held to 2.2 (each by
-itself: 4.4). In the host's extended format."""
+factors, 1.2 in all, times the entries' 1.5. All earlier strips' products are summed apart and taken from
+the entry at once. In the panel's block the strip's own, 3.5 on average, come one by one: sqrt(4.5 / 3 +
+1.85^2) = 2.2, held to 2.4 (each strip's sum taken by itself: 2.5, each product of the last strip too 2.9).
+Below the block these are summed as well: sqrt(2 / 3 + 1.85^2) = 2.0, held to 2.2 (each product by
+itself: 4.4). Over the panel's last four strips; in the host's extended format.
+"""
 import numpy as np
 import pytest
 
@@ -41,4 +42,4 @@ def test_roundings_in_a_panel(cuda):
         below += [e[64:, c] for c in range(32, 64)]
     rms = [np.sqrt(np.mean(np.concatenate(v)**2)) for v in (block, below)]
     print("%.2f %.2f" % tuple(rms))
-    assert rms[0] <= 2.7 and rms[1] <= 2.2
+    assert rms[0] <= 2.4 and rms[1] <= 2.2
